@@ -28,7 +28,7 @@ NVCC_FLAGS = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp
 # Per-file extra flags: the parity-critical kernels forbid FMA contraction outright.
 NVCC_EXTRA = {
     "kernels_trace.cu": ["-fmad=false"],
-    "kernels_render.cu": ["-fmad=false"],
+    "kernels_render.cu": ["-fmad=false", "--split-compile=8"],
     "api.cu": ["-fmad=false"],
 }
 CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-ffp-contract=off", "-fno-fast-math", "-Wall", "-I", CSRC, "-I", INCLUDE]

@@ -31,23 +31,6 @@ using namespace pbrt::api;
 
 namespace {
 
-// The dense-result scratch for `cap` rays: a (id, t) pair per queue slot, one mask bit per
-// ray, one queue base per 1,024-ray chunk.
-int alloc_dense(pbrt_ctx* c, DenseScratch* d, uint64_t cap) {
-  if (!d->res) PBRT_TRY(c->cuda(cudaMalloc(&d->res, sizeof(uint2) * cap), "cudaMalloc(dense results)"));
-  const uint64_t chunks = (cap + kDenseChunk - 1) / kDenseChunk;
-  if (!d->mask) PBRT_TRY(c->cuda(cudaMalloc(&d->mask, sizeof(uint32_t) * 32 * chunks), "cudaMalloc(dense mask)"));
-  if (!d->bases) PBRT_TRY(c->cuda(cudaMalloc(&d->bases, sizeof(uint32_t) * chunks), "cudaMalloc(dense bases)"));
-  return PBRT_OK;
-}
-
-void free_dense(DenseScratch* d) {
-  cudaFree(d->res);
-  cudaFree(d->mask);
-  cudaFree(d->bases);
-  *d = DenseScratch{};
-}
-
 int ensure_slots(pbrt_ctx* c) {
   if (c->slots_ready) return PBRT_OK;
   for (Slot& s : c->slots) {
@@ -59,7 +42,6 @@ int ensure_slots(pbrt_ctx* c) {
     PBRT_TRY(c->cuda(cudaMalloc(&s.occ, kSlotRays), "cudaMalloc(staging)"));
     PBRT_TRY(c->cuda(cudaMalloc(&s.queue, sizeof(uint32_t) * kSlotRays), "cudaMalloc(staging)"));
     PBRT_TRY(c->cuda(cudaMalloc(&s.rec, sizeof(float4) * 2 * kSlotRays), "cudaMalloc(staging)"));
-    PBRT_TRY(alloc_dense(c, &s.dense, kSlotRays));
     PBRT_TRY(c->cuda(cudaMalloc(&s.fetch, 2 * sizeof(unsigned long long)), "cudaMalloc(staging)"));
   }
   c->slots_ready = true;
@@ -67,11 +49,25 @@ int ensure_slots(pbrt_ctx* c) {
 }
 
 int ensure_queue(pbrt_ctx* c) {
-  if (c->queue && c->queue_rec && c->queue_dense.bases) return PBRT_OK;
+  if (c->queue && c->queue_rec) return PBRT_OK;
   if (!c->queue) PBRT_TRY(c->cuda(cudaMalloc(&c->queue, sizeof(uint32_t) * kDevChunk), "cudaMalloc(survivor queue)"));
   if (!c->queue_rec)
     PBRT_TRY(c->cuda(cudaMalloc(&c->queue_rec, sizeof(float4) * 2 * kDevChunk), "cudaMalloc(survivor records)"));
-  return alloc_dense(c, &c->queue_dense, kDevChunk);
+  return PBRT_OK;
+}
+
+// The survivor queue is the context's: a call on another stream than the last asynchronous one
+// waits for that one's use of it.
+int acquire_queue(pbrt_ctx* c, cudaStream_t st) {
+  if (!c->queue_used || c->queue_stream == st) return PBRT_OK;
+  return c->cuda(cudaStreamWaitEvent(st, c->queue_used, 0), "cudaStreamWaitEvent(survivor queue)");
+}
+
+int release_queue(pbrt_ctx* c, cudaStream_t st) {
+  if (!c->queue_used)
+    PBRT_TRY(c->cuda(cudaEventCreateWithFlags(&c->queue_used, cudaEventDisableTiming), "cudaEventCreate"));
+  c->queue_stream = st;
+  return c->cuda(cudaEventRecord(c->queue_used, st), "cudaEventRecord(survivor queue)");
 }
 
 // Host-to-device copies go on the context's own stream: a plain cudaMemcpy from pageable
@@ -85,8 +81,9 @@ int upload(pbrt_ctx* c, void** dst, const void* src, size_t bytes, uint64_t* tot
 
 void free_mesh(DeviceMesh& m) {
   cudaFree(m.nodes);
-  cudaFree(m.tri_a);
-  cudaFree(m.tri_b);
+  cudaFree(m.wide);
+  cudaFree(m.leaf_node);
+  cudaFree(m.tri);
   cudaFree(m.tri_c);
   m = DeviceMesh{};
 }
@@ -145,7 +142,6 @@ void pbrt_ctx_destroy(pbrt_ctx* c) {
     cudaFree(s.queue);
     cudaFree(s.fetch);
     cudaFree(s.rec);
-    free_dense(&s.dense);
     if (s.s) cudaStreamDestroy(s.s);
   }
   if (c->side) {
@@ -165,11 +161,11 @@ void pbrt_ctx_destroy(pbrt_ctx* c) {
     if (k + 1 < kMaxBatchBranches) cudaFree(c->branch_waves[k].block);
   }
   if (c->branch_fork) cudaEventDestroy(c->branch_fork);
+  if (c->queue_used) cudaEventDestroy(c->queue_used);
   cudaFree(c->d_err);
   cudaFree(c->d_counters);
   cudaFree(c->queue);
   cudaFree(c->queue_rec);
-  free_dense(&c->queue_dense);
   cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -219,24 +215,33 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
     if (dev && i < dev->size() && (*dev)[i].nodes) {  // built on the GPU: take its arrays
       DeviceMeshBuild& b = (*dev)[i];
       dm.nodes = b.nodes;
-      dm.tri_a = b.tri_a;
-      dm.tri_b = b.tri_b;
+      dm.tri = b.tri;
       dm.tri_c = b.tri_c;
       dm.bytes = b.node_slots * sizeof(GpuNode) + ntri * 40;
       dm.view.node_count = uint32_t(b.node_slots);
-      cudaFree(b.tri_index);
+      dm.leaf_node = b.tri_index;  // the triangle order is not needed any more: its words hold the leaves' nodes
       b = DeviceMeshBuild{};
     } else {
       rc = upload(c, &dm.nodes, fm.nodes.data(), fm.nodes.size() * sizeof(GpuNode), &dm.bytes);
-      if (rc == PBRT_OK) rc = upload(c, &dm.tri_a, fm.tri_a.data(), fm.tri_a.size() * sizeof(float), &dm.bytes);
-      if (rc == PBRT_OK) rc = upload(c, &dm.tri_b, fm.tri_b.data(), fm.tri_b.size() * sizeof(float), &dm.bytes);
+      if (rc == PBRT_OK) rc = upload(c, &dm.tri, fm.tri.data(), fm.tri.size() * sizeof(float), &dm.bytes);
       if (rc == PBRT_OK) rc = upload(c, &dm.tri_c, fm.tri_c.data(), fm.tri_c.size() * sizeof(float), &dm.bytes);
       if (rc != PBRT_OK) break;
       dm.view.node_count = uint32_t(fm.nodes.size());
     }
+    dm.view.leaf_direct = ntri <= (uint64_t(1) << 27) && dm.view.node_count <= (1u << 27);
+    rc = c->cuda(cudaMalloc(&dm.wide, wide_bytes(dm.view.node_count)), "cudaMalloc(scene)");
+    if (rc == PBRT_OK && !dm.leaf_node)
+      rc = c->cuda(cudaMalloc(&dm.leaf_node, ntri * sizeof(uint32_t)), "cudaMalloc(scene)");
+    if (rc == PBRT_OK)
+      rc = c->cuda(launch_widen(dm.nodes, dm.view.node_count, dm.view.leaf_direct, dm.wide,
+                                static_cast<uint32_t*>(dm.leaf_node), c->sm_count, c->stream),
+                   "scene upload");
+    if (rc != PBRT_OK) break;
+    dm.bytes += wide_bytes(dm.view.node_count) + ntri * sizeof(uint32_t);
+    dm.view.wide = (const WideNode*)dm.wide;
+    dm.view.leaf_node = (const uint32_t*)dm.leaf_node;
     dm.view.nodes = (const float4*)dm.nodes;
-    dm.view.tri_a = (const float4*)dm.tri_a;
-    dm.view.tri_b = (const float4*)dm.tri_b;
+    dm.view.tri = (const float4*)dm.tri;
     dm.view.tri_c = (const float2*)dm.tri_c;
     views[i] = dm.view;
     void* pv = nullptr;
@@ -617,14 +622,14 @@ int trace_impl(pbrt_scene* s, const float* rays, uint64_t n, uint32_t* prim, flo
   // Nearest hit / any hit of one chunk of `m` rays (planes `stride` apart) on `st`.
   auto launch = [&](const float* r, uint64_t stride, uint64_t m, uint32_t* p, float* tt, uint32_t* ob, uint8_t* oc,
                     unsigned long long* cnt, uint32_t* queue, unsigned long long* qc, float4* rec,
-                    cudaStream_t st, const DenseScratch* dense = nullptr) -> cudaError_t {
+                    cudaStream_t st) -> cudaError_t {
     if (!one_mesh)
       return oc ? launch_scene_any(s->view, r, stride, m, oc, cnt, c->d_err, c->sm_count, st)
                 : launch_scene_closest(s->view, r, stride, m, p, tt, ob, cnt, c->d_err, c->sm_count, st);
-    if (oc) return launch_mesh_any(mv, r, stride, m, oc, c->d_err, c->sm_count, st);
+    if (oc && !queue) return launch_mesh_any(mv, r, stride, m, oc, c->d_err, c->sm_count, st);
+    if (oc) return launch_mesh_any_persistent(mv, r, stride, m, oc, queue, qc, c->d_err, c->sm_count, st, rec);
     if (c->persistent && !cnt)
-      return launch_mesh_closest_persistent(mv, r, stride, m, p, tt, ob, queue, qc, c->d_err, c->sm_count, st, rec,
-                                            dense);
+      return launch_mesh_closest_persistent(mv, r, stride, m, p, tt, ob, queue, qc, c->d_err, c->sm_count, st, rec);
     return launch_mesh_closest(mv, r, stride, m, p, tt, ob, cnt, c->d_err, c->sm_count, st);
   };
 
@@ -643,15 +648,23 @@ int trace_impl(pbrt_scene* s, const float* rays, uint64_t n, uint32_t* prim, flo
 
   if (kr == MemKind::Device) {
     cudaStream_t st = c->work_stream();
-    if (one_mesh && !occ && c->persistent && !counters) {
+    // Occlusion needs no scratch when it runs one thread per ray: a stream under capture takes
+    // that form, since a graph replayed later may run beside another call's use of the queue.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (c->user) PBRT_TRY(c->cuda(cudaStreamIsCapturing(st, &cap), "cudaStreamIsCapturing"));
+    const bool captured = cap != cudaStreamCaptureStatusNone;
+    if (one_mesh && c->persistent && !counters && !(occ && captured)) {
       // Chunks of at most kDevChunk rays bound the survivor queue (scratch) to 64 MiB.
       PBRT_TRY(ensure_queue(c));
+      if (!captured) PBRT_TRY(acquire_queue(c, st));
       for (uint64_t base = 0; base < n; base += kDevChunk) {
         const uint64_t m = std::min<uint64_t>(kDevChunk, n - base);
-        PBRT_TRY(c->cuda(launch(rays + base, n, m, prim + base, t + base, obj ? obj + base : nullptr, nullptr, nullptr,
-                                c->queue, c->d_counters + 4, c->queue_rec, st, &c->queue_dense),
+        PBRT_TRY(c->cuda(launch(rays + base, n, m, occ ? nullptr : prim + base, occ ? nullptr : t + base,
+                                obj ? obj + base : nullptr, occ ? occ + base : nullptr, nullptr, c->queue,
+                                c->d_counters + 4, c->queue_rec, st),
                          "kernel launch"));
       }
+      if (!captured && c->user) PBRT_TRY(release_queue(c, st));
     } else {
       PBRT_TRY(c->cuda(launch(rays, n, n, prim, t, obj, occ, counters, nullptr, nullptr, nullptr, st), "kernel launch"));
     }
@@ -683,7 +696,7 @@ int trace_impl(pbrt_scene* s, const float* rays, uint64_t n, uint32_t* prim, flo
                                        m * sizeof(float), 8, cudaMemcpyHostToDevice, sl.s),
                      "cudaMemcpy2DAsync(rays)"));
     PBRT_TRY(c->cuda(launch(sl.rays, kSlotRays, m, sl.prim, sl.t, obj ? sl.obj : nullptr, occ ? sl.occ : nullptr,
-                            counters, sl.queue, sl.fetch, sl.rec, sl.s, &sl.dense),
+                            counters, c->persistent ? sl.queue : nullptr, sl.fetch, sl.rec, sl.s),
                      "kernel launch"));
     if (occ) {
       PBRT_TRY(c->cuda(cudaMemcpyAsync(occ + base, sl.occ, m, cudaMemcpyDeviceToHost, sl.s), "cudaMemcpyAsync"));

@@ -697,7 +697,7 @@ __global__ void k_layout(const PoolNode* __restrict__ pool, uint32_t n, const ui
 
 // the triangles in leaf order, with their precomputed edges (mesh_bvh.hpp)
 __global__ void k_tri_layout(const TriRec* __restrict__ fin, uint32_t n, const float* __restrict__ v,
-                             const uint32_t* __restrict__ idx, float4* ta, float4* tb, float2* tc, uint32_t* order) {
+                             const uint32_t* __restrict__ idx, float4* tri, float2* tc, uint32_t* order) {
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     const uint32_t t = __float_as_uint(fin[k].c.w);
     const float* p0 = v + 3 * size_t(idx[3 * size_t(t)]);
@@ -705,8 +705,8 @@ __global__ void k_tri_layout(const TriRec* __restrict__ fin, uint32_t n, const f
     const float* p2 = v + 3 * size_t(idx[3 * size_t(t) + 2]);
     const float e1[3] = {__fsub_rn(p1[0], p0[0]), __fsub_rn(p1[1], p0[1]), __fsub_rn(p1[2], p0[2])};
     const float e2[3] = {__fsub_rn(p2[0], p0[0]), __fsub_rn(p2[1], p0[1]), __fsub_rn(p2[2], p0[2])};
-    ta[k] = make_float4(p0[0], p0[1], p0[2], e1[0]);
-    tb[k] = make_float4(e1[1], e1[2], e2[0], e2[1]);
+    tri[2 * size_t(k)] = make_float4(p0[0], p0[1], p0[2], e1[0]);
+    tri[2 * size_t(k) + 1] = make_float4(e1[1], e1[2], e2[0], e2[1]);
     tc[k] = make_float2(e2[2], __uint_as_float(t));
     order[k] = t;
   }
@@ -931,21 +931,18 @@ bool build_mesh_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_idx,
   o.node_slots = uint64_t(nodes) + 1;
   auto fail_free = [&o]() {
     cudaFree(o.nodes);
-    cudaFree(o.tri_a);
-    cudaFree(o.tri_b);
+    cudaFree(o.tri);
     cudaFree(o.tri_c);
     cudaFree(o.tri_index);
   };
-  cudaError_t e = cudaMalloc(&o.tri_a, size_t(n) * sizeof(float4));
-  if (e == cudaSuccess) e = cudaMalloc(&o.tri_b, size_t(n) * sizeof(float4));
+  cudaError_t e = cudaMalloc(&o.tri, size_t(n) * 2 * sizeof(float4));
   if (e == cudaSuccess) e = cudaMalloc(&o.tri_c, size_t(n) * sizeof(float2));
   if (e == cudaSuccess) e = cudaMalloc(&o.tri_index, size_t(n) * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemsetAsync(o.nodes, 0, (size_t(nodes) + 1) * sizeof(GpuNode), st);
   if (e == cudaSuccess) e = cudaMemsetAsync(stats, 0, 4 * sizeof(uint32_t), st);
   if (e == cudaSuccess) {
     k_layout<<<grid_for(nodes, 256, sm_count), 256, 0, st>>>(pool, nodes, ref, o.nodes, stats);
-    k_tri_layout<<<grid_for(n, 256, sm_count), 256, 0, st>>>(fin, n, d_v, d_idx, o.tri_a, o.tri_b, o.tri_c,
-                                                             o.tri_index);
+    k_tri_layout<<<grid_for(n, 256, sm_count), 256, 0, st>>>(fin, n, d_v, d_idx, o.tri, o.tri_c, o.tri_index);
     e = cudaGetLastError();
   }
   uint32_t hs[4] = {0, 0, 0, 0};
@@ -977,8 +974,7 @@ bool build_mesh_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_idx,
 
 void free_device_mesh_build(DeviceMeshBuild* b) {
   cudaFree(b->nodes);
-  cudaFree(b->tri_a);
-  cudaFree(b->tri_b);
+  cudaFree(b->tri);
   cudaFree(b->tri_c);
   cudaFree(b->tri_index);
   *b = DeviceMeshBuild{};

@@ -13,8 +13,7 @@ namespace pbrt {
 struct DeviceMeshBuild {
   GpuNode* nodes = nullptr;     // node_slots records, GPU numbering (root 0, padding 1)
   uint64_t node_slots = 0;
-  float4* tri_a = nullptr;      // the triangle streams of mesh_bvh.hpp, in leaf order
-  float4* tri_b = nullptr;
+  float4* tri = nullptr;        // the triangle streams of mesh_bvh.hpp, in leaf order
   float2* tri_c = nullptr;
   uint32_t* tri_index = nullptr;  // leaf order -> original triangle index
   MeshBuildStats stats;

@@ -62,7 +62,6 @@ struct Slot {
   uint8_t* occ = nullptr;
   uint32_t* queue = nullptr;            // survivor queue of the two-stage nearest-hit pass
   float4* rec = nullptr;                // the survivors' ray records (32 bytes each)
-  pbrt::DenseScratch dense;             // dense results: per-slot (id, t), survivor bitmask, chunk bases
   unsigned long long* fetch = nullptr;  // [queue length, fetch position] of that pass
 };
 
@@ -88,7 +87,8 @@ struct pbrt_ctx {
                                              // [8..10] rays / shadow rays / paths of the last render
   uint32_t* queue = nullptr;                  // survivor queue for device-buffer calls (kDevChunk entries)
   float4* queue_rec = nullptr;                // and their ray records (kDevChunk x 32 bytes)
-  pbrt::DenseScratch queue_dense;             // and the dense-result scratch for kDevChunk rays
+  cudaEvent_t queue_used = nullptr;           // the queue's last asynchronous use,
+  cudaStream_t queue_stream = nullptr;        // and its stream
   bool persistent = true;                     // persistent dynamic-fetch traversal (default)
   uint32_t* noalloc_scratch = nullptr;        // device address of pbrt_trace_closest_noalloc's static
                                               // scratch array on this device, looked up at creation
@@ -124,8 +124,9 @@ struct pbrt_ctx {
 
 struct DeviceMesh {
   void* nodes = nullptr;
-  void* tri_a = nullptr;
-  void* tri_b = nullptr;
+  void* wide = nullptr;
+  void* leaf_node = nullptr;
+  void* tri = nullptr;
   void* tri_c = nullptr;
   pbrt::MeshView view{};
   uint64_t bytes = 0;

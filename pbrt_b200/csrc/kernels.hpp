@@ -16,22 +16,22 @@ cudaError_t launch_mesh_closest(const MeshView& m, const float* rays, uint64_t s
 // Two-stage nearest hit: a streaming root-box cull that answers misses and compacts the
 // survivors' indices into `queue` (scratch, capacity >= n, n < 2^32), then the persistent
 // dynamic-fetch traversal over the queue. `counters` is two 64-bit words of scratch (queue
-// length, fetch position), zeroed on `s` by the launcher. `rec` (optional scratch, 2 x n
-// float4): the survivors' rays copied beside their queue entries, read back coalesced.
-// Dense results (optional scratch, with `rec`): the cull writes no miss answers but a survivor
-// bitmask per ray (`mask`, n/32 words) and the queue position of each 1,024-ray chunk's first
-// survivor (`bases`); the traversal writes each survivor's (id, t) to its queue slot (`res`,
-// capacity n); a last pass writes every ray's answer in ray order, coalesced.
-struct DenseScratch {
-  uint2* res = nullptr;
-  uint32_t* mask = nullptr;
-  uint32_t* bases = nullptr;
-};
-constexpr uint64_t kDenseChunk = 1024;  // rays per bitmask chunk (one cull block iteration)
+// length, fetch position), zeroed on `s` by the launcher. `rec` (scratch, 2 x n float4): the
+// survivors' rays copied beside their queue entries, read back coalesced.
 cudaError_t launch_mesh_closest_persistent(const MeshView& m, const float* rays, uint64_t stride, uint64_t n,
                                            uint32_t* prim, float* t, uint32_t* obj, uint32_t* queue,
                                            unsigned long long* counters, uint32_t* err, int sm_count, cudaStream_t s,
-                                           float4* rec = nullptr, const DenseScratch* dense = nullptr);
+                                           float4* rec);
+// The same two stages for occlusion.
+cudaError_t launch_mesh_any_persistent(const MeshView& m, const float* rays, uint64_t stride, uint64_t n, uint8_t* occ,
+                                       uint32_t* queue, unsigned long long* counters, uint32_t* err, int sm_count,
+                                       cudaStream_t s, float4* rec);
+// A tree's wide nodes (wide_bvh.cuh): their bytes for node_slots binary records, and the
+// kernel that writes them and each leaf's node beside its first triangle (leaf_node, one word
+// per triangle). direct: leaf references hold first and count (at most 2^27 triangles).
+size_t wide_bytes(uint64_t node_slots);
+cudaError_t launch_widen(const void* nodes, uint32_t node_slots, bool direct, void* wide, uint32_t* leaf_node,
+                         int sm_count, cudaStream_t s);
 // Allocation-free form of launch_mesh_closest_persistent for device buffers (plane stride
 // = n): its scratch is a file-scope __device__ array of kNoAllocMaxRays queue entries
 // shared by every call on a device. `scratch` is that array's device address on the current

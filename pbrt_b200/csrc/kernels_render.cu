@@ -1053,11 +1053,11 @@ __global__ void __launch_bounds__(128, PBRT_DEFER_MIN_BLOCKS) k_defer_closest(Wa
           done = true;
         } else {
           for (uint32_t k = lf; k < lf + count; ++k) {
-            const float4 A = __ldg(&m.tri_a[k]);
-            const float4 B = __ldg(&m.tri_b[k]);
+            float4 A, B;
+            load_node(&m.tri[2 * size_t(k)], A, B);
             const float2 C = __ldg(&m.tri_c[k]);
             float t;
-            if (tri_hit(r, A, B, C.x, t) && t < min_t && t >= near && t <= far) {
+            if (tri_hit(r.o, r.d, A, B, C.x, t) && t < min_t && t >= near && t <= far) {
               min_t = t;
               best = __float_as_uint(C.y);
             }
@@ -1185,11 +1185,11 @@ __global__ void __launch_bounds__(128, PBRT_DEFER_MIN_BLOCKS) k_defer_any(WaveBu
       }
       if (!done) {
         for (uint32_t j = lf; j < lf + count && !hit; ++j) {
-          const float4 A = __ldg(&m.tri_a[j]);
-          const float4 B = __ldg(&m.tri_b[j]);
+          float4 A, B;
+          load_node(&m.tri[2 * size_t(j)], A, B);
           const float2 C = __ldg(&m.tri_c[j]);
           float t;
-          if (tri_hit(r, A, B, C.x, t) && t >= kShadowEps && t <= far) hit = true;
+          if (tri_hit(r.o, r.d, A, B, C.x, t) && t >= kShadowEps && t <= far) hit = true;
         }
         if (hit || sp == 0) {
           done = true;

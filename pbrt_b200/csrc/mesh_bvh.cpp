@@ -263,8 +263,7 @@ bool build_mesh_bvh(const float* vertices, uint32_t vertex_count, const uint32_t
   }
   out->stats = st;
 
-  out->tri_a.resize(size_t(tri_count) * 4);
-  out->tri_b.resize(size_t(tri_count) * 4);
+  out->tri.resize(size_t(tri_count) * 8);
   out->tri_c.resize(size_t(tri_count) * 2);
   out->tri_index = order;
   for (uint32_t k = 0; k < tri_count; ++k) {
@@ -274,8 +273,8 @@ bool build_mesh_bvh(const float* vertices, uint32_t vertex_count, const uint32_t
     const float* p2 = vertices + 3 * size_t(indices[3 * size_t(t) + 2]);
     const float e1[3] = {p1[0] - p0[0], p1[1] - p0[1], p1[2] - p0[2]};
     const float e2[3] = {p2[0] - p0[0], p2[1] - p0[1], p2[2] - p0[2]};
-    float* a = &out->tri_a[size_t(k) * 4];
-    float* b = &out->tri_b[size_t(k) * 4];
+    float* a = &out->tri[size_t(k) * 8];
+    float* b = a + 4;
     float* c = &out->tri_c[size_t(k) * 2];
     a[0] = p0[0]; a[1] = p0[1]; a[2] = p0[2]; a[3] = e1[0];
     b[0] = e1[1]; b[1] = e1[2]; b[2] = e2[0]; b[3] = e2[1];

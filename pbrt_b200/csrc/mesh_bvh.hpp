@@ -13,9 +13,9 @@
 //          records starting at left_first; an interior node's children are left_first and
 //          left_first + 1. Index 0 is the root and index 1 is padding, so every sibling pair
 //          starts at an even index and the pair is one aligned 64-byte read.
-//   triangles, in leaf order, as three streams (SoA):
-//          tri_a[k] = {v0.x, v0.y, v0.z, e1.x}
-//          tri_b[k] = {e1.y, e1.z, e2.x, e2.y}
+//   triangles, in leaf order, as two streams (a lane's load of up to 32 bytes costs the same
+//   L1 wavefront, so a triangle is two loads):
+//          tri[k]   = {v0.x, v0.y, v0.z, e1.x, e1.y, e1.z, e2.x, e2.y}
 //          tri_c[k] = {e2.z, bits(original triangle index)}
 //          with e1 = v1 - v0 and e2 = v2 - v0 rounded to FP32 exactly as the reference's
 //          intersect_ray forms them (triangle_mesh.rs:190-191), so precomputing them
@@ -50,8 +50,7 @@ struct MeshBuildStats {
 
 struct FlatMesh {
   std::vector<GpuNode> nodes;      // GPU numbering (root 0, padding 1)
-  std::vector<float> tri_a;        // 4 floats per triangle
-  std::vector<float> tri_b;        // 4 floats per triangle
+  std::vector<float> tri;          // 8 floats per triangle
   std::vector<float> tri_c;        // 2 floats per triangle
   std::vector<uint32_t> tri_index; // leaf order -> original triangle index
   float bounds_min[3], bounds_max[3];  // vertex bounds (TriangleMesh::get_bounding_box)

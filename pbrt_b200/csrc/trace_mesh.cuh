@@ -14,8 +14,7 @@
 //
 // Layout (mesh_bvh.hpp): nodes are 32-byte records read as two float4 (bmin|left_first,
 // bmax|count); a sibling pair is one aligned 64-byte read
-// (two 256-bit loads); triangles are three SoA
-// streams in leaf order.
+// (two 256-bit loads); triangles are two streams in leaf order, 32 and 8 bytes each.
 #pragma once
 
 #include <cfloat>
@@ -40,12 +39,16 @@ PBRT_DEV void load_node(const float4* p, float4& lo, float4& hi) {
       : "l"(p));
 }
 
+struct WideNode;  // wide_bvh.cuh
+
 struct MeshView {
-  const float4* nodes;  // 2 float4 per node
-  const float4* tri_a;
-  const float4* tri_b;
+  const float4* nodes;   // 2 float4 per node
+  const WideNode* wide;  // the same tree two levels at a time
+  const float4* tri;     // 2 float4 per triangle
   const float2* tri_c;
+  const uint32_t* leaf_node;  // at a leaf's first triangle: the leaf's node
   uint32_t node_count;  // GPU numbering, including the padding slot
+  bool leaf_direct;     // leaf references hold first and count (leaf_ref in wide_bvh.cuh)
 };
 
 // A ray prepared for box tests: the reciprocals depend on the ray alone (the reference
@@ -114,19 +117,19 @@ PBRT_DEV bool box_hit(const PRay& r, const float4& lo, const float4& hi, float t
 }
 
 // Möller–Trumbore with e1, e2 precomputed (bit-identical to forming them here).
-PBRT_DEV bool tri_hit(const PRay& r, const float4& A, const float4& B, float e2z, float& t) {
+PBRT_DEV bool tri_hit(const F3& o, const F3& d, const float4& A, const float4& B, float e2z, float& t) {
   const F3 p0 = mk3(A.x, A.y, A.z);
   const F3 e1 = mk3(A.w, B.x, B.y);
   const F3 e2 = mk3(B.z, B.w, e2z);
-  const F3 pv = cross3(r.d, e2);
+  const F3 pv = cross3(d, e2);
   const float det = dot3(e1, pv);
   if (fabsf(det) < 1e-8f) return false;
   const float inv_det = frcp(det);
-  const F3 s = sub3(r.o, p0);
+  const F3 s = sub3(o, p0);
   const float u = fm(inv_det, dot3(s, pv));
   if (u < 0.f || u > 1.f) return false;
   const F3 q = cross3(s, e1);
-  const float v = fm(inv_det, dot3(r.d, q));
+  const float v = fm(inv_det, dot3(d, q));
   if (v < 0.f || fa(u, v) > 1.f) return false;
   t = fm(inv_det, dot3(e2, q));
   return true;
@@ -163,12 +166,12 @@ PBRT_DEV uint32_t mesh_closest(const MeshView& m, const PRay& r, float near, flo
       bool pop = true;
       if (count > 0) {
         for (uint32_t k = lf; k < lf + count; ++k) {
-          const float4 A = __ldg(&m.tri_a[k]);
-          const float4 B = __ldg(&m.tri_b[k]);
+          float4 A, B;
+          load_node(&m.tri[2 * size_t(k)], A, B);
           const float2 C = __ldg(&m.tri_c[k]);
           if (kCount) cnt->triangle_tests++;
           float t;
-          if (tri_hit(r, A, B, C.x, t) && t < min_t && t >= near && t <= far) {
+          if (tri_hit(r.o, r.d, A, B, C.x, t) && t < min_t && t >= near && t <= far) {
             min_t = t;
             best = __float_as_uint(C.y);
           }
@@ -245,11 +248,11 @@ PBRT_DEV bool mesh_any(const MeshView& m, const PRay& r, float near, float far, 
     bool pop = true;
     if (count > 0) {
       for (uint32_t k = lf; k < lf + count; ++k) {
-        const float4 A = __ldg(&m.tri_a[k]);
-        const float4 B = __ldg(&m.tri_b[k]);
+        float4 A, B;
+        load_node(&m.tri[2 * size_t(k)], A, B);
         const float2 C = __ldg(&m.tri_c[k]);
         float t;
-        if (tri_hit(r, A, B, C.x, t) && t >= near && t <= far) return true;
+        if (tri_hit(r.o, r.d, A, B, C.x, t) && t >= near && t <= far) return true;
       }
     } else {
       float4 l0, l1, r0, r1;

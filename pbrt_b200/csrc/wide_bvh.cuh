@@ -1,0 +1,317 @@
+// wide_bvh.cuh — a mesh's binary BVH two levels at a time, with the binary traversal's answers.
+//
+// What bounds an incoherent walk here is the L1 data path: every lane reads another node, so a
+// load costs one wavefront per lane whatever its width up to 32 bytes. A wide node holds the
+// four grandchildren of an interior node (slots 0, 1 under its left child, 2, 3 under the
+// right) in 64 bytes, two loads, where the binary tree takes six (three pairs of 64 bytes):
+// the boxes are rounded outwards to a 256-step grid over the node's own box. The slab test on
+// them is conservative, never missing a box that box_hit takes (the margin m below), so a walk
+// reaches every leaf the binary one reaches, and perhaps a few more.
+//
+// Why the answers are the binary traversal's (trace_mesh.cuh). There a leaf is visited when
+// its own box is hit over [near, far] and its entry distance is below the nearest hit at its
+// turn; the boxes above add nothing, being exact unions under a monotone slab test.
+//   - Any hit: a triangle hit counts only if its leaf's exact box is hit. No order matters.
+//   - Nearest hit: as long as every hit lies at or beyond its leaf's exact entry distance, the
+//     binary answer is the nearest of all hits in exactly-hit leaves, and among equal distances
+//     the first in traversal order, whatever the order of the visits. A triangle that lowers the
+//     nearest distance is therefore checked against its leaf's exact box; a leaf that is not hit
+//     is ignored as the binary walk would; a hit before its leaf's entry, or one that equals the
+//     nearest distance of another leaf, makes the lane start its ray again on the binary nodes,
+//     in the binary order. Nodes are dropped only beyond the nearest distance plus 2^-13 of it,
+//     so that a leaf whose hit comes before its entry by a rounding is seen, not skipped.
+// Rays the grid's arithmetic does not cover (a direction component of zero or outside
+// [2^-40, 2^40], near < 0 or NaN, coordinates beyond 2^40) walk the binary nodes from the start.
+#pragma once
+
+#include <cfloat>
+
+#include "trace_mesh.cuh"
+
+namespace pbrt {
+
+constexpr uint32_t kLeafRef = 0x80000000u;
+constexpr int kWideStack = 96;  // three pending slots per two levels of a tree of depth < 64
+constexpr float kWideLimit = 1.099511627776e12f;  // 2^40
+
+struct __align__(64) WideNode {
+  float org[3];      // the node's own lower corner
+  float step[3];     // the grid's step / 256 (a power of two) per axis
+  uint32_t lo_x, hi_x, lo_y, hi_y, lo_z, hi_z;  // the slots' planes, a byte each
+  uint32_t ref[4];   // 0: empty; kLeafRef | leaf (leaf_ref); else a wide node
+};
+static_assert(sizeof(WideNode) == 64, "a wide node is two 32-byte loads");
+
+// References name a sibling pair of the binary tree by half its first index: the wide node of
+// that pair's parent, and the pair itself for a binary step. A leaf's holds the first triangle
+// and count packed (27 + 4 bits), or, when they do not fit, the index of the leaf's binary node
+// with the count field 15 (`direct`; meshes of more than 2^27 triangles always name the node).
+PBRT_DEV uint32_t leaf_ref(uint32_t first, uint32_t count, uint32_t node, bool direct) {
+  if (!direct) return kLeafRef | node;
+  if (count <= 15u && first < (1u << 27)) return kLeafRef | ((count - 1u) << 27) | first;
+  return kLeafRef | (15u << 27) | node;
+}
+
+PBRT_DEV void leaf_range(const float4* nodes, uint32_t ref, bool direct, uint32_t& first, uint32_t& count) {
+  const uint32_t code = (ref >> 27) & 15u;
+  if (direct && code != 15u) {
+    first = ref & 0x7FFFFFFu;
+    count = code + 1u;
+    return;
+  }
+  const uint32_t node = direct ? ref & 0x7FFFFFFu : ref & 0x7FFFFFFFu;
+  first = __float_as_uint(__ldg(&nodes[2 * size_t(node)]).w);
+  count = __float_as_uint(__ldg(&nodes[2 * size_t(node) + 1]).w);
+}
+
+PBRT_DEV uint32_t node_ref(const float4& lo, const float4& hi, uint32_t node, bool direct) {
+  const uint32_t lf = __float_as_uint(lo.w), count = __float_as_uint(hi.w);
+  return count ? leaf_ref(lf, count, node, direct) : lf >> 1;
+}
+
+PBRT_DEV uint32_t root_ref(const float4* nodes, bool direct) {
+  return node_ref(__ldg(&nodes[0]), __ldg(&nodes[1]), 0, direct);
+}
+
+// Whether every coordinate of a tree lies where the grid's arithmetic holds.
+PBRT_DEV bool tree_bounded(const float4* nodes) {
+  const float4 lo = __ldg(&nodes[0]), hi = __ldg(&nodes[1]);
+  const float a = fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(hi.x)), fmaxf(fabsf(lo.y), fabsf(hi.y))),
+                        fmaxf(fabsf(lo.z), fabsf(hi.z)));
+  return a <= kWideLimit;
+}
+
+// The least float above x; +inf above FLT_MAX, -FLT_MAX above -inf; a NaN gives -inf (nothing
+// is below it: an interval that ends in a NaN holds no hit).
+PBRT_DEV float next_up(float x) {
+  if (!(x == x)) return __int_as_float(0xff800000);
+  if (x == 0.f) return __int_as_float(1);
+  const uint32_t b = __float_as_uint(x);
+  if (x > 0.f) return x > FLT_MAX ? x : __uint_as_float(b + 1u);
+  return __uint_as_float(b - 1u);
+}
+
+struct WRay {
+  F3 o, d, inv;
+  bool exact;  // walks the binary nodes
+};
+
+PBRT_DEV WRay wide_ray(const F3& o, const F3& d, float near, bool bounded) {
+  WRay r;
+  r.o = o;
+  r.d = d;
+  r.inv = mk3(frcp(d.x), frcp(d.y), frcp(d.z));
+  auto in = [](float x) { return fabsf(x) <= kWideLimit && fabsf(x) >= 1.f / kWideLimit; };
+  auto below = [](float x) { return fabsf(x) <= kWideLimit; };
+  r.exact = !(bounded && near >= 0.f && in(r.inv.x) && in(r.inv.y) && in(r.inv.z) && below(o.x) && below(o.y) &&
+              below(o.z));
+  return r;
+}
+
+// Pending slots of a walk: reference and entry distance.
+struct WideStack {
+  uint2 s[kWideStack];
+};
+
+PBRT_DEV void wide_push(WideStack& st, int& sp, uint32_t ref, float e, uint32_t* err) {
+  if (sp >= kWideStack) {
+    atomicOr(err, kErrStack);
+    return;
+  }
+  st.s[sp] = make_uint2(ref, __float_as_uint(e));
+  ++sp;
+}
+
+// The next pending slot whose entry distance is below lim (the pop that drops entries at or
+// beyond the nearest hit, bvh.rs:470-472); 0 when none is left.
+PBRT_DEV uint32_t wide_pop(const WideStack& st, int& sp, float lim) {
+  while (sp > 0) {
+    const uint2 v = st.s[--sp];
+    if (__uint_as_float(v.y) < lim) return v.x;
+  }
+  return 0u;
+}
+
+namespace wide {
+PBRT_DEV unsigned long long pack(float a, float b) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  return v;
+}
+PBRT_DEV void unpack(unsigned long long v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+PBRT_DEV unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long v;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+  return v;
+}
+PBRT_DEV float max3(float a, float b, float c) {
+  float v;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(a), "f"(b), "f"(c));
+  return v;
+}
+PBRT_DEV float min3(float a, float b, float c) {
+  float v;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(a), "f"(b), "f"(c));
+  return v;
+}
+// Byte j of w as the float 2^23 + 256 * byte.
+template <int j>
+PBRT_DEV float grid(uint32_t w) {
+  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7604u | (j << 4)));
+}
+
+// Distances to the four slots' near (t0) and far (t1) planes on one axis, rounded outwards.
+// The plane is at org + 256 * byte * step, its distance fma(2^23 + 256 * byte, k, c) with
+// k = step * inv (exact), p = (org - o) * inv and c = p -+ m - 2^23 * k. The roundings of p, c
+// and the fma stay below 2^-21.9 |p| + 0.51 |k|, the exact test's own roundings and its widening
+// by 2*gamma(3) below 2^-21 of the distance, which is at most |p| + 2^16 |k|: m covers their sum.
+PBRT_DEV void planes(float org, float step, uint32_t lo, uint32_t hi, float o, float inv, float (&t0)[4],
+                     float (&t1)[4]) {
+  const float p = fm(fs(org, o), inv), k = fm(step, inv);
+  const float m = fa(fm(fabsf(p), 0x1p-20f), fabsf(k));
+  float c0, c1;
+  unpack(fma2(pack(-8388608.f, -8388608.f), pack(k, k), pack(fs(p, m), fa(p, m))), c0, c1);
+  const bool neg = inv < 0.f;
+  const uint32_t a = neg ? hi : lo, b = neg ? lo : hi;
+  const unsigned long long kk = pack(k, k), cc0 = pack(c0, c0), cc1 = pack(c1, c1);
+  unpack(fma2(pack(grid<0>(a), grid<1>(a)), kk, cc0), t0[0], t0[1]);
+  unpack(fma2(pack(grid<2>(a), grid<3>(a)), kk, cc0), t0[2], t0[3]);
+  unpack(fma2(pack(grid<0>(b), grid<1>(b)), kk, cc1), t1[0], t1[1]);
+  unpack(fma2(pack(grid<2>(b), grid<3>(b)), kk, cc1), t1[2], t1[3]);
+}
+
+// Entry distances of the four slots of a node (+inf: not hit within [near, lim] or empty).
+PBRT_DEV void slots(const WideNode* nd, const WRay& r, float near, float lim, float (&e)[4], uint32_t (&ref)[4]) {
+  float4 a, b, c, d;
+  load_node(reinterpret_cast<const float4*>(nd), a, b);
+  load_node(reinterpret_cast<const float4*>(nd) + 2, c, d);
+  float x0[4], x1[4], y0[4], y1[4], z0[4], z1[4];
+  planes(a.x, a.w, __float_as_uint(b.z), __float_as_uint(b.w), r.o.x, r.inv.x, x0, x1);
+  planes(a.y, b.x, __float_as_uint(c.x), __float_as_uint(c.y), r.o.y, r.inv.y, y0, y1);
+  planes(a.z, b.y, __float_as_uint(c.z), __float_as_uint(c.w), r.o.z, r.inv.z, z0, z1);
+  ref[0] = __float_as_uint(d.x);
+  ref[1] = __float_as_uint(d.y);
+  ref[2] = __float_as_uint(d.z);
+  ref[3] = __float_as_uint(d.w);
+  const float inf = __int_as_float(0x7f800000);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float t0 = fmaxf(max3(x0[i], y0[i], z0[i]), near);
+    const float t1 = fminf(min3(x1[i], y1[i], z1[i]), lim);
+    e[i] = t0 <= t1 && (i % 2 == 0 || ref[i] != 0u) ? t0 : inf;
+  }
+}
+
+PBRT_DEV void order(bool s, float& a, float& b, uint32_t& p, uint32_t& q) {  // exchanges when s
+  const float t = s ? b : a;
+  const uint32_t u = s ? q : p;
+  b = s ? a : b;
+  q = s ? p : q;
+  a = t;
+  p = u;
+}
+}  // namespace wide
+
+// The limit beyond which a wide walk drops a slot: the nearest distance and a little more.
+PBRT_DEV float wide_limit(float lim) { return fa(lim, fm(fabsf(lim), 0x1p-13f)); }
+
+// Visits one wide node: its slots hit within [near, reach], each pair nearest first and the
+// pair with the nearest slot first. The first is returned, the others are pushed; the next
+// pending one when none is hit; 0 when none is left.
+PBRT_DEV uint32_t wide_step(const WideNode* nd, const WRay& r, float near, float reach, WideStack& st, int& sp,
+                            uint32_t* err) {
+  float k[4];
+  uint32_t f[4];
+  wide::slots(nd, r, near, reach, k, f);
+  wide::order(k[1] < k[0], k[0], k[1], f[0], f[1]);
+  wide::order(k[3] < k[2], k[2], k[3], f[2], f[3]);
+  const bool s = k[2] < k[0];
+  wide::order(s, k[0], k[2], f[0], f[2]);
+  wide::order(s, k[1], k[3], f[1], f[3]);
+  const float inf = __int_as_float(0x7f800000);
+  if (k[3] < inf) wide_push(st, sp, f[3], k[3], err);
+  if (k[2] < inf) wide_push(st, sp, f[2], k[2], err);
+  if (k[1] < inf) wide_push(st, sp, f[1], k[1], err);
+  return k[0] < inf ? f[0] : wide_pop(st, sp, reach);
+}
+
+// Visits a sibling pair of the binary tree as the binary traversal does: the children hit with
+// an entry below lim, the right one first only when strictly nearer (bvh.rs:503-506).
+PBRT_DEV uint32_t binary_step(const float4* nodes, uint32_t pair, bool direct, const WRay& r, float near, float lim,
+                              WideStack& st, int& sp, uint32_t* err) {
+  const float4* n = nodes + 4 * size_t(pair);
+  float4 l0, l1, r0, r1;
+  load_node(n, l0, l1);
+  load_node(n + 2, r0, r1);
+  const PRay p = prepare_ray(r.o, r.d);
+  const float inf = __int_as_float(0x7f800000);
+  float dl, dr;
+  const bool hl = box_hit(p, l0, l1, near, inf, dl);
+  const bool hr = box_hit(p, r0, r1, near, inf, dr);
+  const bool swap = hl && hr && dr < dl;
+  const uint32_t fl = node_ref(l0, l1, 2u * pair, direct), fr = node_ref(r0, r1, 2u * pair + 1u, direct);
+  const bool hn = swap ? hr : hl, hf = swap ? hl : hr;
+  const float dn = swap ? dr : dl, df = swap ? dl : dr;
+  const uint32_t fn = swap ? fr : fl, ff = swap ? fl : fr;
+  const bool take_n = hn && dn < lim, take_f = hf && df < lim;
+  if (take_n) {
+    if (take_f) wide_push(st, sp, ff, df, err);
+    return fn;
+  }
+  return take_f ? ff : wide_pop(st, sp, lim);
+}
+
+// The triangles of one leaf in order. False: the ray must start again on the binary nodes.
+PBRT_DEV bool closest_in_leaf(const MeshView& m, uint32_t ref, const WRay& r, float near, float& lim, uint32_t& best,
+                              bool exact) {
+  uint32_t first, count;
+  leaf_range(m.nodes, ref, m.leaf_direct, first, count);
+  float t1 = lim;
+  uint32_t b1 = best;
+  bool tie = false;
+  for (uint32_t k = first; k < first + count; ++k) {
+    float4 A, B;
+    load_node(&m.tri[2 * size_t(k)], A, B);
+    const float2 C = __ldg(&m.tri_c[k]);
+    float t;
+    if (tri_hit(r.o, r.d, A, B, C.x, t) && t >= near) {
+      tie = tie || (t == lim && best != 0xFFFFFFFFu);
+      if (t < t1) {
+        t1 = t;
+        b1 = __float_as_uint(C.y);
+      }
+    }
+  }
+  if (!exact && (t1 < lim || tie)) {
+    const uint32_t node = __ldg(&m.leaf_node[first]);
+    const float4 lo = __ldg(&m.nodes[2 * size_t(node)]), hi = __ldg(&m.nodes[2 * size_t(node) + 1]);
+    float e;
+    if (!box_hit(prepare_ray(r.o, r.d), lo, hi, near, __int_as_float(0x7f800000), e)) return true;  // not its leaf
+    if (!(t1 < lim) || t1 < e) return false;  // a tie between leaves, or a hit before the leaf's entry
+  }
+  lim = t1;
+  best = b1;
+  return true;
+}
+
+// Whether some triangle of the leaf is hit within [near, lim).
+PBRT_DEV bool any_in_leaf(const MeshView& m, uint32_t ref, const WRay& r, float near, float lim, bool exact) {
+  uint32_t first, count;
+  leaf_range(m.nodes, ref, m.leaf_direct, first, count);
+  for (uint32_t k = first; k < first + count; ++k) {
+    float4 A, B;
+    load_node(&m.tri[2 * size_t(k)], A, B);
+    const float2 C = __ldg(&m.tri_c[k]);
+    float t;
+    if (tri_hit(r.o, r.d, A, B, C.x, t) && t < lim && t >= near) {
+      if (exact) return true;
+      const uint32_t node = __ldg(&m.leaf_node[first]);
+      const float4 lo = __ldg(&m.nodes[2 * size_t(node)]), hi = __ldg(&m.nodes[2 * size_t(node) + 1]);
+      float e;
+      return box_hit(prepare_ray(r.o, r.d), lo, hi, near, __int_as_float(0x7f800000), e) && e < lim;
+    }
+  }
+  return false;
+}
+
+}  // namespace pbrt
