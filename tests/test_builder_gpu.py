@@ -59,6 +59,20 @@ def test_degenerate_meshes():
     _same(v[:3], i[:1], 8, 1)
 
 
+@pytest.mark.parametrize("n", [2, 3, 32, 33, 127, 128, 129, 257, 2047, 2048, 2049, 4097])
+@pytest.mark.parametrize("bins,max_leaf", [(8, 1), (64, 3)])
+def test_sizes_around_the_kernels_limits(n, bins, max_leaf):
+    """Subtrees of one warp (128 triangles), chunks of the level kernels (2,048), and rows whose
+    partition is one long chain of moves (a triangle of the right side before all of the left)."""
+    rng = np.random.default_rng(n)
+    soup = (rng.random((n, 1, 3)) + 0.1 * rng.random((n, 3, 3))).astype(np.float32)
+    row = np.arange(n, dtype=np.float32)
+    row[0] = n + 1.5 * n  # far on the right, first in the order
+    line = (np.stack([row, 0 * row, 0 * row], 1)[:, None, :] + np.array([[0, 0, 0], [0.5, 0, 0], [0, 1, 0]])).astype(np.float32)
+    for t in (soup, line, line[::-1]):
+        _same(np.ascontiguousarray(t).reshape(-1, 3), np.arange(3 * n, dtype=np.uint32).reshape(-1, 3), bins, max_leaf)
+
+
 def test_large_mesh_and_speed():
     v, i = workloads.displaced_icosphere(8)  # 1,310,720 triangles
     ms = _same(v, i, 16, 4)
