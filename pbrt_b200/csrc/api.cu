@@ -74,7 +74,7 @@ int release_queue(pbrt_ctx* c, cudaStream_t st) {
 // memory may return before its DMA lands, and kernels on a non-blocking stream would not wait
 // for it. Scene creation synchronises that stream once all copies are queued.
 int upload(pbrt_ctx* c, void** dst, const void* src, size_t bytes, uint64_t* total) {
-  PBRT_TRY(c->cuda(cudaMalloc(dst, bytes), "cudaMalloc(scene)"));
+  PBRT_TRY(c->cuda(cudaMallocFromPoolAsync(dst, bytes, c->pool, c->stream), "cudaMalloc(scene)"));
   *total += bytes;
   return c->cuda(cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, c->stream), "cudaMemcpy(scene)");
 }
@@ -110,6 +110,15 @@ int pbrt_ctx_create(int device, pbrt_ctx** out) {
   // PBRT_TRACE_KERNEL=simple selects the one-thread-per-ray kernel (same results) for A/B runs.
   if (const char* k = std::getenv("PBRT_TRACE_KERNEL")) c->persistent = std::strcmp(k, "simple") != 0;
   if (c->cuda(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "cudaStreamCreate") != PBRT_OK)
+    return PBRT_ERR_CUDA;
+  cudaMemPoolProps pp{};
+  pp.allocType = cudaMemAllocationTypePinned;
+  pp.location.type = cudaMemLocationTypeDevice;
+  pp.location.id = device;
+  if (c->cuda(cudaMemPoolCreate(&c->pool, &pp), "cudaMemPoolCreate") != PBRT_OK) return PBRT_ERR_CUDA;
+  uint64_t keep = kPoolKeep;
+  if (c->cuda(cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute") !=
+      PBRT_OK)
     return PBRT_ERR_CUDA;
   if (c->cuda(cudaMalloc(&c->d_err, sizeof(uint32_t)), "cudaMalloc") != PBRT_OK) return PBRT_ERR_OUT_OF_MEMORY;
   if (c->cuda(cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), c->stream), "cudaMemset") != PBRT_OK)
@@ -167,6 +176,7 @@ void pbrt_ctx_destroy(pbrt_ctx* c) {
   cudaFree(c->queue);
   cudaFree(c->queue_rec);
   cudaStreamDestroy(c->stream);
+  if (c->pool) cudaMemPoolDestroy(c->pool);  // (memory of scenes still alive goes with them)
   delete c;
 }
 
@@ -211,7 +221,10 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
   for (uint32_t i = 0; i < fs.meshes.size() && rc == PBRT_OK; ++i) {
     const FlatMesh& fm = fs.meshes[i];
     DeviceMesh& dm = s->meshes[i];
-    const uint64_t ntri = d->meshes[i].triangle_count;
+    const pbrt_mesh_desc& md = d->meshes[i];
+    const uint64_t ntri = md.triangle_count;
+    void* pv = nullptr;
+    void* pi = nullptr;
     if (dev && i < dev->size() && (*dev)[i].nodes) {  // built on the GPU: take its arrays
       DeviceMeshBuild& b = (*dev)[i];
       dm.nodes = b.nodes;
@@ -220,6 +233,11 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
       dm.bytes = b.node_slots * sizeof(GpuNode) + ntri * 40;
       dm.view.node_count = uint32_t(b.node_slots);
       dm.leaf_node = b.tri_index;  // the triangle order is not needed any more: its words hold the leaves' nodes
+      pv = b.v;
+      pi = b.idx;
+      s->allocs.push_back(pv);
+      s->allocs.push_back(pi);
+      s->extra_bytes += size_t(md.vertex_count) * 12 + ntri * 12;
       b = DeviceMeshBuild{};
     } else {
       rc = upload(c, &dm.nodes, fm.nodes.data(), fm.nodes.size() * sizeof(GpuNode), &dm.bytes);
@@ -229,9 +247,11 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
       dm.view.node_count = uint32_t(fm.nodes.size());
     }
     dm.view.leaf_direct = ntri <= (uint64_t(1) << 27) && dm.view.node_count <= (1u << 27);
-    rc = c->cuda(cudaMalloc(&dm.wide, wide_bytes(dm.view.node_count)), "cudaMalloc(scene)");
+    rc = c->cuda(cudaMallocFromPoolAsync(&dm.wide, wide_bytes(dm.view.node_count), c->pool, c->stream),
+                 "cudaMalloc(scene)");
     if (rc == PBRT_OK && !dm.leaf_node)
-      rc = c->cuda(cudaMalloc(&dm.leaf_node, ntri * sizeof(uint32_t)), "cudaMalloc(scene)");
+      rc = c->cuda(cudaMallocFromPoolAsync(&dm.leaf_node, ntri * sizeof(uint32_t), c->pool, c->stream),
+                   "cudaMalloc(scene)");
     if (rc == PBRT_OK)
       rc = c->cuda(launch_widen(dm.nodes, dm.view.node_count, dm.view.leaf_direct, dm.wide,
                                 static_cast<uint32_t*>(dm.leaf_node), c->sm_count, c->stream),
@@ -244,13 +264,10 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
     dm.view.tri = (const float4*)dm.tri;
     dm.view.tri_c = (const float2*)dm.tri_c;
     views[i] = dm.view;
-    void* pv = nullptr;
-    void* pi = nullptr;
-    rc = s->upload(&pv, fs.mesh_v[i].data(), fs.mesh_v[i].size() * sizeof(float));
-    if (rc == PBRT_OK) rc = s->upload(&pi, fs.mesh_idx[i].data(), fs.mesh_idx[i].size() * sizeof(uint32_t));
+    if (!pv) rc = s->upload(&pv, md.vertices, size_t(md.vertex_count) * 3 * sizeof(float));
+    if (rc == PBRT_OK && !pi) rc = s->upload(&pi, md.indices, ntri * 3 * sizeof(uint32_t));
     void* pf = nullptr;
-    if (rc == PBRT_OK && !fs.mesh_fmat[i].empty())
-      rc = s->upload(&pf, fs.mesh_fmat[i].data(), fs.mesh_fmat[i].size() * sizeof(uint32_t));
+    if (rc == PBRT_OK && md.face_materials) rc = s->upload(&pf, md.face_materials, ntri * sizeof(uint32_t));
     shades[i] = MeshShade{(const float*)pv, (const uint32_t*)pi, (const uint32_t*)pf};
     s->info.triangle_count += ntri;
     s->info.mesh_node_count += fm.stats.node_count;
@@ -361,23 +378,21 @@ int build_meshes_on_device(pbrt_ctx* c, const pbrt_scene_desc* d, std::vector<pb
     float* dv = nullptr;
     uint32_t* di = nullptr;
     int rc = PBRT_OK;
-    if (vdev) {
-      dv = const_cast<float*>(m.vertices);
+    // the mesh's own copies: the build reads them, and the scene keeps them for shading
+    rc = c->cuda(cudaMallocFromPoolAsync(&dv, std::max<size_t>(vb, 4), c->pool, st), "cudaMalloc(build vertices)");
+    if (rc == PBRT_OK)
+      rc = c->cuda(cudaMallocFromPoolAsync(&di, std::max<size_t>(ib, 4), c->pool, st), "cudaMalloc(build indices)");
+    if (rc == PBRT_OK) rc = c->cuda(cudaMemcpyAsync(dv, m.vertices, vb, cudaMemcpyDefault, st), "cudaMemcpy(vertices)");
+    if (rc == PBRT_OK) rc = c->cuda(cudaMemcpyAsync(di, m.indices, ib, cudaMemcpyDefault, st), "cudaMemcpy(indices)");
+    if (rc == PBRT_OK && vdev) {  // the scene's host part reads them too
       (*hv)[i].resize(size_t(m.vertex_count) * 3);
       rc = c->cuda(cudaMemcpyAsync((*hv)[i].data(), m.vertices, vb, cudaMemcpyDeviceToHost, st), "cudaMemcpy(vertices)");
       (*md)[i].vertices = (*hv)[i].data();
-    } else {
-      rc = c->cuda(cudaMalloc(&dv, std::max<size_t>(vb, 4)), "cudaMalloc(build vertices)");
-      if (rc == PBRT_OK) rc = c->cuda(cudaMemcpyAsync(dv, m.vertices, vb, cudaMemcpyHostToDevice, st), "cudaMemcpy");
     }
     if (rc == PBRT_OK && idev) {
-      di = const_cast<uint32_t*>(m.indices);
       (*hi)[i].resize(size_t(m.triangle_count) * 3);
       rc = c->cuda(cudaMemcpyAsync((*hi)[i].data(), m.indices, ib, cudaMemcpyDeviceToHost, st), "cudaMemcpy(indices)");
       (*md)[i].indices = (*hi)[i].data();
-    } else if (rc == PBRT_OK) {
-      rc = c->cuda(cudaMalloc(&di, std::max<size_t>(ib, 4)), "cudaMalloc(build indices)");
-      if (rc == PBRT_OK) rc = c->cuda(cudaMemcpyAsync(di, m.indices, ib, cudaMemcpyHostToDevice, st), "cudaMemcpy");
     }
     if (rc == PBRT_OK && m.face_materials && mem_kind(m.face_materials) == MemKind::Device) {
       (*hf)[i].resize(m.triangle_count);
@@ -388,11 +403,12 @@ int build_meshes_on_device(pbrt_ctx* c, const pbrt_scene_desc* d, std::vector<pb
     }
     std::string e;
     if (rc == PBRT_OK &&
-        !build_mesh_bvh_device(dv, m.vertex_count, di, m.triangle_count, bp, st, c->sm_count, &(*builds)[i], &e))
+        !build_mesh_bvh_device(dv, m.vertex_count, di, m.triangle_count, bp, st, c->pool, c->sm_count, &(*builds)[i], &e))
       rc = c->fail(PBRT_ERR_INVALID_ARGUMENT, "mesh " + std::to_string(i) + ": " + e);
-    if (!vdev) cudaFree(dv);
-    if (!idev) cudaFree(di);
+    (*builds)[i].v = dv;
+    (*builds)[i].idx = di;
     if (rc != PBRT_OK) {
+      cudaStreamSynchronize(st);
       for (DeviceMeshBuild& b : *builds) free_device_mesh_build(&b);
       return rc;
     }
@@ -514,7 +530,9 @@ int pbrt_scene_create_many(pbrt_ctx* c, const pbrt_scene_desc* descs, uint32_t n
 void pbrt_scene_destroy(pbrt_scene* s) {
   if (!s) return;
   DeviceGuard g(s->ctx->device);
-  cudaStreamSynchronize(s->ctx->work_stream());
+  // every stream's work: a call may still run on a stream the context used before (and pool
+  // memory, unlike cudaMalloc's, is freed without waiting for anyone)
+  cudaDeviceSynchronize();
   for (auto& m : s->meshes) free_mesh(m);
   for (void* p : s->allocs) cudaFree(p);
   delete s;

@@ -894,15 +894,23 @@ __global__ void k_tri_layout(const uint32_t* __restrict__ order, uint32_t n, con
 
 // ---- host driver ------------------------------------------------------------------------------
 struct Scratch {
+  cudaStream_t st;
+  cudaMemPool_t mem;
   std::vector<void*> ptrs;
+  Scratch(cudaStream_t s, cudaMemPool_t m) : st(s), mem(m) {}
   ~Scratch() {
-    for (void* p : ptrs) cudaFree(p);
+    for (void* p : ptrs) cudaFreeAsync(p, st);
   }
   template <class T>
   cudaError_t alloc(T** p, size_t count) {
+    const cudaError_t e = keep(p, count);
+    if (e == cudaSuccess) ptrs.push_back(*p);
+    return e;
+  }
+  template <class T>
+  cudaError_t keep(T** p, size_t count) {  // not freed here
     void* q = nullptr;
-    const cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
-    if (e == cudaSuccess) ptrs.push_back(q);
+    const cudaError_t e = cudaMallocFromPoolAsync(&q, std::max<size_t>(count, 1) * sizeof(T), mem, st);
     *p = static_cast<T*>(q);
     return e;
   }
@@ -928,13 +936,13 @@ unsigned grid_for(uint64_t n, int threads, int sm_count) {
 }  // namespace
 
 bool build_mesh_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_idx, uint32_t n,
-                           const MeshBuildParams& p, cudaStream_t st, int sm_count, DeviceMeshBuild* out,
-                           std::string* err) {
+                           const MeshBuildParams& p, cudaStream_t st, cudaMemPool_t mem, int sm_count,
+                           DeviceMeshBuild* out, std::string* err) {
   *out = DeviceMeshBuild{};
   if (n == 0) { *err = "a TriangleMesh needs at least one triangle"; return false; }
   if (p.bins < 2 || p.bins > kMaxBins) { *err = "bvh_bins must be in [2, 64]"; return false; }
   const int B = p.bins;
-  Scratch s;
+  Scratch s(st, mem);
   // large nodes hold more than kSmall triangles each; a job at least two
   const size_t cap_nodes = size_t(n) / (kSmall + 1) + 1, cap_chunks = size_t(n) / kChunk + cap_nodes + 1;
   TriRec* bufs[2];
@@ -971,7 +979,7 @@ bool build_mesh_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_idx,
       if (b) free_device_mesh_build(b);
     }
   } guard{&o};
-  BUILD_TRY(cudaMalloc(&o.tri_index, size_t(n) * sizeof(uint32_t)));
+  BUILD_TRY(s.keep(&o.tri_index, n));
 
   // large nodes, level by level; `small` jobs follow
   int cur = 0;
@@ -1070,10 +1078,10 @@ bool build_mesh_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_idx,
   BUILD_TRY(cudaGetLastError());
 
   // outputs
-  BUILD_TRY(cudaMalloc(&o.nodes, (size_t(made) + 1) * sizeof(GpuNode)));
+  BUILD_TRY(s.keep(&o.nodes, size_t(made) + 1));
   o.node_slots = uint64_t(made) + 1;
-  BUILD_TRY(cudaMalloc(&o.tri, size_t(n) * 2 * sizeof(float4)));
-  BUILD_TRY(cudaMalloc(&o.tri_c, size_t(n) * sizeof(float2)));
+  BUILD_TRY(s.keep(&o.tri, size_t(n) * 2));
+  BUILD_TRY(s.keep(&o.tri_c, n));
   BUILD_TRY(cudaMemsetAsync(o.nodes + 1, 0, sizeof(GpuNode), st));  // the padding slot
   BUILD_TRY(cudaMemsetAsync(stats, 0, 4 * sizeof(uint32_t), st));
   k_layout<<<grid_for(made, 256, sm_count), 256, 0, st>>>(pool, made, ref, o.nodes, stats);
@@ -1102,6 +1110,8 @@ bool build_mesh_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_idx,
 }
 
 void free_device_mesh_build(DeviceMeshBuild* b) {
+  cudaFree(b->v);
+  cudaFree(b->idx);
   cudaFree(b->nodes);
   cudaFree(b->tri);
   cudaFree(b->tri_c);

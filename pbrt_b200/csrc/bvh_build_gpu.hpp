@@ -16,16 +16,18 @@ struct DeviceMeshBuild {
   float4* tri = nullptr;        // the triangle streams of mesh_bvh.hpp, in leaf order
   float2* tri_c = nullptr;
   uint32_t* tri_index = nullptr;  // leaf order -> original triangle index
+  float* v = nullptr;             // the mesh's own copy of its vertices and indices, for shading
+  uint32_t* idx = nullptr;
   MeshBuildStats stats;
   float bounds_min[3] = {0, 0, 0}, bounds_max[3] = {0, 0, 0};  // vertex bounds
 };
 
 // vertices (3 floats each) and indices (3 per triangle) in device memory of the current
-// device; runs on `st` and returns when the build is complete. On failure returns false with
-// `err` set (bad input is reported, not read out of range).
+// device; runs on `st` and returns when the build is complete (its memory comes from `pool`).
+// On failure returns false with `err` set (bad input is reported, not read out of range).
 bool build_mesh_bvh_device(const float* vertices, uint32_t vertex_count, const uint32_t* indices, uint32_t tri_count,
-                           const MeshBuildParams& params, cudaStream_t st, int sm_count, DeviceMeshBuild* out,
-                           std::string* err);
+                           const MeshBuildParams& params, cudaStream_t st, cudaMemPool_t pool, int sm_count,
+                           DeviceMeshBuild* out, std::string* err);
 void free_device_mesh_build(DeviceMeshBuild* build);
 
 }  // namespace pbrt

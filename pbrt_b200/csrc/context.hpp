@@ -20,6 +20,7 @@ namespace api {
 
 constexpr uint64_t kSlotRays = uint64_t(1) << 20;  // rays per pipelined chunk (32 MiB of rays)
 constexpr int kSlots = 3;
+constexpr uint64_t kPoolKeep = uint64_t(1) << 30;  // bytes the context's memory pool keeps mapped when free
 constexpr uint64_t kDevChunk = uint64_t(1) << 24;  // rays per launch pair on device buffers
 // Concurrent branches of a wavefront batch frame (pbrt_ctx_set_batch_branches).
 constexpr uint32_t kMaxBatchBranches = 8;
@@ -81,6 +82,11 @@ struct pbrt_ctx {
   int sm_count = 0;
   cudaStream_t stream = nullptr;  // internal stream
   cudaStream_t user = nullptr;    // caller's stream (asynchronous device-buffer calls)
+  // Scenes and the device tree build take their memory here: a mapping costs 0.1-1 ms and a
+  // rebuilt mesh needs some 30. Up to kPoolKeep bytes stay mapped between scenes; what is freed
+  // beyond that goes back to the device when the stream next synchronises, all of it with the
+  // context.
+  cudaMemPool_t pool = nullptr;
   std::string err;
   uint32_t* d_err = nullptr;
   unsigned long long* d_counters = nullptr;  // [0..2] traversal counters, [4..5] queue length / fetch position,
@@ -146,7 +152,7 @@ struct pbrt_scene {
 
   int upload(void** dst, const void* src, size_t bytes) {
     if (bytes == 0) return PBRT_OK;
-    int rc = ctx->cuda(cudaMalloc(dst, bytes), "cudaMalloc(scene)");
+    int rc = ctx->cuda(cudaMallocFromPoolAsync(dst, bytes, ctx->pool, ctx->stream), "cudaMalloc(scene)");
     if (rc != PBRT_OK) return rc;
     allocs.push_back(*dst);
     extra_bytes += bytes;

@@ -466,9 +466,6 @@ bool build_scene(const pbrt_scene_desc& d, FlatScene* out, std::string* err, con
   bp.max_leaf = d.bvh_max_leaf ? d.bvh_max_leaf : 1;
 
   out->meshes.resize(d.mesh_count);
-  out->mesh_v.resize(d.mesh_count);
-  out->mesh_idx.resize(d.mesh_count);
-  out->mesh_fmat.resize(d.mesh_count);
   for (uint32_t i = 0; i < d.mesh_count; ++i) {
     const pbrt_mesh_desc& md = d.meshes[i];
     std::string e;
@@ -484,15 +481,12 @@ bool build_scene(const pbrt_scene_desc& d, FlatScene* out, std::string* err, con
       *err = "mesh " + std::to_string(i) + ": " + e;
       return false;
     }
-    out->mesh_v[i].assign(md.vertices, md.vertices + 3 * size_t(md.vertex_count));
-    out->mesh_idx[i].assign(md.indices, md.indices + 3 * size_t(md.triangle_count));
     if (md.face_materials) {
       for (uint32_t t = 0; t < md.triangle_count; ++t)
         if (md.face_materials[t] >= d.material_count) {
           *err = "mesh " + std::to_string(i) + ": triangle " + std::to_string(t) + " has a bad material";
           return false;
         }
-      out->mesh_fmat[i].assign(md.face_materials, md.face_materials + md.triangle_count);
     }
   }
 
@@ -656,12 +650,12 @@ bool build_scene(const pbrt_scene_desc& d, FlatScene* out, std::string* err, con
       }
       if (em.texture != PBRT_TEXTURE_COLOR) { *err = who + "an area light's emission must be a plain colour"; return false; }
       if (ob.shape == PBRT_SHAPE_MESH) {
-        const std::vector<float>& v = out->mesh_v[ob.mesh];
-        const std::vector<uint32_t>& ix = out->mesh_idx[ob.mesh];
+        const float* v = d.meshes[ob.mesh].vertices;
+        const uint32_t* ix = d.meshes[ob.mesh].indices;
         r.tri_first = uint32_t(out->light_cdf.size());
-        r.tri_count = uint32_t(ix.size() / 3);
+        r.tri_count = d.meshes[ob.mesh].triangle_count;
         float run = 0.0f;
-        for (size_t t = 0; t < ix.size() / 3; ++t) {
+        for (size_t t = 0; t < r.tri_count; ++t) {
           V3f p[3];
           for (int k = 0; k < 3; ++k) {
             const uint32_t vi = ix[3 * t + k];

@@ -23,9 +23,6 @@ namespace pbrt {
 
 struct FlatScene {
   std::vector<FlatMesh> meshes;
-  std::vector<std::vector<float>> mesh_v;       // original vertices (shading)
-  std::vector<std::vector<uint32_t>> mesh_idx;  // original indices (shading)
-  std::vector<std::vector<uint32_t>> mesh_fmat; // per-triangle material, empty when absent
   std::vector<ObjRec> objects;                  // leaves: placed Simple objects
   std::vector<XfRec> xforms;                    // transform chains beyond each leaf's first
   std::vector<CsgRec> csg;                      // constructive solids' elements
