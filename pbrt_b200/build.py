@@ -25,12 +25,9 @@ NVCC = os.environ.get("PBRT_NVCC", shutil.which("nvcc") or "/usr/local/cuda/bin/
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off", "-ccbin", "g++",
                      "-I", CSRC, "-I", INCLUDE]
-# Per-file extra flags: the parity-critical kernels forbid FMA contraction outright.
-NVCC_EXTRA = {
-    "kernels_trace.cu": ["-fmad=false"],
-    "kernels_render.cu": ["-fmad=false", "--split-compile=8"],
-    "api.cu": ["-fmad=false"],
-}
+# The parity-critical kernels forbid FMA contraction outright.
+NVCC_EXTRA = {f: ["-fmad=false"] for f in ("kernels_trace.cu", "kernels_render.cu", "kernels_walk_one.cu",
+                                           "kernels_walk_many.cu", "kernels_scene_rays.cu", "api.cu")}
 CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-ffp-contract=off", "-fno-fast-math", "-Wall", "-I", CSRC, "-I", INCLUDE]
 
 

@@ -70,24 +70,6 @@ int release_queue(pbrt_ctx* c, cudaStream_t st) {
   return c->cuda(cudaEventRecord(c->queue_used, st), "cudaEventRecord(survivor queue)");
 }
 
-// Host-to-device copies go on the context's own stream: a plain cudaMemcpy from pageable
-// memory may return before its DMA lands, and kernels on a non-blocking stream would not wait
-// for it. Scene creation synchronises that stream once all copies are queued.
-int upload(pbrt_ctx* c, void** dst, const void* src, size_t bytes, uint64_t* total) {
-  PBRT_TRY(c->cuda(cudaMallocFromPoolAsync(dst, bytes, c->pool, c->stream), "cudaMalloc(scene)"));
-  *total += bytes;
-  return c->cuda(cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, c->stream), "cudaMemcpy(scene)");
-}
-
-void free_mesh(DeviceMesh& m) {
-  cudaFree(m.nodes);
-  cudaFree(m.wide);
-  cudaFree(m.leaf_node);
-  cudaFree(m.tri);
-  cudaFree(m.tri_c);
-  m = DeviceMesh{};
-}
-
 }  // namespace
 
 extern "C" {
@@ -198,8 +180,6 @@ int pbrt_ctx_sync(pbrt_ctx* c) {
 
 namespace {
 
-constexpr uint64_t kDeferMinTriangles = 4096;
-
 // The device half of scene creation: checks the built structure, uploads it, fills the view.
 // Meshes listed in `dev` (non-null nodes) were built on the GPU: their arrays are taken over.
 int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbrt_scene** out,
@@ -214,71 +194,120 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
 
   std::unique_ptr<pbrt_scene> s(new pbrt_scene);
   s->ctx = c;
-  s->meshes.resize(fs.meshes.size());
-  std::vector<MeshView> views(fs.meshes.size());
-  std::vector<MeshShade> shades(fs.meshes.size());
-  int rc = PBRT_OK;
-  for (uint32_t i = 0; i < fs.meshes.size() && rc == PBRT_OK; ++i) {
-    const FlatMesh& fm = fs.meshes[i];
-    DeviceMesh& dm = s->meshes[i];
+  const uint32_t nm = uint32_t(fs.meshes.size());
+  auto built = [&](uint32_t i) { return dev && i < dev->size() && (*dev)[i].nodes; };  // on the GPU
+  // All meshes' nodes and triangles end to end, and one wide tree: the top level's nodes first
+  // (index 0 stays unused), then each mesh's.
+  std::vector<uint64_t> node_at(nm + 1, 0), tri_at(nm + 1, 0), wide_at(nm + 1, 0);
+  wide_at[0] = fs.top.size() / 2 + 1;
+  uint32_t deepest = 0;
+  for (uint32_t i = 0; i < nm; ++i) {
+    const uint64_t slots = built(i) ? (*dev)[i].node_slots : fs.meshes[i].nodes.size();
+    node_at[i + 1] = node_at[i] + slots;
+    tri_at[i + 1] = tri_at[i] + d->meshes[i].triangle_count;
+    wide_at[i + 1] = wide_at[i] + slots / 2 + 1;
+    deepest = std::max(deepest, fs.meshes[i].stats.max_depth);
+  }
+  const uint64_t total_nodes = node_at[nm], total_tris = tri_at[nm], total_wide = wide_at[nm];
+  if (total_tris >= (uint64_t(1) << 30) || total_nodes >= (uint64_t(1) << 32) || total_wide >= (uint64_t(1) << 31))
+    return c->fail(PBRT_ERR_CAPACITY, "a scene holds at most 2^30 triangles");
+  const bool direct = total_tris <= (uint64_t(1) << 26);
+  s->meshes.resize(nm);
+  std::vector<MeshView> views(nm);
+  std::vector<MeshShade> shades(nm);
+  void *nodes = nullptr, *tri = nullptr, *tri_c = nullptr, *wide = nullptr, *leaf = nullptr;
+  int rc = s->alloc(&wide, total_wide * sizeof(WideNode));
+  if (rc == PBRT_OK && nm) rc = s->alloc(&leaf, total_tris * sizeof(uint2));
+  if (rc == PBRT_OK && nm == 1 && built(0)) {  // the only mesh's arrays are the scene's
+    DeviceMeshBuild& b = (*dev)[0];
+    s->take(nodes = b.nodes, total_nodes * sizeof(GpuNode));
+    s->take(tri = b.tri, total_tris * 32);
+    s->take(tri_c = b.tri_c, total_tris * 8);
+    b.nodes = nullptr;
+    b.tri = nullptr;
+    b.tri_c = nullptr;
+  } else if (rc == PBRT_OK && nm) {
+    rc = s->alloc(&nodes, total_nodes * sizeof(GpuNode));
+    if (rc == PBRT_OK) rc = s->alloc(&tri, total_tris * 32);
+    if (rc == PBRT_OK) rc = s->alloc(&tri_c, total_tris * 8);
+    for (uint32_t i = 0; i < nm && rc == PBRT_OK; ++i) {
+      const FlatMesh& fm = fs.meshes[i];
+      const bool on_gpu = built(i);
+      const size_t nt = d->meshes[i].triangle_count;
+      auto put = [&](void* dst, size_t at, const void* src, size_t bytes) {
+        return c->cuda(cudaMemcpyAsync(static_cast<char*>(dst) + at, src, bytes, cudaMemcpyDefault, c->stream),
+                       "cudaMemcpy(scene)");
+      };
+      rc = put(nodes, node_at[i] * sizeof(GpuNode), on_gpu ? (const void*)(*dev)[i].nodes : fm.nodes.data(),
+               (node_at[i + 1] - node_at[i]) * sizeof(GpuNode));
+      if (rc == PBRT_OK) rc = put(tri, tri_at[i] * 32, on_gpu ? (const void*)(*dev)[i].tri : fm.tri.data(), nt * 32);
+      if (rc == PBRT_OK) rc = put(tri_c, tri_at[i] * 8, on_gpu ? (const void*)(*dev)[i].tri_c : fm.tri_c.data(), nt * 8);
+    }
+  }
+  // The primitives' references: a mesh placed untransformed, once, is merged (its wide root),
+  // anything else is an object leaf.
+  std::vector<uint32_t> slot_ref(fs.order.size()), owner(nm, 0xFFFFFFFFu);
+  bool objects = !fs.unbounded.empty();
+  for (uint32_t k = 0; k < fs.order.size(); ++k) {
+    const uint32_t ref = fs.order[k];
+    const ObjRec* ob = ref & kGroupBit ? nullptr : &fs.objects[ref];
+    if (ob && ob->shape == kShapeMesh && ob->xf_count == 0 && owner[ob->mesh] == 0xFFFFFFFFu) {
+      const uint32_t m = ob->mesh;
+      owner[m] = ref;
+      const uint32_t count = uint32_t(tri_at[m + 1] - tri_at[m]);
+      slot_ref[k] = node_at[m + 1] - node_at[m] > 2 ? uint32_t(wide_at[m]) + 1u  // the root's pair
+                                                    : triangle_ref(uint32_t(tri_at[m]), count, direct);
+    } else {
+      slot_ref[k] = kLeafRef | kObjectRef | k;
+      objects = true;
+    }
+  }
+  for (uint32_t i = 0; i < nm && rc == PBRT_OK; ++i) {
     const pbrt_mesh_desc& md = d->meshes[i];
-    const uint64_t ntri = md.triangle_count;
+    MeshView& v = views[i];
+    v.nodes = static_cast<const float4*>(nodes) + 2 * node_at[i];
+    v.tri = static_cast<const float4*>(tri) + 2 * tri_at[i];
+    v.tri_c = static_cast<const float2*>(tri_c) + tri_at[i];
+    v.node_count = uint32_t(node_at[i + 1] - node_at[i]);
+    s->meshes[i] = v;
+    WidenArgs a{};
+    a.nodes = v.nodes;
+    a.count = v.node_count;
+    a.wide = static_cast<WideNode*>(wide);
+    a.wide_base = uint32_t(wide_at[i]);
+    a.direct = direct;
+    a.tri_base = uint32_t(tri_at[i]);
+    a.node_base = uint32_t(node_at[i]);
+    a.owner = owner[i];
+    a.leaf = static_cast<uint2*>(leaf);
+    rc = c->cuda(launch_widen(a, c->sm_count, c->stream), "scene upload");
     void* pv = nullptr;
     void* pi = nullptr;
-    if (dev && i < dev->size() && (*dev)[i].nodes) {  // built on the GPU: take its arrays
+    if (built(i) || (dev && i < dev->size() && (*dev)[i].v)) {  // the build's copies of the mesh's arrays
       DeviceMeshBuild& b = (*dev)[i];
-      dm.nodes = b.nodes;
-      dm.tri = b.tri;
-      dm.tri_c = b.tri_c;
-      dm.bytes = b.node_slots * sizeof(GpuNode) + ntri * 40;
-      dm.view.node_count = uint32_t(b.node_slots);
-      dm.leaf_node = b.tri_index;  // the triangle order is not needed any more: its words hold the leaves' nodes
-      pv = b.v;
-      pi = b.idx;
-      s->allocs.push_back(pv);
-      s->allocs.push_back(pi);
-      s->extra_bytes += size_t(md.vertex_count) * 12 + ntri * 12;
-      b = DeviceMeshBuild{};
+      s->take(pv = b.v, size_t(md.vertex_count) * 12);
+      s->take(pi = b.idx, size_t(md.triangle_count) * 12);
+      b.v = nullptr;
+      b.idx = nullptr;
     } else {
-      rc = upload(c, &dm.nodes, fm.nodes.data(), fm.nodes.size() * sizeof(GpuNode), &dm.bytes);
-      if (rc == PBRT_OK) rc = upload(c, &dm.tri, fm.tri.data(), fm.tri.size() * sizeof(float), &dm.bytes);
-      if (rc == PBRT_OK) rc = upload(c, &dm.tri_c, fm.tri_c.data(), fm.tri_c.size() * sizeof(float), &dm.bytes);
-      if (rc != PBRT_OK) break;
-      dm.view.node_count = uint32_t(fm.nodes.size());
+      if (rc == PBRT_OK) rc = s->upload(&pv, md.vertices, size_t(md.vertex_count) * 3 * sizeof(float));
+      if (rc == PBRT_OK) rc = s->upload(&pi, md.indices, size_t(md.triangle_count) * 3 * sizeof(uint32_t));
     }
-    dm.view.leaf_direct = ntri <= (uint64_t(1) << 27) && dm.view.node_count <= (1u << 27);
-    rc = c->cuda(cudaMallocFromPoolAsync(&dm.wide, wide_bytes(dm.view.node_count), c->pool, c->stream),
-                 "cudaMalloc(scene)");
-    if (rc == PBRT_OK && !dm.leaf_node)
-      rc = c->cuda(cudaMallocFromPoolAsync(&dm.leaf_node, ntri * sizeof(uint32_t), c->pool, c->stream),
-                   "cudaMalloc(scene)");
-    if (rc == PBRT_OK)
-      rc = c->cuda(launch_widen(dm.nodes, dm.view.node_count, dm.view.leaf_direct, dm.wide,
-                                static_cast<uint32_t*>(dm.leaf_node), c->sm_count, c->stream),
-                   "scene upload");
-    if (rc != PBRT_OK) break;
-    dm.bytes += wide_bytes(dm.view.node_count) + ntri * sizeof(uint32_t);
-    dm.view.wide = (const WideNode*)dm.wide;
-    dm.view.leaf_node = (const uint32_t*)dm.leaf_node;
-    dm.view.nodes = (const float4*)dm.nodes;
-    dm.view.tri = (const float4*)dm.tri;
-    dm.view.tri_c = (const float2*)dm.tri_c;
-    views[i] = dm.view;
-    if (!pv) rc = s->upload(&pv, md.vertices, size_t(md.vertex_count) * 3 * sizeof(float));
-    if (rc == PBRT_OK && !pi) rc = s->upload(&pi, md.indices, ntri * 3 * sizeof(uint32_t));
     void* pf = nullptr;
-    if (rc == PBRT_OK && md.face_materials) rc = s->upload(&pf, md.face_materials, ntri * sizeof(uint32_t));
+    if (rc == PBRT_OK && md.face_materials) rc = s->upload(&pf, md.face_materials, size_t(md.triangle_count) * 4);
     shades[i] = MeshShade{(const float*)pv, (const uint32_t*)pi, (const uint32_t*)pf};
-    s->info.triangle_count += ntri;
+    const FlatMesh& fm = fs.meshes[i];
+    s->info.triangle_count += md.triangle_count;
     s->info.mesh_node_count += fm.stats.node_count;
     s->info.mesh_leaf_count += fm.stats.leaf_count;
     s->info.mesh_max_depth = std::max(s->info.mesh_max_depth, fm.stats.max_depth);
     s->info.mesh_max_leaf_tris = std::max(s->info.mesh_max_leaf_tris, fm.stats.max_leaf_tris);
-    s->info.device_bytes += dm.bytes;
   }
   void *top = nullptr, *order = nullptr, *objs = nullptr, *mviews = nullptr, *mshades = nullptr, *mats = nullptr,
        *lights = nullptr, *ltris = nullptr, *lcdf = nullptr, *unb = nullptr, *xfs = nullptr, *grps = nullptr,
-       *csgs = nullptr;
+       *csgs = nullptr, *srefs = nullptr, *snodes = nullptr;
+  if (rc == PBRT_OK && !slot_ref.empty()) rc = s->upload(&srefs, slot_ref.data(), slot_ref.size() * sizeof(uint32_t));
+  if (rc == PBRT_OK && !slot_ref.empty()) rc = s->alloc(&snodes, slot_ref.size() * sizeof(uint32_t));
   if (rc == PBRT_OK && !fs.top.empty()) rc = s->upload(&top, fs.top.data(), fs.top.size() * sizeof(GpuNode));
   if (rc == PBRT_OK && !fs.order.empty()) rc = s->upload(&order, fs.order.data(), fs.order.size() * sizeof(uint32_t));
   if (rc == PBRT_OK) rc = s->upload(&objs, fs.objects.data(), fs.objects.size() * sizeof(ObjRec));
@@ -318,18 +347,36 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
   v.light_cdf = (const float*)lcdf;
   v.has_csg = 0;
   for (const ObjRec& ob : fs.objects) v.has_csg |= ob.shape == kShapeCsg ? 1u : 0u;
-  // The leaf the renderer answers in passes of its own: the largest untransformed mesh placed
-  // directly in the top-level tree, of at least kDeferMinTriangles triangles.
-  v.defer_leaf = kNoLeaf;
-  uint64_t defer_tris = kDeferMinTriangles - 1;
-  for (const uint32_t ref : fs.order) {
-    if (ref & kGroupBit) continue;
-    const ObjRec& ob = fs.objects[ref];
-    if (ob.shape != kShapeMesh || ob.xf_count != 0) continue;
-    const uint64_t nt = d->meshes[ob.mesh].triangle_count;
-    if (nt > defer_tris) {
-      defer_tris = nt;
-      v.defer_leaf = ref;
+  v.has_objects = objects ? 1u : 0u;
+  WideView& w = v.wide;
+  w.wide = (const WideNode*)wide;
+  w.tri = (const float4*)tri;
+  w.tri_c = (const float2*)tri_c;
+  w.leaf = (const uint2*)leaf;
+  w.nodes = (const float4*)nodes;
+  w.slot_node = (const uint32_t*)snodes;
+  w.count = uint32_t(total_wide);
+  w.direct = direct;
+  // (a top level of one leaf has no wide node: its primitive's reference is the root)
+  w.root = fs.top.empty() ? 0u : (fs.top.size() > 2 ? 1u : slot_ref[0]);
+  // The wide walk needs its coordinates inside the grid's arithmetic and its pending slots,
+  // three per two levels, inside its stack; otherwise every ray takes the binary nodes.
+  w.bounded = 3 * ((fs.top_depth + 1) / 2 + (deepest + 1) / 2 + 2) <= uint32_t(kWideStack);
+  for (const GpuNode& g : fs.top)
+    for (int x = 0; x < 3; ++x)
+      if (!(std::fabs(g.bmin[x]) <= kWideLimit) || !(std::fabs(g.bmax[x]) <= kWideLimit)) w.bounded = false;
+  if (!fs.top.empty()) {
+    WidenArgs a{};
+    a.nodes = (const float4*)top;
+    a.count = uint32_t(fs.top.size());
+    a.wide = static_cast<WideNode*>(wide);
+    a.direct = direct;
+    a.slot_ref = (const uint32_t*)srefs;
+    a.slot_node = (uint32_t*)snodes;
+    const int rc1 = c->cuda(launch_widen(a, c->sm_count, c->stream), "scene upload");
+    if (rc1 != PBRT_OK) {
+      pbrt_scene_destroy(s.release());
+      return rc1;
     }
   }
   s->info.object_count = fs.primitive_count;
@@ -533,7 +580,6 @@ void pbrt_scene_destroy(pbrt_scene* s) {
   // every stream's work: a call may still run on a stream the context used before (and pool
   // memory, unlike cudaMalloc's, is freed without waiting for anyone)
   cudaDeviceSynchronize();
-  for (auto& m : s->meshes) free_mesh(m);
   for (void* p : s->allocs) cudaFree(p);
   delete s;
 }
@@ -636,7 +682,8 @@ int trace_impl(pbrt_scene* s, const float* rays, uint64_t n, uint32_t* prim, flo
   if (stats && !scene_stats && s->single_mesh < 0)
     return c->fail(PBRT_ERR_UNSUPPORTED, "work counters are reported for scenes made of one untransformed mesh");
   const bool one_mesh = s->single_mesh >= 0 && !scene_stats;
-  const MeshView mv = one_mesh ? s->meshes[s->single_mesh].view : MeshView{};
+  const MeshView mv = one_mesh ? s->meshes[s->single_mesh] : MeshView{};
+  const WideView& wv = s->view.wide;
   // Nearest hit / any hit of one chunk of `m` rays (planes `stride` apart) on `st`.
   auto launch = [&](const float* r, uint64_t stride, uint64_t m, uint32_t* p, float* tt, uint32_t* ob, uint8_t* oc,
                     unsigned long long* cnt, uint32_t* queue, unsigned long long* qc, float4* rec,
@@ -645,9 +692,9 @@ int trace_impl(pbrt_scene* s, const float* rays, uint64_t n, uint32_t* prim, flo
       return oc ? launch_scene_any(s->view, r, stride, m, oc, cnt, c->d_err, c->sm_count, st)
                 : launch_scene_closest(s->view, r, stride, m, p, tt, ob, cnt, c->d_err, c->sm_count, st);
     if (oc && !queue) return launch_mesh_any(mv, r, stride, m, oc, c->d_err, c->sm_count, st);
-    if (oc) return launch_mesh_any_persistent(mv, r, stride, m, oc, queue, qc, c->d_err, c->sm_count, st, rec);
+    if (oc) return launch_mesh_any_persistent(mv, wv, r, stride, m, oc, queue, qc, c->d_err, c->sm_count, st, rec);
     if (c->persistent && !cnt)
-      return launch_mesh_closest_persistent(mv, r, stride, m, p, tt, ob, queue, qc, c->d_err, c->sm_count, st, rec);
+      return launch_mesh_closest_persistent(mv, wv, r, stride, m, p, tt, ob, queue, qc, c->d_err, c->sm_count, st, rec);
     return launch_mesh_closest(mv, r, stride, m, p, tt, ob, cnt, c->d_err, c->sm_count, st);
   };
 
@@ -781,9 +828,9 @@ int pbrt_trace_closest_noalloc(pbrt_scene* s, const float* rays, uint64_t n, uin
                    "pbrt_trace_closest_noalloc takes device buffers only (host buffers need staging memory)");
   if (s->single_mesh < 0)
     return c->fail(PBRT_ERR_UNSUPPORTED, "pbrt_trace_closest_noalloc traces scenes made of one untransformed mesh");
-  const MeshView& mv = s->meshes[s->single_mesh].view;
+  const MeshView& mv = s->meshes[s->single_mesh];
   uint32_t* scratch = c->noalloc_scratch;
-  PBRT_TRY(c->cuda(launch_mesh_closest_noalloc(mv, rays, n, prim_id, t, scratch, c->sm_count, st),
+  PBRT_TRY(c->cuda(launch_mesh_closest_noalloc(mv, s->view.wide, rays, n, prim_id, t, scratch, c->sm_count, st),
                    "pbrt_trace_closest_noalloc"));
   uint32_t h = 0;  // the error word, read back on the same stream (no legacy-stream wait)
   PBRT_TRY(c->cuda(cudaMemcpyAsync(&h, scratch + 4, sizeof(h), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync"));

@@ -128,20 +128,10 @@ struct pbrt_ctx {
   cudaStream_t work_stream() const { return user ? user : stream; }
 };
 
-struct DeviceMesh {
-  void* nodes = nullptr;
-  void* wide = nullptr;
-  void* leaf_node = nullptr;
-  void* tri = nullptr;
-  void* tri_c = nullptr;
-  pbrt::MeshView view{};
-  uint64_t bytes = 0;
-};
-
 struct pbrt_scene {
   pbrt_ctx* ctx = nullptr;
-  std::vector<DeviceMesh> meshes;
-  std::vector<void*> allocs;  // every other device array of the scene
+  std::vector<pbrt::MeshView> meshes;  // one mesh's binary tree and triangles each
+  std::vector<void*> allocs;           // every device array of the scene
   uint64_t extra_bytes = 0;
   pbrt::SceneView view{};
   pbrt_scene_info info{};
@@ -150,13 +140,22 @@ struct pbrt_scene {
   float max_radiance = 0.f;              // bound of reflected radiance (see FlatScene)
   bool has_dielectric = false;
 
+  void take(void* p, size_t bytes) {  // an array allocated elsewhere becomes the scene's
+    allocs.push_back(p);
+    extra_bytes += bytes;
+  }
+  int alloc(void** dst, size_t bytes) {
+    const int rc = ctx->cuda(cudaMallocFromPoolAsync(dst, bytes, ctx->pool, ctx->stream), "cudaMalloc(scene)");
+    if (rc == 0) take(*dst, bytes);
+    return rc;
+  }
+  // Host-to-device copies go on the context's own stream: a plain cudaMemcpy from pageable
+  // memory may return before its DMA lands, and kernels on a non-blocking stream would not wait
+  // for it. Scene creation synchronises that stream once all copies are queued.
   int upload(void** dst, const void* src, size_t bytes) {
     if (bytes == 0) return PBRT_OK;
-    int rc = ctx->cuda(cudaMallocFromPoolAsync(dst, bytes, ctx->pool, ctx->stream), "cudaMalloc(scene)");
+    const int rc = alloc(dst, bytes);
     if (rc != PBRT_OK) return rc;
-    allocs.push_back(*dst);
-    extra_bytes += bytes;
-    // ordered on the context's stream (see upload in api.cu); scene creation synchronises it
     return ctx->cuda(cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream), "cudaMemcpy(scene)");
   }
 };

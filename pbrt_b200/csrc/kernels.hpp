@@ -7,6 +7,8 @@
 namespace pbrt {
 
 struct MeshView;
+struct WideView;
+struct WideNode;
 
 // Ray buffers: eight planes (ox oy oz dx dy dz tmin tmax) of `stride` floats each, of which
 // the first `n` are used.
@@ -18,27 +20,35 @@ cudaError_t launch_mesh_closest(const MeshView& m, const float* rays, uint64_t s
 // dynamic-fetch traversal over the queue. `counters` is two 64-bit words of scratch (queue
 // length, fetch position), zeroed on `s` by the launcher. `rec` (scratch, 2 x n float4): the
 // survivors' rays copied beside their queue entries, read back coalesced.
-cudaError_t launch_mesh_closest_persistent(const MeshView& m, const float* rays, uint64_t stride, uint64_t n,
+cudaError_t launch_mesh_closest_persistent(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
                                            uint32_t* prim, float* t, uint32_t* obj, uint32_t* queue,
                                            unsigned long long* counters, uint32_t* err, int sm_count, cudaStream_t s,
                                            float4* rec);
 // The same two stages for occlusion.
-cudaError_t launch_mesh_any_persistent(const MeshView& m, const float* rays, uint64_t stride, uint64_t n, uint8_t* occ,
+cudaError_t launch_mesh_any_persistent(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n, uint8_t* occ,
                                        uint32_t* queue, unsigned long long* counters, uint32_t* err, int sm_count,
                                        cudaStream_t s, float4* rec);
-// A tree's wide nodes (wide_bvh.cuh): their bytes for node_slots binary records, and the
-// kernel that writes them and each leaf's node beside its first triangle (leaf_node, one word
-// per triangle). direct: leaf references hold first and count (at most 2^27 triangles).
-size_t wide_bytes(uint64_t node_slots);
-cudaError_t launch_widen(const void* nodes, uint32_t node_slots, bool direct, void* wide, uint32_t* leaf_node,
-                         int sm_count, cudaStream_t s);
+// One binary tree's part of a scene's wide tree (wide_bvh.cuh): a mesh's (slot_ref NULL), or the
+// top level's. A tree of `count` records (GPU numbering) takes count / 2 + 1 wide nodes.
+struct WidenArgs {
+  const float4* nodes;
+  uint32_t count;
+  WideNode* wide;
+  uint32_t wide_base;
+  bool direct;
+  uint32_t tri_base, node_base, owner;  // a mesh: its first triangle, first node and object in the scene's arrays
+  uint2* leaf;
+  const uint32_t* slot_ref;  // the top level: each primitive's reference
+  uint32_t* slot_node;
+};
+cudaError_t launch_widen(const WidenArgs& a, int sm_count, cudaStream_t s);
 // Allocation-free form of launch_mesh_closest_persistent for device buffers (plane stride
 // = n): its scratch is a file-scope __device__ array of kNoAllocMaxRays queue entries
 // shared by every call on a device. `scratch` is that array's device address on the current
 // device, from noalloc_scratch_lookup (word 4 is the error word). cudaErrorInvalidValue when
 // n > kNoAllocMaxRays. Calls that overlap on the GPU race.
 constexpr uint64_t kNoAllocMaxRays = uint64_t(1) << 20;
-cudaError_t launch_mesh_closest_noalloc(const MeshView& m, const float* rays, uint64_t n, uint32_t* prim, float* t,
+cudaError_t launch_mesh_closest_noalloc(const MeshView& m, const WideView& w, const float* rays, uint64_t n, uint32_t* prim, float* t,
                                         uint32_t* scratch, int sm_count, cudaStream_t s);
 // Device address of the allocation-free pass's scratch array on the current device. The
 // lookup loads this file's module there (under lazy loading), which commits the array.

@@ -1,10 +1,10 @@
 // kernels_render.cu — wavefront path tracing and general-scene ray casting.
 //
-// A wave of paths (up to the context's wave size, 2^22 by default) lives in SoA buffers. Each bounce runs three kernels over
-// queues of path indices: extend (nearest hit), shade (emission, light sampling, BSDF
+// A wave of paths (up to the context's wave size, 2^26 by default) lives in SoA buffers. Each bounce runs three kernels over
+// queues of path indices: nearest (persistent walk, walk_kernels.cuh), shade (emission, light sampling, BSDF
 // sampling, Russian roulette; pushes the surviving paths to the next queue and at most one
 // shadow ray per path to the shadow queue, both with one atomicAdd per warp) and shadow
-// (any hit; adds the light sample's contribution when unoccluded). Radiance is added to a
+// (any hit, persistent walk; adds the light sample's contribution when unoccluded). Radiance is added to a
 // path in exactly the order PathIntegrator::li adds it (src/integrators/path.rs:55-113):
 // emission, then the light sample, then the next vertex's emission or the background. At
 // the end of a wave, accumulate adds every path's FP32 radiance into the FP64 film.
@@ -17,11 +17,15 @@
 #include "kernels.hpp"
 #include "render.hpp"
 #include "scene_device.cuh"
+#include "walk.cuh"
 
 namespace pbrt {
 
+#ifndef PBRT_SHADE_BLOCKS
+#define PBRT_SHADE_BLOCKS 3
+#endif
+
 constexpr float kPiF = 3.14159265358979323846f;
-constexpr float kShadowEps = 0.00001f;  // SHADOW_RAY_EPSILON (src/lights.rs:21)
 constexpr uint32_t kSpecularBit = 0x80000000u;
 
 // ---- sampler: PCG32, one stream per pixel, re-keyed per (pixel, sample) ------------------
@@ -307,30 +311,6 @@ PBRT_DEV void write_record(float* rec, const F3& p, float rough, const F3& wo, c
   r[3] = make_float4(alb.x, alb.y, alb.z, 0.f);
 }
 
-// ---- where a path's scene comes from ------------------------------------------------------------
-// The wavefront kernels are written once over a scene source: one scene passed as a kernel
-// parameter (pbrt_render, the cached render), or the batch table indexed by the path's scene.
-struct PathSettings {
-  uint32_t max_depth, rr_start, integrator;  // integrator: 0 path, 1 naive, 2 normal
-  float near, far;
-};
-
-struct OneScene {
-  SceneView v;
-  PathSettings ps;
-  PBRT_DEV const SceneView& view(const WaveBuffers&, uint32_t) const { return v; }
-  PBRT_DEV PathSettings settings(const WaveBuffers&, uint32_t) const { return ps; }
-};
-
-struct ManyScenes {
-  const BatchScene* b;
-  PBRT_DEV const SceneView& view(const WaveBuffers& w, uint32_t p) const { return b[w.scene[p]].view; }
-  PBRT_DEV PathSettings settings(const WaveBuffers& w, uint32_t p) const {
-    const BatchScene& e = b[w.scene[p]];
-    return PathSettings{e.max_depth, e.rr_start, e.integrator, e.cam.near, e.cam.far};
-  }
-};
-
 // ---- kernels ---------------------------------------------------------------------------------
 // A new path for image pixel `pixel`, sample `sample`: jitter, camera ray, fresh state.
 PBRT_DEV void begin_path(const CameraRec& cam, unsigned long long seed, uint32_t pixel, uint32_t sample,
@@ -394,7 +374,10 @@ __global__ void __launch_bounds__(256) k_generate(WaveBuffers w, CameraRec cam, 
     }
     start_path(w, i, cam, seed, pixel, sample);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) w.counts[0] = n;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    w.counts[0] = n;
+    w.counts[3] = 0u;
+  }
 }
 
 __global__ void __launch_bounds__(256) k_generate_batch(WaveBuffers w, const BatchScene* __restrict__ b,
@@ -411,201 +394,9 @@ __global__ void __launch_bounds__(256) k_generate_batch(WaveBuffers w, const Bat
     start_path(w, i, e.cam, e.seed, pixel, sample);
     w.scene[i] = lo;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) w.counts[0] = n;
-}
-
-// Scene::find_nearest for the queued paths, one thread per path (scene_closest). At least 4
-// resident 256-thread blocks per SM (at most 64 registers a thread) for the traversal kernels:
-// measured 2-4% faster than the compiler's 86 registers on the Cornell, many-spheres and
-// torus-knot renders.
-template <class Src, bool kCsg>
-__global__ void __launch_bounds__(256, 4) k_extend(WaveBuffers w, Src src, const uint32_t* __restrict__ q,
-                                                const uint32_t* __restrict__ qcount, uint32_t* err,
-                                                unsigned long long* stats, uint32_t defer) {
-  const uint32_t n = *qcount;
-  if (stats && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(stats, (unsigned long long)n);
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const uint32_t p = q[k];
-    const SceneView& s = src.view(w, p);
-    const PathSettings ps = src.settings(w, p);
-    const F3 o = mk3(w.ox[p], w.oy[p], w.oz[p]), d = mk3(w.dx[p], w.dy[p], w.dz[p]);
-    float t = 0.f;
-    uint32_t obj = 0xFFFFFFFFu, prim = 0;
-    if (!scene_closest<kCsg>(s, o, d, ps.near, ps.far, t, obj, prim, err, defer ? s.defer_leaf : kNoLeaf))
-      obj = 0xFFFFFFFFu;
-    w.ht[p] = t;
-    w.hobj[p] = obj;
-    w.hprim[p] = prim;
-  }
-}
-
-// Scene::find_nearest for the queued paths (scene_closest_t, visit for visit), restated as a
-// persistent walk of the top-level BVH with one warp-voted step per iteration: a node step
-// (or a pop) for the lanes not standing on a leaf, or, once at least `leaf_min` lanes stand on
-// a leaf they must visit (or no lane has anything else to do), a leaf step for those; idle
-// lanes take the next queued paths (one atomicAdd on `fetch` per warp) once at least
-// `refill_min` of them are idle. Hit t / object / primitive are those of scene_closest: the
-// same boxes, the same order, the same adoptions. It pays where the top-level tree is deep
-// (10,000 spheres) and costs where a path's query is a few nodes (a 4-object box), hence
-// kWalkMinTopNodes. At 2 resident blocks per SM it keeps its walk state in registers.
-template <class Src, bool kCsg>
-__global__ void __launch_bounds__(256, 2) k_extend_walk(WaveBuffers w, Src src, const uint32_t* __restrict__ q,
-                                                     const uint32_t* __restrict__ qcount, uint32_t* __restrict__ fetch,
-                                                     uint32_t* err, unsigned long long* stats, int leaf_min,
-                                                     int refill_min, uint32_t defer) {
-  const uint32_t n = *qcount;
-  if (stats && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(stats, (unsigned long long)n);
-  const unsigned lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
-  bool active = false, exhausted = false;  // exhausted is warp-uniform
-  uint32_t p = 0;
-  F3 o = mk3(0.f, 0.f, 0.f), d = o;
-  PRay r;
-  float near = 0.f, min_t = 0.f, cur_e = 0.f;
-  bool have = false;
-  uint32_t leaf_out = 0, prim_out = 0, lf = 0, count = 0, budget = 0;
-  int sp = 0;
-  uint32_t stk_lf[kTraceStack], stk_cnt[kTraceStack];
-  float stk_e[kTraceStack];
-  for (;;) {
-    const unsigned idle = __ballot_sync(0xffffffffu, !active);
-    if (!exhausted && idle && (__popc(idle) >= refill_min || idle == 0xffffffffu)) {
-      const int leader = __ffs(idle) - 1;
-      uint32_t base = 0;
-      if (int(lane) == leader) base = atomicAdd(fetch, uint32_t(__popc(idle)));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      exhausted = uint64_t(base) + __popc(idle) >= n;
-      const uint64_t k = uint64_t(base) + __popc(idle & lt_mask);
-      if (!active && k < n) {
-        p = q[k];
-        const SceneView& s = src.view(w, p);
-        const PathSettings ps = src.settings(w, p);
-        o = mk3(w.ox[p], w.oy[p], w.oz[p]);
-        d = mk3(w.dx[p], w.dy[p], w.dz[p]);
-        near = ps.near;
-        min_t = ps.far;
-        have = false;
-        prim_out = 0;
-        for (uint32_t u = 0; u < s.unbounded_count; ++u) {  // nearest_among + closer (scene.rs:222-249)
-          float t;
-          uint32_t leaf, prim;
-          if (prim_closest<kCsg>(s, __ldg(&s.unbounded[u]), o, d, near, ps.far, t, leaf, prim, err) &&
-              (!have || t < min_t)) {
-            have = true;
-            min_t = t;
-            leaf_out = leaf;
-            prim_out = prim;
-          }
-        }
-        bool walk = false;
-        if (s.top_node_count != 0) {
-          r = prepare_ray(o, d);
-          const float4 rlo = __ldg(&s.top[0]);
-          const float4 rhi = __ldg(&s.top[1]);
-          float entry;
-          if (box_hit(r, rlo, rhi, near, min_t, entry)) {
-            lf = __float_as_uint(rlo.w);
-            count = __float_as_uint(rhi.w);
-            cur_e = entry;
-            sp = 0;
-            budget = 2u * s.top_node_count + 2u;  // every node is pushed (and popped) at most once
-            walk = true;
-          }
-        }
-        if (walk) {
-          active = true;
-        } else {
-          w.ht[p] = have ? min_t : 0.f;
-          w.hobj[p] = have ? leaf_out : 0xFFFFFFFFu;
-          w.hprim[p] = prim_out;
-        }
-      }
-    }
-    const unsigned act = __ballot_sync(0xffffffffu, active);
-    if (act == 0) {
-      if (exhausted) break;
-      continue;  // all idle and the queue not yet drained: the next iteration refills
-    }
-    const bool at_leaf = active && cur_e < min_t && count > 0;  // a leaf this lane must visit
-    const unsigned on_leaf = __ballot_sync(0xffffffffu, at_leaf);
-    const bool leaf_step = __popc(on_leaf) >= leaf_min || on_leaf == act;
-    bool done = false;
-    if (active && at_leaf == leaf_step) {
-      const SceneView& s = src.view(w, p);
-      if (budget-- == 0) {
-        atomicOr(err, kErrBudget);
-        done = true;
-      } else if (leaf_step) {
-        // A leaf: its primitives over [near, min_t], a candidate adopted only when strictly nearer.
-        for (uint32_t k = lf; k < lf + count; ++k) {
-          const uint32_t ref = __ldg(&s.order[k]);
-          if (defer && ref == s.defer_leaf) continue;  // answered by k_defer_closest
-          float t;
-          uint32_t leaf, prim;
-          if (prim_closest<kCsg>(s, ref, o, d, near, min_t, t, leaf, prim, err) && (!have || t < min_t)) {
-            have = true;
-            min_t = t;
-            leaf_out = leaf;
-            prim_out = prim;
-          }
-        }
-        if (sp == 0) {
-          done = true;
-        } else {
-          --sp;
-          lf = stk_lf[sp];
-          count = stk_cnt[sp];
-          cur_e = stk_e[sp];
-        }
-      } else {
-        // One node of the walk: an interior node's children (the farther pushed, the nearer
-        // taken), or a pop when the current entry is dropped (>= min_t) or no child was hit.
-        bool pop = true;
-        if (cur_e < min_t) {
-          float4 l0, l1, r0, r1;
-          load_node(&s.top[2 * lf], l0, l1);
-          load_node(&s.top[2 * lf + 2], r0, r1);
-          float dl, dr;
-          const bool hl = box_hit(r, l0, l1, near, min_t, dl);
-          const bool hr = box_hit(r, r0, r1, near, min_t, dr);
-          const bool swap = hl && hr && dr < dl;
-          const bool hn = swap ? hr : hl, hf = swap ? hl : hr;
-          const float dn = swap ? dr : dl, df = swap ? dl : dr;
-          if (hf) {
-            if (sp >= kTraceStack) {
-              atomicOr(err, kErrStack);
-              done = true;
-            } else {
-              stk_lf[sp] = __float_as_uint(swap ? l0.w : r0.w);
-              stk_cnt[sp] = __float_as_uint(swap ? l1.w : r1.w);
-              stk_e[sp] = df;
-              ++sp;
-            }
-          }
-          if (hn) {
-            lf = __float_as_uint(swap ? r0.w : l0.w);
-            count = __float_as_uint(swap ? r1.w : l1.w);
-            cur_e = dn;
-            pop = false;
-          }
-        }
-        if (pop && !done) {
-          if (sp == 0) {
-            done = true;
-          } else {
-            --sp;
-            lf = stk_lf[sp];
-            count = stk_cnt[sp];
-            cur_e = stk_e[sp];
-          }
-        }
-      }
-    }
-    if (done) {
-      w.ht[p] = have ? min_t : 0.f;  // the adopted hit's distance (min_t = c.d)
-      w.hobj[p] = have ? leaf_out : 0xFFFFFFFFu;
-      w.hprim[p] = prim_out;
-      active = false;
-    }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    w.counts[0] = n;
+    w.counts[3] = 0u;
   }
 }
 
@@ -736,7 +527,7 @@ PBRT_DEV void shade_vertex(const SceneView& s, const PathSettings& ps, PathState
 }
 
 template <class Src, bool kStage>
-__global__ void __launch_bounds__(256) k_shade(WaveBuffers w, Src src, const uint32_t* __restrict__ q,
+__global__ void __launch_bounds__(256, PBRT_SHADE_BLOCKS) k_shade(WaveBuffers w, Src src, const uint32_t* __restrict__ q,
                                                const uint32_t* __restrict__ qcount, uint32_t* __restrict__ qout,
                                                uint32_t* __restrict__ qout_count, CacheWave cw, uint32_t cache_mode,
                                                uint32_t term_hit) {
@@ -745,6 +536,7 @@ __global__ void __launch_bounds__(256) k_shade(WaveBuffers w, Src src, const uin
   __shared__ uint32_t st_path[kStage ? kMaxThreads : 1];
   __shared__ float st_rec[kStage ? 10 : 1][kStage ? kMaxThreads : 1];
   const uint32_t n = *qcount;
+  if (blockIdx.x == 0 && threadIdx.x == 0) w.counts[3] = 0u;  // the next nearest walk's fetch position
   // every lane runs the same trip count so the warp-aggregated pushes see full warps
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t iters = (n + stride - 1) / stride;
@@ -758,8 +550,9 @@ __global__ void __launch_bounds__(256) k_shade(WaveBuffers w, Src src, const uin
     float crough = 0.f;
     if (k < n) {
       p = q[k];
-      const SceneView& s = src.view(w, p);
-      const PathSettings ps = src.settings(w, p);
+      const typename Src::Cursor c = src.cursor(w, p);
+      const SceneView& s = src.view(c);
+      const PathSettings ps = src.settings(c);
       PathState P;
       P.o = mk3(w.ox[p], w.oy[p], w.oz[p]);
       P.d = mk3(w.dx[p], w.dy[p], w.dz[p]);
@@ -891,322 +684,6 @@ __global__ void __launch_bounds__(256) k_train_batch(WaveBuffers w, CacheWave cw
     for (int c = 0; c < 3; ++c) {
       const float b = ts[3 + c];
       tgt[3 * size_t(i) + c] = b > 0.f ? cache_value(fdv(fs(le[c], ts[c]), b), max_l) : 0.f;
-    }
-  }
-}
-
-// 3 resident blocks per SM (the torus-knot frame 54.1 -> 52.9 ms against 4; 2 gained nothing
-// more; with the solids' code, 48 of 770 bytes still spill).
-// With `defer`, a scene's deferred leaf is left out: an occluded entry is resolved (its t_max
-// set to -1), an unoccluded one of a scene without a deferred leaf adds its light sample and
-// is resolved, and the others wait for k_defer_any.
-template <class Src, bool kCsg>
-__global__ void __launch_bounds__(256, 3) k_shadow(WaveBuffers w, Src src, uint32_t* err, unsigned long long* stats,
-                                                uint32_t defer) {
-  const uint32_t n = w.counts[2];
-  if (stats && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(stats + 1, (unsigned long long)n);
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const uint32_t p = w.s_path[k];
-    const SceneView& s = src.view(w, p);
-    const F3 o = mk3(w.s_ox[k], w.s_oy[k], w.s_oz[k]), d = mk3(w.s_dx[k], w.s_dy[k], w.s_dz[k]);
-    const uint32_t skip = defer ? s.defer_leaf : kNoLeaf;
-    if (scene_any<kCsg>(s, o, d, kShadowEps, w.s_tmax[k], err, skip)) {
-      if (defer) w.s_tmax[k] = -1.f;
-    } else if (skip == kNoLeaf) {  // VisibilityTester::unoccluded (lights.rs:67-69)
-      w.lr[p] = fa(w.lr[p], w.s_cr[k]);
-      w.lg[p] = fa(w.lg[p], w.s_cg[k]);
-      w.lb[p] = fa(w.lb[p], w.s_cb[k]);
-      if (defer) w.s_tmax[k] = -1.f;
-    }
-  }
-}
-
-// ---- the deferred leaf ----------------------------------------------------------------------
-// Resident 128-thread blocks per SM the deferred passes are compiled for (8: at most 64
-// registers a thread).
-#ifndef PBRT_DEFER_MIN_BLOCKS
-#define PBRT_DEFER_MIN_BLOCKS 8
-#endif
-
-// A scene's largest mesh, when it is placed untransformed in the top-level tree, is left out
-// of the per-path queries above and answered here for all queued paths at once by persistent
-// warps over the paths (the ray-cast kernel's while-while schedule: idle lanes refilled with
-// one atomicAdd per warp, interior nodes walked until every lane stands on a leaf, the leaves
-// of all lanes tested in one pass). Each lane walks its own scene's mesh (batches mix scenes).
-//
-// Nearest hit: the mesh is offered [near, nearest hit so far] and its hit adopted only when
-// strictly nearer, which is what Scene::find_nearest does with it wherever it comes in the
-// top-level order (scene.rs:186-220); an object's own answer does not depend on the interval
-// it is offered as long as its hit lies inside, so the result is the per-path query's, up to
-// which of two objects hit at exactly the same distance is kept.
-template <class Src>
-__global__ void __launch_bounds__(128, PBRT_DEFER_MIN_BLOCKS) k_defer_closest(WaveBuffers w, Src src, const uint32_t* __restrict__ q,
-                                                       const uint32_t* __restrict__ qcount,
-                                                       uint32_t* __restrict__ fetch, uint32_t* err) {
-  const uint32_t n = *qcount;
-  const unsigned lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
-  bool active = false;
-  uint32_t p = 0, leaf = 0, best = 0xFFFFFFFFu, lf = 0, count = 0, budget = 0;
-  MeshView m{};
-  PRay r;
-  float near = 0.f, far = 0.f, min_t = FLT_MAX;
-  bool have = false;
-  int sp = 0;
-  uint32_t stk_lf[kTraceStack], stk_cnt[kTraceStack];
-  float stk_e[kTraceStack];
-  for (;;) {
-    const unsigned idle = __ballot_sync(0xffffffffu, !active);
-    bool exhausted = false;
-    if (idle) {
-      const int leader = __ffs(idle) - 1;
-      uint32_t base = 0;
-      if (int(lane) == leader) base = atomicAdd(fetch, uint32_t(__popc(idle)));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      exhausted = uint64_t(base) + __popc(idle) >= n;
-      const uint64_t k = uint64_t(base) + __popc(idle & lt_mask);
-      if (!active && k < n) {
-        p = q[k];
-        const SceneView& s = src.view(w, p);
-        leaf = s.defer_leaf;
-        if (leaf != kNoLeaf) {
-          const PathSettings ps = src.settings(w, p);
-          m = s.meshes[s.objects[leaf].mesh];
-          r = prepare_ray(mk3(w.ox[p], w.oy[p], w.oz[p]), mk3(w.dx[p], w.dy[p], w.dz[p]));
-          near = ps.near;
-          have = w.hobj[p] != 0xFFFFFFFFu;
-          far = have ? w.ht[p] : ps.far;
-          const float4 rlo = __ldg(&m.nodes[0]);
-          const float4 rhi = __ldg(&m.nodes[1]);
-          float entry;
-          // the root is pushed, then dropped at pop if its entry is >= min_t = FLT_MAX (bvh.rs:462-472)
-          if (box_hit(r, rlo, rhi, near, far, entry) && entry < FLT_MAX) {
-            lf = __float_as_uint(rlo.w);
-            count = __float_as_uint(rhi.w);
-            min_t = FLT_MAX;
-            best = 0xFFFFFFFFu;
-            sp = 0;
-            budget = m.node_count;
-            active = true;
-          }
-        }
-      }
-    }
-    if (__ballot_sync(0xffffffffu, active) == 0) {
-      if (exhausted) break;
-      continue;
-    }
-    if (active) {
-      bool done = false;
-      while (count == 0) {  // interior nodes until this lane stands on a leaf
-        if (budget-- == 0) {
-          atomicOr(err, kErrBudget);
-          done = true;
-          break;
-        }
-        float4 l0, l1, r0, r1;
-        load_node(&m.nodes[2 * lf], l0, l1);
-        load_node(&m.nodes[2 * lf + 2], r0, r1);
-        float dl, dr;
-        const bool hl = box_hit(r, l0, l1, near, far, dl);
-        const bool hr = box_hit(r, r0, r1, near, far, dr);
-        const bool swap = hl && hr && dr < dl;  // right first only when strictly nearer
-        const bool hn = swap ? hr : hl, hf = swap ? hl : hr;
-        const float dn = swap ? dr : dl, df = swap ? dl : dr;
-        const bool take_f = hf && df < min_t, take_n = hn && dn < min_t;
-        if (take_n) {
-          if (take_f) {
-            if (sp >= kTraceStack) {
-              atomicOr(err, kErrStack);
-              done = true;
-              break;
-            }
-            stk_lf[sp] = __float_as_uint(swap ? l0.w : r0.w);
-            stk_cnt[sp] = __float_as_uint(swap ? l1.w : r1.w);
-            stk_e[sp] = df;
-            ++sp;
-          }
-          lf = __float_as_uint(swap ? r0.w : l0.w);
-          count = __float_as_uint(swap ? r1.w : l1.w);
-        } else if (take_f) {
-          lf = __float_as_uint(swap ? l0.w : r0.w);
-          count = __float_as_uint(swap ? l1.w : r1.w);
-        } else {
-          bool found = false;  // pop, dropping entries at or beyond the nearest hit (bvh.rs:470-472)
-          while (sp > 0) {
-            --sp;
-            if (stk_e[sp] < min_t) {
-              lf = stk_lf[sp];
-              count = stk_cnt[sp];
-              found = true;
-              break;
-            }
-          }
-          if (!found) {
-            done = true;
-            break;
-          }
-        }
-      }
-      if (!done) {  // the leaves of every lane standing on one
-        if (budget-- == 0) {
-          atomicOr(err, kErrBudget);
-          done = true;
-        } else {
-          for (uint32_t k = lf; k < lf + count; ++k) {
-            float4 A, B;
-            load_node(&m.tri[2 * size_t(k)], A, B);
-            const float2 C = __ldg(&m.tri_c[k]);
-            float t;
-            if (tri_hit(r.o, r.d, A, B, C.x, t) && t < min_t && t >= near && t <= far) {
-              min_t = t;
-              best = __float_as_uint(C.y);
-            }
-          }
-          bool found = false;
-          while (sp > 0) {
-            --sp;
-            if (stk_e[sp] < min_t) {
-              lf = stk_lf[sp];
-              count = stk_cnt[sp];
-              found = true;
-              break;
-            }
-          }
-          if (!found) done = true;
-        }
-      }
-      if (done) {
-        if (best != 0xFFFFFFFFu && (!have || min_t < far)) {  // adopted only when strictly nearer
-          w.ht[p] = min_t;
-          w.hobj[p] = leaf;
-          w.hprim[p] = best;
-        }
-        active = false;
-      }
-    }
-  }
-}
-
-// Shadow rays against the deferred leaf: the entries k_shadow left open (t_max >= 0) add their
-// light sample when the mesh does not block [kShadowEps, t_max]; any hit ends the walk.
-template <class Src>
-__global__ void __launch_bounds__(128, PBRT_DEFER_MIN_BLOCKS) k_defer_any(WaveBuffers w, Src src, uint32_t* __restrict__ fetch,
-                                                   uint32_t* err) {
-  const uint32_t n = w.counts[2];
-  const unsigned lane = threadIdx.x & 31u, lt_mask = (1u << lane) - 1u;
-  bool active = false;
-  uint32_t k = 0, p = 0, lf = 0, count = 0, budget = 0;
-  MeshView m{};
-  PRay r;
-  float far = 0.f;
-  int sp = 0;
-  uint32_t stk_lf[kTraceStack], stk_cnt[kTraceStack];
-  for (;;) {
-    const unsigned idle = __ballot_sync(0xffffffffu, !active);
-    bool exhausted = false;
-    if (idle) {
-      const int leader = __ffs(idle) - 1;
-      uint32_t base = 0;
-      if (int(lane) == leader) base = atomicAdd(fetch, uint32_t(__popc(idle)));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      exhausted = uint64_t(base) + __popc(idle) >= n;
-      const uint64_t kk = uint64_t(base) + __popc(idle & lt_mask);
-      if (!active && kk < n) {
-        k = uint32_t(kk);
-        far = w.s_tmax[k];
-        if (far >= 0.f) {  // still open
-          p = w.s_path[k];
-          const SceneView& s = src.view(w, p);
-          m = s.meshes[s.objects[s.defer_leaf].mesh];
-          r = prepare_ray(mk3(w.s_ox[k], w.s_oy[k], w.s_oz[k]), mk3(w.s_dx[k], w.s_dy[k], w.s_dz[k]));
-          const float4 rlo = __ldg(&m.nodes[0]);
-          const float4 rhi = __ldg(&m.nodes[1]);
-          float entry;
-          if (box_hit(r, rlo, rhi, kShadowEps, far, entry)) {
-            lf = __float_as_uint(rlo.w);
-            count = __float_as_uint(rhi.w);
-            sp = 0;
-            budget = m.node_count;
-            active = true;
-          } else {  // misses the mesh: unoccluded
-            w.lr[p] = fa(w.lr[p], w.s_cr[k]);
-            w.lg[p] = fa(w.lg[p], w.s_cg[k]);
-            w.lb[p] = fa(w.lb[p], w.s_cb[k]);
-          }
-        }
-      }
-    }
-    if (__ballot_sync(0xffffffffu, active) == 0) {
-      if (exhausted) break;
-      continue;
-    }
-    if (active) {
-      bool done = false, hit = false;
-      while (count == 0) {
-        if (budget-- == 0) {
-          atomicOr(err, kErrBudget);
-          done = true;
-          hit = true;  // a malformed tree: reported, the sample dropped
-          break;
-        }
-        float4 l0, l1, r0, r1;
-        load_node(&m.nodes[2 * lf], l0, l1);
-        load_node(&m.nodes[2 * lf + 2], r0, r1);
-        float dl, dr;
-        const bool hl = box_hit(r, l0, l1, kShadowEps, far, dl);
-        const bool hr = box_hit(r, r0, r1, kShadowEps, far, dr);
-        const bool swap = hl && hr && dr < dl;  // the nearer child first: the likelier blocker
-        const bool hn = swap ? hr : hl, hf = swap ? hl : hr;
-        if (hn) {
-          if (hf) {
-            if (sp >= kTraceStack) {
-              atomicOr(err, kErrStack);
-              done = true;
-              hit = true;
-              break;
-            }
-            stk_lf[sp] = __float_as_uint(swap ? l0.w : r0.w);
-            stk_cnt[sp] = __float_as_uint(swap ? l1.w : r1.w);
-            ++sp;
-          }
-          lf = __float_as_uint(swap ? r0.w : l0.w);
-          count = __float_as_uint(swap ? r1.w : l1.w);
-        } else if (hf) {
-          lf = __float_as_uint(swap ? l0.w : r0.w);
-          count = __float_as_uint(swap ? l1.w : r1.w);
-        } else if (sp > 0) {
-          --sp;
-          lf = stk_lf[sp];
-          count = stk_cnt[sp];
-        } else {
-          done = true;
-          break;
-        }
-      }
-      if (!done) {
-        for (uint32_t j = lf; j < lf + count && !hit; ++j) {
-          float4 A, B;
-          load_node(&m.tri[2 * size_t(j)], A, B);
-          const float2 C = __ldg(&m.tri_c[j]);
-          float t;
-          if (tri_hit(r.o, r.d, A, B, C.x, t) && t >= kShadowEps && t <= far) hit = true;
-        }
-        if (hit || sp == 0) {
-          done = true;
-        } else {
-          --sp;
-          lf = stk_lf[sp];
-          count = stk_cnt[sp];
-        }
-      }
-      if (done) {
-        if (!hit) {
-          w.lr[p] = fa(w.lr[p], w.s_cr[k]);
-          w.lg[p] = fa(w.lg[p], w.s_cg[k]);
-          w.lb[p] = fa(w.lb[p], w.s_cb[k]);
-        }
-        active = false;
-      }
     }
   }
 }
@@ -1367,114 +844,11 @@ __global__ void k_scale_film(double* film, size_t n, double s) {
     film[i] *= s;
 }
 
-// ---- general-scene ray casting ---------------------------------------------------------------
-// Adds a thread's counters to cnt[0..2] (one atomic per warp and counter).
-PBRT_DEV void flush_counts(const SceneCount& c, unsigned long long* cnt) {
-  unsigned long long v[3] = {c.nodes, c.boxes, c.objects};
-  for (int k = 0; k < 3; ++k) {
-    for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_down_sync(0xFFFFFFFFu, v[k], off);
-    if ((threadIdx.x & 31) == 0 && v[k]) atomicAdd(cnt + k, v[k]);
-  }
-}
-
-// Nearest hit per ray; object ids are the description's (the leaf's desc_id). kCount adds
-// the scene accelerator's counters (Scene::intersect_instrumented) into cnt.
-template <bool kCount, bool kCsg>
-__global__ void __launch_bounds__(128) k_scene_closest(SceneView s, const float* __restrict__ rays, uint64_t stride,
-                                                       uint64_t n, uint32_t* __restrict__ prim, float* __restrict__ tout,
-                                                       uint32_t* __restrict__ obj, unsigned long long* cnt,
-                                                       uint32_t* err) {
-  SceneCount c{0, 0, 0};
-  // whole warps run the same trip count so the counter reduction sees full warps
-  const uint64_t step = uint64_t(gridDim.x) * blockDim.x;
-  const uint64_t iters = (n + step - 1) / step;
-  for (uint64_t it = 0; it < iters; ++it) {
-    const uint64_t i = it * step + uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) continue;
-    const F3 o = mk3(__ldcs(rays + i), __ldcs(rays + stride + i), __ldcs(rays + 2 * stride + i));
-    const F3 d = mk3(__ldcs(rays + 3 * stride + i), __ldcs(rays + 4 * stride + i), __ldcs(rays + 5 * stride + i));
-    const float near = __ldcs(rays + 6 * stride + i), far = __ldcs(rays + 7 * stride + i);
-    float t = 0.f;
-    uint32_t leaf = 0, pr = 0;
-    const bool hit = scene_closest_t<kCount, kCsg>(s, o, d, near, far, t, leaf, pr, err, &c);
-    __stcs(prim + i, hit ? pr : 0xFFFFFFFFu);
-    __stcs(tout + i, hit ? t : __int_as_float(0x7f800000));
-    if (obj) __stcs(obj + i, hit ? s.objects[leaf].desc_id : 0xFFFFFFFFu);
-  }
-  if (kCount) flush_counts(c, cnt);
-}
-
-template <bool kCount, bool kCsg>
-__global__ void __launch_bounds__(128) k_scene_any(SceneView s, const float* __restrict__ rays, uint64_t stride,
-                                                   uint64_t n, uint8_t* __restrict__ occ, unsigned long long* cnt,
-                                                   uint32_t* err) {
-  SceneCount c{0, 0, 0};
-  const uint64_t step = uint64_t(gridDim.x) * blockDim.x;
-  const uint64_t iters = (n + step - 1) / step;
-  for (uint64_t it = 0; it < iters; ++it) {
-    const uint64_t i = it * step + uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) continue;
-    const F3 o = mk3(__ldcs(rays + i), __ldcs(rays + stride + i), __ldcs(rays + 2 * stride + i));
-    const F3 d = mk3(__ldcs(rays + 3 * stride + i), __ldcs(rays + 4 * stride + i), __ldcs(rays + 5 * stride + i));
-    occ[i] = scene_any_t<kCount, kCsg>(s, o, d, __ldcs(rays + 6 * stride + i), __ldcs(rays + 7 * stride + i), err, &c)
-                 ? 1
-                 : 0;
-  }
-  if (kCount) flush_counts(c, cnt);
-}
-
 // ---- launchers -------------------------------------------------------------------------------
 static unsigned grid_cap(uint64_t n, int threads, int sm_count, int per_sm) {
   const uint64_t want = (n + threads - 1) / threads;
   const uint64_t cap = uint64_t(sm_count) * per_sm;
   return unsigned(want < cap ? (want ? want : 1) : cap);
-}
-
-cudaError_t launch_scene_closest(const SceneView& s, const float* rays, uint64_t stride, uint64_t n, uint32_t* prim,
-                                 float* t, uint32_t* obj, unsigned long long* cnt, uint32_t* err, int sm_count,
-                                 cudaStream_t st) {
-  if (n == 0) return cudaSuccess;
-  const unsigned g = grid_cap(n, 128, sm_count, 32);
-  if (cnt) k_scene_closest<true, true><<<g, 128, 0, st>>>(s, rays, stride, n, prim, t, obj, cnt, err);
-  else if (s.has_csg) k_scene_closest<false, true><<<g, 128, 0, st>>>(s, rays, stride, n, prim, t, obj, nullptr, err);
-  else k_scene_closest<false, false><<<g, 128, 0, st>>>(s, rays, stride, n, prim, t, obj, nullptr, err);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_scene_any(const SceneView& s, const float* rays, uint64_t stride, uint64_t n, uint8_t* occ,
-                             unsigned long long* cnt, uint32_t* err, int sm_count, cudaStream_t st) {
-  if (n == 0) return cudaSuccess;
-  const unsigned g = grid_cap(n, 128, sm_count, 32);
-  if (cnt) k_scene_any<true, true><<<g, 128, 0, st>>>(s, rays, stride, n, occ, cnt, err);
-  else if (s.has_csg) k_scene_any<false, true><<<g, 128, 0, st>>>(s, rays, stride, n, occ, nullptr, err);
-  else k_scene_any<false, false><<<g, 128, 0, st>>>(s, rays, stride, n, occ, nullptr, err);
-  return cudaGetLastError();
-}
-
-// The persistent walk (k_extend_walk) for scenes whose top-level tree has at least this many
-// nodes; one thread per path (k_extend) below it.
-constexpr uint32_t kWalkMinTopNodes = 64;
-
-// The walk's step schedule: a leaf step once `leaf_min` lanes of a warp stand on a leaf, a
-// refill once `refill_min` lanes are idle. PBRT_WALK_SCHEDULE="leaf_min,refill_min" (each in
-// 1..32) overrides the default for measurements; films do not depend on it.
-struct WalkSchedule {
-  int leaf_min = 8, refill_min = 8;
-};
-
-static WalkSchedule walk_schedule() {
-  static const WalkSchedule v = [] {
-    WalkSchedule d;
-    if (const char* e = std::getenv("PBRT_WALK_SCHEDULE")) {
-      int a = 0, b = 0;
-      if (std::sscanf(e, "%d,%d", &a, &b) == 2 && a >= 1 && a <= 32 && b >= 1 && b <= 32) {
-        d.leaf_min = a;
-        d.refill_min = b;
-      }
-    }
-    return d;
-  }();
-  return v;
 }
 
 // Queue pushes of the shading kernel per block through shared memory (k_shade<.., true>)
@@ -1488,62 +862,30 @@ static bool shade_staging() {
   return v;
 }
 
-// extend -> shade -> shadow, `loops` times, over the ping-pong queues. `top_nodes`: the largest
-// top-level tree among the scenes rendered; `csg`: some scene holds a constructive solid (the
-// traversal kernels are also built without the solids' code, which takes registers and spills
-// from every other query).
-// Scenes' deferred leaves are answered by their own passes (k_defer_closest, k_defer_any)
-// unless PBRT_DEFER=0 (for measurements; the films differ at most where two objects are hit
-// at exactly the same distance).
-static bool defer_enabled() {
-  static const bool v = [] {
-    const char* e = std::getenv("PBRT_DEFER");
-    return !(e && e[0] == '0');
-  }();
-  return v;
-}
-
+// nearest -> shade -> shadow, `loops` times, over the ping-pong queues. objects, csg: some scene
+// rendered has primitives that are not merged meshes, or constructive solids.
 template <class Src>
 static cudaError_t bounce_loop(const WaveBuffers& w, const Src& src, const CacheWave& cw, uint32_t loops, bool shadows,
                                uint32_t cache_mode, uint32_t term_hit, const LaunchShape& sh, unsigned long long* stats,
-                               uint32_t* err, int sm_count, cudaStream_t st, uint32_t top_nodes, bool csg,
-                               bool defer) {
+                               uint32_t* err, int sm_count, cudaStream_t st, bool objects, bool csg, uint32_t nodes, uint32_t paths) {
   cudaError_t e;
-  const unsigned gt = unsigned(sm_count) * sh.trace_blocks_per_sm, gs = unsigned(sm_count) * sh.shade_blocks_per_sm;
-  // the deferred passes: persistent, PBRT_DEFER_MIN_BLOCKS blocks of 128 per SM
-  const unsigned gd = unsigned(sm_count) * unsigned(PBRT_DEFER_MIN_BLOCKS);
-  const uint32_t df = defer ? 1u : 0u;
+  const unsigned gs = unsigned(sm_count) * sh.shade_blocks_per_sm;
+  const WalkLaunch wl{objects, csg, nodes, paths, sh, stats, err, sm_count, st};
   for (uint32_t b = 0; b < loops; ++b) {
     uint32_t* qin = (b & 1) ? w.qb : w.qa;
     uint32_t* qout = (b & 1) ? w.qa : w.qb;
     uint32_t* cin = w.counts + (b & 1);
     uint32_t* cout = w.counts + ((b + 1) & 1);
-    if ((e = cudaMemsetAsync(cout, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-    // counts[2]: shadow rays queued by k_shade; counts[3]: k_extend_walk's fetch position;
-    // counts[4], [5]: the deferred passes' fetch positions
-    if ((e = cudaMemsetAsync(w.counts + 2, 0, 4 * sizeof(uint32_t), st)) != cudaSuccess) return e;
-    const WalkSchedule ws = walk_schedule();
-    if (top_nodes >= kWalkMinTopNodes && csg)
-      k_extend_walk<Src, true><<<gt, sh.trace_threads, 0, st>>>(w, src, qin, cin, w.counts + 3, err, stats,
-                                                                ws.leaf_min, ws.refill_min, df);
-    else if (top_nodes >= kWalkMinTopNodes)
-      k_extend_walk<Src, false><<<gt, sh.trace_threads, 0, st>>>(w, src, qin, cin, w.counts + 3, err, stats,
-                                                                 ws.leaf_min, ws.refill_min, df);
-    else if (csg)
-      k_extend<Src, true><<<gt, sh.trace_threads, 0, st>>>(w, src, qin, cin, err, stats, df);
-    else
-      k_extend<Src, false><<<gt, sh.trace_threads, 0, st>>>(w, src, qin, cin, err, stats, df);
-    if (defer) k_defer_closest<Src><<<gd, 128, 0, st>>>(w, src, qin, cin, w.counts + 4, err);
+    // counts[2]: shadow rays queued by k_shade; counts[3], [4]: the walks' fetch positions. Each
+    // kernel zeroes what the next ones count in (a memset a bounce is another launch): the
+    // nearest walk the shading's and shadow walk's words, generation and shading the walk's.
+    if ((e = launch_nearest(w, src, qin, cin, w.counts + 3, cout, wl)) != cudaSuccess) return e;
     if (shade_staging())
       k_shade<Src, true><<<gs, sh.shade_threads, 0, st>>>(w, src, qin, cin, qout, cout, cw, cache_mode, term_hit);
     else
       k_shade<Src, false><<<gs, sh.shade_threads, 0, st>>>(w, src, qin, cin, qout, cout, cw, cache_mode, term_hit);
-    // (a persistent walk for the shadow rays measured 2.6% slower on 10,000 spheres: any-hit
-    // rays end early, so one thread per ray wastes little)
-    if (shadows && csg) k_shadow<Src, true><<<gt, sh.trace_threads, 0, st>>>(w, src, err, stats, df);
-    else if (shadows) k_shadow<Src, false><<<gt, sh.trace_threads, 0, st>>>(w, src, err, stats, df);
-    if (shadows && defer) k_defer_any<Src><<<gd, 128, 0, st>>>(w, src, w.counts + 5, err);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (shadows && (e = launch_shadow(w, src, w.counts + 4, wl)) != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
@@ -1623,10 +965,11 @@ cudaError_t render_batch(const BatchScene* table, const BatchScene* host_table, 
       if ((e = cudaStreamWaitEvent(bst[k], fork, 0)) != cudaSuccess) return e;
   }
   const ManyScenes src{table};
-  uint32_t top_nodes = 0;
-  bool csg = false;
+  bool objects = false, csg = false;
+  uint32_t nodes = 0;
   for (uint32_t i = 0; i < nscenes; ++i) {
-    top_nodes = top_nodes > host_table[i].view.top_node_count ? top_nodes : host_table[i].view.top_node_count;
+    nodes = nodes > host_table[i].view.wide.count ? nodes : host_table[i].view.wide.count;
+    objects = objects || host_table[i].view.has_objects;
     csg = csg || host_table[i].view.has_csg;
   }
   uint32_t first = 0;
@@ -1647,12 +990,10 @@ cudaError_t render_batch(const BatchScene* table, const BatchScene* host_table, 
       const BatchScene& h = host_table[first];
       const OneScene one{h.view, PathSettings{h.max_depth, h.rr_start, h.integrator, h.cam.near, h.cam.far}};
       e = bounce_loop(w, one, CacheWave{}, h.max_depth, !h.integrator, kCacheOff, 0, shape, stats, err, sm_count, s,
-                      h.view.top_node_count, h.view.has_csg != 0, defer_enabled() && h.view.defer_leaf != kNoLeaf);
+                      h.view.has_objects != 0, h.view.has_csg != 0, h.view.wide.count, n);
     } else {
-      bool defer = false;
-      for (uint32_t i = first; i <= last; ++i) defer = defer || host_table[i].view.defer_leaf != kNoLeaf;
       e = bounce_loop(w, src, CacheWave{}, max_depth, any_path_integrator, kCacheOff, 0, shape, stats, err, sm_count,
-                      s, top_nodes, csg, defer_enabled() && defer);
+                      s, objects, csg, nodes, n);
     }
     if (e != cudaSuccess) return e;
     k_accumulate_batch<<<grid_cap(n, 256, sm_count, 16), 256, 0, s>>>(w, n, table);
@@ -1756,8 +1097,7 @@ cudaError_t trace_wave(const SceneView& s, const WaveBuffers& w, const CacheWave
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const OneScene src{s, PathSettings{rs.max_depth, rs.rr_start, rs.integrator, cam.near, cam.far}};
   return bounce_loop(w, src, cw, rs.loop_depth ? rs.loop_depth : rs.max_depth, !rs.integrator, rs.cache_mode, rs.term_hit,
-                     rs.shape, rs.stats, err, sm_count, st, s.top_node_count, s.has_csg != 0,
-                     defer_enabled() && s.defer_leaf != kNoLeaf);
+                     rs.shape, rs.stats, err, sm_count, st, s.has_objects != 0, s.has_csg != 0, s.wide.count, n);
 }
 
 cudaError_t accumulate_wave(const WaveBuffers& w, uint32_t n, double* film, uint32_t image_w, const RenderSettings& rs,

@@ -290,10 +290,11 @@ __global__ void __launch_bounds__(kCullThreads) k_cull_root_bulk(MeshView m, con
 // the drained queue in their second byte. Each lane tests its triangles in the reference's
 // order, so ids and t are unchanged.
 // kRec: the survivors' rays come from the records stage 1 wrote beside the queue. kAny: the
-// first triangle hit ends a ray, `prim` holds the occlusion bytes.
+// first triangle hit ends a ray, `prim` holds the occlusion bytes. Rays outside the grid's
+// arithmetic, and those whose answer could depend on the order (judge), walk m's binary nodes.
 template <bool kRec, bool kAny>
 __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
-    MeshView m, const float* __restrict__ rays, uint64_t stride, const uint32_t* __restrict__ queue,
+    MeshView m, WideView w, const float* __restrict__ rays, uint64_t stride, const uint32_t* __restrict__ queue,
     const unsigned long long* __restrict__ queue_count, uint32_t* __restrict__ prim, float* __restrict__ tout,
     uint32_t* __restrict__ obj, unsigned long long* __restrict__ next_ray, uint32_t* __restrict__ err,
     const float4* __restrict__ rec, int leaf_min, int refill_min, int burst) {
@@ -303,12 +304,12 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
   bool active = false, exhausted = false;  // exhausted is warp-uniform
   uint32_t idx = 0;
   WRay r;
-  float near = 0.f, lim = 0.f, lim0 = 0.f;
+  float near = 0.f, lim0 = 0.f;
+  Nearest nearest{0.f, 0.f, false};
   uint32_t best = 0xFFFFFFFFu, cur = 0, budget = 0;
   int sp = 0;
   WideStack stk;
-  const bool bounded = tree_bounded(m.nodes);
-  const uint32_t root = root_ref(m.nodes, m.leaf_direct);
+  const uint32_t exact_root = binary_ref(__ldg(&m.nodes[0]), __ldg(&m.nodes[1]), 0u);
 
   for (;;) {
     // Refill the idle lanes: one atomicAdd per warp.
@@ -337,11 +338,13 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
             near = __ldg(rays + 6 * stride + idx);
             far = __ldg(rays + 7 * stride + idx);
           }
-          r = wide_ray(o, d, near, bounded);
+          r = wide_ray(o, d, near, w.bounded);
           // a hit lies below lim: t <= far, and t < min_t (which starts at FLT_MAX, bvh.rs:459)
-          lim0 = lim = kAny ? next_up(far) : fminf(FLT_MAX, next_up(far));
+          lim0 = kAny ? next_up(far) : fminf(FLT_MAX, next_up(far));
+          nearest = nothing_yet(far);
+          nearest.lim = lim0;
           best = 0xFFFFFFFFu;
-          cur = root;  // the root entered the ray's interval in stage 1 (bvh.rs:458-461)
+          cur = r.exact ? exact_root : w.root;  // the root entered the ray's interval in stage 1 (bvh.rs:458-461)
           sp = 0;
           budget = m.node_count;
           active = true;
@@ -359,35 +362,61 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
     const bool leaf_step = __popc(on_leaf) >= lmin || on_leaf == act;
     if (active && at_leaf == leaf_step) {
       if (leaf_step) {
-        if (kAny) {
-          if (any_in_leaf(m, cur, r, near, lim, r.exact)) {
-            best = 0u;
-            cur = 0u;
-          } else {
-            cur = wide_pop(stk, sp, lim);
+        bool done = false, restart = false;
+        if (r.exact) {
+          const uint32_t node = cur & ~kLeafRef;
+          const uint32_t first = __float_as_uint(__ldg(&m.nodes[2 * size_t(node)]).w);
+          const uint32_t count = __float_as_uint(__ldg(&m.nodes[2 * size_t(node) + 1]).w);
+          float t;
+          uint32_t id;
+          if (kAny) {
+            done = blocking_triangle(m.tri, m.tri_c, first, count, r.o, r.d, near, nearest.lim);
+          } else if (nearest_triangle(m.tri, m.tri_c, first, count, r.o, r.d, near, nearest.lim, t, id) &&
+                     t < nearest.lim) {
+            nearest.lim = t;
+            best = id;
           }
-        } else if (closest_in_leaf(m, cur, r, near, lim, best, r.exact)) {
-          cur = wide_pop(stk, sp, r.exact ? lim : wide_limit(lim));
-        } else {  // again, on the binary nodes
+        } else {
+          uint32_t first, count;
+          triangle_range(w, cur, first, count);
+          float t, e;
+          uint32_t id;
+          if (kAny) {
+            done = blocking_triangle(w.tri, w.tri_c, first, count, r.o, r.d, near, nearest.lim) &&
+                   leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e) && e < nearest.lim;
+          } else if (nearest_triangle(w.tri, w.tri_c, first, count, r.o, r.d, near, wide_limit(nearest.lim), t, id) &&
+                     leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e)) {
+            const Verdict v = judge(nearest, t, e);
+            if (v == kAdopt) best = id;
+            restart = v == kRestart;
+          }
+        }
+        if (kAny && done) {
+          best = 0u;
+          cur = 0u;
+        } else if (!kAny && restart) {  // again, on the binary nodes
           r.exact = true;
-          lim = lim0;
+          nearest.lim = lim0;
           best = 0xFFFFFFFFu;
-          cur = root;
+          cur = exact_root;
           sp = 0;
           budget = m.node_count;
+        } else {
+          cur = wide_pop(stk, sp, kAny || r.exact ? nearest.lim : wide_limit(nearest.lim));
         }
       } else {
         // up to `burst` nodes before the next vote (fewer when a leaf is reached)
         const int nb = exhausted ? (burst >> 8) : (burst & 255);
-        const float reach = kAny ? lim : wide_limit(lim);
+        const float reach = kAny ? nearest.lim : wide_limit(nearest.lim);
         for (int b = 0; b < nb && cur != 0u && !(cur & kLeafRef); ++b) {
           if (budget-- == 0) {
             atomicOr(err, kErrBudget);
             cur = 0u;
             break;
           }
-          cur = r.exact ? binary_step(m.nodes, cur, m.leaf_direct, r, near, lim, stk, sp, err)
-                        : wide_step(m.wide + cur, r, near, reach, stk, sp, err);
+          cur = r.exact ? binary_step(m.nodes, cur, r, near, nearest.lim, stk, sp)
+                : kAny  ? wide_step_any(w.wide + cur, r, near, nearest.lim, stk, sp)
+                        : wide_step(w.wide + cur, r, near, reach, stk, sp);
         }
       }
       if (cur == 0u) {
@@ -396,7 +425,7 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
             reinterpret_cast<uint8_t*>(prim)[idx] = 1;
           } else {
             __stcs(prim + idx, best);
-            __stcs(tout + idx, lim);
+            __stcs(tout + idx, nearest.lim);
             if (obj) __stcs(obj + idx, 0u);
           }
         }
@@ -407,66 +436,73 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
 }
 
 // The wide nodes of a tree: one thread per interior node of the binary tree, which writes the
-// wide node of its children's pair (index left_first / 2). Half of them are reached (every
-// second level); the others cost memory, not time. A leaf's thread notes the leaf's node
-// beside its first triangle.
-__global__ void k_widen(const float4* __restrict__ nodes, uint32_t count, bool direct, WideNode* __restrict__ out,
-                        uint32_t* __restrict__ leaf_node) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+// wide node of its children's pair (index base + left_first / 2). Half of them are reached (every
+// second level); the others cost memory, not time. A mesh's leaves become triangle references
+// and note their node and object beside their first triangle; a top-level tree's leaves become
+// their primitive's reference (`slot_ref`: the root of a merged mesh, or an object leaf) and note
+// their node beside the slot.
+__global__ void k_widen(WidenArgs a) {
+  auto ref_of = [&](uint32_t q) -> uint32_t {
+    const uint32_t first = __float_as_uint(__ldg(&a.nodes[2 * size_t(q)]).w);
+    const uint32_t count = __float_as_uint(__ldg(&a.nodes[2 * size_t(q) + 1]).w);
+    if (count == 0u) return a.wide_base + (first >> 1);
+    return a.slot_ref ? __ldg(&a.slot_ref[first]) : triangle_ref(a.tri_base + first, count, a.direct);
+  };
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.count; i += gridDim.x * blockDim.x) {
     if (i == 1u) continue;  // the padding slot
-    const float4 nlo = __ldg(&nodes[2 * size_t(i)]), nhi = __ldg(&nodes[2 * size_t(i) + 1]);
+    const float4 nlo = __ldg(&a.nodes[2 * size_t(i)]), nhi = __ldg(&a.nodes[2 * size_t(i) + 1]);
     const uint32_t pair = __float_as_uint(nlo.w);
     if (__float_as_uint(nhi.w) != 0u) {
-      leaf_node[pair] = i;
+      if (a.slot_ref) a.slot_node[pair] = i;
+      else a.leaf[a.tri_base + pair] = make_uint2(a.node_base + i, a.owner);
       continue;
     }
-    if (pair < 2u || pair + 1u >= count) continue;
+    if (pair < 2u || pair + 1u >= a.count) continue;
     uint32_t slot[4], ref[4];  // the slots' nodes; a leaf child stands in slot 0 (2), slot 1 (3) is empty
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
       const uint32_t c = pair + side;
-      const float4 lo = __ldg(&nodes[2 * size_t(c)]), hi = __ldg(&nodes[2 * size_t(c) + 1]);
-      const uint32_t cl = __float_as_uint(lo.w);
-      const bool leaf = __float_as_uint(hi.w) != 0u || cl + 1u >= count;
+      const uint32_t cl = __float_as_uint(__ldg(&a.nodes[2 * size_t(c)]).w);
+      const bool leaf = __float_as_uint(__ldg(&a.nodes[2 * size_t(c) + 1]).w) != 0u || cl + 1u >= a.count;
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
         const int k = 2 * side + g;
-        const uint32_t q = leaf ? c : cl + g;
-        slot[k] = q;
-        ref[k] = leaf && g == 1 ? 0u : node_ref(__ldg(&nodes[2 * size_t(q)]), __ldg(&nodes[2 * size_t(q) + 1]), q, direct);
+        slot[k] = leaf ? c : cl + g;
+        ref[k] = leaf && g == 1 ? 0u : ref_of(slot[k]);
       }
     }
     WideNode w;
     uint32_t pl[3] = {0u, 0u, 0u}, ph[3] = {0u, 0u, 0u};
     const float blo[3] = {nlo.x, nlo.y, nlo.z}, bhi[3] = {nhi.x, nhi.y, nhi.z};
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      // the least power of two whose 255 steps span the node (at least 2^-70)
-      const double extent = double(bhi[a]) - double(blo[a]);
-      int e = extent > 0.0 ? ilogb(extent / 255.0) : -70;
-      if (ldexp(255.0, e) < extent) ++e;
-      if (e < -70) e = -70;
-      if (e > 100) e = 100;  // beyond kWideLimit: never walked
-      const double s = ldexp(1.0, e);
-      w.org[a] = blo[a];
-      w.step[a] = float(ldexp(1.0, e - 8));
+    for (int x = 0; x < 3; ++x) {
+      // 255 steps span the node (a step of at least 2^-70; beyond kWideLimit: never walked), so
+      // that a plane on the node's own faces stands on the grid: the flat boxes of a room's walls
+      // stay flat
+      const double extent = double(bhi[x]) - double(blo[x]);
+      float step = float(fmin(fmax(extent / 255.0, 0x1p-70), 0x1p100));
+      if (double(step) * 255.0 < extent) step = nextafterf(step, FLT_MAX);
+      const double s = double(step);
+      w.org[x] = blo[x];
+      w.step[x] = step * 0x1p-8f;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const float4 lo = __ldg(&nodes[2 * size_t(slot[k])]), hi = __ldg(&nodes[2 * size_t(slot[k]) + 1]);
-        const float l = a == 0 ? lo.x : (a == 1 ? lo.y : lo.z), h = a == 0 ? hi.x : (a == 1 ? hi.y : hi.z);
-        // (a rounding of the FP64 difference moves a plane by 2^-53 of the extent at most, far
-        // inside the walk's margin of a 256th of a step)
-        const double fl = floor((double(l) - double(blo[a])) / s), fh = ceil((double(h) - double(blo[a])) / s);
+        const float4 lo = __ldg(&a.nodes[2 * size_t(slot[k])]), hi = __ldg(&a.nodes[2 * size_t(slot[k]) + 1]);
+        const float l = x == 0 ? lo.x : (x == 1 ? lo.y : lo.z), h = x == 0 ? hi.x : (x == 1 ? hi.y : hi.z);
+        // (within a thousandth of a step a plane snaps to the grid, inwards too: the walk's margin
+        // of a 256th of a step covers it)
+        const double fl = floor((double(l) - double(blo[x])) / s + 1e-3);
+        const double fh = ceil((double(h) - double(blo[x])) / s - 1e-3);
         const uint32_t ql = uint32_t(fmin(fmax(fl, 0.0), 255.0)), qh = uint32_t(fmin(fmax(fh, 0.0), 255.0));
-        pl[a] |= ql << (8 * k);
-        ph[a] |= qh << (8 * k);
+        pl[x] |= ql << (8 * k);
+        ph[x] |= qh << (8 * k);
       }
     }
     w.lo_x = pl[0]; w.lo_y = pl[1]; w.lo_z = pl[2];
     w.hi_x = ph[0]; w.hi_y = ph[1]; w.hi_z = ph[2];
 #pragma unroll
     for (int k = 0; k < 4; ++k) w.ref[k] = ref[k];
-    out[pair >> 1] = w;
+    a.wide[a.wide_base + (pair >> 1)] = w;
   }
 }
 
@@ -507,12 +543,9 @@ static unsigned grid_for(uint64_t n, int threads, int sm_count) {
   return unsigned(want < cap ? (want ? want : 1) : cap);
 }
 
-size_t wide_bytes(uint64_t node_slots) { return size_t(node_slots / 2 + 1) * sizeof(WideNode); }
-
-cudaError_t launch_widen(const void* nodes, uint32_t node_slots, bool direct, void* wide, uint32_t* leaf_node,
-                         int sm_count, cudaStream_t s) {
-  k_widen<<<grid_for(node_slots, 128, sm_count), 128, 0, s>>>(static_cast<const float4*>(nodes), node_slots, direct,
-                                                              static_cast<WideNode*>(wide), leaf_node);
+cudaError_t launch_widen(const WidenArgs& a, int sm_count, cudaStream_t s) {
+  if (a.count == 0) return cudaSuccess;
+  k_widen<<<grid_for(a.count, 128, sm_count), 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -544,7 +577,7 @@ static int walk_blocks_per_sm() {
 
 // The two stages over n rays; kAny: `prim` is the occlusion buffer, t and obj are NULL.
 template <bool kRec, bool kAny>
-static cudaError_t two_stage(const MeshView& m, const float* rays, uint64_t stride, uint64_t n, uint32_t* prim, float* t,
+static cudaError_t two_stage(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n, uint32_t* prim, float* t,
                              uint32_t* obj, uint32_t* queue, unsigned long long* counters, uint32_t* err, int sm_count,
                              cudaStream_t s, float4* rec) {
   const bool vec = stride % 4 == 0 && aligned(rays, 16) &&
@@ -574,28 +607,28 @@ static cudaError_t two_stage(const MeshView& m, const float* rays, uint64_t stri
   const uint64_t need = (n + 127) / 128;
   const TraversalSchedule ts = traversal_schedule();
   k_mesh_walk<kRec, kAny><<<unsigned(need < full ? need : full), 128, 0, s>>>(
-      m, rays, stride, queue, counters, prim, t, obj, counters + 1, err, rec, ts.leaf_arg(), ts.refill_min,
+      m, w, rays, stride, queue, counters, prim, t, obj, counters + 1, err, rec, ts.leaf_arg(), ts.refill_min,
       ts.burst_arg());
   return cudaGetLastError();
 }
 
-cudaError_t launch_mesh_closest_persistent(const MeshView& m, const float* rays, uint64_t stride, uint64_t n,
+cudaError_t launch_mesh_closest_persistent(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
                                            uint32_t* prim, float* t, uint32_t* obj, uint32_t* queue,
                                            unsigned long long* counters, uint32_t* err, int sm_count, cudaStream_t s,
                                            float4* rec) {
   if (n == 0) return cudaSuccess;
   const cudaError_t e = cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
-  return two_stage<true, false>(m, rays, stride, n, prim, t, obj, queue, counters, err, sm_count, s, rec);
+  return two_stage<true, false>(m, w, rays, stride, n, prim, t, obj, queue, counters, err, sm_count, s, rec);
 }
 
-cudaError_t launch_mesh_any_persistent(const MeshView& m, const float* rays, uint64_t stride, uint64_t n, uint8_t* occ,
+cudaError_t launch_mesh_any_persistent(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n, uint8_t* occ,
                                        uint32_t* queue, unsigned long long* counters, uint32_t* err, int sm_count,
                                        cudaStream_t s, float4* rec) {
   if (n == 0) return cudaSuccess;
   const cudaError_t e = cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
-  return two_stage<true, true>(m, rays, stride, n, reinterpret_cast<uint32_t*>(occ), nullptr, nullptr, queue, counters,
+  return two_stage<true, true>(m, w, rays, stride, n, reinterpret_cast<uint32_t*>(occ), nullptr, nullptr, queue, counters,
                                err, sm_count, s, rec);
 }
 
@@ -621,7 +654,7 @@ cudaError_t noalloc_scratch_lookup(uint32_t** out) {
   return cudaSuccess;
 }
 
-cudaError_t launch_mesh_closest_noalloc(const MeshView& m, const float* rays, uint64_t n, uint32_t* prim, float* t,
+cudaError_t launch_mesh_closest_noalloc(const MeshView& m, const WideView& w, const float* rays, uint64_t n, uint32_t* prim, float* t,
                                         uint32_t* scratch, int sm_count, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   if (n > kNoAllocMaxRays || !scratch) return cudaErrorInvalidValue;
@@ -632,7 +665,7 @@ cudaError_t launch_mesh_closest_noalloc(const MeshView& m, const float* rays, ui
   unsigned long long* counters = reinterpret_cast<unsigned long long*>(scratch);
   uint32_t* err = scratch + 4;
   uint32_t* queue = scratch + 64;
-  return two_stage<false, false>(m, rays, n, n, prim, t, nullptr, queue, counters, err, sm_count, s, nullptr);
+  return two_stage<false, false>(m, w, rays, n, n, prim, t, nullptr, queue, counters, err, sm_count, s, nullptr);
 }
 
 cudaError_t launch_mesh_any(const MeshView& m, const float* rays, uint64_t stride, uint64_t n, uint8_t* occ,

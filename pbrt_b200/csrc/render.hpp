@@ -25,7 +25,8 @@ struct WaveBuffers {
   uint32_t *qa, *qb;                   // ping-pong queues of path indices
   uint32_t* s_path;                    // shadow queue
   float *s_ox, *s_oy, *s_oz, *s_dx, *s_dy, *s_dz, *s_tmax, *s_cr, *s_cg, *s_cb;
-  uint32_t* counts;                    // [0] qa length, [1] qb length, [2] shadow queue length
+  uint32_t* counts;                    // [0] qa length, [1] qb length, [2] shadow queue length, [3], [4] the
+                                       // nearest and shadow walks' fetch positions
 };
 
 // The radiance cache's side of a wave. Query mode: a path that reaches hit `term_hit` on a

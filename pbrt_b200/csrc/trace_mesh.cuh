@@ -39,16 +39,11 @@ PBRT_DEV void load_node(const float4* p, float4& lo, float4& hi) {
       : "l"(p));
 }
 
-struct WideNode;  // wide_bvh.cuh
-
 struct MeshView {
-  const float4* nodes;   // 2 float4 per node
-  const WideNode* wide;  // the same tree two levels at a time
-  const float4* tri;     // 2 float4 per triangle
+  const float4* nodes;  // 2 float4 per node
+  const float4* tri;    // 2 float4 per triangle
   const float2* tri_c;
-  const uint32_t* leaf_node;  // at a leaf's first triangle: the leaf's node
   uint32_t node_count;  // GPU numbering, including the padding slot
-  bool leaf_direct;     // leaf references hold first and count (leaf_ref in wide_bvh.cuh)
 };
 
 // A ray prepared for box tests: the reciprocals depend on the ray alone (the reference

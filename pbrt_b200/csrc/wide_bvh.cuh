@@ -1,4 +1,4 @@
-// wide_bvh.cuh — a mesh's binary BVH two levels at a time, with the binary traversal's answers.
+// wide_bvh.cuh — binary BVHs two levels at a time, with the binary traversal's answers.
 //
 // What bounds an incoherent walk here is the L1 data path: every lane reads another node, so a
 // load costs one wavefront per lane whatever its width up to 32 bytes. A wide node holds the
@@ -8,20 +8,25 @@
 // them is conservative, never missing a box that box_hit takes (the margin m below), so a walk
 // reaches every leaf the binary one reaches, and perhaps a few more.
 //
-// Why the answers are the binary traversal's (trace_mesh.cuh). There a leaf is visited when
-// its own box is hit over [near, far] and its entry distance is below the nearest hit at its
-// turn; the boxes above add nothing, being exact unions under a monotone slab test.
-//   - Any hit: a triangle hit counts only if its leaf's exact box is hit. No order matters.
-//   - Nearest hit: as long as every hit lies at or beyond its leaf's exact entry distance, the
-//     binary answer is the nearest of all hits in exactly-hit leaves, and among equal distances
-//     the first in traversal order, whatever the order of the visits. A triangle that lowers the
-//     nearest distance is therefore checked against its leaf's exact box; a leaf that is not hit
-//     is ignored as the binary walk would; a hit before its leaf's entry, or one that equals the
-//     nearest distance of another leaf, makes the lane start its ray again on the binary nodes,
-//     in the binary order. Nodes are dropped only beyond the nearest distance plus 2^-13 of it,
-//     so that a leaf whose hit comes before its entry by a rounding is seen, not skipped.
+// A scene has one wide tree: the top-level BVH's wide nodes, and below its leaves the wide
+// nodes of every mesh that is placed once and untransformed, so that a walk goes from the
+// scene into its meshes without any per-object work. Other primitives are object leaves.
+//
+// Why the answers are the binary traversal's (trace_mesh.cuh, scene_device.cuh). There a leaf is
+// visited when its own box is hit over [near, far] and its entry distance is below the nearest
+// hit at its turn; the boxes above add nothing, being supersets under a monotone slab test.
+//   - Any hit: a hit counts only if its leaf's exact box is hit. No order matters.
+//   - Nearest hit: a candidate is a leaf's nearest hit t with the leaf's exact entry distance e
+//     (a leaf whose exact box is missed gives none). While t >= e for every candidate, the binary
+//     answer is the candidate with the least t, the first in traversal order among equal ones,
+//     whatever the order of the visits. Rounding can make t < e; the order of the visits then
+//     decides, but only between candidates in [t, e]. So the walk keeps the nearest candidate
+//     and, when its t < e, the window up to e; a second candidate at the same distance or in
+//     that window, or a t below e by more than 2^-13 of it, makes the ray start again on the
+//     binary nodes, in the binary order. Nodes are dropped only beyond the nearest distance plus
+//     2^-13 of it, so that a candidate with t < e is seen, not skipped.
 // Rays the grid's arithmetic does not cover (a direction component of zero or outside
-// [2^-40, 2^40], near < 0 or NaN, coordinates beyond 2^40) walk the binary nodes from the start.
+// [2^-40, 2^40], near < 0 or NaN, coordinates beyond 2^40) use the binary nodes from the start.
 #pragma once
 
 #include <cfloat>
@@ -31,54 +36,47 @@
 namespace pbrt {
 
 constexpr uint32_t kLeafRef = 0x80000000u;
-constexpr int kWideStack = 96;  // three pending slots per two levels of a tree of depth < 64
+constexpr int kWideStack = 128;  // three pending slots per two levels (upload_scene checks the depths)
 constexpr float kWideLimit = 1.099511627776e12f;  // 2^40
 
 struct __align__(64) WideNode {
   float org[3];      // the node's own lower corner
-  float step[3];     // the grid's step / 256 (a power of two) per axis
+  float step[3];     // the grid's step / 256 per axis
   uint32_t lo_x, hi_x, lo_y, hi_y, lo_z, hi_z;  // the slots' planes, a byte each
   uint32_t ref[4];   // 0: empty; kLeafRef | leaf (leaf_ref); else a wide node
 };
 static_assert(sizeof(WideNode) == 64, "a wide node is two 32-byte loads");
 
-// References name a sibling pair of the binary tree by half its first index: the wide node of
-// that pair's parent, and the pair itself for a binary step. A leaf's holds the first triangle
-// and count packed (27 + 4 bits), or, when they do not fit, the index of the leaf's binary node
-// with the count field 15 (`direct`; meshes of more than 2^27 triangles always name the node).
-PBRT_DEV uint32_t leaf_ref(uint32_t first, uint32_t count, uint32_t node, bool direct) {
-  if (!direct) return kLeafRef | node;
-  if (count <= 15u && first < (1u << 27)) return kLeafRef | ((count - 1u) << 27) | first;
-  return kLeafRef | (15u << 27) | node;
+// A reference: 0, a wide node's index, or a leaf. A triangle leaf holds its first triangle and
+// its count in 26 + 4 bits; a count that does not fit (code 15), and every count in scenes of
+// more than 2^26 triangles (then the first triangle takes 30 bits), is read from the leaf's node.
+// An object leaf holds its slot in the scene's primitive order.
+constexpr uint32_t kObjectRef = 0x40000000u;
+
+__host__ PBRT_DEV uint32_t triangle_ref(uint32_t first, uint32_t count, bool direct) {
+  if (!direct) return kLeafRef | first;
+  return kLeafRef | ((count <= 15u ? count - 1u : 15u) << 26) | first;
 }
 
-PBRT_DEV void leaf_range(const float4* nodes, uint32_t ref, bool direct, uint32_t& first, uint32_t& count) {
-  const uint32_t code = (ref >> 27) & 15u;
-  if (direct && code != 15u) {
-    first = ref & 0x7FFFFFFu;
-    count = code + 1u;
-    return;
-  }
-  const uint32_t node = direct ? ref & 0x7FFFFFFu : ref & 0x7FFFFFFFu;
-  first = __float_as_uint(__ldg(&nodes[2 * size_t(node)]).w);
-  count = __float_as_uint(__ldg(&nodes[2 * size_t(node) + 1]).w);
-}
+// A scene's wide tree and what its triangle leaves name, all meshes' arrays end to end.
+struct WideView {
+  const WideNode* wide;
+  const float4* tri;    // 2 float4 per triangle
+  const float2* tri_c;
+  const uint2* leaf;    // at a leaf's first triangle: the leaf's node in `nodes`, the object's leaf index
+  const float4* nodes;  // the meshes' binary nodes
+  const uint32_t* slot_node;  // per primitive slot: the top-level node that is its leaf
+  uint32_t root;        // 0: nothing bounded
+  uint32_t count;       // wide nodes: no walk visits more
+  bool direct;          // triangle references hold their counts
+  bool bounded;         // every coordinate lies where the grid's arithmetic holds
+};
 
-PBRT_DEV uint32_t node_ref(const float4& lo, const float4& hi, uint32_t node, bool direct) {
-  const uint32_t lf = __float_as_uint(lo.w), count = __float_as_uint(hi.w);
-  return count ? leaf_ref(lf, count, node, direct) : lf >> 1;
-}
-
-PBRT_DEV uint32_t root_ref(const float4* nodes, bool direct) {
-  return node_ref(__ldg(&nodes[0]), __ldg(&nodes[1]), 0, direct);
-}
-
-// Whether every coordinate of a tree lies where the grid's arithmetic holds.
-PBRT_DEV bool tree_bounded(const float4* nodes) {
-  const float4 lo = __ldg(&nodes[0]), hi = __ldg(&nodes[1]);
-  const float a = fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(hi.x)), fmaxf(fabsf(lo.y), fabsf(hi.y))),
-                        fmaxf(fabsf(lo.z), fabsf(hi.z)));
-  return a <= kWideLimit;
+PBRT_DEV void triangle_range(const WideView& w, uint32_t ref, uint32_t& first, uint32_t& count) {
+  const uint32_t code = (ref >> 26) & 15u;
+  first = w.direct ? ref & 0x3FFFFFFu : ref & 0x3FFFFFFFu;
+  count = code + 1u;
+  if (!w.direct || code == 15u) count = __float_as_uint(__ldg(&w.nodes[2 * size_t(__ldg(&w.leaf[first]).x) + 1]).w);
 }
 
 // The least float above x; +inf above FLT_MAX, -FLT_MAX above -inf; a NaN gives -inf (nothing
@@ -101,10 +99,10 @@ PBRT_DEV WRay wide_ray(const F3& o, const F3& d, float near, bool bounded) {
   r.o = o;
   r.d = d;
   r.inv = mk3(frcp(d.x), frcp(d.y), frcp(d.z));
-  auto in = [](float x) { return fabsf(x) <= kWideLimit && fabsf(x) >= 1.f / kWideLimit; };
-  auto below = [](float x) { return fabsf(x) <= kWideLimit; };
-  r.exact = !(bounded && near >= 0.f && in(r.inv.x) && in(r.inv.y) && in(r.inv.z) && below(o.x) && below(o.y) &&
-              below(o.z));
+  // (sums of magnitudes: a NaN or an infinity anywhere fails them)
+  const float so = fabsf(o.x) + fabsf(o.y) + fabsf(o.z), si = fabsf(r.inv.x) + fabsf(r.inv.y) + fabsf(r.inv.z);
+  const float least = fminf(fminf(fabsf(r.inv.x), fabsf(r.inv.y)), fabsf(r.inv.z));
+  r.exact = !(bounded && near >= 0.f && so <= kWideLimit && si <= kWideLimit && least >= 1.f / kWideLimit);
   return r;
 }
 
@@ -113,11 +111,9 @@ struct WideStack {
   uint2 s[kWideStack];
 };
 
-PBRT_DEV void wide_push(WideStack& st, int& sp, uint32_t ref, float e, uint32_t* err) {
-  if (sp >= kWideStack) {
-    atomicOr(err, kErrStack);
-    return;
-  }
+// (No check against kWideStack: a walk has at most three slots pending per two levels, and
+// upload_scene lets no ray walk a scene whose trees are too deep for that.)
+PBRT_DEV void wide_push(WideStack& st, int& sp, uint32_t ref, float e) {
   st.s[sp] = make_uint2(ref, __float_as_uint(e));
   ++sp;
 }
@@ -162,9 +158,10 @@ PBRT_DEV float grid(uint32_t w) {
 
 // Distances to the four slots' near (t0) and far (t1) planes on one axis, rounded outwards.
 // The plane is at org + 256 * byte * step, its distance fma(2^23 + 256 * byte, k, c) with
-// k = step * inv (exact), p = (org - o) * inv and c = p -+ m - 2^23 * k. The roundings of p, c
-// and the fma stay below 2^-21.9 |p| + 0.51 |k|, the exact test's own roundings and its widening
-// by 2*gamma(3) below 2^-21 of the distance, which is at most |p| + 2^16 |k|: m covers their sum.
+// k = step * inv, p = (org - o) * inv and c = p -+ m - 2^23 * k. The roundings of k, p, c and the
+// fma stay below 2^-21.9 |p| + 0.52 |k|, the exact test's own roundings and its widening by
+// 2*gamma(3) below 2^-21 of the distance, which is at most |p| + 2^16 |k| (0.03 |k|), and a plane
+// stands at most 0.26 |k| inside its box's (k_widen): m covers their sum.
 PBRT_DEV void planes(float org, float step, uint32_t lo, uint32_t hi, float o, float inv, float (&t0)[4],
                      float (&t1)[4]) {
   const float p = fm(fs(org, o), inv), k = fm(step, inv);
@@ -218,8 +215,7 @@ PBRT_DEV float wide_limit(float lim) { return fa(lim, fm(fabsf(lim), 0x1p-13f));
 // Visits one wide node: its slots hit within [near, reach], each pair nearest first and the
 // pair with the nearest slot first. The first is returned, the others are pushed; the next
 // pending one when none is hit; 0 when none is left.
-PBRT_DEV uint32_t wide_step(const WideNode* nd, const WRay& r, float near, float reach, WideStack& st, int& sp,
-                            uint32_t* err) {
+PBRT_DEV uint32_t wide_step(const WideNode* nd, const WRay& r, float near, float reach, WideStack& st, int& sp) {
   float k[4];
   uint32_t f[4];
   wide::slots(nd, r, near, reach, k, f);
@@ -229,16 +225,101 @@ PBRT_DEV uint32_t wide_step(const WideNode* nd, const WRay& r, float near, float
   wide::order(s, k[0], k[2], f[0], f[2]);
   wide::order(s, k[1], k[3], f[1], f[3]);
   const float inf = __int_as_float(0x7f800000);
-  if (k[3] < inf) wide_push(st, sp, f[3], k[3], err);
-  if (k[2] < inf) wide_push(st, sp, f[2], k[2], err);
-  if (k[1] < inf) wide_push(st, sp, f[1], k[1], err);
+  if (k[3] < inf) wide_push(st, sp, f[3], k[3]);
+  if (k[2] < inf) wide_push(st, sp, f[2], k[2]);
+  if (k[1] < inf) wide_push(st, sp, f[1], k[1]);
   return k[0] < inf ? f[0] : wide_pop(st, sp, reach);
 }
 
-// Visits a sibling pair of the binary tree as the binary traversal does: the children hit with
-// an entry below lim, the right one first only when strictly nearer (bvh.rs:503-506).
-PBRT_DEV uint32_t binary_step(const float4* nodes, uint32_t pair, bool direct, const WRay& r, float near, float lim,
-                              WideStack& st, int& sp, uint32_t* err) {
+// The same for an any-hit walk, whose answer does not depend on the order: the slots hit, in slot
+// order.
+PBRT_DEV uint32_t wide_step_any(const WideNode* nd, const WRay& r, float near, float lim, WideStack& st, int& sp) {
+  float k[4];
+  uint32_t f[4];
+  wide::slots(nd, r, near, lim, k, f);
+  const float inf = __int_as_float(0x7f800000);
+#pragma unroll
+  for (int i = 3; i > 0; --i)
+    if (k[i] < inf) wide_push(st, sp, f[i], k[i]);
+  if (k[0] < inf) return f[0];
+  return sp > 0 ? st.s[--sp].x : 0u;
+}
+
+// The exact test of a leaf's box (its node) for a ray of the wide walk: box_hit where no
+// direction component is zero.
+PBRT_DEV bool leaf_hit(const float4* node, const WRay& r, float near, float& e) {
+  float4 lo, hi;
+  load_node(node, lo, hi);
+  float x = __int_as_float(0x7f800000);
+  e = near;
+  slab_axis_fast(r.o.x, r.inv.x, r.inv.x < 0.f, lo.x, hi.x, e, x);
+  slab_axis_fast(r.o.y, r.inv.y, r.inv.y < 0.f, lo.y, hi.y, e, x);
+  slab_axis_fast(r.o.z, r.inv.z, r.inv.z < 0.f, lo.z, hi.z, e, x);
+  return !(x < e);
+}
+
+// The nearest candidate of a walk.
+struct Nearest {
+  float lim;     // a candidate counts below it: the nearest distance, or just above far
+  float window;  // the nearest candidate's leaf entry when that is beyond it, else -inf
+  bool have;
+};
+
+PBRT_DEV Nearest nothing_yet(float far) { return Nearest{next_up(far), __int_as_float(0xff800000), false}; }
+
+enum Verdict : int { kIgnore = 0, kAdopt = 1, kRestart = 2 };
+
+// A candidate t of a leaf that is exactly hit with entry e.
+PBRT_DEV Verdict judge(Nearest& n, float t, float e) {
+  if (!(t < n.lim)) return n.have && t <= fmaxf(n.lim, n.window) ? kRestart : kIgnore;
+  if (!((n.have ? e : next_up(e)) < n.lim) || e > wide_limit(t)) return kRestart;
+  n.lim = t;
+  n.window = t < e ? e : __int_as_float(0xff800000);
+  n.have = true;
+  return kAdopt;
+}
+
+// The first of a leaf's nearest triangles within [near, reach]; prim: its original index.
+PBRT_DEV bool nearest_triangle(const float4* tri, const float2* tri_c, uint32_t first, uint32_t count, const F3& o,
+                               const F3& d, float near, float reach, float& t_out, uint32_t& prim) {
+  bool any = false;
+  for (uint32_t k = first; k < first + count; ++k) {
+    float4 A, B;
+    load_node(&tri[2 * size_t(k)], A, B);
+    const float2 C = __ldg(&tri_c[k]);
+    float t;
+    if (tri_hit(o, d, A, B, C.x, t) && t >= near && (any ? t < t_out : t <= reach)) {
+      any = true;
+      t_out = t;
+      prim = __float_as_uint(C.y);
+    }
+  }
+  return any;
+}
+
+// Whether some triangle of a leaf is hit within [near, lim).
+PBRT_DEV bool blocking_triangle(const float4* tri, const float2* tri_c, uint32_t first, uint32_t count, const F3& o,
+                                const F3& d, float near, float lim) {
+  for (uint32_t k = first; k < first + count; ++k) {
+    float4 A, B;
+    load_node(&tri[2 * size_t(k)], A, B);
+    const float2 C = __ldg(&tri_c[k]);
+    float t;
+    if (tri_hit(o, d, A, B, C.x, t) && t >= near && t < lim) return true;
+  }
+  return false;
+}
+
+// ---- one mesh's binary nodes, in the binary order --------------------------------------------
+// References of this walk: a sibling pair by half its first index, or kLeafRef | a node.
+PBRT_DEV uint32_t binary_ref(const float4& lo, const float4& hi, uint32_t node) {
+  return __float_as_uint(hi.w) ? kLeafRef | node : __float_as_uint(lo.w) >> 1;
+}
+
+// Visits a sibling pair: the children hit with an entry below lim, the right one first only when
+// strictly nearer (bvh.rs:503-506).
+PBRT_DEV uint32_t binary_step(const float4* nodes, uint32_t pair, const WRay& r, float near, float lim, WideStack& st,
+                              int& sp) {
   const float4* n = nodes + 4 * size_t(pair);
   float4 l0, l1, r0, r1;
   load_node(n, l0, l1);
@@ -249,69 +330,16 @@ PBRT_DEV uint32_t binary_step(const float4* nodes, uint32_t pair, bool direct, c
   const bool hl = box_hit(p, l0, l1, near, inf, dl);
   const bool hr = box_hit(p, r0, r1, near, inf, dr);
   const bool swap = hl && hr && dr < dl;
-  const uint32_t fl = node_ref(l0, l1, 2u * pair, direct), fr = node_ref(r0, r1, 2u * pair + 1u, direct);
+  const uint32_t fl = binary_ref(l0, l1, 2u * pair), fr = binary_ref(r0, r1, 2u * pair + 1u);
   const bool hn = swap ? hr : hl, hf = swap ? hl : hr;
   const float dn = swap ? dr : dl, df = swap ? dl : dr;
   const uint32_t fn = swap ? fr : fl, ff = swap ? fl : fr;
   const bool take_n = hn && dn < lim, take_f = hf && df < lim;
   if (take_n) {
-    if (take_f) wide_push(st, sp, ff, df, err);
+    if (take_f) wide_push(st, sp, ff, df);
     return fn;
   }
   return take_f ? ff : wide_pop(st, sp, lim);
-}
-
-// The triangles of one leaf in order. False: the ray must start again on the binary nodes.
-PBRT_DEV bool closest_in_leaf(const MeshView& m, uint32_t ref, const WRay& r, float near, float& lim, uint32_t& best,
-                              bool exact) {
-  uint32_t first, count;
-  leaf_range(m.nodes, ref, m.leaf_direct, first, count);
-  float t1 = lim;
-  uint32_t b1 = best;
-  bool tie = false;
-  for (uint32_t k = first; k < first + count; ++k) {
-    float4 A, B;
-    load_node(&m.tri[2 * size_t(k)], A, B);
-    const float2 C = __ldg(&m.tri_c[k]);
-    float t;
-    if (tri_hit(r.o, r.d, A, B, C.x, t) && t >= near) {
-      tie = tie || (t == lim && best != 0xFFFFFFFFu);
-      if (t < t1) {
-        t1 = t;
-        b1 = __float_as_uint(C.y);
-      }
-    }
-  }
-  if (!exact && (t1 < lim || tie)) {
-    const uint32_t node = __ldg(&m.leaf_node[first]);
-    const float4 lo = __ldg(&m.nodes[2 * size_t(node)]), hi = __ldg(&m.nodes[2 * size_t(node) + 1]);
-    float e;
-    if (!box_hit(prepare_ray(r.o, r.d), lo, hi, near, __int_as_float(0x7f800000), e)) return true;  // not its leaf
-    if (!(t1 < lim) || t1 < e) return false;  // a tie between leaves, or a hit before the leaf's entry
-  }
-  lim = t1;
-  best = b1;
-  return true;
-}
-
-// Whether some triangle of the leaf is hit within [near, lim).
-PBRT_DEV bool any_in_leaf(const MeshView& m, uint32_t ref, const WRay& r, float near, float lim, bool exact) {
-  uint32_t first, count;
-  leaf_range(m.nodes, ref, m.leaf_direct, first, count);
-  for (uint32_t k = first; k < first + count; ++k) {
-    float4 A, B;
-    load_node(&m.tri[2 * size_t(k)], A, B);
-    const float2 C = __ldg(&m.tri_c[k]);
-    float t;
-    if (tri_hit(r.o, r.d, A, B, C.x, t) && t < lim && t >= near) {
-      if (exact) return true;
-      const uint32_t node = __ldg(&m.leaf_node[first]);
-      const float4 lo = __ldg(&m.nodes[2 * size_t(node)]), hi = __ldg(&m.nodes[2 * size_t(node) + 1]);
-      float e;
-      return box_hit(prepare_ray(r.o, r.d), lo, hi, near, __int_as_float(0x7f800000), e) && e < lim;
-    }
-  }
-  return false;
 }
 
 }  // namespace pbrt

@@ -12,6 +12,7 @@ import torch
 import oracle
 import pbrt_b200 as pb
 from pbrt_b200 import workloads as W
+from pbrt_b200.scene import Batch, render_params
 
 pytestmark = pytest.mark.gpu
 
@@ -148,3 +149,72 @@ def test_occlusion_under_capture_and_on_several_streams():
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(occ, want[0][1])
+
+
+def _mixed_scene():
+    """Meshes merged into the wide tree, one placed twice, coplanar sheets in different objects,
+    transformed instances, analytic shapes, a compound, a solid and an unbounded plane."""
+    v, f = _ball(1, 0)
+    ball = pb.TriangleMesh(v, f)
+    sv, sf = _sheets()
+    sheet = pb.TriangleMesh(sv * np.float32(3) + np.float32([0, 0, 2]), sf)
+    again = pb.TriangleMesh(sv * np.float32(2) + np.float32([0.5, 0, 2]), sf[:, ::-1])
+    tr = pb.Transform
+    s = pb.Scene()
+    for o in (pb.Simple(ball), pb.Simple(ball), pb.Simple(sheet), pb.Simple(again),
+              pb.Transformed(pb.Simple(ball), tr.translation([3.0, 1.0, 0.5]) * tr.rotation_x(0.4)),
+              pb.Transformed(pb.Simple(pb.Sphere(0.7)), tr.translation([-2.0, 0.0, 0.0])),
+              pb.Transformed(pb.Simple(pb.Sphere(0.7)), tr.translation([-2.0, 0.0, 0.0])),
+              pb.Simple(pb.AABox((1.0, 5.0, 1.0))), pb.Transformed(pb.Simple(pb.Cylinder(0.4, 2.0)), tr.translation([0, 2.0, 1.0])),
+              pb.Transformed(pb.Simple(pb.Rectangle(4.0, 4.0)), tr.translation([0.0, -1.5, 0.0])),
+              pb.Compound([pb.Transformed(pb.Simple(pb.Sphere(0.5)), tr.translation([0.0, 0.0, 3.0])), pb.Simple(ball)]),
+              pb.Simple(pb.Csg("subtraction", [(pb.Sphere(1.2), tr.translation([4.0, 0.0, 4.0])),
+                                               (pb.AABox((1.0, 1.0, 4.0)), tr.translation([4.0, 0.0, 4.0]))])),
+              pb.Transformed(pb.Simple(pb.Plane()), tr.translation([0.0, -2.0, 0.0]))):
+        s.add_object(o)
+    return s
+
+
+def _only_meshes():
+    s = pb.Scene()
+    for k, (scale, shift) in enumerate([(1, 0), (0.5, 0.7), (1e-3, 0.2), (2, 0)]):
+        s.add_object(pb.Simple(pb.TriangleMesh(*_ball(scale, shift))))
+    s.add_object(pb.Simple(pb.TriangleMesh(*_sheets())))
+    s.add_object(pb.Simple(pb.TriangleMesh(*_one())))
+    return s
+
+
+@pytest.mark.parametrize("build", [_mixed_scene, _only_meshes])
+def test_scene_walk_equals_the_counted_queries(build):
+    """Any scene's nearest hits and occlusion by the walk over its one wide tree against the
+    counted queries, which take the binary trees one object at a time: the same objects,
+    primitives and distances, equal distances between objects included."""
+    s = build().commit()
+    v = np.array([[-5, -3, -3], [5, 3, 5]], np.float32)
+    rays = _rays(np.concatenate([v, _sheets()[0], _ball(1, 0)[0]]), np.arange(600, dtype=np.uint32).reshape(-1, 3), 17)
+    for n in (rays.shape[1], 31, 1):
+        r = np.ascontiguousarray(rays[:, :n])
+        bp, bt, bo, _ = s.intersect_counted(r)
+        wp, wt, wo = s.intersect(r, with_object=True)
+        assert np.array_equal(wo, bo) and np.array_equal(wt, bt)
+        hit = bo != pb.PBRT_MISS
+        assert np.array_equal(wp[hit], bp[hit])
+        bocc, _ = s.intersect_p_counted(r)
+        assert np.array_equal(s.intersect_p(r), bocc)
+    assert hit.any() or n == 1
+
+
+def test_small_scenes_by_both_walks():
+    """A closed box, whose waves of at most 786,432 paths run one thread per ray and larger ones
+    persistently: the same film from one wave of 1.05 M paths as from waves of 2^18."""
+    desc, cam = W.cornell_box(256, 256)
+    films = []
+    for wave in (1 << 18, 0):
+        ctx = pb.Context(0)
+        ctx.set_tuning(wave_paths=wave)
+        ctx.set_batch_branches(1)
+        scene = pb.Scene.from_description(desc, ctx).commit()
+        b = Batch([scene], [render_params(cam, 16, 6, seed=5)], ctx)
+        films += [b.render(0)[0], scene.render(cam, 16, 6, seed=5)]
+    for f in films[1:]:
+        np.testing.assert_array_equal(f, films[0])
