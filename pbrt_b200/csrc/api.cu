@@ -102,9 +102,9 @@ int pbrt_ctx_create(int device, pbrt_ctx** out) {
   if (c->cuda(cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute") !=
       PBRT_OK)
     return PBRT_ERR_CUDA;
-  if (c->cuda(cudaMalloc(&c->d_err, sizeof(uint32_t)), "cudaMalloc") != PBRT_OK) return PBRT_ERR_OUT_OF_MEMORY;
-  if (c->cuda(cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), c->stream), "cudaMemset") != PBRT_OK)
-    return PBRT_ERR_CUDA;
+  if (c->cuda(cudaHostAlloc(&c->d_err, sizeof(uint32_t), cudaHostAllocMapped), "cudaHostAlloc") != PBRT_OK)
+    return PBRT_ERR_OUT_OF_MEMORY;
+  *c->d_err = 0;
   if (c->cuda(cudaMalloc(&c->d_counters, 16 * sizeof(unsigned long long)), "cudaMalloc") != PBRT_OK)
     return PBRT_ERR_OUT_OF_MEMORY;
   if (c->cuda(cudaMemsetAsync(c->d_counters, 0, 16 * sizeof(unsigned long long), c->stream), "cudaMemset") !=
@@ -153,7 +153,7 @@ void pbrt_ctx_destroy(pbrt_ctx* c) {
   }
   if (c->branch_fork) cudaEventDestroy(c->branch_fork);
   if (c->queue_used) cudaEventDestroy(c->queue_used);
-  cudaFree(c->d_err);
+  cudaFreeHost(c->d_err);
   cudaFree(c->d_counters);
   cudaFree(c->queue);
   cudaFree(c->queue_rec);

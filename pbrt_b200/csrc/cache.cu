@@ -54,8 +54,8 @@ int pbrt_cache::device_arrays() {
   PBRT_TRY(ctx->cuda(cudaMalloc(&grad, P * 4), "cudaMalloc(cache)"));
   PBRT_TRY(ctx->cuda(cudaMalloc(&wfwd, P * 2), "cudaMalloc(cache)"));
   PBRT_TRY(ctx->cuda(cudaMalloc(&wbwd, P * 2), "cudaMalloc(cache)"));
-  PBRT_TRY(ctx->cuda(cudaMalloc(&loss, 4), "cudaMalloc(cache)"));
-  return PBRT_OK;
+  // pinned host memory: the gradient's last kernel writes the loss where the caller reads it
+  return ctx->cuda(cudaHostAlloc(&loss, 4, cudaHostAllocMapped), "cudaHostAlloc(cache)");
 }
 
 int pbrt_cache::ensure_tiles(uint32_t tiles) {
@@ -198,9 +198,10 @@ int pbrt_cache::ensure_branch_buffers(uint32_t slot, uint32_t queries) {
 }
 
 void pbrt_cache::release() {
-  for (void* p : {(void*)w, (void*)m, (void*)v, (void*)grad, (void*)wfwd, (void*)wbwd, (void*)loss, (void*)partials,
-                  (void*)tile_loss, render_block, frame_block})
+  for (void* p : {(void*)w, (void*)m, (void*)v, (void*)grad, (void*)wfwd, (void*)wbwd, (void*)partials, (void*)tile_loss,
+                  render_block, frame_block})
     cudaFree(p);
+  cudaFreeHost(loss);
   for (void* p : branch_block) cudaFree(p);
 }
 
@@ -323,11 +324,7 @@ int pbrt_cache_gradient(pbrt_cache* k, const float* records, const float* target
   PBRT_TRY(k->gradient_device(rin.ptr, tin.ptr, n, s));
   PBRT_TRY(check_device_error(c, s));
   PBRT_TRY(c->cuda(cudaMemcpy(grad, k->grad, mlp::kParams * 4, cudaMemcpyDefault), "cudaMemcpy(gradient)"));
-  if (loss) {
-    float l = 0.f;
-    PBRT_TRY(c->cuda(cudaMemcpy(&l, k->loss, 4, cudaMemcpyDeviceToHost), "cudaMemcpy(loss)"));
-    *loss = l / (float(n) * float(mlp::kOut));
-  }
+  if (loss) *loss = *static_cast<volatile float*>(k->loss) / (float(n) * float(mlp::kOut));
   return PBRT_OK;
 }
 
@@ -343,11 +340,7 @@ int pbrt_cache_train_step(pbrt_cache* k, const float* records, const float* targ
   PBRT_TRY(k->gradient_device(rin.ptr, tin.ptr, n, s));
   PBRT_TRY(k->adam_device(s));
   PBRT_TRY(check_device_error(c, s));
-  if (loss) {
-    float l = 0.f;
-    PBRT_TRY(c->cuda(cudaMemcpy(&l, k->loss, 4, cudaMemcpyDeviceToHost), "cudaMemcpy(loss)"));
-    *loss = l / (float(n) * float(mlp::kOut));
-  }
+  if (loss) *loss = *static_cast<volatile float*>(k->loss) / (float(n) * float(mlp::kOut));
   return PBRT_OK;
 }
 

@@ -88,6 +88,8 @@ struct pbrt_ctx {
   // context.
   cudaMemPool_t pool = nullptr;
   std::string err;
+  // The error word, in pinned host memory that the kernels reach: they touch it only to report
+  // an error, and a synchronous call reads it without a copy (8 us a call).
   uint32_t* d_err = nullptr;
   unsigned long long* d_counters = nullptr;  // [0..2] traversal counters, [4..5] queue length / fetch position,
                                              // [8..10] rays / shadow rays / paths of the last render
@@ -172,11 +174,10 @@ namespace api {
 // Reads and clears the device error word after the work that may have raised it.
 inline int check_device_error(pbrt_ctx* c, cudaStream_t s) {
   PBRT_TRY(c->cuda(cudaStreamSynchronize(s), "kernel execution"));
-  uint32_t h = 0;
-  PBRT_TRY(c->cuda(cudaMemcpy(&h, c->d_err, sizeof(h), cudaMemcpyDeviceToHost), "cudaMemcpy(error word)"));
+  volatile uint32_t* word = c->d_err;
+  const uint32_t h = *word;
   if (h == 0) return PBRT_OK;
-  PBRT_TRY(c->cuda(cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), s), "cudaMemset(error word)"));
-  PBRT_TRY(c->cuda(cudaStreamSynchronize(s), "cudaStreamSynchronize"));
+  *word = 0;
   if (h & kErrStack) return c->fail(PBRT_ERR_CAPACITY, "traversal stack capacity exceeded");
   if (h & 4u) return c->fail(PBRT_ERR_DEVICE_BUDGET, "a tensor-core completion wait ran out of its budget");
   if (h & kErrCopy) return c->fail(PBRT_ERR_DEVICE_BUDGET, "a wait for a bulk copy into shared memory ran out of its budget");

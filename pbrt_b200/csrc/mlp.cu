@@ -27,14 +27,17 @@
 namespace pbrt {
 namespace mlp {
 
-constexpr uint32_t kErrMma = 4u;  // a tensor-core completion wait ran out of its budget
+constexpr uint32_t kErrMma = 4u;      // a tensor-core completion wait ran out of its budget
+constexpr uint32_t kErrWeights = 8u;  // a wait for the weights' bulk copy ran out of its budget
 constexpr uint32_t kWBytes = kParams * 2;           // 47,104
 constexpr uint32_t kXBytes = kTile * kInPad * 2;    // 24,576
 constexpr uint32_t kHBytes = kTile * kHidden * 2;   // 16,384
 constexpr uint32_t kG16Bytes = kTile * kOutPad * 2;  // 4,096
 constexpr uint32_t kTmemCols = 64;       // one 64-column accumulator
-constexpr uint32_t kTrainTmemCols = 256;  // training: dA in columns 0-63, dW from column 64 (up to 96 wide)
-constexpr uint32_t kWgradCol = 64;
+constexpr uint32_t kTrainTmemCols = 256;  // training: dA in columns 0-63, then two ranges of dW
+constexpr uint32_t kWgradCol = 64, kWgradCols = 96;
+static_assert(kWgradCol + 2 * kWgradCols <= kTrainTmemCols && kWgradCols >= kInPad, "both weight gradients must fit");
+constexpr int kReduceThreads = 128;
 static_assert(kXBytes >= kHBytes, "the inference kernel stores the hidden tile over the input tile");
 
 __device__ __forceinline__ uint16_t to_bf16(float f) { return __bfloat16_as_ushort(__float2bfloat16_rn(f)); }
@@ -93,48 +96,43 @@ __device__ __forceinline__ void next_octave(float& s, float& c) {
   s = s2;
 }
 
-// Encodes one query record into 96 features (82 used, zero padded): sin / cos (pi 2^j x) of the
-// normalised position, j < 12 (the first band by sincospi_poly, the others by next_octave),
-// then wo, n, albedo, roughness.
-__device__ void encode(const float* __restrict__ rec, const Bounds& b, float* f) {
-  const float4 q0 = __ldg(reinterpret_cast<const float4*>(rec));
-  const float4 q1 = __ldg(reinterpret_cast<const float4*>(rec) + 1);
-  const float4 q2 = __ldg(reinterpret_cast<const float4*>(rec) + 2);
-  const float4 q3 = __ldg(reinterpret_cast<const float4*>(rec) + 3);
-  const float p[3] = {q0.x, q0.y, q0.z};
+// Stores 8 values as columns c .. c + 7 of row r of a 128-row tile, as BF16.
+__device__ __forceinline__ void store8(uint8_t* tile, uint32_t r, uint32_t c, const float* v) {
+  uint4 q;
+  q.x = pack2(v[0], v[1]);
+  q.y = pack2(v[2], v[3]);
+  q.z = pack2(v[4], v[5]);
+  q.w = pack2(v[6], v[7]);
+  *reinterpret_cast<uint4*>(tile + tc::tile_offset(r, c, kTile)) = q;
+}
+
+// A query record's 96 features (82 used, zero padded), as row r of the input tile: columns
+// 24 a .. 24 a + 23 are sin / cos (pi 2^j x) of the normalised position along axis a, j < 12
+// (the first band by sincospi_poly, the others by next_octave); columns 72 .. 95 are wo, n,
+// albedo, roughness and the padding.
+__device__ __forceinline__ void encode_axis(uint8_t* tile, uint32_t r, uint32_t a, float p, float lo, float inv_extent,
+                                            bool valid) {
+  float sn, cs;
+  sincospi_poly(__fmul_rn(__fsub_rn(p, lo), inv_extent), sn, cs);
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    float s, c;
-    sincospi_poly(__fmul_rn(__fsub_rn(p[a], b.lo[a]), b.inv_extent[a]), s, c);
+  for (int c = 0; c < 3; ++c) {
+    float v[8];
 #pragma unroll
-    for (int j = 0; j < 12; ++j) {
-      f[a * 24 + 2 * j] = s;
-      f[a * 24 + 2 * j + 1] = c;
-      next_octave(s, c);
+    for (int j = 0; j < 4; ++j) {
+      v[2 * j] = valid ? sn : 0.f;
+      v[2 * j + 1] = valid ? cs : 0.f;
+      next_octave(sn, cs);
     }
-  }
-  f[72] = q1.x; f[73] = q1.y; f[74] = q1.z;
-  f[75] = q2.x; f[76] = q2.y; f[77] = q2.z;
-  f[78] = q3.x; f[79] = q3.y; f[80] = q3.z;
-  f[81] = q0.w;
-#pragma unroll
-  for (int k = kIn; k < kInPad; ++k) f[k] = 0.f;
-}
-
-// Writes `n` (multiple of 8) values of row r into an R=128-row tile as BF16.
-__device__ __forceinline__ void store_row(uint8_t* tile, uint32_t r, const float* v, int n) {
-  for (int c = 0; c < n; c += 8) {
-    uint4 q;
-    q.x = pack2(v[c], v[c + 1]);
-    q.y = pack2(v[c + 2], v[c + 3]);
-    q.z = pack2(v[c + 4], v[c + 5]);
-    q.w = pack2(v[c + 6], v[c + 7]);
-    *reinterpret_cast<uint4*>(tile + tc::tile_offset(r, uint32_t(c), kTile)) = q;
+    store8(tile, r, a * 24u + uint32_t(c) * 8u, v);
   }
 }
-
-__device__ __forceinline__ float tile_at(const uint8_t* tile, uint32_t r, uint32_t k, uint32_t rows) {
-  return from_bf16(*reinterpret_cast<const uint16_t*>(tile + tc::tile_offset(r, k, rows)));
+__device__ __forceinline__ void encode_rest(uint8_t* tile, uint32_t r, const float4& q0, const float4& q1,
+                                            const float4& q2, const float4& q3) {
+  const float va[8] = {q1.x, q1.y, q1.z, q2.x, q2.y, q2.z, q3.x, q3.y};
+  const float vb[8] = {q3.z, q0.w, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  store8(tile, r, 72u, va);
+  store8(tile, r, 80u, vb);
+  *reinterpret_cast<uint4*>(tile + tc::tile_offset(r, 88u, kTile)) = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // D[128 x n] = A[128 x k] · B[n x k]^T, both K-major in the core-matrix layout; thread 0 only.
@@ -166,46 +164,10 @@ __device__ __forceinline__ void issue_gemm_tn(const uint8_t* p, const uint8_t* q
   tc::mma_commit(mbar);
 }
 
-// All threads: waits for the committed GEMM; false (and the error bit) if it never completes.
-__device__ __forceinline__ bool wait_gemm(uint64_t* mbar, uint32_t& phase, uint32_t* err) {
-  bool ok = tc::mbar_wait(mbar, phase);
-  ok = __syncthreads_and(ok);
-  if (!ok && threadIdx.x == 0) atomicOr(err, kErrMma);
-  phase ^= 1u;
-  tc::fence_after_sync();
-  return ok;
-}
-
-// This thread's 64 accumulator columns (its TMEM lane is its row).
-__device__ __forceinline__ void read_acc64(uint32_t tmem, float* v) {
-  const uint32_t lane = (threadIdx.x >> 5) * 32u;
-#pragma unroll
-  for (int c = 0; c < 64; c += 16) tc::tmem_ld16(tmem + (lane << 16) + uint32_t(c), v + c);
-}
-
 __device__ __forceinline__ void load_smem(uint8_t* dst, const uint16_t* src, uint32_t bytes) {
   const uint4* s = reinterpret_cast<const uint4*>(src);
   uint4* d = reinterpret_cast<uint4*>(dst);
   for (uint32_t i = threadIdx.x; i < bytes / 16; i += blockDim.x) d[i] = __ldg(s + i);
-}
-
-__device__ __forceinline__ void setup_tmem(uint64_t* mbar, uint32_t* tslot, uint32_t ncols = kTmemCols) {
-  if (threadIdx.x == 0) tc::mbar_init(mbar, 1);
-  if ((threadIdx.x >> 5) == 0) {
-    tc::tmem_alloc(tslot, ncols);
-    tc::tmem_relinquish();
-  }
-  tc::fence_before_sync();
-  __syncthreads();
-  tc::fence_after_sync();
-}
-
-__device__ __forceinline__ void release_tmem(uint32_t tmem, uint64_t* mbar, uint32_t phase, bool ok,
-                                             uint32_t ncols = kTmemCols) {
-  if (!ok) tc::mbar_wait(mbar, phase, 1u << 20);  // one more bounded wait for a GEMM still in flight
-  tc::fence_before_sync();
-  __syncthreads();
-  if ((threadIdx.x >> 5) == 0) tc::tmem_dealloc(tmem, ncols);
 }
 
 // Inference: one CTA per SM holds the weights once and runs kInferGroups independent tile
@@ -282,46 +244,13 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(Net net, Bounds 
   for (uint64_t tile = uint64_t(blockIdx.x) * kInferGroups + g; tile < tiles && ok; tile += tile_step) {
     const uint64_t row = tile * kTile + r;
     {
-      // encode(): the features in 8-column chunks, 3 axes x 3 chunks of sin/cos bands, then the
-      // 10 record values, without a 96-value array in registers
       const float4 q0 = n0, q1 = n1, q2 = n2, q3 = n3;
       load_record(tile + tile_step, n0, n1, n2, n3);
       const bool valid = row < n;
       const float p[3] = {q0.x, q0.y, q0.z};
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        float sn, cs;
-        sincospi_poly(__fmul_rn(__fsub_rn(p[a], b.lo[a]), b.inv_extent[a]), sn, cs);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          float v[8];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            v[2 * j] = valid ? sn : 0.f;
-            v[2 * j + 1] = valid ? cs : 0.f;
-            next_octave(sn, cs);
-          }
-          uint4 qq;
-          qq.x = pack2(v[0], v[1]);
-          qq.y = pack2(v[2], v[3]);
-          qq.z = pack2(v[4], v[5]);
-          qq.w = pack2(v[6], v[7]);
-          *reinterpret_cast<uint4*>(sX + tc::tile_offset(r, uint32_t(a * 24 + c * 8), kTile)) = qq;
-        }
-      }
-      uint4 qa, qb;
-      const uint4 qz = make_uint4(0u, 0u, 0u, 0u);
-      qa.x = pack2(q1.x, q1.y);
-      qa.y = pack2(q1.z, q2.x);
-      qa.z = pack2(q2.y, q2.z);
-      qa.w = pack2(q3.x, q3.y);
-      qb.x = pack2(q3.z, q0.w);
-      qb.y = 0u;
-      qb.z = 0u;
-      qb.w = 0u;
-      *reinterpret_cast<uint4*>(sX + tc::tile_offset(r, 72u, kTile)) = qa;
-      *reinterpret_cast<uint4*>(sX + tc::tile_offset(r, 80u, kTile)) = qb;
-      *reinterpret_cast<uint4*>(sX + tc::tile_offset(r, 88u, kTile)) = qz;
+      for (int a = 0; a < 3; ++a) encode_axis(sX, r, uint32_t(a), p[a], b.lo[a], b.inv_extent[a], valid);
+      encode_rest(sX, r, q0, q1, q2, q3);
     }
     tc::fence_smem_to_async();
     group_sync(g);
@@ -376,158 +305,243 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(Net net, Bounds 
   if (threadIdx.x < 32) tc::tmem_dealloc(*tslot, kInferTmemCols);
 }
 
-__global__ void __launch_bounds__(kTile, 1) k_mlp_grad(Net net, Bounds b, const float* __restrict__ rec,
-                                                        const float* __restrict__ tgt, uint64_t n, float grad_scale,
-                                                        float* __restrict__ partials, float* __restrict__ tile_loss,
-                                                        uint32_t* err) {
+// One tile's loss, activations and weight gradients: one CTA of 256 threads per 128 samples, a
+// sample's row shared by threads r and r + 128, which take half of the columns each (TMEM lanes
+// belong to a warp's number modulo 4, so both reach the row's lane).
+//
+// A batch is one tile per SM, so what bounds the kernel is its chain of twelve dependent GEMMs
+// (under 0.1 us of tensor-core time each): what stands between two of them decides the time.
+// The weights arrive by bulk copies that the encoding runs under. Going back, a layer's data
+// gradient is masked and stored first and the next layer's GEMMs are issued; only then is the
+// layer's weight gradient read out, under them (its accumulators alternate between two column
+// ranges). The layer gradient replaces the activations it was masked by, whose last reader,
+// the weight gradient's GEMM, has completed by then, each thread its own columns.
+// 16,384 samples (128 tiles), B200: 29.5 us with 128 threads, ordinary loads of the weights and
+// the weight gradients read out in the chain; 17.8 us so.
+constexpr int kGradThreads = 2 * kTile;
+
+__global__ void __launch_bounds__(kGradThreads, 1) k_mlp_grad(Net net, Bounds b, const float* __restrict__ rec,
+                                                              const float* __restrict__ tgt, uint64_t n,
+                                                              float grad_scale, float* __restrict__ partials,
+                                                              float* __restrict__ tile_loss, uint32_t* err) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sWf = smem;
   uint8_t* sWb = sWf + kWBytes;
   uint8_t* sX = sWb + kWBytes;
-  uint8_t* sA = sX + kXBytes;          // activations A_1..A_5, kHBytes each
-  uint8_t* sG = sA + 5 * kHBytes;      // layer gradient (64 wide)
-  uint8_t* sG16 = sG + kHBytes;        // output gradient (16 wide)
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(sG16 + kG16Bytes);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 1);
+  uint8_t* sA = sX + kXBytes;         // activations A_1..A_5, kHBytes each; then the gradients G_0..G_4
+  uint8_t* sG16 = sA + 5 * kHBytes;   // output gradient (16 wide)
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(sG16 + kG16Bytes);  // [0] GEMMs, [1] [2] weight copies
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 3);
   float* s_loss = reinterpret_cast<float*>(tslot + 1);
-  load_smem(sWf, net.wpk_fwd, kWBytes);
-  load_smem(sWb, net.wpk_bwd, kWBytes);
-  if (threadIdx.x == 0) *s_loss = 0.f;
-  setup_tmem(mbar, tslot, kTrainTmemCols);
-  const uint32_t tmem = *tslot;
-  uint32_t phase = 0;
-  bool ok = true;
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < 3; ++k) tc::mbar_init(mbar + k, 1);
+    *s_loss = 0.f;
+    tc::mbar_arrive_expect_tx(mbar + 1, kWBytes);
+    tc::bulk_g2s(sWf, net.wpk_fwd, kWBytes, mbar + 1);
+    tc::mbar_arrive_expect_tx(mbar + 2, kWBytes);
+    tc::bulk_g2s(sWb, net.wpk_bwd, kWBytes, mbar + 2);
+  }
+  const uint32_t half = threadIdx.x / kTile, r = threadIdx.x % kTile;
   const uint64_t tile = blockIdx.x;
-  const uint32_t r = threadIdx.x;
   const uint64_t row = tile * kTile + r;
-  auto act = [&](int l) -> uint8_t* { return l == 0 ? sX : sA + (l - 1) * kHBytes; };
-
   {
-    float f[kInPad];
-    if (row < n) {
-      encode(rec + row * kRecord, b, f);
-    } else {
-#pragma unroll
-      for (int k = 0; k < kInPad; ++k) f[k] = 0.f;
-    }
-    store_row(sX, r, f, kInPad);
-    tc::fence_smem_to_async();
-    __syncthreads();
-  }
-  // forward, keeping every activation
-  float o[3] = {0.f, 0.f, 0.f};
-  for (int l = 0; l < kLayers && ok; ++l) {
-    if (threadIdx.x == 0) {
-      tc::fence_after_sync();
-      issue_gemm(act(l), sWf + 2 * layer_off(l), uint32_t(layer_n(l)), uint32_t(layer_k(l)), tmem, mbar);
-    }
-    ok = wait_gemm(mbar, phase, err);
-    if (!ok) break;
-    if (l < kLayers - 1) {
-      float v[64];
-      read_acc64(tmem, v);
-#pragma unroll
-      for (int c = 0; c < 64; ++c) v[c] = fmaxf(v[c], 0.f);
-      store_row(act(l + 1), r, v, 64);
-      tc::fence_before_sync();
-      tc::fence_smem_to_async();
-      __syncthreads();
-    } else {
-      float v[16];
-      tc::tmem_ld16(tmem + (((threadIdx.x >> 5) * 32u) << 16), v);
-      o[0] = v[0]; o[1] = v[1]; o[2] = v[2];
-      tc::fence_before_sync();
-      __syncthreads();
-    }
-  }
-  if (ok) {
-    // relative L2 loss and its gradient (the denominator is held constant)
-    float g[16];
-#pragma unroll
-    for (int c = 0; c < 16; ++c) g[c] = 0.f;
-    float loss = 0.f;
-    if (row < n) {
-      for (int c = 0; c < 3; ++c) {
-        const float d = o[c] - __ldg(tgt + 3 * row + c);
-        const float w = 1.0f / (o[c] * o[c] + 0.01f);
-        loss += d * d * w;
-        g[c] = 2.0f * d * w * grad_scale;
+    const bool valid = row < n;
+    float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0, q2 = q0, q3 = q0;
+    if (valid) {
+      const float4* qr = reinterpret_cast<const float4*>(rec + row * kRecord);
+      q0 = __ldg(qr);
+      if (half) {
+        q1 = __ldg(qr + 1);
+        q2 = __ldg(qr + 2);
+        q3 = __ldg(qr + 3);
       }
     }
-    for (int off = 16; off > 0; off >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(s_loss, loss);
-    store_row(sG16, r, g, 16);
-    tc::fence_smem_to_async();
-    __syncthreads();
-  }
-  // backward
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t quarter = (warp * 32u) << 16;  // this warp's TMEM lanes
-  for (int l = kLayers - 1; l >= 0 && ok; --l) {
-    const int N = layer_n(l), K = layer_k(l);
-    const uint8_t* G = (l == kLayers - 1) ? sG16 : sG;
-    const uint8_t* A = act(l);
-    if (threadIdx.x == 0) {
-      tc::fence_after_sync();
-      // dA_l = G_l · W_l, (128 x K) with K = 64, into columns 0-63
-      if (l > 0) issue_gemm(G, sWb + 2 * layer_off(l), uint32_t(K), uint32_t(N), tmem, nullptr);
-      // dW_l = G_lᵀ · A_l (64 x K), or for the 16-row output layer dW_lᵀ = A_lᵀ · G_l (64 x 16)
-      if (l < kLayers - 1)
-        issue_gemm_tn(G, A, uint32_t(K), tmem + kWgradCol, mbar);
-      else
-        issue_gemm_tn(A, G, uint32_t(N), tmem + kWgradCol, mbar);
+    if (half == 0) {
+      encode_axis(sX, r, 0, q0.x, b.lo[0], b.inv_extent[0], valid);
+      encode_axis(sX, r, 1, q0.y, b.lo[1], b.inv_extent[1], valid);
+    } else {
+      encode_axis(sX, r, 2, q0.z, b.lo[2], b.inv_extent[2], valid);
+      encode_rest(sX, r, q0, q1, q2, q3);
     }
-    ok = wait_gemm(mbar, phase, err);
-    if (!ok) break;
-    {
-      // M = 64 accumulator: lanes 0-15 of warp q hold rows 16q .. 16q + 15
-      const uint32_t row = warp * 16u + lane;
+    tc::fence_smem_to_async();
+  }
+  if (threadIdx.x < 32) {
+    tc::tmem_alloc(tslot, kTrainTmemCols);
+    tc::tmem_relinquish();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *tslot;
+  const uint32_t warp = (threadIdx.x >> 5) & 3u, lane = threadIdx.x & 31u;
+  const uint32_t quarter = (warp * 32u) << 16;  // this warp's TMEM lanes
+  auto act = [&](int l) -> uint8_t* { return l == 0 ? sX : sA + (l - 1) * kHBytes; };
+  // A wait that runs out sets the error bit and clears `ok`, which every barrier below makes
+  // the block's: nobody issues or reads anything after that.
+  auto await = [&](uint64_t* bar, uint32_t parity, uint32_t bit) {
+    if (tc::mbar_wait(bar, parity)) return true;
+    if (r == 0) atomicOr(err, bit);
+    return false;
+  };
+  uint32_t phase = 0;
+  // the copies' waits by every thread: none exits, or deallocates, under a copy in flight
+  bool ok = __syncthreads_and(await(mbar + 1, 0, kErrWeights) && await(mbar + 2, 0, kErrWeights));
+  const bool copied = ok;
+  if (ok && threadIdx.x == 0) issue_gemm(sX, sWf, uint32_t(layer_n(0)), uint32_t(layer_k(0)), tmem, mbar);
+  // forward, keeping every activation; this thread's 32 columns of its row
+  for (int l = 0; l < kLayers - 1 && ok; ++l) {
+    ok = await(mbar, phase, kErrMma);
+    phase ^= 1u;
+    if (ok) {
+      tc::fence_after_sync();
+      float v[32];
+      tc::tmem_ld16(tmem + quarter + half * 32u, v);
+      tc::tmem_ld16(tmem + quarter + half * 32u + 16u, v + 16);
+#pragma unroll
+      for (int c = 0; c < 32; ++c) v[c] = fmaxf(v[c], 0.f);
+#pragma unroll
+      for (int c = 0; c < 32; c += 8) store8(act(l + 1), r, half * 32u + uint32_t(c), v + c);
+      tc::fence_before_sync();
+      tc::fence_smem_to_async();
+    }
+    ok = __syncthreads_and(ok);
+    if (ok && threadIdx.x == 0) {
+      tc::fence_after_sync();
+      issue_gemm(act(l + 1), sWf + 2 * layer_off(l + 1), uint32_t(layer_n(l + 1)), uint32_t(layer_k(l + 1)), tmem,
+                 mbar);
+    }
+  }
+  // relative L2 loss and its gradient (the denominator is held constant), by the first half
+  if (ok) {
+    ok = await(mbar, phase, kErrMma);
+    phase ^= 1u;
+    if (ok && half == 0) {
+      tc::fence_after_sync();
+      float o[16], g[16];
+      tc::tmem_ld16(tmem + quarter, o);
+#pragma unroll
+      for (int c = 0; c < 16; ++c) g[c] = 0.f;
+      float loss = 0.f;
+      if (row < n) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float d = o[c] - __ldg(tgt + 3 * row + c);
+          const float w = 1.0f / (o[c] * o[c] + 0.01f);
+          loss += d * d * w;
+          g[c] = 2.0f * d * w * grad_scale;
+        }
+      }
+      store8(sG16, r, 0, g);
+      store8(sG16, r, 8, g + 8);
+      for (int off = 16; off > 0; off >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, off);
+      if (lane == 0) atomicAdd(s_loss, loss);
+      tc::fence_before_sync();
+      tc::fence_smem_to_async();
+    }
+    ok = __syncthreads_and(ok);
+  }
+  // Both products of layer l, committed together: dA_l = G_l · W_l (128 x 64) into columns 0-63
+  // and dW_l = G_lᵀ · A_l (64 x K), for the 16-row output layer dW_lᵀ = A_lᵀ · G_l (64 x 16).
+  auto wgrad_col = [&](int l) { return kWgradCol + ((l & 1) ? kWgradCols : 0u); };
+  auto issue_layer = [&](int l) {
+    const uint8_t* G = l == kLayers - 1 ? sG16 : act(l + 1);
+    const uint32_t N = uint32_t(layer_n(l)), K = uint32_t(layer_k(l));
+    tc::fence_after_sync();
+    if (l > 0) issue_gemm(G, sWb + 2 * layer_off(l), K, N, tmem, nullptr);
+    if (l < kLayers - 1)
+      issue_gemm_tn(G, act(l), K, tmem + wgrad_col(l), mbar);
+    else
+      issue_gemm_tn(act(l), G, N, tmem + wgrad_col(l), mbar);
+  };
+  if (ok && threadIdx.x == 0) issue_layer(kLayers - 1);
+  for (int l = kLayers - 1; l >= 0 && ok; --l) {
+    ok = await(mbar, phase, kErrMma);
+    phase ^= 1u;
+    if (ok) tc::fence_after_sync();
+    if (l > 0) {
+      if (ok) {
+        uint8_t* A = act(l);
+        float v[32];
+        tc::tmem_ld16(tmem + quarter + half * 32u, v);
+        tc::tmem_ld16(tmem + quarter + half * 32u + 16u, v + 16);
+#pragma unroll
+        for (int c = 0; c < 32; c += 8) {
+          // an activation is above 0 when its BF16 bits, as a signed number, are: neither zero
+          // nor negative (a NaN never follows a ReLU written as a maximum with 0)
+          const uint4 q = *reinterpret_cast<const uint4*>(A + tc::tile_offset(r, half * 32u + uint32_t(c), kTile));
+          const uint32_t h[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            v[c + 2 * j] = int16_t(h[j] & 0xffffu) > 0 ? v[c + 2 * j] : 0.f;
+            v[c + 2 * j + 1] = int32_t(h[j] & 0xffff0000u) > 0 ? v[c + 2 * j + 1] : 0.f;
+          }
+          store8(A, r, half * 32u + uint32_t(c), v + c);
+        }
+        tc::fence_before_sync();
+        tc::fence_smem_to_async();
+      }
+      ok = __syncthreads_and(ok);
+      if (ok && threadIdx.x == 0) issue_layer(l - 1);
+    }
+    if (ok) {
+      // M = 64 accumulator: lanes 0-15 of the quarter q hold rows 16q .. 16q + 15
+      const int K = layer_k(l);
+      const uint32_t orow = warp * 16u + lane;
       float* dst = partials + tile * uint64_t(kParams) + layer_off(l);
-      const int cols = l < kLayers - 1 ? K : N;
-      for (int c = 0; c < cols; c += 16) {
-        float v[16];
-        tc::tmem_ld16(tmem + quarter + kWgradCol + uint32_t(c), v);
-        if (lane < 16) {
-          if (l < kLayers - 1) {  // row = output unit o, columns = inputs i
+      if (l < kLayers - 1) {  // row = output unit o, columns = inputs i
+        for (int c = int(half) * 16; c < K; c += 32) {
+          float v[16];
+          tc::tmem_ld16(tmem + quarter + wgrad_col(l) + uint32_t(c), v);
+          if (lane < 16) {
 #pragma unroll
             for (int j = 0; j < 16; j += 4)
-              *reinterpret_cast<float4*>(dst + row * uint32_t(K) + uint32_t(c + j)) =
+              *reinterpret_cast<float4*>(dst + orow * uint32_t(K) + uint32_t(c + j)) =
                   make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-          } else {  // transposed: row = input i, columns = outputs o
-#pragma unroll
-            for (int j = 0; j < 16; ++j) dst[uint32_t(c + j) * uint32_t(K) + row] = v[j];
           }
+        }
+      } else if (half == 0) {  // transposed: row = input i, columns = outputs o
+        float v[16];
+        tc::tmem_ld16(tmem + quarter + wgrad_col(l), v);
+        if (lane < 16) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) dst[uint32_t(j) * uint32_t(K) + orow] = v[j];
         }
       }
     }
-    if (l > 0) {
-      float v[64];
-      read_acc64(tmem, v);
-#pragma unroll
-      for (int c = 0; c < 64; ++c) v[c] = tile_at(A, r, uint32_t(c), kTile) > 0.f ? v[c] : 0.f;
-      store_row(sG, r, v, 64);
-      tc::fence_smem_to_async();
-    }
-    tc::fence_before_sync();
-    __syncthreads();
   }
   if (threadIdx.x == 0) tile_loss[tile] = *s_loss;
-  release_tmem(tmem, mbar, phase, ok, kTrainTmemCols);
+  // one more bounded wait for a GEMM or copies still in flight
+  if (!ok) tc::mbar_wait(copied ? mbar : mbar + 2, copied ? phase ^ 1u : 0u, 1u << 20);
+  tc::fence_before_sync();
+  __syncthreads();
+  if (threadIdx.x < 32) tc::tmem_dealloc(tmem, kTrainTmemCols);
 }
 
-__global__ void k_reduce(const float* __restrict__ partials, const float* __restrict__ tile_loss, uint32_t tiles,
-                         float* __restrict__ grad, float* __restrict__ loss) {
+// grad[p] = the sum of the tiles' partials in tile order, a thread per parameter and one for
+// the loss. The order is part of the result, so the additions are one chain, and what bounds
+// the kernel is the loads' latency: kBatch are in flight at a time. (128 tiles are
+// 12 MB, in L2 when the tiles' kernel has just written them.)
+__device__ __forceinline__ float ordered_sum(const float* __restrict__ p, uint64_t stride, uint32_t count) {
+  constexpr uint32_t kBatch = 32;
+  float s = 0.f;
+  uint32_t t = 0;
+  for (; t + kBatch <= count; t += kBatch) {
+    float v[kBatch];
+#pragma unroll
+    for (uint32_t j = 0; j < kBatch; ++j) v[j] = __ldg(p + uint64_t(t + j) * stride);
+#pragma unroll
+    for (uint32_t j = 0; j < kBatch; ++j) s += v[j];
+  }
+  for (; t < count; ++t) s += __ldg(p + uint64_t(t) * stride);
+  return s;
+}
+
+__global__ void __launch_bounds__(kReduceThreads) k_reduce(const float* __restrict__ partials,
+                                                           const float* __restrict__ tile_loss, uint32_t tiles,
+                                                           float* __restrict__ grad, float* __restrict__ loss) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < uint32_t(kParams)) {
-    float s = 0.f;
-    for (uint32_t t = 0; t < tiles; ++t) s += partials[uint64_t(t) * kParams + p];
-    grad[p] = s;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    float s = 0.f;
-    for (uint32_t t = 0; t < tiles; ++t) s += tile_loss[t];
-    *loss = s;
-  }
+  if (p < uint32_t(kParams)) grad[p] = ordered_sum(partials + p, kParams, tiles);
+  if (p == uint32_t(kParams)) *loss = ordered_sum(tile_loss, 1, tiles);
 }
 
 __device__ __forceinline__ void pack_one(uint32_t p, float w, uint16_t* fwd, uint16_t* bwd) {
@@ -565,7 +579,7 @@ __global__ void k_pack(const float* __restrict__ w, uint16_t* fwd, uint16_t* bwd
 }
 
 size_t infer_smem_bytes() { return kWBytes + kInferGroups * kXBytes + kInferGroups * 8 + 16; }
-size_t train_smem_bytes() { return 2 * kWBytes + kXBytes + 5 * kHBytes + kHBytes + kG16Bytes + 64; }
+size_t train_smem_bytes() { return 2 * kWBytes + kXBytes + 5 * kHBytes + kG16Bytes + 64; }
 
 cudaError_t launch_infer(const Net& net, const Bounds& b, const float* records, uint64_t n, float* out, uint32_t* err,
                          int sm_count, cudaStream_t s) {
@@ -605,14 +619,14 @@ cudaError_t launch_grad_tiles(const Net& net, const Bounds& b, const float* reco
   cudaError_t e = allow_smem(configured, reinterpret_cast<const void*>(k_mlp_grad), train_smem_bytes());
   if (e != cudaSuccess) return e;
   const uint64_t tiles = (n + kTile - 1) / kTile;
-  k_mlp_grad<<<unsigned(tiles), kTile, train_smem_bytes(), s>>>(net, b, records, targets, n, grad_scale, partials,
+  k_mlp_grad<<<unsigned(tiles), kGradThreads, train_smem_bytes(), s>>>(net, b, records, targets, n, grad_scale, partials,
                                                                  tile_loss, err);
   return cudaGetLastError();
 }
 
 cudaError_t launch_reduce(const float* partials, const float* tile_loss, uint32_t tiles, float* grad, float* loss,
                           cudaStream_t s) {
-  k_reduce<<<(kParams + 255) / 256, 256, 0, s>>>(partials, tile_loss, tiles, grad, loss);
+  k_reduce<<<kParams / kReduceThreads + 1, kReduceThreads, 0, s>>>(partials, tile_loss, tiles, grad, loss);
   return cudaGetLastError();
 }
 

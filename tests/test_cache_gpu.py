@@ -130,6 +130,36 @@ def test_gradient_is_deterministic(cache):
     np.testing.assert_array_equal(g1, g2)
 
 
+@pytest.mark.parametrize("tiles", [1, 2, 16, 32, 128, 256])
+def test_gradient_is_the_ordered_sum_of_its_tiles(cache, tiles):
+    """A batch of a power of two of 128-sample tiles scales each tile's loss gradient by an exact
+    power of two against the tile alone, so the batch's gradient is, bit for bit, the FP32 sum of
+    the tiles' own scaled gradients in tile order (sums of one tile up to several load batches)."""
+    cache.reset()
+    r = random_records(128 * tiles, LO, HI, seed=40 + tiles)
+    t = _targets(r)
+    g, _ = cache.gradient(r, t)
+    want = np.zeros(PARAMS, np.float32)
+    for k in range(tiles):
+        part, _ = cache.gradient(r[128 * k:128 * (k + 1)], t[128 * k:128 * (k + 1)])
+        want = want + part * np.float32(1.0 / tiles)
+    np.testing.assert_array_equal(g, want)
+
+
+def test_gradient_of_a_ragged_batch_matches_oracle(cache):
+    cache.reset()
+    n = 33 * 128 + 1  # a load batch of tiles, one more, and a tile of one sample
+    r = random_records(n, LO, HI, seed=13)
+    t = _targets(r)
+    g, loss = cache.gradient(r, t)
+    go, lo = oracle.mlp_gradient(cache.weights(), BOUNDS, r, t, emulate=True)
+    assert loss == pytest.approx(lo, rel=2e-2)
+    for layer in range(6):
+        a, b = g[OFFS[layer]:OFFS[layer + 1]], go[OFFS[layer]:OFFS[layer + 1]]
+        rel = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-12)
+        assert rel < 3e-2, (layer, rel)
+
+
 def test_adam_step_bit_exact(cache):
     cache.reset()
     r = random_records(3000, LO, HI, seed=13)
