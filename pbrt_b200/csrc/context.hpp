@@ -20,6 +20,13 @@ namespace api {
 
 constexpr uint64_t kSlotRays = uint64_t(1) << 20;  // rays per pipelined chunk (32 MiB of rays)
 constexpr int kSlots = 3;
+// Rays against one mesh that a single kernel answers, one thread each; more go through the two
+// stages. Us per call, one kernel / two stages, meshes of 1,280 / 20,480 / 327,680 triangles, all
+// rays entering the root: 4,099 rays 34/54, 36/60, 56/83; 262,144 rays 62/74, 83/104, 126/156;
+// 524,288 rays 89/84, 124/116, 159/155; 1,048,576 rays 141/93, 179/131, 218/181.
+constexpr uint64_t kFewRays = 1u << 18;
+constexpr uint64_t kStageRays = 1u << 15;  // rays of a host call that go through the pinned stage
+constexpr uint64_t kStageBytes = kStageRays * (8 + 3) * 4;
 constexpr uint64_t kPoolKeep = uint64_t(1) << 30;  // bytes the context's memory pool keeps mapped when free
 constexpr uint64_t kDevChunk = uint64_t(1) << 24;  // rays per launch pair on device buffers
 // Concurrent branches of a wavefront batch frame (pbrt_ctx_set_batch_branches).
@@ -102,6 +109,7 @@ struct pbrt_ctx {
                                               // scratch array on this device, looked up at creation
   pbrt::api::Slot slots[pbrt::api::kSlots];
   bool slots_ready = false;
+  char* stage = nullptr;  // pinned host memory the kernels read a small host call's rays from
   std::vector<void*> allocs;
   pbrt::LaunchShape shape;          // wavefront launch shape (pbrt_ctx_set_tuning)
   uint32_t wave_paths = 1u << 26;   // paths per wave (136 bytes of path state each, allocated on demand)

@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(128) k_mesh_closest(MeshView m, const float* _
   }
 }
 
-// Occlusion, one thread per ray and no scratch: for streams under capture.
+// Occlusion, one thread per ray on the binary nodes (PBRT_TRACE_KERNEL=simple).
 __global__ void __launch_bounds__(128) k_mesh_any(MeshView m, const float* __restrict__ rays, uint64_t stride, uint64_t n,
                                                   uint8_t* __restrict__ occ, uint32_t* __restrict__ err) {
   const uint64_t step = uint64_t(gridDim.x) * blockDim.x;
@@ -435,6 +435,81 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
   }
 }
 
+// Few rays, one launch and no scratch: `lanes` rays to a warp, each through the root test and its
+// own walk of the wide tree. The answers are the two stages' (see k_mesh_walk). What bounds a
+// small call is the launches and a ray's own chain of node loads, not the lanes left idle: 4,099
+// device rays against 20,480 triangles take 36 us a call so, 60 with a memset and two kernels.
+template <bool kAny>
+__global__ void __launch_bounds__(128) k_mesh_few(MeshView m, WideView w, const float* __restrict__ rays,
+                                                  uint64_t stride, uint64_t n, uint32_t* __restrict__ prim,
+                                                  float* __restrict__ tout, uint32_t* __restrict__ obj,
+                                                  uint32_t* __restrict__ err, uint32_t lanes) {
+  const uint32_t lane = threadIdx.x & 31u;
+  if (lane >= lanes) return;
+  const float4 rlo = __ldg(&m.nodes[0]), rhi = __ldg(&m.nodes[1]);
+  const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x / 32u);
+  for (uint64_t i = (blockIdx.x * uint64_t(blockDim.x / 32u) + threadIdx.x / 32u) * lanes + lane; i < n;
+       i += warps * lanes) {
+    const F3 o = mk3(__ldcs(rays + i), __ldcs(rays + stride + i), __ldcs(rays + 2 * stride + i));
+    const F3 d = mk3(__ldcs(rays + 3 * stride + i), __ldcs(rays + 4 * stride + i), __ldcs(rays + 5 * stride + i));
+    const float near = __ldcs(rays + 6 * stride + i), far = __ldcs(rays + 7 * stride + i);
+    const PRay pr = prepare_ray(o, d);
+    uint32_t best = 0xFFFFFFFFu;
+    float t = 0.f, entry;
+    if (box_hit(pr, rlo, rhi, near, far, entry) && (kAny || entry < FLT_MAX)) {
+      const WRay r = wide_ray(o, d, near, w.bounded);
+      Nearest nearest = nothing_yet(far);
+      nearest.lim = kAny ? next_up(far) : fminf(FLT_MAX, next_up(far));
+      bool restart = r.exact;
+      uint32_t cur = w.root, budget = m.node_count;
+      int sp = 0;
+      WideStack stk;
+      while (cur != 0u && !restart) {
+        const float reach = kAny ? nearest.lim : wide_limit(nearest.lim);
+        while (cur != 0u && !(cur & kLeafRef)) {
+          if (budget-- == 0u) {
+            atomicOr(err, kErrBudget);
+            cur = 0u;
+            break;
+          }
+          cur = kAny ? wide_step_any(w.wide + cur, r, near, reach, stk, sp)
+                     : wide_step(w.wide + cur, r, near, reach, stk, sp);
+        }
+        if (cur == 0u) break;
+        uint32_t first, count, id;
+        triangle_range(w, cur, first, count);
+        float e;
+        if (kAny) {
+          if (blocking_triangle(w.tri, w.tri_c, first, count, o, d, near, nearest.lim) &&
+              leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e) && e < nearest.lim) {
+            best = 0u;
+            break;
+          }
+        } else if (nearest_triangle(w.tri, w.tri_c, first, count, o, d, near, reach, t, id) &&
+                   leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e)) {
+          const Verdict v = judge(nearest, t, e);
+          if (v == kAdopt) best = id;
+          restart = v == kRestart;
+        }
+        cur = wide_pop(stk, sp, kAny ? nearest.lim : wide_limit(nearest.lim));
+      }
+      t = nearest.lim;
+      if (restart) {
+        TraceCounters c{0, 0, 0};
+        best = kAny ? (mesh_any(m, pr, near, far, err) ? 0u : 0xFFFFFFFFu)
+                    : mesh_closest<false>(m, pr, near, far, &t, &c, err);
+      }
+    }
+    if (kAny) {
+      reinterpret_cast<uint8_t*>(prim)[i] = best == 0u ? 1 : 0;
+    } else {
+      prim[i] = best;
+      tout[i] = best == 0xFFFFFFFFu ? __int_as_float(0x7f800000) : t;
+      if (obj) obj[i] = best == 0xFFFFFFFFu ? 0xFFFFFFFFu : 0u;
+    }
+  }
+}
+
 // The wide nodes of a tree: one thread per interior node of the binary tree, which writes the
 // wide node of its children's pair (index base + left_first / 2). Half of them are reached (every
 // second level); the others cost memory, not time. A mesh's leaves become triangle references
@@ -630,6 +705,33 @@ cudaError_t launch_mesh_any_persistent(const MeshView& m, const WideView& w, con
   if (e != cudaSuccess) return e;
   return two_stage<true, true>(m, w, rays, stride, n, reinterpret_cast<uint32_t*>(occ), nullptr, nullptr, queue, counters,
                                err, sm_count, s, rec);
+}
+
+// Rays per warp of k_mesh_few: 8 (a 32-byte sector of each plane) while the GPU has room for the
+// warps, more for more rays.
+static uint32_t few_lanes(uint64_t n, int sm_count) {
+  uint32_t lanes = 8;
+  while (lanes < 32 && n > uint64_t(sm_count) * 32u * lanes) lanes *= 2;
+  return lanes;
+}
+template <bool kAny>
+static cudaError_t launch_few(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
+                              uint32_t* prim, float* t, uint32_t* obj, uint32_t* err, int sm_count, cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  const uint32_t lanes = few_lanes(n, sm_count);
+  k_mesh_few<kAny><<<grid_for(n, int(4 * lanes), sm_count), 128, 0, s>>>(m, w, rays, stride, n, prim, t, obj, err, lanes);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mesh_closest_few(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
+                                    uint32_t* prim, float* t, uint32_t* obj, uint32_t* err, int sm_count,
+                                    cudaStream_t s) {
+  return launch_few<false>(m, w, rays, stride, n, prim, t, obj, err, sm_count, s);
+}
+
+cudaError_t launch_mesh_any_few(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
+                                uint8_t* occ, uint32_t* err, int sm_count, cudaStream_t s) {
+  return launch_few<true>(m, w, rays, stride, n, reinterpret_cast<uint32_t*>(occ), nullptr, nullptr, err, sm_count, s);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -151,6 +151,49 @@ def test_occlusion_under_capture_and_on_several_streams():
     assert torch.equal(occ, want[0][1])
 
 
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 33, 4099, (1 << 15) - 1, 1 << 15, (1 << 15) + 1, 1 << 18, (1 << 18) + 1])
+def test_few_and_many_rays(n):
+    """Host and device calls around the sizes where the staging, the rays per warp and the kernels
+    change: the binary query's answers, object ids, and occlusion from the same hits."""
+    for v, f in (_ball(1, 0), _sheets()):
+        base = _rays(v, f, seed=17)
+        r = np.ascontiguousarray(base[:, np.arange(n) % base.shape[1]])
+        s = pb.Scene().add_object(pb.Simple(pb.TriangleMesh(v, f))).commit(bvh_bins=16, bvh_max_leaf=4)
+        bp, bt, _ = s.intersect_instrumented(r)
+        for rays in (r, torch.from_numpy(r).cuda()):
+            p, t, o = [x if isinstance(x, np.ndarray) else x.cpu().numpy() for x in s.intersect(rays, with_object=True)]
+            assert np.array_equal(p.view(np.uint32), bp) and np.array_equal(t, bt)
+            assert np.array_equal(o.view(np.uint32), np.where(bp == pb.PBRT_MISS, pb.PBRT_MISS, 0).astype(np.uint32))
+        occ = oracle.MeshBVH(v, f, np.float32, bins=16, max_leaf=4).occluded(base)[np.arange(n) % base.shape[1]]
+        assert np.array_equal(s.intersect_p(r), occ)
+        assert np.array_equal(s.intersect_p(torch.from_numpy(r).cuda()).cpu().numpy(), occ)
+
+
+def test_survivor_queue_on_several_streams():
+    """Asynchronous calls of more rays than one kernel takes, on changing streams."""
+    v, f = W.displaced_icosphere(5, seed=4)
+    ctx = pb.Context(0)
+    s = pb.Scene(ctx).add_object(pb.Simple(pb.TriangleMesh(v, f))).commit(bvh_bins=16, bvh_max_leaf=4)
+    n = 600_000
+    r = [torch.from_numpy(W.incoherent_rays(n, v.min(0), v.max(0), seed=k)).cuda() for k in (5, 6)]
+    want = [(s.intersect(x), s.intersect_p(x)) for x in r]
+    st = [torch.cuda.Stream() for _ in r]
+    for _ in range(4):
+        got = []
+        for x, q in zip(r, st):
+            ctx.set_stream(q.cuda_stream)
+            prim, t = torch.zeros(n, dtype=torch.int32, device="cuda"), torch.zeros(n, device="cuda")
+            occ = torch.zeros(n, dtype=torch.uint8, device="cuda")
+            q.wait_stream(torch.cuda.current_stream())
+            ctx.check(ctx.lib.pbrt_trace_any(s.h, x.data_ptr(), n, occ.data_ptr()), "any")
+            ctx.check(ctx.lib.pbrt_trace_closest(s.h, x.data_ptr(), n, prim.data_ptr(), t.data_ptr(), None), "closest")
+            got.append((prim, t, occ))
+        torch.cuda.synchronize()
+        for (prim, t, occ), ((p0, t0), o0) in zip(got, want):
+            assert torch.equal(prim, p0) and torch.equal(t, t0) and torch.equal(occ, o0)
+    ctx.set_stream(None)
+
+
 def _mixed_scene():
     """Meshes merged into the wide tree, one placed twice, coplanar sheets in different objects,
     transformed instances, analytic shapes, a compound, a solid and an unbounded plane."""
