@@ -175,16 +175,19 @@ __device__ __forceinline__ void load_smem(uint8_t* dst, const uint16_t* src, uin
 // barrier and 64 TMEM columns, so six tiles' GEMM chains are in flight per SM: while one
 // group waits on its GEMM the others encode, read TMEM or store activations. (Three CTAs of
 // one tile each, every CTA with its own copy of the weights, was the shared-memory limit.)
-constexpr int kInferGroups = 6;  // 7 (72 registers, spills) measured 4 % slower
+// A group's chain is what the kernel waits for: each thread waits for a GEMM on its own, and the
+// one barrier between two layers is the one that the stored activations need, which also carries
+// whether every wait succeeded. 2,000,003 records through the C call: 196 us with a barrier after
+// each wait and one after each store, 146 us so (the tensor pipe is busy a third of it); 159 us
+// when one lane of a warp waits for all, 150 us with seven groups, 154 us with 32-column TMEM
+// loads, which spill.
+constexpr int kInferGroups = 6;
 constexpr int kInferThreads = kInferGroups * kTile;  // 768
 constexpr uint32_t kInferTmemCols = 512;             // 6 x 64 columns, rounded up to a power of two
 static_assert(kInferGroups * kTmemCols <= kInferTmemCols, "the groups' accumulators must fit the allocation");
 
-// Named barrier g + 1 over the 128 threads of tile group g (barrier 0 is __syncthreads).
-__device__ __forceinline__ void group_sync(uint32_t g) {
-  asm volatile("bar.sync %0, %1;" ::"r"(g + 1u), "r"(uint32_t(kTile)) : "memory");
-}
-// The same barrier, returning whether `v` holds in every thread of the group.
+// Named barrier g + 1 over the 128 threads of tile group g (barrier 0 is __syncthreads),
+// returning whether `v` holds in every thread of the group.
 __device__ __forceinline__ bool group_and(uint32_t g, bool v) {
   uint32_t r;
   asm volatile(
@@ -222,7 +225,7 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(Net net, Bounds 
   const uint32_t tmem = *tslot + g * kTmemCols;                // this group's 64 columns
   const uint32_t lane_base = ((threadIdx.x >> 5) & 3u) * 32u;  // this warp's TMEM lanes = rows
   uint32_t phase = 0;
-  bool ok = true;
+  bool ok = true, late = false;  // late: a wait of this warp ran out
   const uint64_t tiles = (n + kTile - 1) / kTile;
   const uint64_t tile_step = uint64_t(gridDim.x) * kInferGroups;
   // A row's record, loaded one tile ahead: the next tile's loads are in flight while this
@@ -241,7 +244,7 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(Net net, Bounds 
   };
   float4 n0, n1, n2, n3;
   load_record(uint64_t(blockIdx.x) * kInferGroups + g, n0, n1, n2, n3);
-  for (uint64_t tile = uint64_t(blockIdx.x) * kInferGroups + g; tile < tiles && ok; tile += tile_step) {
+  for (uint64_t tile = uint64_t(blockIdx.x) * kInferGroups + g; tile < tiles; tile += tile_step) {
     const uint64_t row = tile * kTile + r;
     {
       const float4 q0 = n0, q1 = n1, q2 = n2, q3 = n3;
@@ -253,53 +256,62 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(Net net, Bounds 
       encode_rest(sX, r, q0, q1, q2, q3);
     }
     tc::fence_smem_to_async();
-    group_sync(g);
-    for (int l = 0; l < kLayers && ok; ++l) {
-      if (r == 0) {
-        tc::fence_after_sync();
-        issue_gemm(sX, sW + 2 * layer_off(l), uint32_t(layer_n(l)), uint32_t(layer_k(l)), tmem, mbar);
-      }
-      ok = group_and(g, tc::mbar_wait(mbar, phase));
-      if (!ok) {
-        if (r == 0) atomicOr(err, kErrMma);
-        break;
-      }
-      phase ^= 1u;
+    tc::fence_before_sync();  // the previous tile's outputs have been read
+    ok = group_and(g, ok);
+    if (!ok) break;
+    if (r == 0) {
       tc::fence_after_sync();
-      if (l < kLayers - 1) {
+      issue_gemm(sX, sW, uint32_t(layer_n(0)), uint32_t(layer_k(0)), tmem, mbar);
+    }
 #pragma unroll
-        for (int c = 0; c < 64; c += 16) {
-          float v[16];
-          tc::tmem_ld16(tmem + (lane_base << 16) + uint32_t(c), v);
-          uint4 lo, hi;
-          lo.x = pack2_relu(v[0], v[1]);
-          lo.y = pack2_relu(v[2], v[3]);
-          lo.z = pack2_relu(v[4], v[5]);
-          lo.w = pack2_relu(v[6], v[7]);
-          hi.x = pack2_relu(v[8], v[9]);
-          hi.y = pack2_relu(v[10], v[11]);
-          hi.z = pack2_relu(v[12], v[13]);
-          hi.w = pack2_relu(v[14], v[15]);
-          *reinterpret_cast<uint4*>(sX + tc::tile_offset(r, uint32_t(c), kTile)) = lo;
-          *reinterpret_cast<uint4*>(sX + tc::tile_offset(r, uint32_t(c + 8), kTile)) = hi;
-        }
-        tc::fence_before_sync();
-        tc::fence_smem_to_async();
-        group_sync(g);
+    for (int l = 0; l < kLayers; ++l) {
+      if (!ok) break;
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(mbar, phase));  // the TMEM loads want whole warps
+      if (ok) {
+        phase ^= 1u;
+        tc::fence_after_sync();
       } else {
-        float v[16];
-        tc::tmem_ld16(tmem + (lane_base << 16), v);
-        if (row < n) {
-          out[3 * row] = v[0];
-          out[3 * row + 1] = v[1];
-          out[3 * row + 2] = v[2];
+        late = true;
+        atomicOr(err, kErrMma);
+      }
+      if (l < kLayers - 1) {
+        if (ok) {
+#pragma unroll
+          for (int c = 0; c < 64; c += 16) {
+            float v[16];
+            tc::tmem_ld16(tmem + (lane_base << 16) + uint32_t(c), v);
+#pragma unroll
+            for (int k = 0; k < 16; k += 8) {
+              uint4 q;
+              q.x = pack2_relu(v[k], v[k + 1]);
+              q.y = pack2_relu(v[k + 2], v[k + 3]);
+              q.z = pack2_relu(v[k + 4], v[k + 5]);
+              q.w = pack2_relu(v[k + 6], v[k + 7]);
+              *reinterpret_cast<uint4*>(sX + tc::tile_offset(r, uint32_t(c + k), kTile)) = q;
+            }
+          }
+          tc::fence_before_sync();
+          tc::fence_smem_to_async();
         }
-        tc::fence_before_sync();
-        group_sync(g);
+        ok = group_and(g, ok);
+        if (ok && r == 0) {
+          tc::fence_after_sync();
+          issue_gemm(sX, sW + 2 * layer_off(l + 1), uint32_t(layer_n(l + 1)), uint32_t(layer_k(l + 1)), tmem, mbar);
+        }
+      } else {
+        if (ok) {
+          float v[16];
+          tc::tmem_ld16(tmem + (lane_base << 16), v);
+          if (row < n) {
+            out[3 * row] = v[0];
+            out[3 * row + 1] = v[1];
+            out[3 * row + 2] = v[2];
+          }
+        }
       }
     }
   }
-  if (!ok) tc::mbar_wait(mbar, phase, 1u << 20);  // one more bounded wait for a GEMM still in flight
+  if (late) tc::mbar_wait(mbar, phase, 1u << 20);  // one more bounded wait for the GEMM still in flight
   tc::fence_before_sync();
   __syncthreads();
   if (threadIdx.x < 32) tc::tmem_dealloc(*tslot, kInferTmemCols);
@@ -376,11 +388,11 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_mlp_grad(Net net, Bounds b,
   const uint32_t warp = (threadIdx.x >> 5) & 3u, lane = threadIdx.x & 31u;
   const uint32_t quarter = (warp * 32u) << 16;  // this warp's TMEM lanes
   auto act = [&](int l) -> uint8_t* { return l == 0 ? sX : sA + (l - 1) * kHBytes; };
-  // A wait that runs out sets the error bit and clears `ok`, which every barrier below makes
-  // the block's: nobody issues or reads anything after that.
+  // A wait that runs out sets the error bit and clears the warp's `ok` (TMEM loads want whole
+  // warps), which every barrier below makes the block's: nobody issues or reads anything then.
   auto await = [&](uint64_t* bar, uint32_t parity, uint32_t bit) {
-    if (tc::mbar_wait(bar, parity)) return true;
-    if (r == 0) atomicOr(err, bit);
+    if (__all_sync(0xffffffffu, tc::mbar_wait(bar, parity))) return true;
+    if (lane == 0) atomicOr(err, bit);
     return false;
   };
   uint32_t phase = 0;
@@ -482,6 +494,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_mlp_grad(Net net, Bounds b,
       }
       ok = __syncthreads_and(ok);
       if (ok && threadIdx.x == 0) issue_layer(l - 1);
+      __syncwarp();
     }
     if (ok) {
       // M = 64 accumulator: lanes 0-15 of the quarter q hold rows 16q .. 16q + 15
