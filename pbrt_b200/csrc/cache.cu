@@ -46,26 +46,41 @@ std::vector<float> initial_weights(uint64_t seed) {
 
 }  // namespace
 
+// Memory comes from the context's pool, as a scene's does: a cached frame's query buffers are
+// hundreds of megabytes, and a new cache whose first frame maps them anew waits for that. The
+// pointer is good on every stream once this returns.
+int pbrt_cache::take_bytes(void** p, size_t bytes) {
+  PBRT_TRY(ctx->cuda(cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream), "cudaMalloc(cache)"));
+  return ctx->cuda(cudaStreamSynchronize(ctx->stream), "cudaMalloc(cache)");
+}
+
+// After every stream's work: freeing pool memory waits for nobody.
+void pbrt_cache::give_back(std::initializer_list<void*> blocks) {
+  bool any = false;
+  for (void* p : blocks) any |= p != nullptr;
+  if (any) cudaDeviceSynchronize();
+  for (void* p : blocks) cudaFree(p);
+}
+
 int pbrt_cache::device_arrays() {
   const size_t P = mlp::kParams;
-  PBRT_TRY(ctx->cuda(cudaMalloc(&w, P * 4), "cudaMalloc(cache)"));
-  PBRT_TRY(ctx->cuda(cudaMalloc(&m, P * 4), "cudaMalloc(cache)"));
-  PBRT_TRY(ctx->cuda(cudaMalloc(&v, P * 4), "cudaMalloc(cache)"));
-  PBRT_TRY(ctx->cuda(cudaMalloc(&grad, P * 4), "cudaMalloc(cache)"));
-  PBRT_TRY(ctx->cuda(cudaMalloc(&wfwd, P * 2), "cudaMalloc(cache)"));
-  PBRT_TRY(ctx->cuda(cudaMalloc(&wbwd, P * 2), "cudaMalloc(cache)"));
+  PBRT_TRY(take(&w, P * 4));
+  PBRT_TRY(take(&m, P * 4));
+  PBRT_TRY(take(&v, P * 4));
+  PBRT_TRY(take(&grad, P * 4));
+  PBRT_TRY(take(&wfwd, P * 2));
+  PBRT_TRY(take(&wbwd, P * 2));
   // pinned host memory: the gradient's last kernel writes the loss where the caller reads it
   return ctx->cuda(cudaHostAlloc(&loss, 4, cudaHostAllocMapped), "cudaHostAlloc(cache)");
 }
 
 int pbrt_cache::ensure_tiles(uint32_t tiles) {
   if (tiles <= tile_cap) return PBRT_OK;
-  cudaFree(partials);
-  cudaFree(tile_loss);
+  give_back({partials, tile_loss});
   partials = nullptr;
   tile_loss = nullptr;
-  PBRT_TRY(ctx->cuda(cudaMalloc(&partials, size_t(tiles) * mlp::kParams * 4), "cudaMalloc(cache gradients)"));
-  PBRT_TRY(ctx->cuda(cudaMalloc(&tile_loss, size_t(tiles) * 4), "cudaMalloc(cache gradients)"));
+  PBRT_TRY(take(&partials, size_t(tiles) * mlp::kParams * 4));
+  PBRT_TRY(take(&tile_loss, size_t(tiles) * 4));
   tile_cap = tiles;
   return PBRT_OK;
 }
@@ -123,7 +138,7 @@ int pbrt_cache::ensure_render_buffers(uint32_t queries, uint32_t train_vertices,
   queries = std::max(queries, qcap);
   train_vertices = std::max(train_vertices, cw.tcap);
   batch = std::max(batch, bcap);
-  cudaFree(render_block);
+  give_back({render_block});
   render_block = nullptr;
   qcap = bcap = 0;
   cw = pbrt::CacheWave{};
@@ -132,20 +147,20 @@ int pbrt_cache::ensure_render_buffers(uint32_t queries, uint32_t train_vertices,
   const size_t bytes = up(64) + up(size_t(queries) * R) + up(size_t(queries) * 12) + up(size_t(queries) * 4) +
                        up(size_t(train_vertices) * R) + up(size_t(train_vertices) * 24) +
                        up(size_t(train_vertices) * 4) + up(size_t(batch) * R) + up(size_t(batch) * 12);
-  PBRT_TRY(ctx->cuda(cudaMalloc(&render_block, bytes), "cudaMalloc(cache render buffers)"));
+  PBRT_TRY(take(&render_block, bytes));
   char* p = static_cast<char*>(render_block);
-  auto take = [&](size_t b) { char* r = p; p += up(b); return r; };
-  cw.counts = reinterpret_cast<uint32_t*>(take(64));
-  cw.qrec = reinterpret_cast<float*>(take(size_t(queries) * R));
-  cw.qout = reinterpret_cast<float*>(take(size_t(queries) * 12));
-  cw.qpath = reinterpret_cast<uint32_t*>(take(size_t(queries) * 4));
-  cw.trec = reinterpret_cast<float*>(take(size_t(train_vertices) * R));
-  cw.tstate = reinterpret_cast<float*>(take(size_t(train_vertices) * 24));
-  cw.tpath = reinterpret_cast<uint32_t*>(take(size_t(train_vertices) * 4));
+  auto part = [&](size_t b) { char* r = p; p += up(b); return r; };
+  cw.counts = reinterpret_cast<uint32_t*>(part(64));
+  cw.qrec = reinterpret_cast<float*>(part(size_t(queries) * R));
+  cw.qout = reinterpret_cast<float*>(part(size_t(queries) * 12));
+  cw.qpath = reinterpret_cast<uint32_t*>(part(size_t(queries) * 4));
+  cw.trec = reinterpret_cast<float*>(part(size_t(train_vertices) * R));
+  cw.tstate = reinterpret_cast<float*>(part(size_t(train_vertices) * 24));
+  cw.tpath = reinterpret_cast<uint32_t*>(part(size_t(train_vertices) * 4));
   cw.tcap = train_vertices;
   cw.qcap = queries;
-  brec = reinterpret_cast<float*>(take(size_t(batch) * R));
-  btgt = reinterpret_cast<float*>(take(size_t(batch) * 12));
+  brec = reinterpret_cast<float*>(part(size_t(batch) * R));
+  btgt = reinterpret_cast<float*>(part(size_t(batch) * 12));
   qcap = queries;
   bcap = batch;
   return PBRT_OK;
@@ -153,7 +168,7 @@ int pbrt_cache::ensure_render_buffers(uint32_t queries, uint32_t train_vertices,
 
 int pbrt_cache::ensure_frame_buffers(uint32_t queries) {
   if (frame_block && fqcap >= queries) return PBRT_OK;
-  cudaFree(frame_block);
+  give_back({frame_block});
   frame_block = nullptr;
   fqcap = 0;
   fcw = pbrt::CacheWave{};
@@ -161,15 +176,15 @@ int pbrt_cache::ensure_frame_buffers(uint32_t queries) {
   auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
   const size_t bytes =
       up(64) + up(size_t(queries) * R) + up(size_t(queries) * 12) + up(size_t(queries) * 4) + up(mlp::kParams * 2);
-  PBRT_TRY(ctx->cuda(cudaMalloc(&frame_block, bytes), "cudaMalloc(cache frame buffers)"));
+  PBRT_TRY(take(&frame_block, bytes));
   char* p = static_cast<char*>(frame_block);
-  auto take = [&](size_t b) { char* r = p; p += up(b); return r; };
-  fcw.counts = reinterpret_cast<uint32_t*>(take(64));
-  fcw.qrec = reinterpret_cast<float*>(take(size_t(queries) * R));
-  fcw.qout = reinterpret_cast<float*>(take(size_t(queries) * 12));
-  fcw.qpath = reinterpret_cast<uint32_t*>(take(size_t(queries) * 4));
+  auto part = [&](size_t b) { char* r = p; p += up(b); return r; };
+  fcw.counts = reinterpret_cast<uint32_t*>(part(64));
+  fcw.qrec = reinterpret_cast<float*>(part(size_t(queries) * R));
+  fcw.qout = reinterpret_cast<float*>(part(size_t(queries) * 12));
+  fcw.qpath = reinterpret_cast<uint32_t*>(part(size_t(queries) * 4));
   fcw.qcap = queries;  // no training vertices: the frame only queries
-  wsnap = reinterpret_cast<uint16_t*>(take(mlp::kParams * 2));
+  wsnap = reinterpret_cast<uint16_t*>(part(mlp::kParams * 2));
   fqcap = queries;
   return PBRT_OK;
 }
@@ -177,7 +192,7 @@ int pbrt_cache::ensure_frame_buffers(uint32_t queries) {
 int pbrt_cache::ensure_branch_buffers(uint32_t slot, uint32_t queries) {
   if (slot >= kBranchSlots) return ctx->fail(PBRT_ERR_INVALID_ARGUMENT, "no such frame branch");
   if (branch_block[slot] && branch_qcap[slot] >= queries) return PBRT_OK;
-  cudaFree(branch_block[slot]);
+  give_back({branch_block[slot]});
   branch_block[slot] = nullptr;
   branch_qcap[slot] = 0;
   pbrt::CacheWave& q = bcw[slot];
@@ -185,24 +200,22 @@ int pbrt_cache::ensure_branch_buffers(uint32_t slot, uint32_t queries) {
   const size_t R = pbrt::kCacheRecordFloats * 4;
   auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
   const size_t bytes = up(64) + up(size_t(queries) * R) + up(size_t(queries) * 12) + up(size_t(queries) * 4);
-  PBRT_TRY(ctx->cuda(cudaMalloc(&branch_block[slot], bytes), "cudaMalloc(cache branch buffers)"));
+  PBRT_TRY(take(&branch_block[slot], bytes));
   char* p = static_cast<char*>(branch_block[slot]);
-  auto take = [&](size_t b) { char* r = p; p += up(b); return r; };
-  q.counts = reinterpret_cast<uint32_t*>(take(64));
-  q.qrec = reinterpret_cast<float*>(take(size_t(queries) * R));
-  q.qout = reinterpret_cast<float*>(take(size_t(queries) * 12));
-  q.qpath = reinterpret_cast<uint32_t*>(take(size_t(queries) * 4));
+  auto part = [&](size_t b) { char* r = p; p += up(b); return r; };
+  q.counts = reinterpret_cast<uint32_t*>(part(64));
+  q.qrec = reinterpret_cast<float*>(part(size_t(queries) * R));
+  q.qout = reinterpret_cast<float*>(part(size_t(queries) * 12));
+  q.qpath = reinterpret_cast<uint32_t*>(part(size_t(queries) * 4));
   q.qcap = queries;  // queries only, like the frame's own buffers
   branch_qcap[slot] = queries;
   return PBRT_OK;
 }
 
 void pbrt_cache::release() {
-  for (void* p : {(void*)w, (void*)m, (void*)v, (void*)grad, (void*)wfwd, (void*)wbwd, (void*)partials, (void*)tile_loss,
-                  render_block, frame_block})
-    cudaFree(p);
+  give_back({w, m, v, grad, wfwd, wbwd, partials, tile_loss, render_block, frame_block});
+  for (void* p : branch_block) give_back({p});
   cudaFreeHost(loss);
-  for (void* p : branch_block) cudaFree(p);
 }
 
 namespace {

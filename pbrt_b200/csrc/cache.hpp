@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <initializer_list>
 #include <vector>
 
 #include "../../include/pbrt_b200.h"
@@ -42,6 +43,12 @@ struct pbrt_cache {
   pbrt::CacheWave bcw[kBranchSlots] = {};
   int ensure_branch_buffers(uint32_t slot, uint32_t queries);
 
+  int take_bytes(void** p, size_t bytes);
+  template <class T>
+  int take(T** p, size_t bytes) {
+    return take_bytes(reinterpret_cast<void**>(p), bytes);
+  }
+  void give_back(std::initializer_list<void*> blocks);
   int device_arrays();
   int ensure_tiles(uint32_t tiles);
   int reset();
