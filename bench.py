@@ -172,14 +172,14 @@ def _per_kernel(launch_ms: float, n_rays: int, box_pr: float, tri_pr: float, pea
     of the captured pass (ncu times are serialised and cold, so only their ratio is used).
     The cull (k_cull_root_bulk, or k_cull_root) streams rays: its figure is its captured DRAM
     bytes over that time.
-    k_mesh_closest_persistent walks the survivors: its algorithmic bytes are the node and
+    k_mesh_walk walks the survivors: its algorithmic bytes are the node and
     triangle fetches beyond the root test, 32 (box tests - 1) + 36 triangle tests per ray."""
     d = _kernel_profile()
     if not d:
         return None
     k = d["kernels"]
     cull_name = "k_cull_root_bulk" if "k_cull_root_bulk" in k else "k_cull_root"
-    cull, trav = k[cull_name], k["k_mesh_closest_persistent"]
+    cull, trav = k[cull_name], k["k_mesh_walk"]
     total_ns = float(cull["ns"] + trav["ns"])
     scale = n_rays / float(d["rays_per_launch"])
     cull_ms, trav_ms = launch_ms * cull["ns"] / total_ns, launch_ms * trav["ns"] / total_ns
@@ -190,12 +190,11 @@ def _per_kernel(launch_ms: float, n_rays: int, box_pr: float, tri_pr: float, pea
         cull_name: {"share": round(cull["ns"] / total_ns, 4), "ms": round(cull_ms, 4),
                         "dram_gbs": round(cull_gbs, 1), "frac": round(cull_gbs / peak, 4),
                         "limiter": "HBM: streams the 32-byte rays and writes every answer"},
-        "k_mesh_closest_persistent": {"share": round(trav["ns"] / total_ns, 4), "ms": round(trav_ms, 4),
+        "k_mesh_walk": {"share": round(trav["ns"] / total_ns, 4), "ms": round(trav_ms, 4),
                                       "algorithmic_bytes_per_ray": round(trav_bytes / n_rays, 2),
                                       "achieved_gbs": round(trav_gbs, 1), "frac": round(trav_gbs / peak, 4),
-                                      "limiter": "instruction issue and latency: 10.0 of 32 lanes active per warp "
-                                                 "instruction, 63 % issue active, 3 % of DRAM throughput; node "
-                                                 "and triangle reads are mostly L1/L2 hits"},
+                                      "limiter": "instruction issue and the latency of node loads; node and triangle "
+                                                 "reads are mostly L1/L2 hits"},
         "shares_from": "profiles/k_mesh_closest_raycast.json (ncu, full-size pass)",
     }
 
@@ -999,7 +998,7 @@ def main():
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "traffic": round(traffic) if traffic else None,
                          "peak_kind": peak_kind,
-                         "kernel": "the nearest-hit pass: k_cull_root + k_mesh_closest_persistent (one "
+                         "kernel": "the nearest-hit pass: k_cull_root + k_mesh_walk (one "
                                    "pbrt_trace_closest call, timed as a whole)",
                          "algorithmic_bytes_per_ray": round(bytes_per_ray, 2), "box_tests_per_ray": round(box_pr, 4),
                          "triangle_tests_per_ray": round(tri_pr, 4), "avg_launch_ms": round(launch_ms, 4),
