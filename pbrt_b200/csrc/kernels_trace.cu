@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kCullThreads) k_cull_root_bulk(MeshView m, con
 // order, so ids and t are unchanged.
 // kRec: the survivors' rays come from the records stage 1 wrote beside the queue. kAny: the
 // first triangle hit ends a ray, `prim` holds the occlusion bytes. Rays outside the grid's
-// arithmetic, and those whose answer could depend on the order (judge), walk m's binary nodes.
+// arithmetic, and those whose answer could depend on the order (weigh), walk m's binary nodes.
 template <bool kRec, bool kAny>
 __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
     MeshView m, WideView w, const float* __restrict__ rays, uint64_t stride, const uint32_t* __restrict__ queue,
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
                    leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e) && e < nearest.lim;
           } else if (nearest_triangle(w.tri, w.tri_c, first, count, r.o, r.d, near, wide_limit(nearest.lim), t, id) &&
                      leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e)) {
-            const Verdict v = judge(nearest, t, e);
+            const Verdict v = weigh(nearest, t, e);
             if (v == kAdopt) best = id;
             restart = v == kRestart;
           }
@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(128) k_mesh_few(MeshView m, WideView w, const 
           }
         } else if (nearest_triangle(w.tri, w.tri_c, first, count, o, d, near, reach, t, id) &&
                    leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e)) {
-          const Verdict v = judge(nearest, t, e);
+          const Verdict v = weigh(nearest, t, e);
           if (v == kAdopt) best = id;
           restart = v == kRestart;
         }

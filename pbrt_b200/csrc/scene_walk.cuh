@@ -161,7 +161,7 @@ PBRT_DEV void walk_nearest(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err
         }
         float e;
         if (node && leaf_hit(node, r, near, e)) {
-          const Verdict v = judge(best, t, e);
+          const Verdict v = weigh(best, t, e);
           restart = v == kRestart;
           if (v == kAdopt) {
             leaf = lf;
@@ -327,7 +327,7 @@ PBRT_DEV bool nearest_in_leaf(const SceneView& s, float near, NearestLane& l, ui
   }
   float e;
   if (!node || !leaf_hit(node, l.r, near, e)) return false;
-  const Verdict v = judge(l.best, t, e);
+  const Verdict v = weigh(l.best, t, e);
   if (v == kAdopt) {
     l.leaf = lf;
     l.prim = pr;

@@ -270,7 +270,7 @@ PBRT_DEV Nearest nothing_yet(float far) { return Nearest{next_up(far), __int_as_
 enum Verdict : int { kIgnore = 0, kAdopt = 1, kRestart = 2 };
 
 // A candidate t of a leaf that is exactly hit with entry e.
-PBRT_DEV Verdict judge(Nearest& n, float t, float e) {
+PBRT_DEV Verdict weigh(Nearest& n, float t, float e) {
   if (!(t < n.lim)) return n.have && t <= fmaxf(n.lim, n.window) ? kRestart : kIgnore;
   if (!((n.have ? e : next_up(e)) < n.lim) || e > wide_limit(t)) return kRestart;
   n.lim = t;
