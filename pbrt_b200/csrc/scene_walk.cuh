@@ -88,6 +88,60 @@ __device__ __noinline__ bool exact_any(const SceneView& s, F3 o, F3 d, float nea
   return scene_any<kCsg>(s, o, d, near, far, err);
 }
 
+// ---- a leaf ---------------------------------------------------------------------------------------
+// The nearest hit of the leaf `cur`, weighed against the best so far. True: the ray must be answered
+// by the exact query. An object is asked up to the nearest distance and a little more (wide_limit),
+// but never beyond the ray's own end: an exit at exactly that distance is no hit (sphere_hit's and
+// the other shapes' last comparison is strict).
+template <bool kObj, bool kCsg, class Job>
+PBRT_DEV bool nearest_in_leaf(const Job& job, const SceneView& s, const WRay& r, float near, uint32_t cur,
+                              Nearest& best, uint32_t& leaf, uint32_t& prim, uint32_t* err) {
+  const float reach = wide_limit(best.lim);
+  float t;
+  uint32_t lf = 0, pr = 0;
+  const float4* node = nullptr;
+  if (kObj && (cur & kObjectRef)) {
+    const uint32_t slot = cur & 0x3FFFFFFFu;
+    if (prim_closest<kCsg>(s, __ldg(&s.order[slot]), r.o, r.d, near, fminf(reach, job.far()), t, lf, pr, err))
+      node = s.top + 2 * size_t(__ldg(&s.wide.slot_node[slot]));
+  } else {
+    uint32_t first, count;
+    triangle_range(s.wide, cur, first, count);
+    if (nearest_triangle(s.wide.tri, s.wide.tri_c, first, count, r.o, r.d, near, reach, t, pr)) {
+      const uint2 info = __ldg(&s.wide.leaf[first]);
+      node = s.wide.nodes + 2 * size_t(info.x);
+      lf = info.y;
+    }
+  }
+  float e;
+  if (!node || !leaf_hit(node, r, near, e)) return false;
+  const Verdict v = weigh(best, t, e);
+  if (v == kAdopt) {
+    leaf = lf;
+    prim = pr;
+  }
+  return v == kRestart;
+}
+
+// Whether the leaf `cur` blocks the ray (lim: just above its far end).
+template <bool kObj, bool kCsg, class Job>
+PBRT_DEV bool blocked_in_leaf(const Job& job, const SceneView& s, const WRay& r, float near, float lim, uint32_t cur,
+                              uint32_t* err) {
+  const float4* node = nullptr;
+  if (kObj && (cur & kObjectRef)) {
+    const uint32_t slot = cur & 0x3FFFFFFFu;
+    if (prim_any<kCsg>(s, __ldg(&s.order[slot]), r.o, r.d, near, job.far(), err))
+      node = s.top + 2 * size_t(__ldg(&s.wide.slot_node[slot]));
+  } else {
+    uint32_t first, count;
+    triangle_range(s.wide, cur, first, count);
+    if (blocking_triangle(s.wide.tri, s.wide.tri_c, first, count, r.o, r.d, near, lim))
+      node = s.wide.nodes + 2 * size_t(__ldg(&s.wide.leaf[first]).x);
+  }
+  float e;
+  return node && leaf_hit(node, r, near, e) && e < lim;
+}
+
 // ---- many rays: persistent warps ----------------------------------------------------------------
 // kObj: some primitive of some scene is not a mesh merged into its wide tree (kCsg: or is a
 // constructive solid).
@@ -142,32 +196,7 @@ PBRT_DEV void walk_nearest(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err
       const float near = job.near();
       bool restart = r.exact;
       if (leaf_step && at_leaf && !restart) {
-        const float reach = wide_limit(best.lim);
-        float t;
-        uint32_t lf = 0, pr = 0;
-        const float4* node = nullptr;
-        if (kObj && (cur & kObjectRef)) {
-          const uint32_t slot = cur & 0x3FFFFFFFu;
-          if (prim_closest<kCsg>(s, __ldg(&s.order[slot]), r.o, r.d, near, reach, t, lf, pr, err))
-            node = s.top + 2 * size_t(__ldg(&s.wide.slot_node[slot]));
-        } else {
-          uint32_t first, count;
-          triangle_range(s.wide, cur, first, count);
-          if (nearest_triangle(s.wide.tri, s.wide.tri_c, first, count, r.o, r.d, near, reach, t, pr)) {
-            const uint2 info = __ldg(&s.wide.leaf[first]);
-            node = s.wide.nodes + 2 * size_t(info.x);
-            lf = info.y;
-          }
-        }
-        float e;
-        if (node && leaf_hit(node, r, near, e)) {
-          const Verdict v = weigh(best, t, e);
-          restart = v == kRestart;
-          if (v == kAdopt) {
-            leaf = lf;
-            prim = pr;
-          }
-        }
+        restart = nearest_in_leaf<kObj, kCsg>(job, s, r, near, cur, best, leaf, prim, err);
         cur = wide_pop(stk, sp, wide_limit(best.lim));
       }
       if (!leaf_step || q.drained) {
@@ -239,19 +268,7 @@ PBRT_DEV void walk_any(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err) {
         hit = exact_any<Job, kObj, kCsg, false>(s, r.o, r.d, near, job.far(), err);
         cur = 0u;
       } else if (leaf_step && at_leaf) {
-        const float4* node = nullptr;
-        if (kObj && (cur & kObjectRef)) {
-          const uint32_t slot = cur & 0x3FFFFFFFu;
-          if (prim_any<kCsg>(s, __ldg(&s.order[slot]), r.o, r.d, near, job.far(), err))
-            node = s.top + 2 * size_t(__ldg(&s.wide.slot_node[slot]));
-        } else {
-          uint32_t first, count;
-          triangle_range(s.wide, cur, first, count);
-          if (blocking_triangle(s.wide.tri, s.wide.tri_c, first, count, r.o, r.d, near, lim))
-            node = s.wide.nodes + 2 * size_t(__ldg(&s.wide.leaf[first]).x);
-        }
-        float e;
-        hit = node && leaf_hit(node, r, near, e) && e < lim;
+        hit = blocked_in_leaf<kObj, kCsg>(job, s, r, near, lim, cur, err);
         cur = hit ? 0u : wide_pop(stk, sp, lim);
       }
       if (!leaf_step || q.drained) {
@@ -272,168 +289,71 @@ PBRT_DEV void walk_any(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err) {
 }
 
 // ---- one thread per ray -------------------------------------------------------------------------
-// For scenes of a few wide nodes: their walks are too short for the votes and refills to pay.
-struct NearestLane {
-  WRay r;
-  Nearest best;
-  uint32_t leaf, prim, cur;
-  int sp;
-};
-
-template <bool kObj, bool kCsg, class Job>
-PBRT_DEV void start_nearest(Job& job, uint64_t k, NearestLane& l, uint32_t* err) {
-  F3 o, d;
-  job.load(k, o, d);
-  const SceneView& s = job.scene();
-  const float near = job.near(), far = job.far();
-  l.r = wide_ray(o, d, near, s.wide.bounded);
-  l.best = nothing_yet(far);
-  if (kObj && !l.r.exact) {
-    for (uint32_t u = 0; u < s.unbounded_count; ++u) {  // nearest_among + closer (scene.rs:222-249)
-      float t;
-      uint32_t lf, pr;
-      if (prim_closest<kCsg>(s, __ldg(&s.unbounded[u]), o, d, near, far, t, lf, pr, err) &&
-          (!l.best.have || t < l.best.lim)) {
-        l.best.have = true;
-        l.best.lim = t;
-        l.leaf = lf;
-        l.prim = pr;
-      }
-    }
-  }
-  l.cur = s.wide.root;
-  l.sp = 0;
-}
-
-// The leaf the lane stands on. True: the ray must be answered by the exact query.
-template <bool kObj, bool kCsg>
-PBRT_DEV bool nearest_in_leaf(const SceneView& s, float near, NearestLane& l, uint32_t* err) {
-  const float reach = wide_limit(l.best.lim);
-  float t;
-  uint32_t lf = 0, pr = 0;
-  const float4* node = nullptr;
-  if (kObj && (l.cur & kObjectRef)) {
-    const uint32_t slot = l.cur & 0x3FFFFFFFu;
-    if (prim_closest<kCsg>(s, __ldg(&s.order[slot]), l.r.o, l.r.d, near, reach, t, lf, pr, err))
-      node = s.top + 2 * size_t(__ldg(&s.wide.slot_node[slot]));
-  } else {
-    uint32_t first, count;
-    triangle_range(s.wide, l.cur, first, count);
-    if (nearest_triangle(s.wide.tri, s.wide.tri_c, first, count, l.r.o, l.r.d, near, reach, t, pr)) {
-      const uint2 info = __ldg(&s.wide.leaf[first]);
-      node = s.wide.nodes + 2 * size_t(info.x);
-      lf = info.y;
-    }
-  }
-  float e;
-  if (!node || !leaf_hit(node, l.r, near, e)) return false;
-  const Verdict v = weigh(l.best, t, e);
-  if (v == kAdopt) {
-    l.leaf = lf;
-    l.prim = pr;
-  }
-  return v == kRestart;
-}
-
-struct AnyLane {
-  WRay r;
-  float lim;  // a hit lies below it: just above far
-  uint32_t cur;
-  int sp;
-};
-
-// False: blocked by an unbounded primitive.
-template <bool kObj, bool kCsg, class Job>
-PBRT_DEV bool start_any(Job& job, uint64_t k, AnyLane& l, uint32_t* err) {
-  F3 o, d;
-  job.load(k, o, d);
-  const SceneView& s = job.scene();
-  const float near = job.near(), far = job.far();
-  l.r = wide_ray(o, d, near, s.wide.bounded);
-  l.lim = next_up(far);
-  l.cur = s.wide.root;
-  l.sp = 0;
-  if (kObj && !l.r.exact)
-    for (uint32_t u = 0; u < s.unbounded_count; ++u)  // any_blocks (scene.rs:170-184)
-      if (prim_any<kCsg>(s, __ldg(&s.unbounded[u]), o, d, near, far, err)) return false;
-  return true;
-}
-
-// Whether the leaf the lane stands on blocks its ray.
-template <bool kObj, bool kCsg>
-PBRT_DEV bool blocked_in_leaf(const SceneView& s, float near, float far, AnyLane& l, uint32_t* err) {
-  const float4* node = nullptr;
-  if (kObj && (l.cur & kObjectRef)) {
-    const uint32_t slot = l.cur & 0x3FFFFFFFu;
-    if (prim_any<kCsg>(s, __ldg(&s.order[slot]), l.r.o, l.r.d, near, far, err))
-      node = s.top + 2 * size_t(__ldg(&s.wide.slot_node[slot]));
-  } else {
-    uint32_t first, count;
-    triangle_range(s.wide, l.cur, first, count);
-    if (blocking_triangle(s.wide.tri, s.wide.tri_c, first, count, l.r.o, l.r.d, near, l.lim))
-      node = s.wide.nodes + 2 * size_t(__ldg(&s.wide.leaf[first]).x);
-  }
-  float e;
-  return node && leaf_hit(node, l.r, near, e) && e < l.lim;
-}
-
-template <bool kObj, bool kCsg, class Job>
+// For scenes of a few wide nodes, merged meshes only: their walks are too short for the votes and
+// refills to pay.
+template <class Job>
 PBRT_DEV void each_nearest(Job& job, uint64_t n, uint32_t* err) {
   for (uint64_t k = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; k < n; k += uint64_t(gridDim.x) * blockDim.x) {
-    NearestLane l{};
-    WideStack stk;
-    start_nearest<kObj, kCsg>(job, k, l, err);
+    F3 o, d;
+    job.load(k, o, d);
     const SceneView& s = job.scene();
     const float near = job.near();
-    bool restart = l.r.exact;
-    uint32_t budget = 2u * s.wide.count + 2u;
-    while (l.cur != 0u && !restart) {
-      const float reach = wide_limit(l.best.lim);
-      while (l.cur != 0u && !(l.cur & kLeafRef)) {
-        l.cur = wide_step(s.wide.wide + l.cur, l.r, near, reach, stk, l.sp);
+    const WRay r = wide_ray(o, d, near, s.wide.bounded);
+    Nearest best = nothing_yet(job.far());
+    uint32_t leaf = 0, prim = 0, cur = s.wide.root, budget = 2u * s.wide.count + 2u;
+    int sp = 0;
+    WideStack stk;
+    bool restart = r.exact;
+    while (cur != 0u && !restart) {
+      const float reach = wide_limit(best.lim);
+      while (cur != 0u && !(cur & kLeafRef)) {
+        cur = wide_step(s.wide.wide + cur, r, near, reach, stk, sp);
         if (--budget == 0u) {
           atomicOr(err, kErrBudget);
-          l.cur = 0u;
+          cur = 0u;
         }
       }
-      if (l.cur == 0u) break;
-      restart = nearest_in_leaf<kObj, kCsg>(s, near, l, err);
-      l.cur = wide_pop(stk, l.sp, wide_limit(l.best.lim));
+      if (cur == 0u) break;
+      restart = nearest_in_leaf<false, false>(job, s, r, near, cur, best, leaf, prim, err);
+      cur = wide_pop(stk, sp, wide_limit(best.lim));
     }
     if (restart) {
       float t = 0.f;
-      l.best.have = exact_nearest<Job, kObj, kCsg, true>(s, l.r.o, l.r.d, near, job.far(), t, l.leaf, l.prim, err);
-      l.best.lim = t;
+      best.have = exact_nearest<Job, false, false, true>(s, r.o, r.d, near, job.far(), t, leaf, prim, err);
+      best.lim = t;
     }
-    job.store(l.best.have, l.best.lim, l.leaf, l.prim);
+    job.store(best.have, best.lim, leaf, prim);
   }
 }
 
-template <bool kObj, bool kCsg, class Job>
+template <class Job>
 PBRT_DEV void each_any(Job& job, uint64_t n, uint32_t* err) {
   for (uint64_t k = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; k < n; k += uint64_t(gridDim.x) * blockDim.x) {
-    AnyLane l{};
-    WideStack stk;
-    bool hit = !start_any<kObj, kCsg>(job, k, l, err);
+    F3 o, d;
+    job.load(k, o, d);
     const SceneView& s = job.scene();
-    const float near = job.near();
-    if (!hit && l.r.exact) {
-      hit = exact_any<Job, kObj, kCsg, true>(s, l.r.o, l.r.d, near, job.far(), err);
-      l.cur = 0u;
+    const float near = job.near(), lim = next_up(job.far());
+    const WRay r = wide_ray(o, d, near, s.wide.bounded);
+    uint32_t cur = s.wide.root, budget = 2u * s.wide.count + 2u;
+    int sp = 0;
+    WideStack stk;
+    bool hit = false;
+    if (r.exact) {
+      hit = exact_any<Job, false, false, true>(s, r.o, r.d, near, job.far(), err);
+      cur = 0u;
     }
-    uint32_t budget = 2u * s.wide.count + 2u;
-    while (l.cur != 0u && !hit) {
-      while (l.cur != 0u && !(l.cur & kLeafRef)) {
-        l.cur = wide_step_any(s.wide.wide + l.cur, l.r, near, l.lim, stk, l.sp);
+    while (cur != 0u && !hit) {
+      while (cur != 0u && !(cur & kLeafRef)) {
+        cur = wide_step_any(s.wide.wide + cur, r, near, lim, stk, sp);
         if (--budget == 0u) {
           atomicOr(err, kErrBudget);
-          l.cur = 0u;
+          cur = 0u;
           hit = true;  // reported, the sample dropped
         }
       }
-      if (l.cur == 0u) break;
-      hit = blocked_in_leaf<kObj, kCsg>(s, near, kObj ? job.far() : 0.f, l, err);
-      if (!hit) l.cur = wide_pop(stk, l.sp, l.lim);
+      if (cur == 0u) break;
+      hit = blocked_in_leaf<false, false>(job, s, r, near, lim, cur, err);
+      if (!hit) cur = wide_pop(stk, sp, lim);
     }
     job.store(hit);
   }

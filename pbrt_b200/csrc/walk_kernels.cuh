@@ -59,7 +59,8 @@ __global__ void __launch_bounds__(256, kObj ? PBRT_WALK_OBJ_BLOCKS : PBRT_WALK_B
     if (stats) atomicAdd(stats, (unsigned long long)n);
   }
   PathRays<Src> job{w, src, q, 0u, {}};
-  if constexpr (kEach) each_nearest<kObj, kCsg>(job, n, err);
+  static_assert(!kEach || !kObj, "one thread per ray: merged meshes only");
+  if constexpr (kEach) each_nearest(job, n, err);
   else walk_nearest<kObj, kCsg>(job, walk_queue(fetch, n), ws, err);
 }
 
@@ -97,7 +98,8 @@ __global__ void __launch_bounds__(256, kObj ? PBRT_WALK_OBJ_BLOCKS : PBRT_WALK_B
   const uint32_t n = w.counts[2];
   if (stats && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(stats + 1, (unsigned long long)n);
   ShadowRays<Src> job{w, src, 0u, {}};
-  if constexpr (kEach) each_any<kObj, kCsg>(job, n, err);
+  static_assert(!kEach || !kObj, "one thread per ray: merged meshes only");
+  if constexpr (kEach) each_any(job, n, err);
   else walk_any<kObj, kCsg>(job, walk_queue(fetch, n), ws, err);
 }
 
