@@ -366,6 +366,7 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
   for (const GpuNode& g : fs.top)
     for (int x = 0; x < 3; ++x)
       if (!(std::fabs(g.bmin[x]) <= kWideLimit) || !(std::fabs(g.bmax[x]) <= kWideLimit)) w.bounded = false;
+  w.ordered = fs.ordered;
   if (!fs.top.empty()) {
     WidenArgs a{};
     a.nodes = (const float4*)top;

@@ -88,6 +88,14 @@ __device__ __noinline__ bool exact_any(const SceneView& s, F3 o, F3 d, float nea
   return scene_any<kCsg>(s, o, d, near, far, err);
 }
 
+// A ray of a nearest walk. Among objects it must be one whose distances are in order (wide_bvh.cuh):
+// the scene's transforms keep lengths, and so does its direction.
+template <bool kObj>
+PBRT_DEV WRay nearest_ray(const WideView& w, const F3& o, const F3& d, float near) {
+  const bool ordered = !kObj || (w.ordered && fabsf(fs(dot3(d, d), 1.f)) <= 0x1p-12f);
+  return wide_ray(o, d, near, w.bounded && ordered);
+}
+
 // ---- a leaf ---------------------------------------------------------------------------------------
 // The nearest hit of the leaf `cur`, weighed against the best so far. True: the ray must be answered
 // by the exact query. An object is asked up to the nearest distance and a little more (wide_limit),
@@ -162,7 +170,7 @@ PBRT_DEV void walk_nearest(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err
         job.load(k, o, d);
         const SceneView& s = job.scene();
         const float near = job.near(), far = job.far();
-        r = wide_ray(o, d, near, s.wide.bounded);
+        r = nearest_ray<kObj>(s.wide, o, d, near);
         best = nothing_yet(far);
         if (kObj && !r.exact) {
           for (uint32_t u = 0; u < s.unbounded_count; ++u) {  // nearest_among + closer (scene.rs:222-249)
@@ -298,7 +306,7 @@ PBRT_DEV void each_nearest(Job& job, uint64_t n, uint32_t* err) {
     job.load(k, o, d);
     const SceneView& s = job.scene();
     const float near = job.near();
-    const WRay r = wide_ray(o, d, near, s.wide.bounded);
+    const WRay r = nearest_ray<false>(s.wide, o, d, near);
     Nearest best = nothing_yet(job.far());
     uint32_t leaf = 0, prim = 0, cur = s.wide.root, budget = 2u * s.wide.count + 2u;
     int sp = 0;

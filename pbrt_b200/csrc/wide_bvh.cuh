@@ -25,6 +25,11 @@
 //     that window, or a t below e by more than 2^-13 of it, makes the ray start again on the
 //     binary nodes, in the binary order. Nodes are dropped only beyond the nearest distance plus
 //     2^-13 of it, so that a candidate with t < e is seen, not skipped.
+// Objects' distances keep to that as long as they are the ray's own: a placed object's is measured
+// along a unit vector again, so its transforms must keep lengths and the ray's direction be a unit
+// vector, and a plane inside a solid measures another way. A leaf whose hit lies far before its
+// entry could be dropped unseen, where the binary order may take it; nearest hits of scenes with
+// such objects (`ordered` false), and of other directions, use the binary nodes from the start.
 // Rays the grid's arithmetic does not cover (a direction component of zero or outside
 // [2^-40, 2^40], near < 0 or NaN, coordinates beyond 2^40) use the binary nodes from the start.
 #pragma once
@@ -70,6 +75,7 @@ struct WideView {
   uint32_t count;       // wide nodes: no walk visits more
   bool direct;          // triangle references hold their counts
   bool bounded;         // every coordinate lies where the grid's arithmetic holds
+  bool ordered;         // no object's hit is nearer than its box's entry, beyond rounding
 };
 
 PBRT_DEV void triangle_range(const WideView& w, uint32_t ref, uint32_t& first, uint32_t& count) {
