@@ -216,8 +216,9 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
   s->meshes.resize(nm);
   std::vector<MeshView> views(nm);
   std::vector<MeshShade> shades(nm);
-  void *nodes = nullptr, *tri = nullptr, *tri_c = nullptr, *wide = nullptr, *leaf = nullptr;
+  void *nodes = nullptr, *tri = nullptr, *tri_c = nullptr, *wide = nullptr, *exact = nullptr, *leaf = nullptr;
   int rc = s->alloc(&wide, total_wide * sizeof(WideNode));
+  if (rc == PBRT_OK) rc = s->alloc(&exact, total_wide * sizeof(ExactNode));
   if (rc == PBRT_OK && nm) rc = s->alloc(&leaf, total_tris * sizeof(uint2));
   if (rc == PBRT_OK && nm == 1 && built(0)) {  // the only mesh's arrays are the scene's
     DeviceMeshBuild& b = (*dev)[0];
@@ -275,6 +276,7 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
     a.nodes = v.nodes;
     a.count = v.node_count;
     a.wide = static_cast<WideNode*>(wide);
+    a.exact = static_cast<ExactNode*>(exact);
     a.wide_base = uint32_t(wide_at[i]);
     a.direct = direct;
     a.tri_base = uint32_t(tri_at[i]);
@@ -350,6 +352,7 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
   for (const ObjRec& ob : fs.objects) v.has_csg |= ob.shape == kShapeCsg ? 1u : 0u;
   v.has_objects = objects ? 1u : 0u;
   WideView& w = v.wide;
+  w.exact = (const ExactNode*)exact;
   w.wide = (const WideNode*)wide;
   w.tri = (const float4*)tri;
   w.tri_c = (const float2*)tri_c;
@@ -366,12 +369,12 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
   for (const GpuNode& g : fs.top)
     for (int x = 0; x < 3; ++x)
       if (!(std::fabs(g.bmin[x]) <= kWideLimit) || !(std::fabs(g.bmax[x]) <= kWideLimit)) w.bounded = false;
-  w.ordered = fs.ordered;
   if (!fs.top.empty()) {
     WidenArgs a{};
     a.nodes = (const float4*)top;
     a.count = uint32_t(fs.top.size());
     a.wide = static_cast<WideNode*>(wide);
+    a.exact = static_cast<ExactNode*>(exact);
     a.direct = direct;
     a.slot_ref = (const uint32_t*)srefs;
     a.slot_node = (uint32_t*)snodes;

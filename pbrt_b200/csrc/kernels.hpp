@@ -9,6 +9,7 @@ namespace pbrt {
 struct MeshView;
 struct WideView;
 struct WideNode;
+struct ExactNode;
 
 // Ray buffers: eight planes (ox oy oz dx dy dz tmin tmax) of `stride` floats each, of which
 // the first `n` are used.
@@ -40,6 +41,7 @@ struct WidenArgs {
   const float4* nodes;
   uint32_t count;
   WideNode* wide;
+  ExactNode* exact;
   uint32_t wide_base;
   bool direct;
   uint32_t tri_base, node_base, owner;  // a mesh: its first triangle, first node and object in the scene's arrays

@@ -290,8 +290,8 @@ __global__ void __launch_bounds__(kCullThreads) k_cull_root_bulk(MeshView m, con
 // the drained queue in their second byte. Each lane tests its triangles in the reference's
 // order, so ids and t are unchanged.
 // kRec: the survivors' rays come from the records stage 1 wrote beside the queue. kAny: the
-// first triangle hit ends a ray, `prim` holds the occlusion bytes. Rays outside the grid's
-// arithmetic, and those whose answer could depend on the order (weigh), walk m's binary nodes.
+// first triangle hit ends a ray, `prim` holds the occlusion bytes. Rays outside the wide nodes'
+// arithmetic walk m's binary nodes.
 template <bool kRec, bool kAny>
 __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
     MeshView m, WideView w, const float* __restrict__ rays, uint64_t stride, const uint32_t* __restrict__ queue,
@@ -304,8 +304,7 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
   bool active = false, exhausted = false;  // exhausted is warp-uniform
   uint32_t idx = 0;
   WRay r;
-  float near = 0.f, lim0 = 0.f;
-  Nearest nearest{0.f, 0.f, false};
+  float near = 0.f, lim = 0.f;  // a hit counts below lim
   uint32_t best = 0xFFFFFFFFu, cur = 0, budget = 0;
   int sp = 0;
   WideStack stk;
@@ -340,9 +339,7 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
           }
           r = wide_ray(o, d, near, w.bounded);
           // a hit lies below lim: t <= far, and t < min_t (which starts at FLT_MAX, bvh.rs:459)
-          lim0 = kAny ? next_up(far) : fminf(FLT_MAX, next_up(far));
-          nearest = nothing_yet(far);
-          nearest.lim = lim0;
+          lim = kAny ? next_up(far) : fminf(FLT_MAX, next_up(far));
           best = 0xFFFFFFFFu;
           cur = r.exact ? exact_root : w.root;  // the root entered the ray's interval in stage 1 (bvh.rs:458-461)
           sp = 0;
@@ -362,61 +359,47 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
     const bool leaf_step = __popc(on_leaf) >= lmin || on_leaf == act;
     if (active && at_leaf == leaf_step) {
       if (leaf_step) {
-        bool done = false, restart = false;
+        uint32_t first, count;
         if (r.exact) {
           const uint32_t node = cur & ~kLeafRef;
-          const uint32_t first = __float_as_uint(__ldg(&m.nodes[2 * size_t(node)]).w);
-          const uint32_t count = __float_as_uint(__ldg(&m.nodes[2 * size_t(node) + 1]).w);
+          first = __float_as_uint(__ldg(&m.nodes[2 * size_t(node)]).w);
+          count = __float_as_uint(__ldg(&m.nodes[2 * size_t(node) + 1]).w);
+        } else {
+          triangle_range(w, cur, first, count);
+        }
+        const float4* tri = r.exact ? m.tri : w.tri;
+        const float2* tri_c = r.exact ? m.tri_c : w.tri_c;
+        bool done = false;
+        if (kAny) {  // (the grid's boxes are wider than a leaf's own)
+          float e;
+          done = blocking_triangle(tri, tri_c, first, count, r.o, r.d, near, lim) &&
+                 (r.exact || (leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e) && e < lim));
+        } else {
           float t;
           uint32_t id;
-          if (kAny) {
-            done = blocking_triangle(m.tri, m.tri_c, first, count, r.o, r.d, near, nearest.lim);
-          } else if (nearest_triangle(m.tri, m.tri_c, first, count, r.o, r.d, near, nearest.lim, t, id) &&
-                     t < nearest.lim) {
-            nearest.lim = t;
+          if (nearest_triangle(tri, tri_c, first, count, r.o, r.d, near, lim, t, id) && t < lim) {
+            lim = t;
             best = id;
           }
-        } else {
-          uint32_t first, count;
-          triangle_range(w, cur, first, count);
-          float t, e;
-          uint32_t id;
-          if (kAny) {
-            done = blocking_triangle(w.tri, w.tri_c, first, count, r.o, r.d, near, nearest.lim) &&
-                   leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e) && e < nearest.lim;
-          } else if (nearest_triangle(w.tri, w.tri_c, first, count, r.o, r.d, near, wide_limit(nearest.lim), t, id) &&
-                     leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e)) {
-            const Verdict v = weigh(nearest, t, e);
-            if (v == kAdopt) best = id;
-            restart = v == kRestart;
-          }
         }
-        if (kAny && done) {
+        if (done) {
           best = 0u;
           cur = 0u;
-        } else if (!kAny && restart) {  // again, on the binary nodes
-          r.exact = true;
-          nearest.lim = lim0;
-          best = 0xFFFFFFFFu;
-          cur = exact_root;
-          sp = 0;
-          budget = m.node_count;
         } else {
-          cur = wide_pop(stk, sp, kAny || r.exact ? nearest.lim : wide_limit(nearest.lim));
+          cur = wide_pop(stk, sp, lim);
         }
       } else {
         // up to `burst` nodes before the next vote (fewer when a leaf is reached)
         const int nb = exhausted ? (burst >> 8) : (burst & 255);
-        const float reach = kAny ? nearest.lim : wide_limit(nearest.lim);
         for (int b = 0; b < nb && cur != 0u && !(cur & kLeafRef); ++b) {
           if (budget-- == 0) {
             atomicOr(err, kErrBudget);
             cur = 0u;
             break;
           }
-          cur = r.exact ? binary_step(m.nodes, cur, r, near, nearest.lim, stk, sp)
-                : kAny  ? wide_step_any(w.wide + cur, r, near, nearest.lim, stk, sp)
-                        : wide_step(w.wide + cur, r, near, reach, stk, sp);
+          cur = r.exact ? binary_step(m.nodes, cur, r, near, lim, stk, sp)
+                : kAny  ? wide_step_any(w.wide + cur, r, near, lim, stk, sp)
+                        : wide_step(w.exact + cur, r, near, lim, stk, sp);
         }
       }
       if (cur == 0u) {
@@ -425,7 +408,7 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
             reinterpret_cast<uint8_t*>(prim)[idx] = 1;
           } else {
             __stcs(prim + idx, best);
-            __stcs(tout + idx, nearest.lim);
+            __stcs(tout + idx, lim);
             if (obj) __stcs(obj + idx, 0u);
           }
         }
@@ -458,43 +441,38 @@ __global__ void __launch_bounds__(128) k_mesh_few(MeshView m, WideView w, const 
     float t = 0.f, entry;
     if (box_hit(pr, rlo, rhi, near, far, entry) && (kAny || entry < FLT_MAX)) {
       const WRay r = wide_ray(o, d, near, w.bounded);
-      Nearest nearest = nothing_yet(far);
-      nearest.lim = kAny ? next_up(far) : fminf(FLT_MAX, next_up(far));
-      bool restart = r.exact;
-      uint32_t cur = w.root, budget = m.node_count;
+      float lim = kAny ? next_up(far) : fminf(FLT_MAX, next_up(far));
+      uint32_t cur = r.exact ? 0u : w.root, budget = m.node_count;
       int sp = 0;
       WideStack stk;
-      while (cur != 0u && !restart) {
-        const float reach = kAny ? nearest.lim : wide_limit(nearest.lim);
+      while (cur != 0u) {
         while (cur != 0u && !(cur & kLeafRef)) {
           if (budget-- == 0u) {
             atomicOr(err, kErrBudget);
             cur = 0u;
             break;
           }
-          cur = kAny ? wide_step_any(w.wide + cur, r, near, reach, stk, sp)
-                     : wide_step(w.wide + cur, r, near, reach, stk, sp);
+          cur = kAny ? wide_step_any(w.wide + cur, r, near, lim, stk, sp)
+                     : wide_step(w.exact + cur, r, near, lim, stk, sp);
         }
         if (cur == 0u) break;
         uint32_t first, count, id;
         triangle_range(w, cur, first, count);
-        float e;
         if (kAny) {
-          if (blocking_triangle(w.tri, w.tri_c, first, count, o, d, near, nearest.lim) &&
-              leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e) && e < nearest.lim) {
+          float e;
+          if (blocking_triangle(w.tri, w.tri_c, first, count, o, d, near, lim) &&
+              leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e) && e < lim) {
             best = 0u;
             break;
           }
-        } else if (nearest_triangle(w.tri, w.tri_c, first, count, o, d, near, reach, t, id) &&
-                   leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e)) {
-          const Verdict v = weigh(nearest, t, e);
-          if (v == kAdopt) best = id;
-          restart = v == kRestart;
+        } else if (nearest_triangle(w.tri, w.tri_c, first, count, o, d, near, lim, t, id) && t < lim) {
+          lim = t;
+          best = id;
         }
-        cur = wide_pop(stk, sp, kAny ? nearest.lim : wide_limit(nearest.lim));
+        cur = wide_pop(stk, sp, lim);
       }
-      t = nearest.lim;
-      if (restart) {
+      t = lim;
+      if (r.exact) {
         TraceCounters c{0, 0, 0};
         best = kAny ? (mesh_any(m, pr, near, far, err) ? 0u : 0xFFFFFFFFu)
                     : mesh_closest<false>(m, pr, near, far, &t, &c, err);
@@ -547,6 +525,7 @@ __global__ void k_widen(WidenArgs a) {
       }
     }
     WideNode w;
+    ExactNode x4;
     uint32_t pl[3] = {0u, 0u, 0u}, ph[3] = {0u, 0u, 0u};
     const float blo[3] = {nlo.x, nlo.y, nlo.z}, bhi[3] = {nhi.x, nhi.y, nhi.z};
 #pragma unroll
@@ -564,6 +543,8 @@ __global__ void k_widen(WidenArgs a) {
       for (int k = 0; k < 4; ++k) {
         const float4 lo = __ldg(&a.nodes[2 * size_t(slot[k])]), hi = __ldg(&a.nodes[2 * size_t(slot[k]) + 1]);
         const float l = x == 0 ? lo.x : (x == 1 ? lo.y : lo.z), h = x == 0 ? hi.x : (x == 1 ? hi.y : hi.z);
+        (x == 0 ? x4.lo_x : (x == 1 ? x4.lo_y : x4.lo_z))[k] = l;
+        (x == 0 ? x4.hi_x : (x == 1 ? x4.hi_y : x4.hi_z))[k] = h;
         // (within a thousandth of a step a plane snaps to the grid, inwards too: the walk's margin
         // of a 256th of a step covers it)
         const double fl = floor((double(l) - double(blo[x])) / s + 1e-3);
@@ -576,8 +557,12 @@ __global__ void k_widen(WidenArgs a) {
     w.lo_x = pl[0]; w.lo_y = pl[1]; w.lo_z = pl[2];
     w.hi_x = ph[0]; w.hi_y = ph[1]; w.hi_z = ph[2];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) w.ref[k] = ref[k];
+    for (int k = 0; k < 4; ++k) {
+      w.ref[k] = x4.ref[k] = ref[k];
+      x4.pad[k] = 0u;
+    }
     a.wide[a.wide_base + (pair >> 1)] = w;
+    a.exact[a.wide_base + (pair >> 1)] = x4;
   }
 }
 
@@ -587,7 +572,7 @@ __global__ void k_widen(WidenArgs a) {
 // [,tail_burst]]]" (each in 1..32; without tail values the bulk's apply) overrides it for
 // measurements; results do not depend on it.
 struct TraversalSchedule {
-  int leaf_min = 16, refill_min = 8, burst = 4;
+  int leaf_min = 12, refill_min = 12, burst = 4;
   int tail_leaf_min = 1, tail_burst = 4;  // once the queue is drained (no refill can come)
   int leaf_arg() const { return leaf_min | (tail_leaf_min << 8); }
   int burst_arg() const { return burst | (tail_burst << 8); }

@@ -400,58 +400,6 @@ class Flattener {
   std::vector<uint8_t>* grouped_ = nullptr;
 };
 
-// Whether a chain of transforms (outermost first) keeps lengths and has to_local undo to_world, to
-// within what rounding the matrices to FP32 leaves (2^-24 an entry, so 2^-22 in these products): a
-// distance along the local ray, whose direction is a unit vector again, is then the world's.
-bool keeps_lengths(const std::vector<Xf>& chain) {
-  double w[3][4] = {{1, 0, 0, 0}, {0, 1, 0, 0}, {0, 0, 1, 0}}, l[3][4] = {{1, 0, 0, 0}, {0, 1, 0, 0}, {0, 0, 1, 0}};
-  auto times = [](const double (&a)[3][4], const double (&b)[3][4], double (&out)[3][4]) {
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 4; ++j) {
-        out[i][j] = j == 3 ? a[i][3] : 0.0;
-        for (int k = 0; k < 3; ++k) out[i][j] += a[i][k] * b[k][j];
-      }
-  };
-  for (const Xf& x : chain) {
-    double tw[3][4], tl[3][4], r[3][4];
-    for (int i = 0; i < 12; ++i) {
-      tw[i / 4][i % 4] = x.to_world[i];
-      tl[i / 4][i % 4] = x.to_local[i];
-    }
-    times(w, tw, r);
-    std::memcpy(w, r, sizeof(w));
-    times(tl, l, r);
-    std::memcpy(l, r, sizeof(l));
-  }
-  double undone[3][4], far = 0.0;
-  times(w, l, undone);
-  for (int i = 0; i < 3; ++i) far = std::max(far, std::fabs(w[i][3]));
-  for (int i = 0; i < 3; ++i) {
-    if (!(std::fabs(undone[i][3]) <= 0x1p-18 * far)) return false;
-    for (int j = 0; j < 3; ++j) {
-      double rows = 0.0;
-      for (int k = 0; k < 3; ++k) rows += l[i][k] * l[j][k];
-      if (!(std::fabs(rows - (i == j)) <= 0x1p-14) || !(std::fabs(undone[i][j] - (i == j)) <= 0x1p-18)) return false;
-    }
-  }
-  return true;
-}
-
-// Whether a leaf's hits are never nearer than the entry into its box, beyond rounding (a plane inside
-// a solid measures its distance another way: plane.rs:19-45).
-bool leaf_ordered(const FlatScene& s, const ObjRec& ob) {
-  std::vector<Xf> chain;
-  for (uint32_t k = 0; k < ob.xf_count; ++k) {
-    if (k == 0) chain.push_back(Xf{ob.to_world, ob.to_local});
-    else chain.push_back(Xf{s.xforms[ob.xf_rest + k - 1].to_world, s.xforms[ob.xf_rest + k - 1].to_local});
-  }
-  if (!keeps_lengths(chain)) return false;
-  if (ob.shape == kShapeCsg)
-    for (uint32_t e = ob.csg_first; e < ob.csg_first + ob.csg_count; ++e)
-      if (s.csg[e].shape == kShapePlane || !keeps_lengths({Xf{s.csg[e].to_world, s.csg[e].to_local}})) return false;
-  return true;
-}
-
 // The box of a plain shape before any transform (its get_bounding_box), with its sizes checked.
 bool plain_shape_box(const pbrt_object_desc& o, const pbrt_scene_desc& d, const FlatScene* out, const std::string& who,
                    Box3* bp, std::string* err) {
@@ -654,10 +602,6 @@ bool build_scene(const pbrt_scene_desc& d, FlatScene* out, std::string* err, con
     if (is_bounded(boxes[i])) {
       bounded_refs.push_back(refs[i]);
       bounded_boxes.push_back(boxes[i]);
-      const bool group = refs[i] & kGroupBit;
-      const GroupRec g = group ? out->groups[refs[i] & ~kGroupBit] : GroupRec{refs[i], 1};
-      for (uint32_t k = g.first; k < g.first + g.count; ++k)
-        out->ordered = out->ordered && leaf_ordered(*out, out->objects[k]);
     } else {
       out->unbounded.push_back(refs[i]);
     }

@@ -32,9 +32,6 @@ struct FlatScene {
                                                 // primitive is bounded
   std::vector<uint32_t> order;                  // leaf slot -> primitive (leaf, or kGroupBit | group)
   uint32_t top_depth = 0;
-  // No bounded primitive's hit is nearer than the entry into its box, beyond rounding: every
-  // transform of it keeps lengths, and no solid of it holds a plane.
-  bool ordered = true;
   uint64_t primitive_count = 0;                 // bounded + unbounded
   int single_mesh = -1;                         // the mesh, when the scene is one untransformed mesh
   std::vector<MatRec> materials;

@@ -88,47 +88,44 @@ __device__ __noinline__ bool exact_any(const SceneView& s, F3 o, F3 d, float nea
   return scene_any<kCsg>(s, o, d, near, far, err);
 }
 
-// A ray of a nearest walk. Among objects it must be one whose distances are in order (wide_bvh.cuh):
-// the scene's transforms keep lengths, and so does its direction.
-template <bool kObj>
-PBRT_DEV WRay nearest_ray(const WideView& w, const F3& o, const F3& d, float near) {
-  const bool ordered = !kObj || (w.ordered && fabsf(fs(dot3(d, d), 1.f)) <= 0x1p-12f);
-  return wide_ray(o, d, near, w.bounded && ordered);
-}
+// The nearest hit of a walk so far: `t` is the ray's far end before there is one.
+struct Nearest {
+  float t;
+  bool have;
+};
 
 // ---- a leaf ---------------------------------------------------------------------------------------
-// The nearest hit of the leaf `cur`, weighed against the best so far. True: the ray must be answered
-// by the exact query. An object is asked up to the nearest distance and a little more (wide_limit),
-// but never beyond the ray's own end: an exit at exactly that distance is no hit (sphere_hit's and
-// the other shapes' last comparison is strict).
-template <bool kObj, bool kCsg, class Job>
-PBRT_DEV bool nearest_in_leaf(const Job& job, const SceneView& s, const WRay& r, float near, uint32_t cur,
-                              Nearest& best, uint32_t& leaf, uint32_t& prim, uint32_t* err) {
-  const float reach = wide_limit(best.lim);
+// The nearest hit of the leaf `cur`, whose slot is entered at `e`, adopted when it is nearer than the
+// best so far, as scene_closest_t does. Slots are entered up to and including best.t, as a mesh's own
+// boxes are; an object is asked when its box is entered below best.t only. A merged mesh's leaf
+// entered at exactly best.t is asked or not as the box of the whole mesh has it: true, the ray must be
+// answered by the exact query.
+template <bool kObj, bool kCsg>
+PBRT_DEV bool nearest_in_leaf(const SceneView& s, const WRay& r, float near, uint32_t cur, float e, Nearest& best,
+                              uint32_t& leaf, uint32_t& prim, uint32_t* err) {
   float t;
   uint32_t lf = 0, pr = 0;
-  const float4* node = nullptr;
   if (kObj && (cur & kObjectRef)) {
-    const uint32_t slot = cur & 0x3FFFFFFFu;
-    if (prim_closest<kCsg>(s, __ldg(&s.order[slot]), r.o, r.d, near, fminf(reach, job.far()), t, lf, pr, err))
-      node = s.top + 2 * size_t(__ldg(&s.wide.slot_node[slot]));
+    if (!(e < best.t) || !prim_closest<kCsg>(s, __ldg(&s.order[cur & 0x3FFFFFFFu]), r.o, r.d, near, best.t, t, lf, pr, err) ||
+        (best.have && !(t < best.t)))
+      return false;
   } else {
     uint32_t first, count;
     triangle_range(s.wide, cur, first, count);
-    if (nearest_triangle(s.wide.tri, s.wide.tri_c, first, count, r.o, r.d, near, reach, t, pr)) {
-      const uint2 info = __ldg(&s.wide.leaf[first]);
-      node = s.wide.nodes + 2 * size_t(info.x);
-      lf = info.y;
-    }
+    // (a mesh's own search starts at FLT_MAX, bvh.rs:459: its hits lie below that)
+    if (!nearest_triangle(s.wide.tri, s.wide.tri_c, first, count, r.o, r.d, near, fminf(best.t, 0x1.fffffcp127f), t, pr) ||
+        (best.have && !(t < best.t)))
+      return false;
+    const uint2 info = __ldg(&s.wide.leaf[first]);
+    // (the slot of a mesh of one leaf is its top-level box: the leaf's own is asked)
+    if (!leaf_hit(s.wide.nodes + 2 * size_t(info.x), r, near, e) || e > best.t) return false;
+    if (e == best.t) return true;
+    lf = info.y;
   }
-  float e;
-  if (!node || !leaf_hit(node, r, near, e)) return false;
-  const Verdict v = weigh(best, t, e);
-  if (v == kAdopt) {
-    leaf = lf;
-    prim = pr;
-  }
-  return v == kRestart;
+  best = Nearest{t, true};
+  leaf = lf;
+  prim = pr;
+  return false;
 }
 
 // Whether the leaf `cur` blocks the ray (lim: just above its far end).
@@ -157,8 +154,9 @@ template <bool kObj, bool kCsg, class Job>
 PBRT_DEV void walk_nearest(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err) {
   bool active = false;
   WRay r;
-  Nearest best{0.f, 0.f, false};
+  Nearest best{0.f, false};
   uint32_t leaf = 0, prim = 0, cur = 0, budget = 0;
+  float e = 0.f;  // the entry into the slot of `cur`
   int sp = 0;
   WideStack stk;
   for (;;) {
@@ -170,22 +168,22 @@ PBRT_DEV void walk_nearest(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err
         job.load(k, o, d);
         const SceneView& s = job.scene();
         const float near = job.near(), far = job.far();
-        r = nearest_ray<kObj>(s.wide, o, d, near);
-        best = nothing_yet(far);
+        r = wide_ray(o, d, near, s.wide.bounded);
+        best = Nearest{far, false};
         if (kObj && !r.exact) {
           for (uint32_t u = 0; u < s.unbounded_count; ++u) {  // nearest_among + closer (scene.rs:222-249)
             float t;
             uint32_t lf, pr;
             if (prim_closest<kCsg>(s, __ldg(&s.unbounded[u]), o, d, near, far, t, lf, pr, err) &&
-                (!best.have || t < best.lim)) {
-              best.have = true;
-              best.lim = t;
+                (!best.have || t < best.t)) {
+              best = Nearest{t, true};
               leaf = lf;
               prim = pr;
             }
           }
         }
         cur = s.wide.root;
+        if (kObj && (cur & kObjectRef) && (cur & kLeafRef) && !leaf_hit(s.top, r, near, e)) cur = 0u;  // the only primitive
         sp = 0;
         budget = 2u * s.wide.count + 2u;  // every iteration visits a node or a leaf it has not visited
         active = true;
@@ -204,13 +202,13 @@ PBRT_DEV void walk_nearest(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err
       const float near = job.near();
       bool restart = r.exact;
       if (leaf_step && at_leaf && !restart) {
-        restart = nearest_in_leaf<kObj, kCsg>(job, s, r, near, cur, best, leaf, prim, err);
-        cur = wide_pop(stk, sp, wide_limit(best.lim));
+        restart = nearest_in_leaf<kObj, kCsg>(s, r, near, cur, e, best, leaf, prim, err);
+        cur = wide_pop(stk, sp, next_up(best.t), e);
       }
       if (!leaf_step || q.drained) {
-        const float reach = wide_limit(best.lim);
+        const float reach = next_up(best.t);
         for (int b = 0; b < ws.burst && cur != 0u && !(cur & kLeafRef); ++b)
-          cur = wide_step(s.wide.wide + cur, r, near, reach, stk, sp);
+          cur = wide_step(s.wide.exact + cur, r, near, reach, stk, sp, e);
         if (--budget == 0u) {
           atomicOr(err, kErrBudget);
           cur = 0u;
@@ -219,11 +217,11 @@ PBRT_DEV void walk_nearest(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err
       if (restart) {
         float t = 0.f;
         best.have = exact_nearest<Job, kObj, kCsg, false>(s, r.o, r.d, near, job.far(), t, leaf, prim, err);
-        best.lim = t;
+        best.t = t;
         cur = 0u;
       }
       if (cur == 0u) {
-        job.store(best.have, best.lim, leaf, prim);
+        job.store(best.have, best.t, leaf, prim);
         active = false;
       }
     }
@@ -306,31 +304,31 @@ PBRT_DEV void each_nearest(Job& job, uint64_t n, uint32_t* err) {
     job.load(k, o, d);
     const SceneView& s = job.scene();
     const float near = job.near();
-    const WRay r = nearest_ray<false>(s.wide, o, d, near);
-    Nearest best = nothing_yet(job.far());
+    const WRay r = wide_ray(o, d, near, s.wide.bounded);
+    Nearest best{job.far(), false};
     uint32_t leaf = 0, prim = 0, cur = s.wide.root, budget = 2u * s.wide.count + 2u;
     int sp = 0;
     WideStack stk;
     bool restart = r.exact;
     while (cur != 0u && !restart) {
-      const float reach = wide_limit(best.lim);
+      const float reach = next_up(best.t);
       while (cur != 0u && !(cur & kLeafRef)) {
-        cur = wide_step(s.wide.wide + cur, r, near, reach, stk, sp);
+        cur = wide_step(s.wide.exact + cur, r, near, reach, stk, sp);
         if (--budget == 0u) {
           atomicOr(err, kErrBudget);
           cur = 0u;
         }
       }
       if (cur == 0u) break;
-      restart = nearest_in_leaf<false, false>(job, s, r, near, cur, best, leaf, prim, err);
-      cur = wide_pop(stk, sp, wide_limit(best.lim));
+      restart = nearest_in_leaf<false, false>(s, r, near, cur, 0.f, best, leaf, prim, err);
+      cur = wide_pop(stk, sp, next_up(best.t));
     }
     if (restart) {
       float t = 0.f;
       best.have = exact_nearest<Job, false, false, true>(s, r.o, r.d, near, job.far(), t, leaf, prim, err);
-      best.lim = t;
+      best.t = t;
     }
-    job.store(best.have, best.lim, leaf, prim);
+    job.store(best.have, best.t, leaf, prim);
   }
 }
 

@@ -140,3 +140,71 @@ def test_directions_that_are_not_unit_vectors(scale):
     rays = _rays(rng, 100_000, 3.0, at)
     rays[3:6] *= np.float32(scale)
     _same(_commit(objects + [pb.Simple(pb.TriangleMesh(*W.displaced_icosphere(3, seed=9)))]), rays)
+
+
+def _towards(rng, tgt, dist):
+    """Rays of a set length from random directions to the points `tgt` (n, 3)."""
+    o = rng.normal(size=tgt.shape)
+    o = tgt + o / np.linalg.norm(o, axis=1, keepdims=True) * dist
+    r = np.empty((8, len(tgt)), np.float32)
+    r[0:3] = o.T.astype(np.float32)
+    r[3:6], r[6], r[7] = W.normalize_f32((tgt.T - r[0:3].astype(np.float64)).astype(np.float32)), 0.0, 1e30
+    return r
+
+
+@pytest.mark.parametrize("ratio", [1e-3, 1e-4, 1e-5])
+def test_small_spheres_far_away(ratio):
+    """A sphere's distance loses as many digits as the sphere is far in its radii: hits before their boxes."""
+    rng = np.random.default_rng(11)
+    c, r = rng.normal(size=(400, 3)) * 8 * ratio, ratio * 10 ** rng.uniform(-0.5, 0.5, 400)
+    s = _commit([pb.Transformed(pb.Simple(pb.Sphere(float(q))), TR.translation([float(x) for x in p])) for p, q in zip(c, r)])
+    n = 2_000_000
+    tgt = c[rng.integers(0, 400, n)] + rng.normal(size=(n, 3)) * ratio
+    hit, _ = _same(s, _towards(rng, tgt, rng.uniform(0.5, 1.5, (n, 1))))
+    assert hit.mean() > 0.5
+
+
+def _sheet(n, half, turn, lift):
+    g = np.linspace(-half, half, n + 1)
+    x, z = np.meshgrid(g, g, indexing="ij")
+    i, j = np.meshgrid(np.arange(n), np.arange(n), indexing="ij")
+    a = (i * (n + 1) + j).reshape(-1)
+    f = np.stack([a, a + n + 1, a + n + 2, a, a + n + 2, a + 1], -1).reshape(-1, 3)
+    v = np.stack([x, np.full_like(x, lift), z], -1).reshape(-1, 3) @ turn.T
+    return v.astype(np.float32), f.astype(np.uint32)
+
+
+def _grazing(rng, n, turn, half, least):
+    """Rays that meet the plane y = 0 (turned) at angles down to `least`."""
+    at = rng.uniform(-half, half, (3, n))
+    at[1] = 0
+    phi, c = rng.uniform(0, 2 * np.pi, n), 10 ** rng.uniform(np.log10(least), -1, n) * rng.choice([-1, 1], n)
+    d = np.stack([np.cos(phi) * np.sqrt(1 - c * c), c, np.sin(phi) * np.sqrt(1 - c * c)])
+    r = np.empty((8, n), np.float32)
+    r[0:3] = turn @ (at - d * (0.01 + 8 * rng.random(n) ** 2))
+    r[3:6], r[6], r[7] = W.normalize_f32((turn @ d).astype(np.float32)), 0.0, np.where(rng.random(n) < 0.2, np.inf, 1e30)
+    return r
+
+
+@pytest.mark.parametrize("merged", ["one mesh", "a mesh each", "instances"])
+@pytest.mark.parametrize("seed", [0, 1])
+def test_sheets_met_at_grazing_angles(merged, seed):
+    """Sheets in nearly the same tilted plane: a triangle's distance is off by 2^-24 over the cosine, so that
+    which sheet is met first, and whether before its box, is left to rounding and the order."""
+    rng = np.random.default_rng(seed)
+    turn = (TR.rotation_x(rng.uniform(0, 3)) * TR.rotation_z(rng.uniform(0, 3))).mat[:3, :3]
+    sheets = [_sheet(12 + k, 2.0, turn, 1e-7 * rng.normal()) for k in range(8)]
+    if merged == "one mesh":
+        base = np.cumsum([0] + [len(v) for v, _ in sheets])
+        objects = [pb.Simple(pb.TriangleMesh(np.concatenate([v for v, _ in sheets]),
+                                             np.concatenate([f + b for (_, f), b in zip(sheets, base)]).astype(np.uint32)))]
+    elif merged == "a mesh each":
+        objects = [pb.Simple(pb.TriangleMesh(v, f)) for v, f in sheets]
+    else:
+        sheet = pb.TriangleMesh(*_sheet(6, 1.0, turn, 0.0))
+        objects = [pb.Transformed(pb.Simple(sheet), TR.translation([float(x) for x in turn @ [a, 0, b]]))
+                   for a, b in rng.uniform(-2, 2, (16, 2))]
+    s = _commit(objects, bvh_bins=16)
+    for _ in range(6):
+        hit, _ = _same(s, _grazing(rng, 2_000_000, turn, 2.0, 1e-5))
+        assert hit.mean() > 0.3
