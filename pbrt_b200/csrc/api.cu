@@ -697,16 +697,17 @@ int trace_impl(pbrt_scene* s, const float* rays, uint64_t n, uint32_t* prim, flo
     if (!one_mesh)
       return oc ? launch_scene_any(s->view, r, stride, m, oc, cnt, c->d_err, c->sm_count, st)
                 : launch_scene_closest(s->view, r, stride, m, p, tt, ob, cnt, c->d_err, c->sm_count, st);
-    const bool two_stage = queue && m > kFewRays;
-    if (oc)
-      return !c->persistent ? launch_mesh_any(mv, r, stride, m, oc, c->d_err, c->sm_count, st)
-             : two_stage    ? launch_mesh_any_persistent(mv, wv, r, stride, m, oc, queue, qc, c->d_err, c->sm_count, st, rec)
-                            : launch_mesh_any_few(mv, wv, r, stride, m, oc, c->d_err, c->sm_count, st);
-    if (c->persistent && !cnt)
-      return two_stage
-                 ? launch_mesh_closest_persistent(mv, wv, r, stride, m, p, tt, ob, queue, qc, c->d_err, c->sm_count, st, rec)
-                 : launch_mesh_closest_few(mv, wv, r, stride, m, p, tt, ob, c->d_err, c->sm_count, st);
-    return launch_mesh_closest(mv, r, stride, m, p, tt, ob, cnt, c->d_err, c->sm_count, st);
+    if (!c->persistent || cnt)
+      return oc ? launch_mesh_any(mv, r, stride, m, oc, c->d_err, c->sm_count, st)
+                : launch_mesh_closest(mv, r, stride, m, p, tt, ob, cnt, c->d_err, c->sm_count, st);
+    if (m <= kFewRays)
+      return oc ? launch_mesh_any_few(mv, wv, r, stride, m, oc, c->d_err, c->sm_count, st)
+                : launch_mesh_closest_few(mv, wv, r, stride, m, p, tt, ob, c->d_err, c->sm_count, st);
+    if (!queue)
+      return oc ? launch_mesh_any_planes(mv, wv, r, stride, m, oc, c->d_err, c->sm_count, st)
+                : launch_mesh_closest_planes(mv, wv, r, stride, m, p, tt, ob, c->d_err, c->sm_count, st);
+    return oc ? launch_mesh_any_persistent(mv, wv, r, stride, m, oc, queue, qc, c->d_err, c->sm_count, st, rec)
+              : launch_mesh_closest_persistent(mv, wv, r, stride, m, p, tt, ob, queue, qc, c->d_err, c->sm_count, st, rec);
   };
 
   const MemKind kr = mem_kind(rays);
@@ -724,26 +725,25 @@ int trace_impl(pbrt_scene* s, const float* rays, uint64_t n, uint32_t* prim, flo
 
   if (kr == MemKind::Device) {
     cudaStream_t st = c->work_stream();
-    // Few rays take one kernel without scratch. So does occlusion on a stream under capture, of
-    // any size, since a graph replayed later may run beside another call's use of the queue.
+    // Few rays take one kernel without scratch. So does a call on a stream under capture, of any
+    // size: a graph replayed later may run beside another call's use of the queue.
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (c->user) PBRT_TRY(c->cuda(cudaStreamIsCapturing(st, &cap), "cudaStreamIsCapturing"));
-    const bool captured = cap != cudaStreamCaptureStatusNone;
-    if (one_mesh && c->persistent && !counters && n > kFewRays && !(occ && captured)) {
-      // Chunks of at most kDevChunk rays bound the survivor queue (scratch) to 64 MiB.
+    const bool queued = one_mesh && c->persistent && !counters && n > kFewRays && cap == cudaStreamCaptureStatusNone;
+    if (queued) {
       PBRT_TRY(ensure_queue(c));
-      if (!captured) PBRT_TRY(acquire_queue(c, st));
-      for (uint64_t base = 0; base < n; base += kDevChunk) {
-        const uint64_t m = std::min<uint64_t>(kDevChunk, n - base);
-        PBRT_TRY(c->cuda(launch(rays + base, n, m, occ ? nullptr : prim + base, occ ? nullptr : t + base,
-                                obj ? obj + base : nullptr, occ ? occ + base : nullptr, nullptr, c->queue,
-                                c->d_counters + 4, c->queue_rec, st),
-                         "kernel launch"));
-      }
-      if (!captured && c->user) PBRT_TRY(release_queue(c, st));
-    } else {
-      PBRT_TRY(c->cuda(launch(rays, n, n, prim, t, obj, occ, counters, nullptr, nullptr, nullptr, st), "kernel launch"));
+      PBRT_TRY(acquire_queue(c, st));
     }
+    // Chunks of at most kDevChunk rays bound the survivor queue (scratch) to 64 MiB.
+    const uint64_t chunk = one_mesh ? kDevChunk : n;
+    for (uint64_t base = 0; base < n; base += chunk) {
+      const uint64_t m = std::min<uint64_t>(chunk, n - base);
+      PBRT_TRY(c->cuda(launch(rays + base, n, m, occ ? nullptr : prim + base, occ ? nullptr : t + base,
+                              obj ? obj + base : nullptr, occ ? occ + base : nullptr, counters,
+                              queued ? c->queue : nullptr, c->d_counters + 4, c->queue_rec, st),
+                       "kernel launch"));
+    }
+    if (queued && c->user) PBRT_TRY(release_queue(c, st));
     if (stats) {
       unsigned long long h[3];
       PBRT_TRY(c->cuda(cudaMemcpyAsync(h, counters, sizeof(h), cudaMemcpyDeviceToHost, st), "cudaMemcpy"));

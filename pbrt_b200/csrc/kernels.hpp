@@ -29,6 +29,12 @@ cudaError_t launch_mesh_closest_persistent(const MeshView& m, const WideView& w,
 cudaError_t launch_mesh_any_persistent(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n, uint8_t* occ,
                                        uint32_t* queue, unsigned long long* counters, uint32_t* err, int sm_count,
                                        cudaStream_t s, float4* rec);
+// Both queries for many rays without scratch: one launch that tests the root itself (n <= 2^32).
+cudaError_t launch_mesh_closest_planes(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
+                                       uint32_t* prim, float* t, uint32_t* obj, uint32_t* err, int sm_count,
+                                       cudaStream_t s);
+cudaError_t launch_mesh_any_planes(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
+                                   uint8_t* occ, uint32_t* err, int sm_count, cudaStream_t s);
 // Both queries for few rays: one launch, no scratch; the rays and answers may be pinned host memory.
 cudaError_t launch_mesh_closest_few(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
                                     uint32_t* prim, float* t, uint32_t* obj, uint32_t* err, int sm_count,

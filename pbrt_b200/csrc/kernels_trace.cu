@@ -90,6 +90,25 @@ PBRT_DEV bool enters_root(const float (&v)[8][kCullRays], int j, const float4& r
   return box_hit(r, rlo, rhi, v[6][j], v[7][j], entry) && (kAny || entry < FLT_MAX);
 }
 
+// The same for ray i of the planes, whose miss answer is written.
+template <bool kAny>
+PBRT_DEV bool enters_root_of(const MeshView& m, const float* rays, uint64_t stride, uint64_t i, uint32_t* prim, float* tout,
+                             uint32_t* obj) {
+  const F3 o = mk3(__ldg(rays + i), __ldg(rays + stride + i), __ldg(rays + 2 * stride + i));
+  const F3 d = mk3(__ldg(rays + 3 * stride + i), __ldg(rays + 4 * stride + i), __ldg(rays + 5 * stride + i));
+  const float near = __ldg(rays + 6 * stride + i), far = __ldg(rays + 7 * stride + i);
+  if (kAny) {
+    reinterpret_cast<uint8_t*>(prim)[i] = 0;
+  } else {
+    __stcs(prim + i, 0xFFFFFFFFu);
+    __stcs(tout + i, __int_as_float(0x7f800000));
+    if (obj) __stcs(obj + i, 0xFFFFFFFFu);
+  }
+  float entry;
+  return box_hit(prepare_ray(o, d), __ldg(&m.nodes[0]), __ldg(&m.nodes[1]), near, far, entry) &&
+         (kAny || entry < FLT_MAX);
+}
+
 // The miss answer of rays i0 .. i0 + 3 (those below n); stage 2 overwrites the hits. For an
 // any-hit pass `prim` holds the occlusion bytes.
 template <bool kVec, bool kAny>
@@ -289,18 +308,29 @@ __global__ void __launch_bounds__(kCullThreads) k_cull_root_bulk(MeshView m, con
 // at least `refill_min` of them are idle (or all are). leaf_min and burst carry the schedule of
 // the drained queue in their second byte. Each lane tests its triangles in the reference's
 // order, so ids and t are unchanged.
-// kRec: the survivors' rays come from the records stage 1 wrote beside the queue. kAny: the
+// kFrom: the survivors' rays come from the records stage 1 wrote beside the queue, from the planes
+// by the queue's indices, or (kPlanes: no scratch, for a stream under capture) from the planes of
+// `n_planes` rays: warp w of W then culls its own chunks of 128, w, w + W, ..., into a queue of its
+// own in shared memory. (16,777,216 rays, 327,680 triangles, nearest hits, recorded: 943 us; 1,419
+// with a warp's rays tested as its lanes take them, 2,496 by k_mesh_few.) kAny: the
 // first triangle hit ends a ray, `prim` holds the occlusion bytes. Rays outside the wide nodes'
 // arithmetic walk m's binary nodes.
-template <bool kRec, bool kAny>
+constexpr uint32_t kOwnChunk = 128;
+enum RaySource : int { kRecords, kQueue, kPlanes };
+template <int kFrom, bool kAny>
 __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
     MeshView m, WideView w, const float* __restrict__ rays, uint64_t stride, const uint32_t* __restrict__ queue,
     const unsigned long long* __restrict__ queue_count, uint32_t* __restrict__ prim, float* __restrict__ tout,
     uint32_t* __restrict__ obj, unsigned long long* __restrict__ next_ray, uint32_t* __restrict__ err,
-    const float4* __restrict__ rec, int leaf_min, int refill_min, int burst) {
+    const float4* __restrict__ rec, uint64_t n_planes, int leaf_min, int refill_min, int burst) {
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
-  const uint64_t n = *queue_count;
+  const uint64_t n = kFrom == kPlanes ? n_planes : *queue_count;
+  // kPlanes: the warp's queue, its length, and its next chunk
+  __shared__ uint32_t own_queue[kFrom == kPlanes ? 4 : 1][kFrom == kPlanes ? kOwnChunk + 32 : 1];
+  uint32_t* own = own_queue[kFrom == kPlanes ? threadIdx.x >> 5 : 0];
+  uint32_t held = 0;
+  uint64_t chunk = uint64_t(blockIdx.x) * 4u + (threadIdx.x >> 5);
   bool active = false, exhausted = false;  // exhausted is warp-uniform
   uint32_t idx = 0;
   WRay r;
@@ -314,38 +344,58 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
     // Refill the idle lanes: one atomicAdd per warp.
     const unsigned idle = __ballot_sync(0xffffffffu, !active);
     if (!exhausted && idle && (__popc(idle) >= refill_min || idle == 0xffffffffu)) {
-      const int leader = __ffs(idle) - 1;
-      unsigned long long base = 0;
-      if (int(lane) == leader) base = atomicAdd(next_ray, (unsigned long long)__popc(idle));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      exhausted = base + __popc(idle) >= n;
-      if (!active) {
-        const uint64_t k = base + __popc(idle & lt_mask);
-        if (k < n) {
-          idx = __ldg(queue + k);
-          F3 o, d;
-          float far;
-          if (kRec) {  // the copy stage 1 wrote: consecutive lanes read consecutive records
-            const float4 a = __ldcs(rec + 2 * k), b = __ldcs(rec + 2 * k + 1);
-            o = mk3(a.x, a.y, a.z);
-            d = mk3(b.x, b.y, b.z);
-            near = a.w;
-            far = b.w;
-          } else {
-            o = mk3(__ldg(rays + idx), __ldg(rays + stride + idx), __ldg(rays + 2 * stride + idx));
-            d = mk3(__ldg(rays + 3 * stride + idx), __ldg(rays + 4 * stride + idx), __ldg(rays + 5 * stride + idx));
-            near = __ldg(rays + 6 * stride + idx);
-            far = __ldg(rays + 7 * stride + idx);
+      uint64_t k = __popc(idle & lt_mask);
+      if (kFrom == kPlanes) {
+        const uint32_t want = __popc(idle);
+        for (; held < want && chunk * kOwnChunk < n; chunk += uint64_t(gridDim.x) * 4u) {
+#pragma unroll 2
+          for (uint32_t j = 0; j < kOwnChunk; j += 32u) {
+            const uint64_t i = chunk * kOwnChunk + j + lane;
+            const bool enters = i < n && enters_root_of<kAny>(m, rays, stride, i, prim, tout, obj);
+            const unsigned in = __ballot_sync(0xffffffffu, enters);
+            if (enters) own[held + __popc(in & lt_mask)] = uint32_t(i);
+            held += __popc(in);
           }
-          r = wide_ray(o, d, near, w.bounded);
-          // a hit lies below lim: t <= far, and t < min_t (which starts at FLT_MAX, bvh.rs:459)
-          lim = kAny ? next_up(far) : fminf(FLT_MAX, next_up(far));
-          best = 0xFFFFFFFFu;
-          cur = r.exact ? exact_root : w.root;  // the root entered the ray's interval in stage 1 (bvh.rs:458-461)
-          sp = 0;
-          budget = m.node_count;
-          active = true;
         }
+        __syncwarp();
+        k = k < held ? uint64_t(own[held - 1u - uint32_t(k)]) : n;
+        __syncwarp();
+        held -= held < want ? held : want;
+        exhausted = held == 0u && chunk * kOwnChunk >= n;
+      } else {
+        const int leader = __ffs(idle) - 1;
+        unsigned long long base = 0;
+        if (int(lane) == leader) base = atomicAdd(next_ray, (unsigned long long)__popc(idle));
+        base = __shfl_sync(0xffffffffu, base, leader);
+        exhausted = base + __popc(idle) >= n;
+        k += base;
+      }
+      if (!active && k < n) {
+        F3 o, d;
+        float far;
+        if (kFrom == kRecords) {  // the copy stage 1 wrote: consecutive lanes read consecutive records
+          idx = __ldg(queue + k);
+          const float4 a = __ldcs(rec + 2 * k), b = __ldcs(rec + 2 * k + 1);
+          o = mk3(a.x, a.y, a.z);
+          d = mk3(b.x, b.y, b.z);
+          near = a.w;
+          far = b.w;
+        } else {
+          const uint64_t i = kFrom == kPlanes ? k : uint64_t(__ldg(queue + k));
+          o = mk3(__ldg(rays + i), __ldg(rays + stride + i), __ldg(rays + 2 * stride + i));
+          d = mk3(__ldg(rays + 3 * stride + i), __ldg(rays + 4 * stride + i), __ldg(rays + 5 * stride + i));
+          near = __ldg(rays + 6 * stride + i);
+          far = __ldg(rays + 7 * stride + i);
+          idx = uint32_t(i);
+        }
+        r = wide_ray(o, d, near, w.bounded);
+        // a hit lies below lim: t <= far, and t < min_t (which starts at FLT_MAX, bvh.rs:459)
+        lim = kAny ? next_up(far) : fminf(FLT_MAX, next_up(far));
+        best = 0xFFFFFFFFu;
+        cur = r.exact ? exact_root : w.root;  // the root has been entered (bvh.rs:458-461)
+        sp = 0;
+        budget = m.node_count;
+        active = true;
       }
     }
     const unsigned act = __ballot_sync(0xffffffffu, active);
@@ -403,7 +453,7 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
         }
       }
       if (cur == 0u) {
-        if (best != 0xFFFFFFFFu) {  // stage 1 already wrote the miss answer
+        if (best != 0xFFFFFFFFu) {  // the miss answer has been written
           if (kAny) {
             reinterpret_cast<uint8_t*>(prim)[idx] = 1;
           } else {
@@ -625,14 +675,28 @@ static bool aligned(const void* p, uintptr_t a) { return (reinterpret_cast<uintp
 
 // Resident 128-thread blocks per SM of the persistent traversal (the same on every B200);
 // computed once, thread-safely, by the first launch.
-template <bool kRec, bool kAny>
+template <int kFrom, bool kAny>
 static int walk_blocks_per_sm() {
   static const int v = [] {
     int b = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_mesh_walk<kRec, kAny>, 128, 0);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_mesh_walk<kFrom, kAny>, 128, 0);
     return e == cudaSuccess && b > 0 ? b : 4;
   }();
   return v;
+}
+
+// The walk over the survivors of n rays (kPlanes: over all of them).
+template <int kFrom, bool kAny>
+static cudaError_t walk(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
+                        uint32_t* prim, float* t, uint32_t* obj, const uint32_t* queue, unsigned long long* counters,
+                        uint32_t* err, int sm_count, cudaStream_t s, const float4* rec) {
+  const uint64_t full = uint64_t(sm_count) * walk_blocks_per_sm<kFrom, kAny>();
+  const uint64_t need = (n + 127) / 128;
+  const TraversalSchedule ts = traversal_schedule();
+  k_mesh_walk<kFrom, kAny><<<unsigned(need < full ? need : full), 128, 0, s>>>(
+      m, w, rays, stride, queue, counters, prim, t, obj, counters + 1, err, rec, n, ts.leaf_arg(), ts.refill_min,
+      ts.burst_arg());
+  return cudaGetLastError();
 }
 
 // The two stages over n rays; kAny: `prim` is the occlusion buffer, t and obj are NULL.
@@ -663,13 +727,7 @@ static cudaError_t two_stage(const MeshView& m, const WideView& w, const float* 
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  const uint64_t full = uint64_t(sm_count) * walk_blocks_per_sm<kRec, kAny>();
-  const uint64_t need = (n + 127) / 128;
-  const TraversalSchedule ts = traversal_schedule();
-  k_mesh_walk<kRec, kAny><<<unsigned(need < full ? need : full), 128, 0, s>>>(
-      m, w, rays, stride, queue, counters, prim, t, obj, counters + 1, err, rec, ts.leaf_arg(), ts.refill_min,
-      ts.burst_arg());
-  return cudaGetLastError();
+  return walk<kRec ? kRecords : kQueue, kAny>(m, w, rays, stride, n, prim, t, obj, queue, counters, err, sm_count, s, rec);
 }
 
 cudaError_t launch_mesh_closest_persistent(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
@@ -706,6 +764,20 @@ static cudaError_t launch_few(const MeshView& m, const WideView& w, const float*
   const uint32_t lanes = few_lanes(n, sm_count);
   k_mesh_few<kAny><<<grid_for(n, int(4 * lanes), sm_count), 128, 0, s>>>(m, w, rays, stride, n, prim, t, obj, err, lanes);
   return cudaGetLastError();
+}
+
+cudaError_t launch_mesh_closest_planes(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
+                                       uint32_t* prim, float* t, uint32_t* obj, uint32_t* err, int sm_count,
+                                       cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  return walk<kPlanes, false>(m, w, rays, stride, n, prim, t, obj, nullptr, nullptr, err, sm_count, s, nullptr);
+}
+
+cudaError_t launch_mesh_any_planes(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
+                                   uint8_t* occ, uint32_t* err, int sm_count, cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  return walk<kPlanes, true>(m, w, rays, stride, n, reinterpret_cast<uint32_t*>(occ), nullptr, nullptr, nullptr, nullptr, err,
+                             sm_count, s, nullptr);
 }
 
 cudaError_t launch_mesh_closest_few(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,

@@ -208,3 +208,60 @@ def test_sheets_met_at_grazing_angles(merged, seed):
     for _ in range(6):
         hit, _ = _same(s, _grazing(rng, 2_000_000, turn, 2.0, 1e-5))
         assert hit.mean() > 0.3
+
+
+def _call(ctx, s, rays, out):
+    """One asynchronous query on the context's stream: nearest hits into (prim, t, obj) or occlusion into (occ,)."""
+    n = rays.shape[1]
+    if len(out) == 1:
+        ctx.check(ctx.lib.pbrt_trace_any(s.h, rays.data_ptr(), n, out[0].data_ptr()), "any")
+    else:
+        ctx.check(ctx.lib.pbrt_trace_closest(s.h, rays.data_ptr(), n, *[x.data_ptr() for x in out]), "closest")
+
+
+def _outputs(n, kind):
+    if kind == "any":
+        return (torch.full((n,), 7, dtype=torch.uint8, device="cuda"),)
+    return (torch.full((n,), 7, dtype=torch.int32, device="cuda"), torch.full((n,), 7.0, device="cuda"),
+            torch.full((n,), 7, dtype=torch.int32, device="cuda"))
+
+
+@pytest.mark.parametrize("n", [(1 << 18) + 1, 600_000, (1 << 24) + 300_001])
+def test_captured_calls_use_nothing_shared(n):
+    """Nearest hits and occlusion of more rays than one small kernel takes, recorded into graphs, replayed
+    on one stream while eager calls of other rays run on another: each its own answers, every time."""
+    v, f = W.displaced_icosphere(5, seed=4)
+    ctx = pb.Context(0)
+    s = pb.Scene(ctx).add_object(pb.Simple(pb.TriangleMesh(v, f))).commit(bvh_bins=16, bvh_max_leaf=4)
+    base = [W.incoherent_rays(600_000, v.min(0), v.max(0), seed=k) for k in (5, 6)]
+    mine = torch.from_numpy(base[0]).cuda()[:, torch.arange(n, device="cuda") % 600_000].contiguous()
+    other = torch.from_numpy(base[1]).cuda()
+    torch.cuda.synchronize()
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    want = {}
+    for kind in ("closest", "any"):
+        for name, rays in (("mine", mine), ("other", other)):
+            want[kind, name] = [x.clone() for x in (s.intersect(rays, with_object=True) if kind == "closest" else
+                                                    [s.intersect_p(rays)])]
+    for kind in ("closest", "any"):
+        out = _outputs(n, kind)
+        torch.cuda.synchronize()
+        ctx.set_stream(first.cuda_stream)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=first):
+            _call(ctx, s, mine, out)
+        ctx.set_stream(second.cuda_stream)
+        for eager in ("any", "closest"):
+            for _ in range(3):
+                for x in out:
+                    x.fill_(7)
+                beside = _outputs(600_000, eager)
+                torch.cuda.synchronize()
+                with torch.cuda.stream(first):
+                    g.replay()
+                _call(ctx, s, other, beside)
+                torch.cuda.synchronize()
+                assert all(torch.equal(a, b) for a, b in zip(out, want[kind, "mine"]))
+                assert all(torch.equal(a, b) for a, b in zip(beside, want[eager, "other"]))
+        ctx.set_stream(None)
+        del g
