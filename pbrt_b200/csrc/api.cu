@@ -56,17 +56,16 @@ int ensure_queue(pbrt_ctx* c) {
   return PBRT_OK;
 }
 
-// The survivor queue is the context's: a call on another stream than the last asynchronous one
-// waits for that one's use of it.
+// The survivor queue is the context's: a call waits for the last asynchronous call's use of it,
+// whatever the stream (one created after that call's was destroyed may have the same handle).
 int acquire_queue(pbrt_ctx* c, cudaStream_t st) {
-  if (!c->queue_used || c->queue_stream == st) return PBRT_OK;
+  if (!c->queue_used) return PBRT_OK;
   return c->cuda(cudaStreamWaitEvent(st, c->queue_used, 0), "cudaStreamWaitEvent(survivor queue)");
 }
 
 int release_queue(pbrt_ctx* c, cudaStream_t st) {
   if (!c->queue_used)
     PBRT_TRY(c->cuda(cudaEventCreateWithFlags(&c->queue_used, cudaEventDisableTiming), "cudaEventCreate"));
-  c->queue_stream = st;
   return c->cuda(cudaEventRecord(c->queue_used, st), "cudaEventRecord(survivor queue)");
 }
 

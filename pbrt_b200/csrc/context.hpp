@@ -102,8 +102,7 @@ struct pbrt_ctx {
                                              // [8..10] rays / shadow rays / paths of the last render
   uint32_t* queue = nullptr;                  // survivor queue for device-buffer calls (kDevChunk entries)
   float4* queue_rec = nullptr;                // and their ray records (kDevChunk x 32 bytes)
-  cudaEvent_t queue_used = nullptr;           // the queue's last asynchronous use,
-  cudaStream_t queue_stream = nullptr;        // and its stream
+  cudaEvent_t queue_used = nullptr;           // the queue's last asynchronous use
   bool persistent = true;                     // persistent dynamic-fetch traversal (default)
   uint32_t* noalloc_scratch = nullptr;        // device address of pbrt_trace_closest_noalloc's static
                                               // scratch array on this device, looked up at creation

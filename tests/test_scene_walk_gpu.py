@@ -265,3 +265,33 @@ def test_captured_calls_use_nothing_shared(n):
                 assert all(torch.equal(a, b) for a, b in zip(beside, want[eager, "other"]))
         ctx.set_stream(None)
         del g
+
+
+def test_survivor_queue_across_streams_that_come_and_go():
+    """Asynchronous calls on streams that are destroyed while their work runs: a new stream, which may have
+    an old one's handle, waits for that work's use of the survivor queue all the same."""
+    import ctypes
+
+    import torch.cuda
+
+    rt = torch.cuda.cudart()
+    v, f = W.displaced_icosphere(5, seed=4)
+    ctx = pb.Context(0)
+    s = pb.Scene(ctx).add_object(pb.Simple(pb.TriangleMesh(v, f))).commit(bvh_bins=16, bvh_max_leaf=4)
+    n = 1_500_000
+    rays = [torch.from_numpy(W.incoherent_rays(n, v.min(0), v.max(0), seed=k)).cuda() for k in (5, 6)]
+    torch.cuda.synchronize()
+    want = [s.intersect(r, with_object=True) for r in rays]
+    for _ in range(6):
+        outs = [_outputs(n, "closest") for _ in rays]
+        torch.cuda.synchronize()
+        for r, out in zip(rays, outs):
+            st = ctypes.c_void_p()
+            assert int(rt.cudaStreamCreate(ctypes.addressof(st))) == 0
+            ctx.set_stream(st.value)
+            _call(ctx, s, r, out)
+            ctx.set_stream(None)
+            assert int(rt.cudaStreamDestroy(st.value)) == 0
+        torch.cuda.synchronize()
+        for out, w in zip(outs, want):
+            assert all(torch.equal(a, b) for a, b in zip(out, w))
