@@ -581,9 +581,7 @@ int pbrt_scene_create_many(pbrt_ctx* c, const pbrt_scene_desc* descs, uint32_t n
 void pbrt_scene_destroy(pbrt_scene* s) {
   if (!s) return;
   DeviceGuard g(s->ctx->device);
-  // every stream's work: a call may still run on a stream the context used before (and pool
-  // memory, unlike cudaMalloc's, is freed without waiting for anyone)
-  cudaDeviceSynchronize();
+  wait_for_device();
   for (void* p : s->allocs) cudaFree(p);
   delete s;
 }

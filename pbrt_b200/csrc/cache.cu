@@ -54,11 +54,10 @@ int pbrt_cache::take_bytes(void** p, size_t bytes) {
   return ctx->cuda(cudaStreamSynchronize(ctx->stream), "cudaMalloc(cache)");
 }
 
-// After every stream's work: freeing pool memory waits for nobody.
 void pbrt_cache::give_back(std::initializer_list<void*> blocks) {
   bool any = false;
   for (void* p : blocks) any |= p != nullptr;
-  if (any) cudaDeviceSynchronize();
+  if (any) wait_for_device();
   for (void* p : blocks) cudaFree(p);
 }
 

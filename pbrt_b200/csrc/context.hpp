@@ -178,6 +178,20 @@ struct pbrt_scene {
 namespace pbrt {
 namespace api {
 
+// Waits for all of the device's work, as freeing ordinary memory does: memory of a pool is freed
+// without waiting for anyone, and a call may still run on a stream the context used before.
+// (cudaDeviceSynchronize would break off a capture that another thread has under way in its own
+// mode; this does not. 4 us on an idle device.)
+inline void wait_for_device() {
+  void* p = nullptr;
+  if (cudaMalloc(&p, 1) == cudaSuccess) {
+    cudaFree(p);
+  } else {
+    cudaGetLastError();
+    cudaDeviceSynchronize();
+  }
+}
+
 // Reads and clears the device error word after the work that may have raised it.
 inline int check_device_error(pbrt_ctx* c, cudaStream_t s) {
   PBRT_TRY(c->cuda(cudaStreamSynchronize(s), "kernel execution"));

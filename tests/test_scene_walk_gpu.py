@@ -295,3 +295,31 @@ def test_survivor_queue_across_streams_that_come_and_go():
         torch.cuda.synchronize()
         for out, w in zip(outs, want):
             assert all(torch.equal(a, b) for a, b in zip(out, w))
+
+
+def test_scenes_and_caches_destroyed_while_another_thread_captures():
+    """A thread that destroys a scene and a cache leaves another thread's capture alone."""
+    import threading
+
+    from pbrt_b200.cache import RadianceCache
+
+    v, f = W.displaced_icosphere(4, seed=4)
+    scene = pb.Scene(pb.Context(0)).add_object(pb.Simple(pb.TriangleMesh(v, f))).commit()
+    other = pb.Context(0)
+    doomed = pb.Scene(other).add_object(pb.Simple(pb.TriangleMesh(v, f))).commit()
+    cache = RadianceCache((0.0,) * 3, (1.0,) * 3, ctx=other)
+    rays = torch.from_numpy(W.incoherent_rays(5000, v.min(0), v.max(0), seed=3)).cuda()
+    torch.cuda.synchronize()
+    want = scene.intersect(rays, with_object=True)
+    out, st, g = _outputs(5000, "closest"), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    scene.ctx.set_stream(st.cuda_stream)
+    with torch.cuda.graph(g, stream=st, capture_error_mode="thread_local"):
+        _call(scene.ctx, scene, rays, out)
+        t = threading.Thread(target=lambda: (doomed.release(), cache.close()))
+        t.start()
+        t.join()
+    scene.ctx.set_stream(None)
+    g.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(out, want))
