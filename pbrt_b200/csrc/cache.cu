@@ -46,9 +46,8 @@ std::vector<float> initial_weights(uint64_t seed) {
 
 }  // namespace
 
-// Memory comes from the context's pool, as a scene's does: a cached frame's query buffers are
-// hundreds of megabytes, and a new cache whose first frame maps them anew waits for that. The
-// pointer is good on every stream once this returns.
+// Memory comes from the context's pool, as a scene's does: a new cache maps none. The pointer is
+// good on every stream once this returns.
 int pbrt_cache::take_bytes(void** p, size_t bytes) {
   PBRT_TRY(ctx->cuda(cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream), "cudaMalloc(cache)"));
   return ctx->cuda(cudaStreamSynchronize(ctx->stream), "cudaMalloc(cache)");
@@ -69,6 +68,7 @@ int pbrt_cache::device_arrays() {
   PBRT_TRY(take(&grad, P * 4));
   PBRT_TRY(take(&wfwd, P * 2));
   PBRT_TRY(take(&wbwd, P * 2));
+  PBRT_TRY(take(&wsnap, P * 2));
   // pinned host memory: the gradient's last kernel writes the loss where the caller reads it
   return ctx->cuda(cudaHostAlloc(&loss, 4, cudaHostAllocMapped), "cudaHostAlloc(cache)");
 }
@@ -132,88 +132,34 @@ int pbrt_cache::query_device(const float* records, uint64_t n, float* rgb, cudaS
   return ctx->cuda(mlp::launch_infer(net, bounds(), records, n, rgb, ctx->d_err, ctx->sm_count, s), "cache query");
 }
 
-int pbrt_cache::ensure_render_buffers(uint32_t queries, uint32_t train_vertices, uint32_t batch) {
-  if (render_block && qcap >= queries && cw.tcap >= train_vertices && bcap >= batch) return PBRT_OK;
-  queries = std::max(queries, qcap);
+int pbrt_cache::ensure_train_buffers(uint32_t train_vertices, uint32_t batch) {
+  if (train_block && cw.tcap >= train_vertices && bcap >= batch) return PBRT_OK;
   train_vertices = std::max(train_vertices, cw.tcap);
   batch = std::max(batch, bcap);
-  give_back({render_block});
-  render_block = nullptr;
-  qcap = bcap = 0;
+  give_back({train_block});
+  train_block = nullptr;
+  bcap = 0;
   cw = pbrt::CacheWave{};
   const size_t R = pbrt::kCacheRecordFloats * 4;
   auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
-  const size_t bytes = up(64) + up(size_t(queries) * R) + up(size_t(queries) * 12) + up(size_t(queries) * 4) +
-                       up(size_t(train_vertices) * R) + up(size_t(train_vertices) * 24) +
+  const size_t bytes = up(64) + up(size_t(train_vertices) * R) + up(size_t(train_vertices) * 24) +
                        up(size_t(train_vertices) * 4) + up(size_t(batch) * R) + up(size_t(batch) * 12);
-  PBRT_TRY(take(&render_block, bytes));
-  char* p = static_cast<char*>(render_block);
+  PBRT_TRY(take(&train_block, bytes));
+  char* p = static_cast<char*>(train_block);
   auto part = [&](size_t b) { char* r = p; p += up(b); return r; };
   cw.counts = reinterpret_cast<uint32_t*>(part(64));
-  cw.qrec = reinterpret_cast<float*>(part(size_t(queries) * R));
-  cw.qout = reinterpret_cast<float*>(part(size_t(queries) * 12));
-  cw.qpath = reinterpret_cast<uint32_t*>(part(size_t(queries) * 4));
   cw.trec = reinterpret_cast<float*>(part(size_t(train_vertices) * R));
   cw.tstate = reinterpret_cast<float*>(part(size_t(train_vertices) * 24));
   cw.tpath = reinterpret_cast<uint32_t*>(part(size_t(train_vertices) * 4));
   cw.tcap = train_vertices;
-  cw.qcap = queries;
   brec = reinterpret_cast<float*>(part(size_t(batch) * R));
   btgt = reinterpret_cast<float*>(part(size_t(batch) * 12));
-  qcap = queries;
   bcap = batch;
   return PBRT_OK;
 }
 
-int pbrt_cache::ensure_frame_buffers(uint32_t queries) {
-  if (frame_block && fqcap >= queries) return PBRT_OK;
-  give_back({frame_block});
-  frame_block = nullptr;
-  fqcap = 0;
-  fcw = pbrt::CacheWave{};
-  const size_t R = pbrt::kCacheRecordFloats * 4;
-  auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
-  const size_t bytes =
-      up(64) + up(size_t(queries) * R) + up(size_t(queries) * 12) + up(size_t(queries) * 4) + up(mlp::kParams * 2);
-  PBRT_TRY(take(&frame_block, bytes));
-  char* p = static_cast<char*>(frame_block);
-  auto part = [&](size_t b) { char* r = p; p += up(b); return r; };
-  fcw.counts = reinterpret_cast<uint32_t*>(part(64));
-  fcw.qrec = reinterpret_cast<float*>(part(size_t(queries) * R));
-  fcw.qout = reinterpret_cast<float*>(part(size_t(queries) * 12));
-  fcw.qpath = reinterpret_cast<uint32_t*>(part(size_t(queries) * 4));
-  fcw.qcap = queries;  // no training vertices: the frame only queries
-  wsnap = reinterpret_cast<uint16_t*>(part(mlp::kParams * 2));
-  fqcap = queries;
-  return PBRT_OK;
-}
-
-int pbrt_cache::ensure_branch_buffers(uint32_t slot, uint32_t queries) {
-  if (slot >= kBranchSlots) return ctx->fail(PBRT_ERR_INVALID_ARGUMENT, "no such frame branch");
-  if (branch_block[slot] && branch_qcap[slot] >= queries) return PBRT_OK;
-  give_back({branch_block[slot]});
-  branch_block[slot] = nullptr;
-  branch_qcap[slot] = 0;
-  pbrt::CacheWave& q = bcw[slot];
-  q = pbrt::CacheWave{};
-  const size_t R = pbrt::kCacheRecordFloats * 4;
-  auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
-  const size_t bytes = up(64) + up(size_t(queries) * R) + up(size_t(queries) * 12) + up(size_t(queries) * 4);
-  PBRT_TRY(take(&branch_block[slot], bytes));
-  char* p = static_cast<char*>(branch_block[slot]);
-  auto part = [&](size_t b) { char* r = p; p += up(b); return r; };
-  q.counts = reinterpret_cast<uint32_t*>(part(64));
-  q.qrec = reinterpret_cast<float*>(part(size_t(queries) * R));
-  q.qout = reinterpret_cast<float*>(part(size_t(queries) * 12));
-  q.qpath = reinterpret_cast<uint32_t*>(part(size_t(queries) * 4));
-  q.qcap = queries;  // queries only, like the frame's own buffers
-  branch_qcap[slot] = queries;
-  return PBRT_OK;
-}
-
 void pbrt_cache::release() {
-  give_back({w, m, v, grad, wfwd, wbwd, partials, tile_loss, render_block, frame_block});
-  for (void* p : branch_block) give_back({p});
+  give_back({w, m, v, grad, wfwd, wbwd, wsnap, partials, tile_loss, train_block});
   cudaFreeHost(loss);
 }
 

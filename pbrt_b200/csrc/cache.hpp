@@ -21,27 +21,14 @@ struct pbrt_cache {
   uint32_t step = 0;
   uint64_t rounds = 0;  // training rounds run by cached renders (keys their path streams)
 
-  // the cached render's buffers: queries, training vertices and one training batch
-  void* render_block = nullptr;
-  uint32_t qcap = 0, bcap = 0;
+  // the cached render's training vertices and one training batch (its queries are the context's)
+  void* train_block = nullptr;
+  uint32_t bcap = 0;
   pbrt::CacheWave cw{};
   float *brec = nullptr, *btgt = nullptr;
-  int ensure_render_buffers(uint32_t queries, uint32_t train_vertices, uint32_t batch);
-
-  // A call that trains and renders: the frame's own query buffers and the snapshot of the
-  // forward weights it reads, while the training rounds (with `cw`) update the weights.
-  void* frame_block = nullptr;
-  uint32_t fqcap = 0;
-  pbrt::CacheWave fcw{};
+  int ensure_train_buffers(uint32_t train_vertices, uint32_t batch);
+  // the weights a frame reads while training rounds beside it update them
   uint16_t* wsnap = nullptr;
-  int ensure_frame_buffers(uint32_t queries);
-
-  // The query buffers of a frame's concurrent branches 1.. (branch 0 takes fcw or cw).
-  static constexpr uint32_t kBranchSlots = 7;
-  void* branch_block[kBranchSlots] = {};
-  uint32_t branch_qcap[kBranchSlots] = {};
-  pbrt::CacheWave bcw[kBranchSlots] = {};
-  int ensure_branch_buffers(uint32_t slot, uint32_t queries);
 
   int take_bytes(void** p, size_t bytes);
   template <class T>

@@ -79,6 +79,14 @@ struct WaveAlloc {
   void* block = nullptr;
   uint32_t capacity = 0;
   WaveBuffers w{};
+  // a cached render's queries: one per path at most (ensure_queries), whichever cache they are for
+  void* qblock = nullptr;
+  uint32_t qcap = 0;
+  CacheWave q{};
+  void release() {
+    cudaFree(block);
+    cudaFree(qblock);
+  }
 };
 
 }  // namespace api
@@ -211,6 +219,7 @@ inline int check_device_error(pbrt_ctx* c, cudaStream_t s) {
 namespace pbrt {
 namespace api {
 int ensure_wave(pbrt_ctx* c, WaveAlloc* wa, uint32_t cap);
+int ensure_queries(pbrt_ctx* c, WaveAlloc* wa, uint32_t cap);
 // Validation of render parameters shared by every render entry point.
 int check_render_params(pbrt_ctx* c, const pbrt_render_params* p, bool allow_no_samples);
 // The kernels' settings for these parameters on this context (tuning, counters).

@@ -142,3 +142,24 @@ def test_training_beside_the_frame(cornell):
         np.testing.assert_allclose(got, want, rtol=1e-12, atol=1e-15)
         w1 = a.weights()
         assert np.isfinite(w1).all() and not np.array_equal(w1, w0)
+
+
+def test_a_cached_frame_holds_what_it_uses():
+    """A frame that trains beside itself holds a query (80 bytes) and a path's state (136 bytes) per path,
+    in two halves, and the rounds' own buffers: no block sized for a frame that another one serves."""
+    import torch
+
+    from pbrt_b200 import Context
+
+    desc, cam = cornell_box(960, 540)
+    ctx = Context(0)
+    scene = Scene.from_description(desc, ctx).commit()
+    lo, hi = np.float32([-1.5] * 3), np.float32([1.5] * 3)
+    paths = 960 * 540 * 2
+    film = torch.zeros(540, 960, 3, dtype=torch.float64, device="cuda")
+    cache = RadianceCache(lo, hi, ctx=ctx)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    scene.render_cached(cache, cam, 2, 8, seed=1, film=film)
+    used = before - torch.cuda.mem_get_info()[0]
+    assert used < 1.1 * paths * (80 + 136) + (96 << 20), f"{used / 1e6:.0f} MB for {paths} paths"
