@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
   bool active = false, exhausted = false;  // exhausted is warp-uniform
   uint32_t idx = 0;
   WRay r;
-  float near = 0.f, lim = 0.f;  // a hit counts below lim
+  float near = 0.f, lim = 0.f;  // a nearest hit counts below lim, any hit up to it
   uint32_t best = 0xFFFFFFFFu, cur = 0, budget = 0;
   int sp = 0;
   WideStack stk;
@@ -388,9 +388,9 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
           far = __ldg(rays + 7 * stride + i);
           idx = uint32_t(i);
         }
-        r = wide_ray(o, d, near, w.bounded);
-        // a hit lies below lim: t <= far, and t < min_t (which starts at FLT_MAX, bvh.rs:459)
-        lim = kAny ? next_up(far) : fminf(FLT_MAX, next_up(far));
+        r = wide_ray(o, d, near, far, w.bounded);
+        // a nearest hit: t <= far, and t < min_t (which starts at FLT_MAX, bvh.rs:459)
+        lim = kAny ? far : fminf(FLT_MAX, next_up(far));
         best = 0xFFFFFFFFu;
         cur = r.exact ? exact_root : w.root;  // the root has been entered (bvh.rs:458-461)
         sp = 0;
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
         if (kAny) {  // (the grid's boxes are wider than a leaf's own)
           float e;
           done = blocking_triangle(tri, tri_c, first, count, r.o, r.d, near, lim) &&
-                 (r.exact || (leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e) && e < lim));
+                 (r.exact || (leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e) && e <= lim));
         } else {
           float t;
           uint32_t id;
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
           best = 0u;
           cur = 0u;
         } else {
-          cur = wide_pop(stk, sp, lim);
+          cur = kAny ? wide_pop_any(stk, sp) : wide_pop(stk, sp, lim);
         }
       } else {
         // up to `burst` nodes before the next vote (fewer when a leaf is reached)
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
             cur = 0u;
             break;
           }
-          cur = r.exact ? binary_step(m.nodes, cur, r, near, lim, stk, sp)
+          cur = r.exact ? binary_step<kAny>(m.nodes, cur, r, near, lim, stk, sp)
                 : kAny  ? wide_step_any(w.wide + cur, r, near, lim, stk, sp)
                         : wide_step(w.exact + cur, r, near, lim, stk, sp);
         }
@@ -490,8 +490,8 @@ __global__ void __launch_bounds__(128) k_mesh_few(MeshView m, WideView w, const 
     uint32_t best = 0xFFFFFFFFu;
     float t = 0.f, entry;
     if (box_hit(pr, rlo, rhi, near, far, entry) && (kAny || entry < FLT_MAX)) {
-      const WRay r = wide_ray(o, d, near, w.bounded);
-      float lim = kAny ? next_up(far) : fminf(FLT_MAX, next_up(far));
+      const WRay r = wide_ray(o, d, near, far, w.bounded);
+      float lim = kAny ? far : fminf(FLT_MAX, next_up(far));
       uint32_t cur = r.exact ? 0u : w.root, budget = m.node_count;
       int sp = 0;
       WideStack stk;
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(128) k_mesh_few(MeshView m, WideView w, const 
         if (kAny) {
           float e;
           if (blocking_triangle(w.tri, w.tri_c, first, count, o, d, near, lim) &&
-              leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e) && e < lim) {
+              leaf_hit(w.nodes + 2 * size_t(__ldg(&w.leaf[first]).x), r, near, e) && e <= lim) {
             best = 0u;
             break;
           }
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(128) k_mesh_few(MeshView m, WideView w, const 
           lim = t;
           best = id;
         }
-        cur = wide_pop(stk, sp, lim);
+        cur = kAny ? wide_pop_any(stk, sp) : wide_pop(stk, sp, lim);
       }
       t = lim;
       if (r.exact) {

@@ -128,23 +128,22 @@ PBRT_DEV bool nearest_in_leaf(const SceneView& s, const WRay& r, float near, uin
   return false;
 }
 
-// Whether the leaf `cur` blocks the ray (lim: just above its far end).
-template <bool kObj, bool kCsg, class Job>
-PBRT_DEV bool blocked_in_leaf(const Job& job, const SceneView& s, const WRay& r, float near, float lim, uint32_t cur,
-                              uint32_t* err) {
+// Whether the leaf `cur` blocks the ray.
+template <bool kObj, bool kCsg>
+PBRT_DEV bool blocked_in_leaf(const SceneView& s, const WRay& r, float near, float far, uint32_t cur, uint32_t* err) {
   const float4* node = nullptr;
   if (kObj && (cur & kObjectRef)) {
     const uint32_t slot = cur & 0x3FFFFFFFu;
-    if (prim_any<kCsg>(s, __ldg(&s.order[slot]), r.o, r.d, near, job.far(), err))
+    if (prim_any<kCsg>(s, __ldg(&s.order[slot]), r.o, r.d, near, far, err))
       node = s.top + 2 * size_t(__ldg(&s.wide.slot_node[slot]));
   } else {
     uint32_t first, count;
     triangle_range(s.wide, cur, first, count);
-    if (blocking_triangle(s.wide.tri, s.wide.tri_c, first, count, r.o, r.d, near, lim))
+    if (blocking_triangle(s.wide.tri, s.wide.tri_c, first, count, r.o, r.d, near, far))
       node = s.wide.nodes + 2 * size_t(__ldg(&s.wide.leaf[first]).x);
   }
   float e;
-  return node && leaf_hit(node, r, near, e) && e < lim;
+  return node && leaf_hit(node, r, near, e) && e <= far;
 }
 
 // ---- many rays: persistent warps ----------------------------------------------------------------
@@ -168,7 +167,7 @@ PBRT_DEV void walk_nearest(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err
         job.load(k, o, d);
         const SceneView& s = job.scene();
         const float near = job.near(), far = job.far();
-        r = wide_ray(o, d, near, s.wide.bounded);
+        r = wide_ray(o, d, near, far, s.wide.bounded);
         best = Nearest{far, false};
         if (kObj && !r.exact) {
           for (uint32_t u = 0; u < s.unbounded_count; ++u) {  // nearest_among + closer (scene.rs:222-249)
@@ -232,7 +231,7 @@ template <bool kObj, bool kCsg, class Job>
 PBRT_DEV void walk_any(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err) {
   bool active = false;
   WRay r;
-  float lim = 0.f;  // a hit lies below it: just above far
+  float far = 0.f;
   uint32_t cur = 0, budget = 0;
   int sp = 0;
   WideStack stk;
@@ -244,9 +243,9 @@ PBRT_DEV void walk_any(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err) {
       if (!active && k < q.n) {
         job.load(k, o, d);
         const SceneView& s = job.scene();
-        const float near = job.near(), far = job.far();
-        r = wide_ray(o, d, near, s.wide.bounded);
-        lim = next_up(far);
+        const float near = job.near();
+        far = job.far();
+        r = wide_ray(o, d, near, far, s.wide.bounded);
         bool hit = false;
         if (kObj && !r.exact)
           for (uint32_t u = 0; u < s.unbounded_count && !hit; ++u)  // any_blocks (scene.rs:170-184)
@@ -271,15 +270,15 @@ PBRT_DEV void walk_any(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err) {
       const float near = job.near();
       bool hit = false;
       if (r.exact) {
-        hit = exact_any<Job, kObj, kCsg, false>(s, r.o, r.d, near, job.far(), err);
+        hit = exact_any<Job, kObj, kCsg, false>(s, r.o, r.d, near, far, err);
         cur = 0u;
       } else if (leaf_step && at_leaf) {
-        hit = blocked_in_leaf<kObj, kCsg>(job, s, r, near, lim, cur, err);
-        cur = hit ? 0u : wide_pop(stk, sp, lim);
+        hit = blocked_in_leaf<kObj, kCsg>(s, r, near, far, cur, err);
+        cur = hit ? 0u : wide_pop_any(stk, sp);
       }
       if (!leaf_step || q.drained) {
         for (int b = 0; b < ws.burst && cur != 0u && !(cur & kLeafRef); ++b)
-          cur = wide_step_any(s.wide.wide + cur, r, near, lim, stk, sp);
+          cur = wide_step_any(s.wide.wide + cur, r, near, far, stk, sp);
         if (--budget == 0u) {
           atomicOr(err, kErrBudget);
           cur = 0u;
@@ -303,9 +302,9 @@ PBRT_DEV void each_nearest(Job& job, uint64_t n, uint32_t* err) {
     F3 o, d;
     job.load(k, o, d);
     const SceneView& s = job.scene();
-    const float near = job.near();
-    const WRay r = wide_ray(o, d, near, s.wide.bounded);
-    Nearest best{job.far(), false};
+    const float near = job.near(), far = job.far();
+    const WRay r = wide_ray(o, d, near, far, s.wide.bounded);
+    Nearest best{far, false};
     uint32_t leaf = 0, prim = 0, cur = s.wide.root, budget = 2u * s.wide.count + 2u;
     int sp = 0;
     WideStack stk;
@@ -338,19 +337,19 @@ PBRT_DEV void each_any(Job& job, uint64_t n, uint32_t* err) {
     F3 o, d;
     job.load(k, o, d);
     const SceneView& s = job.scene();
-    const float near = job.near(), lim = next_up(job.far());
-    const WRay r = wide_ray(o, d, near, s.wide.bounded);
+    const float near = job.near(), far = job.far();
+    const WRay r = wide_ray(o, d, near, far, s.wide.bounded);
     uint32_t cur = s.wide.root, budget = 2u * s.wide.count + 2u;
     int sp = 0;
     WideStack stk;
     bool hit = false;
     if (r.exact) {
-      hit = exact_any<Job, false, false, true>(s, r.o, r.d, near, job.far(), err);
+      hit = exact_any<Job, false, false, true>(s, r.o, r.d, near, far, err);
       cur = 0u;
     }
     while (cur != 0u && !hit) {
       while (cur != 0u && !(cur & kLeafRef)) {
-        cur = wide_step_any(s.wide.wide + cur, r, near, lim, stk, sp);
+        cur = wide_step_any(s.wide.wide + cur, r, near, far, stk, sp);
         if (--budget == 0u) {
           atomicOr(err, kErrBudget);
           cur = 0u;
@@ -358,8 +357,8 @@ PBRT_DEV void each_any(Job& job, uint64_t n, uint32_t* err) {
         }
       }
       if (cur == 0u) break;
-      hit = blocked_in_leaf<false, false>(job, s, r, near, lim, cur, err);
-      if (!hit) cur = wide_pop(stk, sp, lim);
+      hit = blocked_in_leaf<false, false>(s, r, near, far, cur, err);
+      if (!hit) cur = wide_pop_any(stk, sp);
     }
     job.store(hit);
   }

@@ -25,7 +25,8 @@
 //     hit, may be one that the binary order visits first and hits nearer: 1 in 1,000 of the rays
 //     aimed at spheres 10^4 radii away, whose distances round that far.)
 // Rays this arithmetic does not cover (a direction component of zero or outside
-// [2^-40, 2^40], near < 0 or NaN, coordinates beyond 2^40) use the binary nodes from the start.
+// [2^-40, 2^40], near < 0, coordinates beyond 2^40) or whose interval is empty or ends in a NaN use
+// the binary nodes from the start.
 #pragma once
 
 #include <cfloat>
@@ -105,7 +106,7 @@ struct WRay {
   bool exact;  // walks the binary nodes
 };
 
-PBRT_DEV WRay wide_ray(const F3& o, const F3& d, float near, bool bounded) {
+PBRT_DEV WRay wide_ray(const F3& o, const F3& d, float near, float far, bool bounded) {
   WRay r;
   r.o = o;
   r.d = d;
@@ -113,7 +114,7 @@ PBRT_DEV WRay wide_ray(const F3& o, const F3& d, float near, bool bounded) {
   // (sums of magnitudes: a NaN or an infinity anywhere fails them)
   const float so = fabsf(o.x) + fabsf(o.y) + fabsf(o.z), si = fabsf(r.inv.x) + fabsf(r.inv.y) + fabsf(r.inv.z);
   const float least = fminf(fminf(fabsf(r.inv.x), fabsf(r.inv.y)), fabsf(r.inv.z));
-  r.exact = !(bounded && near >= 0.f && so <= kWideLimit && si <= kWideLimit && least >= 1.f / kWideLimit);
+  r.exact = !(bounded && near >= 0.f && near <= far && so <= kWideLimit && si <= kWideLimit && least >= 1.f / kWideLimit);
   return r;
 }
 
@@ -266,8 +267,8 @@ PBRT_DEV void planes(float org, float step, uint32_t lo, uint32_t hi, float o, f
   unpack(fma2(pack(grid<2>(b), grid<3>(b)), kk, cc1), t1[2], t1[3]);
 }
 
-// Entry distances of the four slots of a node (+inf: not hit within [near, lim] or empty).
-PBRT_DEV void slots(const WideNode* nd, const WRay& r, float near, float lim, float (&e)[4], uint32_t (&ref)[4]) {
+// Entry distances of the four slots of a node (+inf: not hit within [near, far] or empty).
+PBRT_DEV void slots(const WideNode* nd, const WRay& r, float near, float far, float (&e)[4], uint32_t (&ref)[4]) {
   float4 a, b, c, d;
   load_node(reinterpret_cast<const float4*>(nd), a, b);
   load_node(reinterpret_cast<const float4*>(nd) + 2, c, d);
@@ -283,7 +284,7 @@ PBRT_DEV void slots(const WideNode* nd, const WRay& r, float near, float lim, fl
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float t0 = fmaxf(max3(x0[i], y0[i], z0[i]), near);
-    const float t1 = fminf(min3(x1[i], y1[i], z1[i]), lim);
+    const float t1 = fminf(min3(x1[i], y1[i], z1[i]), far);
     e[i] = t0 <= t1 && (i % 2 == 0 || ref[i] != 0u) ? t0 : inf;
   }
 }
@@ -324,18 +325,20 @@ PBRT_DEV uint32_t wide_step(const ExactNode* nd, const WRay& r, float near, floa
   return wide_step(nd, r, near, reach, st, sp, e);
 }
 
-// The same for an any-hit walk, whose answer does not depend on the order: the slots hit, in slot
-// order.
-PBRT_DEV uint32_t wide_step_any(const WideNode* nd, const WRay& r, float near, float lim, WideStack& st, int& sp) {
+// The next pending slot of an any-hit walk, whose far end does not change; 0 when none is left.
+PBRT_DEV uint32_t wide_pop_any(const WideStack& st, int& sp) { return sp > 0 ? st.s[--sp].x : 0u; }
+
+// Visits one wide node of an any-hit walk, whose answer does not depend on the order: the slots
+// entered within [near, far], in slot order.
+PBRT_DEV uint32_t wide_step_any(const WideNode* nd, const WRay& r, float near, float far, WideStack& st, int& sp) {
   float k[4];
   uint32_t f[4];
-  wide::slots(nd, r, near, lim, k, f);
+  wide::slots(nd, r, near, far, k, f);
   const float inf = __int_as_float(0x7f800000);
 #pragma unroll
   for (int i = 3; i > 0; --i)
     if (k[i] < inf) wide_push(st, sp, f[i], k[i]);
-  if (k[0] < inf) return f[0];
-  return sp > 0 ? st.s[--sp].x : 0u;
+  return k[0] < inf ? f[0] : wide_pop_any(st, sp);
 }
 
 // The exact test of a leaf's box (its node) for a ray of the wide walk: box_hit where no
@@ -369,15 +372,15 @@ PBRT_DEV bool nearest_triangle(const float4* tri, const float2* tri_c, uint32_t 
   return any;
 }
 
-// Whether some triangle of a leaf is hit within [near, lim).
+// Whether some triangle of a leaf is hit within [near, far].
 PBRT_DEV bool blocking_triangle(const float4* tri, const float2* tri_c, uint32_t first, uint32_t count, const F3& o,
-                                const F3& d, float near, float lim) {
+                                const F3& d, float near, float far) {
   for (uint32_t k = first; k < first + count; ++k) {
     float4 A, B;
     load_node(&tri[2 * size_t(k)], A, B);
     const float2 C = __ldg(&tri_c[k]);
     float t;
-    if (tri_hit(o, d, A, B, C.x, t) && t >= near && t < lim) return true;
+    if (tri_hit(o, d, A, B, C.x, t) && t >= near && t <= far) return true;
   }
   return false;
 }
@@ -388,8 +391,9 @@ PBRT_DEV uint32_t binary_ref(const float4& lo, const float4& hi, uint32_t node) 
   return __float_as_uint(hi.w) ? kLeafRef | node : __float_as_uint(lo.w) >> 1;
 }
 
-// Visits a sibling pair: the children hit with an entry below lim, the right one first only when
-// strictly nearer (bvh.rs:503-506).
+// Visits a sibling pair: the children hit with an entry below lim (any hit: up to it), the right one
+// first only when strictly nearer (bvh.rs:503-506).
+template <bool kAny>
 PBRT_DEV uint32_t binary_step(const float4* nodes, uint32_t pair, const WRay& r, float near, float lim, WideStack& st,
                               int& sp) {
   const float4* n = nodes + 4 * size_t(pair);
@@ -406,12 +410,12 @@ PBRT_DEV uint32_t binary_step(const float4* nodes, uint32_t pair, const WRay& r,
   const bool hn = swap ? hr : hl, hf = swap ? hl : hr;
   const float dn = swap ? dr : dl, df = swap ? dl : dr;
   const uint32_t fn = swap ? fr : fl, ff = swap ? fl : fr;
-  const bool take_n = hn && dn < lim, take_f = hf && df < lim;
+  const bool take_n = hn && (kAny ? !(lim < dn) : dn < lim), take_f = hf && (kAny ? !(lim < df) : df < lim);
   if (take_n) {
     if (take_f) wide_push(st, sp, ff, df);
     return fn;
   }
-  return take_f ? ff : wide_pop(st, sp, lim);
+  return take_f ? ff : kAny ? wide_pop_any(st, sp) : wide_pop(st, sp, lim);
 }
 
 }  // namespace pbrt

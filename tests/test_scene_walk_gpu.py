@@ -323,3 +323,33 @@ def test_scenes_and_caches_destroyed_while_another_thread_captures():
     g.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(out, want))
+
+
+@pytest.mark.parametrize("n", [1000, 300_000])
+def test_occlusion_at_an_infinite_distance(n):
+    """A short direction puts a hit's parameter beyond the largest float: it lies within [tmin, inf]."""
+    v = np.array([[-1, -1, 1], [1, -1, 1], [0, 1, 1]], np.float32) * np.float32(1e15)
+    s = _commit([pb.Simple(pb.TriangleMesh(v, np.array([[0, 1, 2]], np.uint32)))])
+    rng = np.random.default_rng(3)
+    base = np.zeros((8, 1000), np.float32)
+    base[0:2] = rng.uniform(-1e14, 1e14, (2, 1000))
+    base[5] = 10.0 ** rng.uniform(-30, -15, 1000)
+    base[7] = np.where(rng.random(1000) < 0.5, np.inf, 1e30)
+    r = np.ascontiguousarray(base[:, np.arange(n) % 1000])
+    want, _ = s.intersect_p_counted(r)
+    assert np.array_equal(s.intersect_p(r), want)
+    assert np.array_equal(s.intersect_p(torch.from_numpy(r).cuda()).cpu().numpy(), want)
+    assert 0 < want.sum() < n and want[np.isinf(r[7]) & (r[5] < 1e-24)].any()
+
+
+def test_intervals_that_are_not_numbers_among_objects():
+    rng = np.random.default_rng(9)
+    objects, at = _analytic(rng)
+    objects = objects + [pb.Simple(pb.TriangleMesh(*W.displaced_icosphere(3, seed=9)))]
+    plane = [pb.Transformed(pb.Simple(pb.Plane()), TR.translation([0.0, -2.0, 0.0]))]
+    for scene in (objects, objects + plane, [pb.Simple(pb.Sphere(1.0))]):
+        rays = _rays(rng, 24_000, 3.0, at)
+        for k, (row, x) in enumerate([(6, np.nan), (7, np.nan), (7, np.inf), (7, -np.inf), (6, np.inf), (6, -np.inf),
+                                      (7, -1.0), (7, 0.0)]):
+            rays[row, k::8] = x
+        _same(_commit(scene), rays)
