@@ -199,27 +199,25 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
   // All meshes' nodes and triangles end to end, and one wide tree: the top level's nodes first
   // (index 0 stays unused), then each mesh's.
   std::vector<uint64_t> node_at(nm + 1, 0), tri_at(nm + 1, 0), wide_at(nm + 1, 0);
-  wide_at[0] = fs.top.size() / 2 + 1;
+  wide_at[0] = 1 + fs.top_wide_count;
   uint32_t deepest = 0;
   for (uint32_t i = 0; i < nm; ++i) {
     const uint64_t slots = built(i) ? (*dev)[i].node_slots : fs.meshes[i].nodes.size();
     node_at[i + 1] = node_at[i] + slots;
     tri_at[i + 1] = tri_at[i] + d->meshes[i].triangle_count;
-    wide_at[i + 1] = wide_at[i] + slots / 2 + 1;
+    wide_at[i + 1] = wide_at[i] + (built(i) ? (*dev)[i].wide_count : fs.meshes[i].wide_count);
     deepest = std::max(deepest, fs.meshes[i].stats.max_depth);
   }
   const uint64_t total_nodes = node_at[nm], total_tris = tri_at[nm], total_wide = wide_at[nm];
-  if (total_tris >= (uint64_t(1) << 30) || total_nodes >= (uint64_t(1) << 32) || total_wide >= (uint64_t(1) << 31))
+  if (total_tris >= (uint64_t(1) << 30) || total_nodes >= (uint64_t(1) << 32) || total_wide >= (uint64_t(1) << 30))
     return c->fail(PBRT_ERR_CAPACITY, "a scene holds at most 2^30 triangles");
   const bool direct = total_tris <= (uint64_t(1) << 26);
   s->meshes.resize(nm);
   std::vector<MeshView> views(nm);
   std::vector<MeshShade> shades(nm);
   void *nodes = nullptr, *tri = nullptr, *tri_c = nullptr, *wide = nullptr, *exact = nullptr, *leaf = nullptr;
-  int rc = s->alloc(&wide, total_wide * sizeof(WideNode));
-  if (rc == PBRT_OK) rc = s->alloc(&exact, total_wide * sizeof(ExactNode));
-  if (rc == PBRT_OK && nm) rc = s->alloc(&leaf, total_tris * sizeof(uint2));
-  if (rc == PBRT_OK && nm == 1 && built(0)) {  // the only mesh's arrays are the scene's
+  int rc = PBRT_OK;
+  if (nm == 1 && built(0)) {  // the only mesh's arrays are the scene's
     DeviceMeshBuild& b = (*dev)[0];
     s->take(nodes = b.nodes, total_nodes * sizeof(GpuNode));
     s->take(tri = b.tri, total_tris * 32);
@@ -227,24 +225,54 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
     b.nodes = nullptr;
     b.tri = nullptr;
     b.tri_c = nullptr;
-  } else if (rc == PBRT_OK && nm) {
-    rc = s->alloc(&nodes, total_nodes * sizeof(GpuNode));
-    if (rc == PBRT_OK) rc = s->alloc(&tri, total_tris * 32);
-    if (rc == PBRT_OK) rc = s->alloc(&tri_c, total_tris * 8);
-    for (uint32_t i = 0; i < nm && rc == PBRT_OK; ++i) {
-      const FlatMesh& fm = fs.meshes[i];
-      const bool on_gpu = built(i);
-      const size_t nt = d->meshes[i].triangle_count;
-      auto put = [&](void* dst, size_t at, const void* src, size_t bytes) {
-        return c->cuda(cudaMemcpyAsync(static_cast<char*>(dst) + at, src, bytes, cudaMemcpyDefault, c->stream),
-                       "cudaMemcpy(scene)");
-      };
-      rc = put(nodes, node_at[i] * sizeof(GpuNode), on_gpu ? (const void*)(*dev)[i].nodes : fm.nodes.data(),
-               (node_at[i + 1] - node_at[i]) * sizeof(GpuNode));
-      if (rc == PBRT_OK) rc = put(tri, tri_at[i] * 32, on_gpu ? (const void*)(*dev)[i].tri : fm.tri.data(), nt * 32);
-      if (rc == PBRT_OK) rc = put(tri_c, tri_at[i] * 8, on_gpu ? (const void*)(*dev)[i].tri_c : fm.tri_c.data(), nt * 8);
+  } else if (nm) {
+    // One kind of array after another, a build's own given back behind its copy: no more than one
+    // kind is held twice, and what was given back serves the wide nodes below (as far as the pool
+    // finds it in one piece).
+    std::vector<char> on_gpu(nm);
+    for (uint32_t i = 0; i < nm; ++i) on_gpu[i] = built(i);
+    for (int part = 0; part < 3 && rc == PBRT_OK; ++part) {
+      void** dst = part == 0 ? &nodes : (part == 1 ? &tri : &tri_c);
+      const std::vector<uint64_t>& at = part == 0 ? node_at : tri_at;
+      const size_t each = part == 2 ? 8 : 32;
+      rc = s->alloc(dst, at[nm] * each);
+      for (uint32_t i = 0; i < nm && rc == PBRT_OK; ++i) {
+        const FlatMesh& fm = fs.meshes[i];
+        const void* src = part == 0 ? (const void*)fm.nodes.data() : (part == 1 ? fm.tri.data() : fm.tri_c.data());
+        if (on_gpu[i]) {
+          DeviceMeshBuild& b = (*dev)[i];
+          src = part == 0 ? (const void*)b.nodes : (part == 1 ? (const void*)b.tri : b.tri_c);
+        }
+        rc = c->cuda(cudaMemcpyAsync(static_cast<char*>(*dst) + at[i] * each, src, (at[i + 1] - at[i]) * each,
+                                     cudaMemcpyDefault, c->stream),
+                     "cudaMemcpy(scene)");
+        if (rc == PBRT_OK && on_gpu[i]) {
+          DeviceMeshBuild& b = (*dev)[i];
+          rc = c->cuda(cudaFreeAsync(const_cast<void*>(src), c->stream), "cudaFree(scene)");
+          if (part == 0) b.nodes = nullptr;
+          if (part == 1) b.tri = nullptr;
+          if (part == 2) b.tri_c = nullptr;
+        }
+      }
     }
   }
+  if (rc == PBRT_OK) rc = s->alloc(&wide, total_wide * sizeof(WideNode));
+  if (rc == PBRT_OK) rc = s->alloc(&exact, total_wide * sizeof(ExactNode));
+  if (rc == PBRT_OK && nm) rc = s->alloc(&leaf, total_tris * sizeof(uint2));
+  // A tree's wide nodes, by its own device array of their numbers or a host one.
+  auto widen = [&](WidenArgs a, const std::vector<uint32_t>& id) -> int {
+    void* copy = nullptr;
+    if (!a.wide_id) {
+      PBRT_TRY(c->cuda(cudaMallocFromPoolAsync(&copy, id.size() * 4, c->pool, c->stream), "cudaMalloc(scene)"));
+      a.wide_id = static_cast<const uint32_t*>(copy);
+    }
+    int r = copy ? c->cuda(cudaMemcpyAsync(copy, id.data(), id.size() * 4, cudaMemcpyHostToDevice, c->stream),
+                           "cudaMemcpy(scene)")
+                 : PBRT_OK;
+    if (r == PBRT_OK) r = c->cuda(launch_widen(a, c->sm_count, c->stream), "scene upload");
+    if (copy) cudaFreeAsync(copy, c->stream);
+    return r;
+  };
   // The primitives' references: a mesh placed untransformed, once, is merged (its wide root),
   // anything else is an object leaf.
   std::vector<uint32_t> slot_ref(fs.order.size()), owner(nm, 0xFFFFFFFFu);
@@ -256,7 +284,7 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
       const uint32_t m = ob->mesh;
       owner[m] = ref;
       const uint32_t count = uint32_t(tri_at[m + 1] - tri_at[m]);
-      slot_ref[k] = node_at[m + 1] - node_at[m] > 2 ? uint32_t(wide_at[m]) + 1u  // the root's pair
+      slot_ref[k] = node_at[m + 1] - node_at[m] > 2 ? uint32_t(wide_at[m])  // the root's
                                                     : triangle_ref(uint32_t(tri_at[m]), count, direct);
     } else {
       slot_ref[k] = kLeafRef | kObjectRef | k;
@@ -282,7 +310,8 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
     a.node_base = uint32_t(node_at[i]);
     a.owner = owner[i];
     a.leaf = static_cast<uint2*>(leaf);
-    rc = c->cuda(launch_widen(a, c->sm_count, c->stream), "scene upload");
+    a.wide_id = dev && i < dev->size() ? (*dev)[i].wide_id : nullptr;
+    rc = widen(a, fs.meshes[i].wide_id);
     void* pv = nullptr;
     void* pi = nullptr;
     if (built(i) || (dev && i < dev->size() && (*dev)[i].v)) {  // the build's copies of the mesh's arrays
@@ -375,9 +404,10 @@ int upload_scene(pbrt_ctx* c, const pbrt_scene_desc* d, const FlatScene& fs, pbr
     a.wide = static_cast<WideNode*>(wide);
     a.exact = static_cast<ExactNode*>(exact);
     a.direct = direct;
+    a.wide_base = 1;
     a.slot_ref = (const uint32_t*)srefs;
     a.slot_node = (uint32_t*)snodes;
-    const int rc1 = c->cuda(launch_widen(a, c->sm_count, c->stream), "scene upload");
+    const int rc1 = widen(a, fs.top_wide);
     if (rc1 != PBRT_OK) {
       pbrt_scene_destroy(s.release());
       return rc1;

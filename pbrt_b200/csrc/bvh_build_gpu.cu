@@ -819,19 +819,22 @@ __global__ void k_depth_scatter(const PoolNode* __restrict__ pool, uint32_t n, u
     by_depth[base + __popc(peers & ((1u << lane) - 1u))] = i;
   }
 }
-// subtree sizes, deepest level first
-__global__ void k_sizes(const PoolNode* __restrict__ pool, const uint32_t* __restrict__ ids, uint32_t n,
-                        uint32_t* size) {
+// subtree sizes, deepest level first; and how many of a subtree's nodes become wide nodes (`wide`:
+// this level's interior nodes do)
+__global__ void k_sizes(const PoolNode* __restrict__ pool, const uint32_t* __restrict__ ids, uint32_t n, uint32_t wide,
+                        uint32_t* size, uint32_t* wsize) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const uint32_t i = ids[k];
   const uint32_t c = pool[i].child;
   size[i] = c == kNone ? 1u : 1u + size[c] + size[c + 1];
+  wsize[i] = c == kNone ? 0u : wide + wsize[c] + wsize[c + 1];
 }
 // depth-first indexes, root level first: a node's children take the next two free indexes,
-// its left subtree's descendants follow, then the right's
-__global__ void k_number(const PoolNode* __restrict__ pool, const uint32_t* __restrict__ ids, uint32_t n,
-                         const uint32_t* __restrict__ size, uint32_t* ref, uint32_t* cbase) {
+// its left subtree's descendants follow, then the right's; wide nodes likewise, the node itself first
+__global__ void k_number(const PoolNode* __restrict__ pool, const uint32_t* __restrict__ ids, uint32_t n, uint32_t wide,
+                         const uint32_t* __restrict__ size, const uint32_t* __restrict__ wsize, uint32_t* ref,
+                         uint32_t* cbase, uint32_t* wbase) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const uint32_t i = ids[k];
@@ -842,9 +845,11 @@ __global__ void k_number(const PoolNode* __restrict__ pool, const uint32_t* __re
   ref[c + 1] = b + 1;
   cbase[c] = b + 2;
   cbase[c + 1] = b + 2 + (size[c] - 1u);
+  wbase[c] = wbase[i] + wide;
+  wbase[c + 1] = wbase[c] + wsize[c];
 }
 __global__ void k_layout(const PoolNode* __restrict__ pool, uint32_t n, const uint32_t* __restrict__ ref,
-                         GpuNode* out, uint32_t* stats) {
+                         const uint32_t* __restrict__ wbase, GpuNode* out, uint32_t* wide_id, uint32_t* stats) {
   uint32_t leaves = 0, most = 0, deepest = 0;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const PoolNode& p = pool[i];
@@ -865,6 +870,7 @@ __global__ void k_layout(const PoolNode* __restrict__ pool, uint32_t n, const ui
     }
     deepest = max(deepest, p.depth);
     out[r == 0 ? 0 : r + 1] = g;
+    wide_id[r == 0 ? 0 : r + 1] = p.child != kNone && (p.depth & 1u) ? wbase[i] : kNoWide;
   }
   leaves = __reduce_add_sync(0xFFFFFFFFu, leaves);  // one atomic per warp and figure
   most = __reduce_max_sync(0xFFFFFFFFu, most);
@@ -1042,12 +1048,14 @@ bool build_mesh_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_idx,
   const uint32_t made = h.pool;  // nodes
 
   // renumbering: nodes grouped by depth, subtree sizes bottom-up, indexes top-down
-  uint32_t *hist, *by_depth, *size, *ref, *cbase, *stats;
+  uint32_t *hist, *by_depth, *size, *wsize, *ref, *cbase, *wbase, *stats;
   BUILD_TRY(s.alloc(&hist, 512));
   BUILD_TRY(s.alloc(&by_depth, made));
   BUILD_TRY(s.alloc(&size, made));
+  BUILD_TRY(s.alloc(&wsize, made));
   BUILD_TRY(s.alloc(&ref, made));
   BUILD_TRY(s.alloc(&cbase, made));
+  BUILD_TRY(s.alloc(&wbase, made));
   BUILD_TRY(s.alloc(&stats, 4));
   BUILD_TRY(cudaMemsetAsync(hist, 0, 512 * sizeof(uint32_t), st));
   k_depth_hist<<<grid_for(made, 256, sm_count), 256, 0, st>>>(pool, made, hist);
@@ -1066,25 +1074,29 @@ bool build_mesh_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_idx,
   k_depth_scatter<<<grid_for(made, 256, sm_count), 256, 0, st>>>(pool, made, hist + 256, by_depth);
   for (uint32_t d = maxd; d >= 1; --d) {
     const uint32_t cnt = hh[d];
-    if (cnt) k_sizes<<<(cnt + 255) / 256, 256, 0, st>>>(pool, by_depth + off[d], cnt, size);
+    if (cnt) k_sizes<<<(cnt + 255) / 256, 256, 0, st>>>(pool, by_depth + off[d], cnt, d & 1u, size, wsize);
   }
   const uint32_t zero = 0, one = 1;
   BUILD_TRY(cudaMemcpyAsync(ref, &zero, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   BUILD_TRY(cudaMemcpyAsync(cbase, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+  BUILD_TRY(cudaMemcpyAsync(wbase, &zero, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
   for (uint32_t d = 1; d <= maxd; ++d) {
     const uint32_t cnt = hh[d];
-    if (cnt) k_number<<<(cnt + 255) / 256, 256, 0, st>>>(pool, by_depth + off[d], cnt, size, ref, cbase);
+    if (cnt)
+      k_number<<<(cnt + 255) / 256, 256, 0, st>>>(pool, by_depth + off[d], cnt, d & 1u, size, wsize, ref, cbase, wbase);
   }
   BUILD_TRY(cudaGetLastError());
 
   // outputs
   BUILD_TRY(s.keep(&o.nodes, size_t(made) + 1));
+  BUILD_TRY(s.keep(&o.wide_id, size_t(made) + 1));
   o.node_slots = uint64_t(made) + 1;
   BUILD_TRY(s.keep(&o.tri, size_t(n) * 2));
   BUILD_TRY(s.keep(&o.tri_c, n));
   BUILD_TRY(cudaMemsetAsync(o.nodes + 1, 0, sizeof(GpuNode), st));  // the padding slot
   BUILD_TRY(cudaMemsetAsync(stats, 0, 4 * sizeof(uint32_t), st));
-  k_layout<<<grid_for(made, 256, sm_count), 256, 0, st>>>(pool, made, ref, o.nodes, stats);
+  BUILD_TRY(cudaMemcpyAsync(stats + 3, wsize, sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
+  k_layout<<<grid_for(made, 256, sm_count), 256, 0, st>>>(pool, made, ref, wbase, o.nodes, o.wide_id, stats);
   k_tri_layout<<<grid_for(n, 256, sm_count), 256, 0, st>>>(o.tri_index, n, d_v, d_idx, o.tri, o.tri_c);
   BUILD_TRY(cudaGetLastError());
   uint32_t hs[4] = {0, 0, 0, 0};
@@ -1094,6 +1106,7 @@ bool build_mesh_bvh_device(const float* d_v, uint32_t nv, const uint32_t* d_idx,
   o.stats.leaf_count = hs[0];
   o.stats.max_leaf_tris = hs[1];
   o.stats.max_depth = hs[2];
+  o.wide_count = hs[3];
   for (int a = 0; a < 3; ++a) {
     auto dec = [](uint32_t x) {
       const uint32_t u = (x & 0x80000000u) ? (x & 0x7FFFFFFFu) : ~x;
@@ -1116,6 +1129,7 @@ void free_device_mesh_build(DeviceMeshBuild* b) {
   cudaFree(b->tri);
   cudaFree(b->tri_c);
   cudaFree(b->tri_index);
+  cudaFree(b->wide_id);
   *b = DeviceMeshBuild{};
 }
 

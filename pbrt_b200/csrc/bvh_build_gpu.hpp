@@ -18,6 +18,8 @@ struct DeviceMeshBuild {
   uint32_t* tri_index = nullptr;  // leaf order -> original triangle index
   float* v = nullptr;             // the mesh's own copy of its vertices and indices, for shading
   uint32_t* idx = nullptr;
+  uint32_t* wide_id = nullptr;    // per node: its wide node (number_wide, in an order of its own)
+  uint32_t wide_count = 0;
   MeshBuildStats stats;
   float bounds_min[3] = {0, 0, 0}, bounds_max[3] = {0, 0, 0};  // vertex bounds
 };

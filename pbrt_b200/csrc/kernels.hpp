@@ -42,12 +42,13 @@ cudaError_t launch_mesh_closest_few(const MeshView& m, const WideView& w, const 
 cudaError_t launch_mesh_any_few(const MeshView& m, const WideView& w, const float* rays, uint64_t stride, uint64_t n,
                                 uint8_t* occ, uint32_t* err, int sm_count, cudaStream_t s);
 // One binary tree's part of a scene's wide tree (wide_bvh.cuh): a mesh's (slot_ref NULL), or the
-// top level's. A tree of `count` records (GPU numbering) takes count / 2 + 1 wide nodes.
+// top level's: `wide_id` names each node's wide node (number_wide), from wide_base on.
 struct WidenArgs {
   const float4* nodes;
   uint32_t count;
   WideNode* wide;
   ExactNode* exact;
+  const uint32_t* wide_id;
   uint32_t wide_base;
   bool direct;
   uint32_t tri_base, node_base, owner;  // a mesh: its first triangle, first node and object in the scene's arrays

@@ -22,6 +22,7 @@
 #include <cstring>
 
 #include "kernels.hpp"
+#include "mesh_bvh.hpp"
 #include "tcgen05.cuh"
 #include "trace_mesh.cuh"
 #include "wide_bvh.cuh"
@@ -538,17 +539,16 @@ __global__ void __launch_bounds__(128) k_mesh_few(MeshView m, WideView w, const 
   }
 }
 
-// The wide nodes of a tree: one thread per interior node of the binary tree, which writes the
-// wide node of its children's pair (index base + left_first / 2). Half of them are reached (every
-// second level); the others cost memory, not time. A mesh's leaves become triangle references
-// and note their node and object beside their first triangle; a top-level tree's leaves become
-// their primitive's reference (`slot_ref`: the root of a merged mesh, or an object leaf) and note
-// their node beside the slot.
+// The wide nodes of a tree: one thread per node of the binary tree; those of every second level write
+// the wide node of their grandchildren. A mesh's leaves become triangle references and note their
+// node and object beside their first triangle; a top-level tree's leaves become their primitive's
+// reference (`slot_ref`: the root of a merged mesh, or an object leaf) and note their node beside the
+// slot.
 __global__ void k_widen(WidenArgs a) {
   auto ref_of = [&](uint32_t q) -> uint32_t {
     const uint32_t first = __float_as_uint(__ldg(&a.nodes[2 * size_t(q)]).w);
     const uint32_t count = __float_as_uint(__ldg(&a.nodes[2 * size_t(q) + 1]).w);
-    if (count == 0u) return a.wide_base + (first >> 1);
+    if (count == 0u) return a.wide_base + __ldg(&a.wide_id[q]);
     return a.slot_ref ? __ldg(&a.slot_ref[first]) : triangle_ref(a.tri_base + first, count, a.direct);
   };
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.count; i += gridDim.x * blockDim.x) {
@@ -560,13 +560,14 @@ __global__ void k_widen(WidenArgs a) {
       else a.leaf[a.tri_base + pair] = make_uint2(a.node_base + i, a.owner);
       continue;
     }
-    if (pair < 2u || pair + 1u >= a.count) continue;
+    const uint32_t id = __ldg(&a.wide_id[i]);
+    if (id == kNoWide) continue;
     uint32_t slot[4], ref[4];  // the slots' nodes; a leaf child stands in slot 0 (2), slot 1 (3) is empty
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
       const uint32_t c = pair + side;
       const uint32_t cl = __float_as_uint(__ldg(&a.nodes[2 * size_t(c)]).w);
-      const bool leaf = __float_as_uint(__ldg(&a.nodes[2 * size_t(c) + 1]).w) != 0u || cl + 1u >= a.count;
+      const bool leaf = __float_as_uint(__ldg(&a.nodes[2 * size_t(c) + 1]).w) != 0u;
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
         const int k = 2 * side + g;
@@ -611,8 +612,8 @@ __global__ void k_widen(WidenArgs a) {
       w.ref[k] = x4.ref[k] = ref[k];
       x4.pad[k] = 0u;
     }
-    a.wide[a.wide_base + (pair >> 1)] = w;
-    a.exact[a.wide_base + (pair >> 1)] = x4;
+    a.wide[a.wide_base + id] = w;
+    a.exact[a.wide_base + id] = x4;
   }
 }
 

@@ -228,6 +228,19 @@ class Builder {
 
 }  // namespace
 
+uint32_t number_wide(const std::vector<GpuNode>& nodes, std::vector<uint32_t>* id) {
+  id->assign(nodes.size(), kNoWide);
+  std::vector<uint8_t> odd(nodes.size(), 0);
+  uint32_t next = 0;
+  for (size_t i = 0; i < nodes.size(); ++i) {  // children come after their parent
+    if (i == 1 || nodes[i].count > 0) continue;
+    const uint32_t pair = nodes[i].left_first;
+    odd[pair] = odd[pair + 1] = !odd[i];
+    if (!odd[i]) (*id)[i] = next++;
+  }
+  return next;
+}
+
 bool build_mesh_bvh(const float* vertices, uint32_t vertex_count, const uint32_t* indices, uint32_t tri_count,
                     const MeshBuildParams& params, FlatMesh* out, std::string* err) {
   if (tri_count == 0) { *err = "a TriangleMesh needs at least one triangle"; return false; }
@@ -287,6 +300,7 @@ bool build_mesh_bvh(const float* vertices, uint32_t vertex_count, const uint32_t
       out->bounds_min[a] = std::fmin(vertices[3 * size_t(i) + a], out->bounds_min[a]);
       out->bounds_max[a] = std::fmax(vertices[3 * size_t(i) + a], out->bounds_max[a]);
     }
+  out->wide_count = number_wide(out->nodes, &out->wide_id);
   for (int a = 0; a < 3; ++a) {
     out->bounds_min[a] = canon(out->bounds_min[a]);
     out->bounds_max[a] = canon(out->bounds_max[a]);

@@ -55,7 +55,14 @@ struct FlatMesh {
   std::vector<uint32_t> tri_index; // leaf order -> original triangle index
   float bounds_min[3], bounds_max[3];  // vertex bounds (TriangleMesh::get_bounding_box)
   MeshBuildStats stats;
+  std::vector<uint32_t> wide_id;  // per node: its wide node (number_wide)
+  uint32_t wide_count = 0;
 };
+
+// The interior nodes that a walk two levels at a time visits: those of every second level from the
+// root's on, numbered in the nodes' order (the root 0); kNoWide for the others.
+constexpr uint32_t kNoWide = 0xFFFFFFFFu;
+uint32_t number_wide(const std::vector<GpuNode>& nodes, std::vector<uint32_t>* id);
 
 // Builds and flattens. Returns false with `err` set on invalid input (no triangle, an index
 // out of range, a non-finite vertex).

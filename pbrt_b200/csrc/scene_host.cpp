@@ -609,6 +609,7 @@ bool build_scene(const pbrt_scene_desc& d, FlatScene* out, std::string* err, con
   if (!bounded_boxes.empty()) {
     std::vector<uint32_t> slot;
     TopBuilder(bounded_boxes).run(&out->top, &slot, &out->top_depth);
+    out->top_wide_count = number_wide(out->top, &out->top_wide);
     out->order.resize(slot.size());
     for (size_t k = 0; k < slot.size(); ++k) out->order[k] = bounded_refs[slot[k]];
   }

@@ -30,6 +30,8 @@ struct FlatScene {
   std::vector<uint32_t> unbounded;              // primitives kept out of the BVH, in scene order
   std::vector<GpuNode> top;                     // GPU numbering (root 0, padding 1); empty when no
                                                 // primitive is bounded
+  std::vector<uint32_t> top_wide;               // its nodes' wide nodes (number_wide)
+  uint32_t top_wide_count = 0;
   std::vector<uint32_t> order;                  // leaf slot -> primitive (leaf, or kGroupBit | group)
   uint32_t top_depth = 0;
   uint64_t primitive_count = 0;                 // bounded + unbounded

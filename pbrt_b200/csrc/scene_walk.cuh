@@ -184,7 +184,7 @@ PBRT_DEV void walk_nearest(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err
         cur = s.wide.root;
         if (kObj && (cur & kObjectRef) && (cur & kLeafRef) && !leaf_hit(s.top, r, near, e)) cur = 0u;  // the only primitive
         sp = 0;
-        budget = 2u * s.wide.count + 2u;  // every iteration visits a node or a leaf it has not visited
+        budget = 4u * s.wide.count + 4u;  // every iteration visits a node or a leaf it has not visited
         active = true;
       }
     }
@@ -252,7 +252,7 @@ PBRT_DEV void walk_any(Job& job, WalkQueue q, WalkSchedule ws, uint32_t* err) {
             hit = prim_any<kCsg>(s, __ldg(&s.unbounded[u]), o, d, near, far, err);
         cur = s.wide.root;
         sp = 0;
-        budget = 2u * s.wide.count + 2u;  // every iteration visits a node or a leaf it has not visited
+        budget = 4u * s.wide.count + 4u;  // every iteration visits a node or a leaf it has not visited
         active = !hit;
         if (hit) job.store(true);
       }
@@ -305,7 +305,7 @@ PBRT_DEV void each_nearest(Job& job, uint64_t n, uint32_t* err) {
     const float near = job.near(), far = job.far();
     const WRay r = wide_ray(o, d, near, far, s.wide.bounded);
     Nearest best{far, false};
-    uint32_t leaf = 0, prim = 0, cur = s.wide.root, budget = 2u * s.wide.count + 2u;
+    uint32_t leaf = 0, prim = 0, cur = s.wide.root, budget = 4u * s.wide.count + 4u;
     int sp = 0;
     WideStack stk;
     bool restart = r.exact;
@@ -339,7 +339,7 @@ PBRT_DEV void each_any(Job& job, uint64_t n, uint32_t* err) {
     const SceneView& s = job.scene();
     const float near = job.near(), far = job.far();
     const WRay r = wide_ray(o, d, near, far, s.wide.bounded);
-    uint32_t cur = s.wide.root, budget = 2u * s.wide.count + 2u;
+    uint32_t cur = s.wide.root, budget = 4u * s.wide.count + 4u;
     int sp = 0;
     WideStack stk;
     bool hit = false;

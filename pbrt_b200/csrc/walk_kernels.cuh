@@ -129,11 +129,11 @@ unsigned walk_blocks(const WalkLaunch& l) {
 }
 
 // One thread per ray for a wave of at most kEachMaxPaths in mesh scenes of at most kEachMaxNodes
-// wide nodes. A closed box of 34 triangles (some 40 nodes), two chains of waves, persistent
+// wide nodes. A closed box of 34 triangles (some 20 nodes), two chains of waves, persistent
 // against one thread per ray: 0.52 M paths a wave 1.50 / 1.47 ms, 0.37 M at depth 20 2.48 / 2.19,
 // 0.56 M at depth 6 0.610 / 0.546; but 0.86 M 2.55 / 2.60, 1.7 M 4.23 / 4.86, 3.5 M 7.68 / 9.61.
 // Larger trees are persistent throughout (a torus knot of 95,000 triangles 5.9 / 7.2 ms).
-constexpr uint32_t kEachMaxNodes = 256, kEachMaxPaths = 3u << 18;
+constexpr uint32_t kEachMaxNodes = 128, kEachMaxPaths = 3u << 18;
 inline bool walk_each(const WalkLaunch& l) { return l.nodes <= kEachMaxNodes && l.paths <= kEachMaxPaths; }
 
 template <bool kObj, bool kCsg, bool kEach, class Src>

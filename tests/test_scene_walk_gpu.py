@@ -353,3 +353,16 @@ def test_intervals_that_are_not_numbers_among_objects():
                                       (7, -1.0), (7, 0.0)]):
             rays[row, k::8] = x
         _same(_commit(scene), rays)
+
+
+@pytest.mark.parametrize("device_build", [False, True])
+@pytest.mark.parametrize("leaf", [1, 4])
+def test_memory_of_a_mesh(device_build, leaf):
+    """A mesh's device memory: 58 bytes of arrays and 8 of leaf notes a triangle, 32 a node, and 192 a wide
+    node, of which no interior node of every second level has one."""
+    v, f = W.displaced_icosphere(6, seed=4)
+    s = _commit([pb.Simple(pb.TriangleMesh(v, f))], device_build=device_build, bvh_bins=16, bvh_max_leaf=leaf)
+    i = s.info()
+    interior = i["mesh_node_count"] - i["mesh_leaf_count"]
+    wide = i["device_bytes"] - 66 * len(f) - 32 * i["mesh_node_count"]
+    assert wide < 192 * interior * 0.7, f"{wide / interior:.0f} bytes an interior node"
