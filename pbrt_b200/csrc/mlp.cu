@@ -41,7 +41,6 @@ constexpr int kReduceThreads = 128;
 static_assert(kXBytes >= kHBytes, "the inference kernel stores the hidden tile over the input tile");
 
 __device__ __forceinline__ uint16_t to_bf16(float f) { return __bfloat16_as_ushort(__float2bfloat16_rn(f)); }
-__device__ __forceinline__ float from_bf16(uint16_t b) { return __uint_as_float(uint32_t(b) << 16); }
 // Two values to BF16 (round to nearest even), `a` in the low half: one cvt.rn.bf16x2.f32,
 // whose first source goes to the high half.
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
@@ -524,7 +523,11 @@ __global__ void __launch_bounds__(kGradThreads, 1) k_mlp_grad(Net net, Bounds b,
   }
   if (threadIdx.x == 0) tile_loss[tile] = *s_loss;
   // one more bounded wait for a GEMM or copies still in flight
-  if (!ok) tc::mbar_wait(copied ? mbar : mbar + 2, copied ? phase ^ 1u : 0u, 1u << 20);
+  if (!ok && copied) tc::mbar_wait(mbar, phase ^ 1u, 1u << 20);
+  if (!copied) {
+    tc::mbar_wait(mbar + 1, 0u, 1u << 20);
+    tc::mbar_wait(mbar + 2, 0u, 1u << 20);
+  }
   tc::fence_before_sync();
   __syncthreads();
   if (threadIdx.x < 32) tc::tmem_dealloc(tmem, kTrainTmemCols);
