@@ -239,7 +239,7 @@ int pbrt_mesh_bvh_build_host(const pbrt_mesh_desc* mesh, uint32_t bvh_bins, uint
                              uint64_t node_capacity, uint32_t* tri_order, uint64_t* node_count);
 /* pbrt_mesh_bvh_build_host on the context's GPU: the binned-SAH build of
  * src/shapes/triangle_mesh/bvh.rs:221-309, 609-735 with every node split level by level by
- * many thread blocks (small subtrees by one thread each); it yields the same nodes, in the
+ * many thread blocks (small subtrees by one warp each); it yields the same nodes, in the
  * same numbering, and the same triangle order. The mesh arrays may be host or device
  * memory; nodes and tri_order are host memory. build_ms (may be NULL) receives the device
  * time of the build, input copies included. */

@@ -785,7 +785,7 @@ int trace_impl(pbrt_scene* s, const float* rays, uint64_t n, uint32_t* prim, flo
   // A small host call on one mesh: the rays are copied into pinned memory that one kernel reads,
   // and it writes its answers there, so that no copy engine, no second kernel and no memset stand
   // in its way. (20,480 triangles, nearest hits through the Python call, staged against chunks:
-  // 100 rays 25 / 61 us, 4,099 rays 50 / 106, 32,768 rays 156 / 198.)
+  // 100 rays 26 / 54 us, 4,099 rays 50 / 79, 32,768 rays 160 / 168.)
   if (one_mesh && c->persistent && !counters && n <= kStageRays) {
     if (!c->stage) PBRT_TRY(c->cuda(cudaHostAlloc(&c->stage, kStageBytes, cudaHostAllocMapped), "cudaHostAlloc(stage)"));
     if (c->user) PBRT_TRY(c->cuda(cudaStreamSynchronize(c->user), "cudaStreamSynchronize"));

@@ -22,8 +22,8 @@ constexpr uint64_t kSlotRays = uint64_t(1) << 20;  // rays per pipelined chunk (
 constexpr int kSlots = 3;
 // Rays against one mesh that a single kernel answers, one thread each; more go through the two
 // stages. Us per call, one kernel / two stages, meshes of 1,280 / 20,480 / 327,680 triangles, all
-// rays entering the root: 4,099 rays 34/54, 36/60, 56/83; 262,144 rays 62/74, 83/104, 126/156;
-// 524,288 rays 89/84, 124/116, 159/155; 1,048,576 rays 141/93, 179/131, 218/181.
+// rays entering the root: 4,099 rays 40/59, 40/61, 37/71; 262,144 rays 60/72, 80/101, 123/153;
+// 524,288 rays 85/79, 119/112, 154/154; 1,048,576 rays 134/87, 172/131, 214/182.
 constexpr uint64_t kFewRays = 1u << 18;
 constexpr uint64_t kStageRays = 1u << 15;  // rays of a host call that go through the pinned stage
 constexpr uint64_t kStageBytes = kStageRays * (8 + 3) * 4;

@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(128, PBRT_TRAVERSAL_MIN_BLOCKS) k_mesh_walk(
 // Few rays, one launch and no scratch: `lanes` rays to a warp, each through the root test and its
 // own walk of the wide tree. The answers are the two stages' (see k_mesh_walk). What bounds a
 // small call is the launches and a ray's own chain of node loads, not the lanes left idle: 4,099
-// device rays against 20,480 triangles take 36 us a call so, 60 with a memset and two kernels.
+// device rays against 20,480 triangles take 40 us a call so, 61 with a memset and two kernels.
 template <bool kAny>
 __global__ void __launch_bounds__(128) k_mesh_few(MeshView m, WideView w, const float* __restrict__ rays,
                                                   uint64_t stride, uint64_t n, uint32_t* __restrict__ prim,

@@ -5,10 +5,10 @@
 // idle (or all are). Each iteration is one warp-voted step: up to `burst` wide nodes for the
 // lanes standing on one or, once `leaf_min` lanes stand on a leaf (or no lane has a node to
 // visit), a leaf for those. Once the warp can take no more rays an iteration is both, the leaf
-// first: a lane that waits then only lengthens the launch. One thread per ray left 3-5 of 32 lanes active per instruction on
-// the torus-knot and 10,000-sphere renders and 10 on a closed box; and a mesh answered in a
-// kernel of its own, or a per-object query inside the top-level walk, repeated the set-up of
-// every ray for every object.
+// first: a lane that waits then only lengthens the launch. One thread per ray left 3-5 of 32 lanes
+// active per instruction on the torus-knot and 10,000-sphere renders and 10 on a closed box; and a
+// mesh answered in a kernel of its own, or a per-object query inside the top-level walk, repeated
+// the set-up of every ray for every object.
 //
 // A Job names the rays:
 //   void load(k, o, d): fetches ray k into the lane
@@ -29,10 +29,9 @@ struct WalkSchedule {
 // stream under capture) its own chunks of 32, warp w of W taking chunks w, w + W, ... When the
 // grid has a lane for every ray a warp takes rays once; and 8 to 16 of them instead of 32 when
 // they are few (up to half the grid's lanes): the launch then lasts as long as its slowest warp,
-// and a warp as long as its lanes' different paths one after another. Frames of a closed box
-// (81x431, 3 samples, depth 19; 948x110, 2 samples, depth 12) took 1.36 and 0.88 ms with 32,
-// 1.24 and 0.80 ms with 8 at least; between half and all of the lanes 32 was faster (a 1.1 M-path
-// frame 0.587 ms against 0.611).
+// and a warp as long as its lanes' different paths one after another. Frames of a torus knot of
+// 164,000 triangles (81x431, 3 samples, depth 19; 948x110, 2 samples, depth 12) took 2.35 and 1.99 ms
+// with 32, 2.09 and 1.75 with 8 at least; between half and all of the lanes 32 was faster.
 struct WalkQueue {
   uint32_t* fetch;
   uint64_t n, own;  // own: rays this warp has taken (fetch NULL)

@@ -32,7 +32,8 @@ enum DeviceError : uint32_t {
 };
 
 // One 32-byte node record (bmin|left_first, bmax|count) as a single 256-bit load. Node
-// arrays come from cudaMalloc and records are 32 bytes, so every record is 32-byte aligned.
+// arrays come from the context's pool, 256-byte aligned, and records are 32 bytes, so every record is
+// 32-byte aligned.
 PBRT_DEV void load_node(const float4* p, float4& lo, float4& hi) {
   asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
       : "=f"(lo.x), "=f"(lo.y), "=f"(lo.z), "=f"(lo.w), "=f"(hi.x), "=f"(hi.y), "=f"(hi.z), "=f"(hi.w)

@@ -130,9 +130,9 @@ unsigned walk_blocks(const WalkLaunch& l) {
 
 // One thread per ray for a wave of at most kEachMaxPaths in mesh scenes of at most kEachMaxNodes
 // wide nodes. A closed box of 34 triangles (some 20 nodes), two chains of waves, persistent
-// against one thread per ray: 0.52 M paths a wave 1.50 / 1.47 ms, 0.37 M at depth 20 2.48 / 2.19,
-// 0.56 M at depth 6 0.610 / 0.546; but 0.86 M 2.55 / 2.60, 1.7 M 4.23 / 4.86, 3.5 M 7.68 / 9.61.
-// Larger trees are persistent throughout (a torus knot of 95,000 triangles 5.9 / 7.2 ms).
+// against one thread per ray: 0.52 M paths a wave 1.82 / 1.78 ms, 0.36 M at depth 20 2.72 / 2.43,
+// 0.56 M at depth 6 1.51 / 1.50; but 0.85 M 2.68 / 2.77, 1.7 M 5.06 / 5.94, 3.4 M 9.82 / 13.2.
+// Larger trees are persistent throughout.
 constexpr uint32_t kEachMaxNodes = 128, kEachMaxPaths = 3u << 18;
 inline bool walk_each(const WalkLaunch& l) { return l.nodes <= kEachMaxNodes && l.paths <= kEachMaxPaths; }
 
