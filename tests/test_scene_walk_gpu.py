@@ -7,6 +7,7 @@ import torch
 
 import pbrt_b200 as pb
 from pbrt_b200 import workloads as W
+from pbrt_b200.scene import Batch, render_params
 
 pytestmark = pytest.mark.gpu
 TR = pb.Transform
@@ -366,3 +367,28 @@ def test_memory_of_a_mesh(device_build, leaf):
     interior = i["mesh_node_count"] - i["mesh_leaf_count"]
     wide = i["device_bytes"] - 66 * len(f) - 32 * i["mesh_node_count"]
     assert wide < 192 * interior * 0.7, f"{wide / interior:.0f} bytes an interior node"
+
+
+def test_films_by_the_walk_and_by_the_per_object_queries():
+    """A render's queries walk the wide tree; a persistent batch asks the top level and each object's own
+    tree, one thread per path: the same film, of objects of every kind, a large mesh among them."""
+    rng = np.random.default_rng(4)
+    objects, at = _unordered(rng)
+    objects += _analytic(rng)[0] + [pb.Simple(pb.TriangleMesh(*W.displaced_icosphere(5, seed=9)))]
+    ctx = pb.Context(0)
+    s = pb.Scene(ctx)
+    for o in objects:
+        s.add_object(o)
+    s.add_light(pb.BackgroundInfiniteLight([1.0, 1.0, 1.0], [0.5, 0.7, 1.0]))
+    s.add_light(pb.PointLight([0.0, 8.0, 0.0], [40.0, 40.0, 40.0]))
+    s.commit()
+    _, cam = W.many_spheres(10, width=128, height=96)
+    film = s.render(cam, 8, 8, seed=3, rr_start=4)
+    ctx.set_batch_kernel("persistent")
+    try:
+        b = Batch([s], [render_params(cam, 8, 8, seed=3, rr_start=4)], ctx)
+        other = b.render(0)[0]
+    finally:
+        ctx.set_batch_kernel("wavefront")
+    np.testing.assert_array_equal(film, other)
+    assert film.std() > 0.01
