@@ -172,7 +172,7 @@ def _per_kernel(launch_ms: float, n_rays: int, box_pr: float, tri_pr: float, pea
     of the captured pass (ncu times are serialised and cold, so only their ratio is used).
     The cull (k_cull_root_bulk, or k_cull_root) streams rays: its figure is its captured DRAM
     bytes over that time.
-    k_mesh_walk walks the survivors: its algorithmic bytes are the node and
+    k_mesh_walk walks the survivors: its algorithmic bytes are the binary walk's node and
     triangle fetches beyond the root test, 32 (box tests - 1) + 36 triangle tests per ray."""
     d = _kernel_profile()
     if not d:
@@ -988,7 +988,7 @@ def main():
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {"workload": WORKLOAD, "rays_per_gpu": N_RAYS, "triangles": int(info["triangle_count"]),
                        "bvh_nodes": int(info["mesh_node_count"]), "bvh_max_depth": int(info["mesh_max_depth"]),
-                       "l2": "no flush: each step streams 512 MiB of rays (> 126 MB L2); the 16 MB tree stays L2-resident "
+                       "l2": "no flush: each step streams 512 MiB of rays (> 126 MB L2); the 20 MB tree stays L2-resident "
                              "by design", "parallelism": f"replicas x{ws}"},
             "e2e": {"value": round(e2e_value, 2), "unit": UNIT, "h2d_bytes_per_step": 32 * N_RAYS,
                     "d2h_bytes_per_step": 8 * N_RAYS, "steps": e2e_steps,
